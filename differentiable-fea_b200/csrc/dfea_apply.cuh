@@ -26,6 +26,7 @@
 #include <mutex>
 
 #include "dfea_common.cuh"
+#include "dfea_frame.cuh"
 
 namespace dfea {
 
@@ -311,8 +312,14 @@ template <typename T>
 __device__ __forceinline__ v2_t<T> node_sum(const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
                                             const v2_t<T>* __restrict__ fe2, int64_t n) {
     T sx = T(0), sy = T(0);
+    int j = inc_ptr[n];
     const int j1 = inc_ptr[n + 1];
-    for (int j = inc_ptr[n]; j < j1; ++j) {
+    for (; j + 4 <= j1; j += 4) {  // four loads in flight, added in order
+        const v2_t<T> f0 = fe2[inc[j]], f1 = fe2[inc[j + 1]], f2 = fe2[inc[j + 2]], f3 = fe2[inc[j + 3]];
+        sx = sx + f0.x + f1.x + f2.x + f3.x;
+        sy = sy + f0.y + f1.y + f2.y + f3.y;
+    }
+    for (; j < j1; ++j) {
         const v2_t<T> f = fe2[inc[j]];
         sx += f.x;
         sy += f.y;
@@ -358,12 +365,8 @@ struct RefApplyCfg {
 template <int NEN, int NQ, typename T, bool DOT, typename Start, typename Gather, typename Scatter>
 __device__ __forceinline__ bool apply_tiles_ref(const Mesh& m, int64_t e0, int64_t e1, const float* __restrict__ C,
                                                 const RefGrad<NEN, NQ>& rg, unsigned char* smem, double& curv,
-                                                Start&& start, Gather&& gather, Scatter&& scatter,
-                                                int64_t blk = -1, int64_t nblk = -1) {
-    if (blk < 0) {  // the whole launch walks [e0, e1)
-        blk = blockIdx.x;
-        nblk = gridDim.x;
-    }
+                                                Start&& start, Gather&& gather, Scatter&& scatter) {
+    const int64_t blk = blockIdx.x, nblk = gridDim.x;
     using Cfg = RefApplyCfg<NEN>;
     using T2 = v2_t<T>;
     constexpr int NT = Cfg::NT, ST = Cfg::STAGES;
@@ -514,18 +517,21 @@ k_apply_ref(Mesh m, int64_t e0, int64_t e1, const float* __restrict__ C, const R
     }
 }
 
-template <int NEN, int NQ, typename T, bool DOT>
-__global__ void __launch_bounds__(128)
-k_apply_ref_elem(Mesh m, const float* __restrict__ C, const RefGrad<NEN, NQ> rg, const T* __restrict__ v,
+// Gather form, element pass from reference-frame moduli (SD: float DFEA_F32REF, double DFEA_F64REF) by the frame
+// walk: one warp per Gauss point, results into fe[a][e].
+template <int NEN, int NQ, typename SD, typename T, bool DOT>
+__global__ void __launch_bounds__(FrameCfg<NEN, NQ>::NT, FrameCfg<NEN, NQ>::MINB)
+k_apply_ref_elem(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const T* __restrict__ v,
                  T* __restrict__ fe, RedSite site, const int* __restrict__ done) {
     using T2 = v2_t<T>;
-    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NT = FrameCfg<NEN, NQ>::NT;
+    __shared__ FrameShared<NEN, NQ, T> sh;
     T2* fe2 = reinterpret_cast<T2*>(fe);
     const int64_t S = m.stride;
     double curv = 0.0;
     const T2* v2 = reinterpret_cast<const T2*>(v);
-    const bool ran = apply_tiles_ref<NEN, NQ, T, DOT>(
-        m, 0, m.n_el, C, rg, smem, curv,
+    const bool ran = frame_product<NEN, NQ, SD, T, DOT>(
+        m, C, rg, sh, curv,
         [&]() -> bool {
             grid_dependency_wait();
             if (DOT && done != nullptr && *done) return false;
@@ -533,15 +539,12 @@ k_apply_ref_elem(Mesh m, const float* __restrict__ C, const RefGrad<NEN, NQ> rg,
             return true;
         },
         [&](int n) { return __ldg(v2 + n); },
-        [&](int64_t e, const int (&)[NEN], const int (&)[NEN], const T (&fx)[NEN], const T (&fy)[NEN]) {
-#pragma unroll
-            for (int a = 0; a < NEN; ++a) fe2[(int64_t)a * S + e] = make_v2<T>(fx[a], fy[a]);
-        });
+        [&](int a, int64_t e, T2 f) { fe2[(int64_t)a * S + e] = f; }, blockIdx.x, gridDim.x);
     if (!ran) return;
     if (DOT) {
-        const double vals[1] = {block_sum<128>(curv)};
+        const double vals[1] = {block_sum<NT>(curv)};
         double tot[1];
-        if (last_block_sum<128, 1>(vals, site, tot) && threadIdx.x == 0) site.result[0] = tot[0];
+        if (last_block_sum<NT, 1>(vals, site, tot) && threadIdx.x == 0) site.result[0] = tot[0];
     }
 }
 
@@ -569,6 +572,15 @@ int resident_grid(int64_t n_elements) {
     return (int)(grid < 1 ? 1 : grid);
 }
 
+// The same for the frame walk: tiles of FrameCfg::EB elements, static shared memory.
+template <auto Kernel, int NEN, int NQ>
+int frame_resident_grid(int64_t n_elements) {
+    constexpr int EB = FrameCfg<NEN, NQ>::EB, NT = FrameCfg<NEN, NQ>::NT;
+    const int64_t grid = resident_grid<Kernel, 0, NT>((int64_t)kMaxBlocks * NT);   // as many as fit
+    const int64_t tiles = (n_elements + EB - 1) / EB;
+    return (int)(tiles < 1 ? 1 : (tiles < grid ? tiles : grid));
+}
+
 // A grid limited to `cap` blocks (0: no limit).  Solves that share the GPU with other streams run
 // with fewer, longer-lived blocks per launch, so that launches of different streams fit side by side.
 inline int capped(int grid, int cap) { return (cap > 0 && grid > cap) ? cap : grid; }
@@ -590,9 +602,9 @@ int apply_ref_grid(int64_t n_elements) {
     return resident_grid<k_apply_ref<NEN, NQ, T, DOT>, RefApplyCfg<NEN>::SMEM, 128>(n_elements);
 }
 
-template <int NEN, int NQ, typename T, bool DOT>
+template <int NEN, int NQ, typename SD, typename T, bool DOT>
 int apply_ref_elem_grid(int64_t n_elements) {
-    return resident_grid<k_apply_ref_elem<NEN, NQ, T, DOT>, RefApplyCfg<NEN>::SMEM, 128>(n_elements);
+    return frame_resident_grid<k_apply_ref_elem<NEN, NQ, SD, T, DOT>, NEN, NQ>(n_elements);
 }
 
 // The byte range of the DOF vectors a product gathers (v) and scatters (y): both when they are
@@ -640,11 +652,12 @@ int launch_apply_colours(const dfea_mesh_view& mv, const SD* C, const SD* G, con
     return launch_check("k_apply");
 }
 
-// Gather form: the element pass over all elements (results into fe), launched with PDL and the L2
-// window on v.  The node pass is launched by the caller.
+// Gather form: the element pass over all elements (results into fe), launched with the L2 window on v.  The node
+// pass is launched by the caller.  pdl: the pass requests its first moduli before it waits for its predecessor, so
+// it may overlap one only where that predecessor cannot be the writer of the moduli.
 template <int NEN, int NQ, typename SD, typename T, bool DOT>
 int launch_apply_elem(const dfea_mesh_view& mv, const SD* C, const SD* G, const T* v, T* fe, RedSite site,
-                      const int* done, cudaStream_t stream, int grid_cap = 0) {
+                      const int* done, cudaStream_t stream, int grid_cap = 0, bool pdl = true) {
     using Cfg = ApplyCfg<NEN, SD>;
     const Mesh m = kernel_mesh(mv);
     long long max_window = 0;
@@ -652,7 +665,7 @@ int launch_apply_elem(const dfea_mesh_view& mv, const SD* C, const SD* G, const 
     size_t wb = (size_t)(2 * mv.n_nodes) * sizeof(T);
     if ((long long)wb > max_window) wb = (size_t)max_window;
     LaunchOpts opts;
-    opts.pdl = true;
+    opts.pdl = pdl;
     if (setaside > 0 && wb > 0) {
         opts.win_base = v;
         opts.win_bytes = wb;
@@ -665,7 +678,8 @@ int launch_apply_elem(const dfea_mesh_view& mv, const SD* C, const SD* G, const 
     return launch_check("k_apply_elem");
 }
 
-// Reference-frame launches: colour passes (y read-modify-write) or the element pass (results into fe).
+// Reference-frame launches: colour passes (y read-modify-write) or the element pass (results into fe).  The element
+// pass marks nothing persisting: it reads v once, and the L2 the set-aside would take keeps fe for the node pass.
 template <int NEN, int NQ, typename T, bool DOT>
 int launch_apply_ref_colours(const dfea_mesh_view& mv, const float* C, const T* v, T* y, const RedSite* sites,
                              const int* done, cudaStream_t stream, int grid_cap = 0) {
@@ -694,34 +708,25 @@ int launch_apply_ref_colours(const dfea_mesh_view& mv, const float* C, const T* 
     return launch_check("k_apply_ref");
 }
 
-template <int NEN, int NQ, typename T, bool DOT>
-int launch_apply_ref_elem(const dfea_mesh_view& mv, const float* C, const T* v, T* fe, RedSite site, const int* done,
-                          cudaStream_t stream, int grid_cap = 0) {
+template <int NEN, int NQ, typename SD, typename T, bool DOT>
+int launch_apply_ref_elem(const dfea_mesh_view& mv, const SD* C, const T* v, T* fe, RedSite site, const int* done,
+                          cudaStream_t stream, int grid_cap = 0, bool pdl = true) {
     const Mesh m = kernel_mesh(mv);
     const RefGrad<NEN, NQ> rg = ref_grad_of<NEN, NQ>(mv);
-    long long max_window = 0;
-    const long long setaside = persisting_l2_bytes(&max_window);
-    size_t wb = (size_t)(2 * mv.n_nodes) * sizeof(T);
-    if ((long long)wb > max_window) wb = (size_t)max_window;
     LaunchOpts opts;
-    opts.pdl = true;
-    if (setaside > 0 && wb > 0) {
-        opts.win_base = v;
-        opts.win_bytes = wb;
-        opts.hit_ratio = setaside >= (long long)wb ? 1.0f : (float)((double)setaside / (double)wb);
-    }
-    const int grid = capped(apply_ref_elem_grid<NEN, NQ, T, DOT>(mv.n_el), grid_cap);
-    const int rc = launch_kernel(k_apply_ref_elem<NEN, NQ, T, DOT>, dim3(grid), dim3(128), RefApplyCfg<NEN>::SMEM, stream,
+    opts.pdl = pdl;
+    const int grid = capped(apply_ref_elem_grid<NEN, NQ, SD, T, DOT>(mv.n_el), grid_cap);
+    const int rc = launch_kernel(k_apply_ref_elem<NEN, NQ, SD, T, DOT>, dim3(grid), dim3(FrameCfg<NEN, NQ>::NT), 0, stream,
                                  opts, m, C, rg, v, fe, site, done);
     if (rc) return rc;
     return launch_check("k_apply_ref_elem");
 }
 
 // Configure the instantiations a solver launches (shared-memory size, occupancy) before any stream capture.
-template <int NEN, int NQ, typename T>
+template <int NEN, int NQ, typename SD, typename T>
 void prepare_apply_ref() {
-    (void)apply_ref_grid<NEN, NQ, T, true>(1);
-    (void)apply_ref_elem_grid<NEN, NQ, T, true>(1);
+    if constexpr (sizeof(SD) == 4) (void)apply_ref_grid<NEN, NQ, T, true>(1);
+    (void)apply_ref_elem_grid<NEN, NQ, SD, T, true>(1);
     (void)persisting_l2_bytes(nullptr);
 }
 

@@ -1150,15 +1150,15 @@ extern "C" int dfea_tangent_apply_gather(const dfea_mesh_view* mesh, const void*
                                          const void* v, void* y, int32_t vec_dtype, void* fe_work, void* stream) {
     int rc = validate_mesh(mesh, moduli_dtype == DFEA_F32);
     if (rc) return rc;
-    if (moduli_dtype == DFEA_F32REF && vec_dtype != DFEA_F64)
-        return set_error(DFEA_ERR_INVALID, "DFEA_F32REF moduli apply to f64 vectors");
+    if ((moduli_dtype == DFEA_F32REF || moduli_dtype == DFEA_F64REF) && vec_dtype != DFEA_F64)
+        return set_error(DFEA_ERR_INVALID, "reference-frame moduli apply to f64 vectors");
     if (!mesh->node_elem_ptr || !mesh->node_elem)
         return set_error(DFEA_ERR_INVALID, "dfea_tangent_apply_gather: the mesh has no node incidence");
     if (!moduli || !v || !y || !fe_work) return set_error(DFEA_ERR_INVALID, "dfea_tangent_apply_gather: NULL pointer");
     if (v == y) return set_error(DFEA_ERR_INVALID, "dfea_tangent_apply_gather: y must not alias v");
     if (!aligned16(moduli) || !aligned16(v) || !aligned16(y) || !aligned16(fe_work))
         return set_error(DFEA_ERR_INVALID, "dfea_tangent_apply_gather: moduli, v, y and fe_work must be 16-byte aligned");
-    if (moduli_dtype != DFEA_F64 && moduli_dtype != DFEA_F32 && moduli_dtype != DFEA_F32REF)
+    if (moduli_dtype != DFEA_F64 && moduli_dtype != DFEA_F32 && moduli_dtype != DFEA_F32REF && moduli_dtype != DFEA_F64REF)
         return set_error(DFEA_ERR_INVALID, "bad moduli dtype");
     if (vec_dtype != DFEA_F64 && vec_dtype != DFEA_F32) return set_error(DFEA_ERR_INVALID, "bad vector dtype");
     if (vec_dtype == DFEA_F32 && moduli_dtype != DFEA_F32)
@@ -1171,11 +1171,14 @@ extern "C" int dfea_tangent_apply_gather(const dfea_mesh_view* mesh, const void*
     pdl.pdl = true;
     rc = dispatch_element(mesh->nen, mesh->n_q, [&](auto nen_c, auto nq_c) -> int {
         constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
-        if (moduli_dtype == DFEA_F32REF) {
+        if (moduli_dtype == DFEA_F32REF || moduli_dtype == DFEA_F64REF) {
             const double* vv = static_cast<const double*>(v);
             double* fe = static_cast<double*>(fe_work);
-            int r = launch_apply_ref_elem<NEN, NQ, double, false>(*mesh, static_cast<const float*>(moduli), vv, fe, none,
-                                                                 nullptr, s);
+            const int r = moduli_dtype == DFEA_F64REF
+                              ? launch_apply_ref_elem<NEN, NQ, double, double, false>(
+                                    *mesh, static_cast<const double*>(moduli), vv, fe, none, nullptr, s, 0, false)
+                              : launch_apply_ref_elem<NEN, NQ, float, double, false>(
+                                    *mesh, static_cast<const float*>(moduli), vv, fe, none, nullptr, s, 0, false);
             if (r) return r;
             return launch_kernel(k_node_gather<double>, dim3(gn), dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr,
                                  mesh->node_elem, (const double*)fe, vv, static_cast<double*>(y));
@@ -1185,9 +1188,9 @@ extern "C" int dfea_tangent_apply_gather(const dfea_mesh_view* mesh, const void*
             double* fe = static_cast<double*>(fe_work);
             int r = (moduli_dtype == DFEA_F64)
                         ? launch_apply_elem<NEN, NQ, double, double, false>(*mesh, static_cast<const double*>(moduli),
-                                                                           mesh->grad, vv, fe, none, nullptr, s)
+                                                                           mesh->grad, vv, fe, none, nullptr, s, 0, false)
                         : launch_apply_elem<NEN, NQ, float, double, false>(*mesh, static_cast<const float*>(moduli),
-                                                                          mesh->grad32, vv, fe, none, nullptr, s);
+                                                                          mesh->grad32, vv, fe, none, nullptr, s, 0, false);
             if (r) return r;
             return launch_kernel(k_node_gather<double>, dim3(gn), dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr,
                                  mesh->node_elem, (const double*)fe, vv, static_cast<double*>(y));
@@ -1195,7 +1198,7 @@ extern "C" int dfea_tangent_apply_gather(const dfea_mesh_view* mesh, const void*
         const float* vv = static_cast<const float*>(v);
         float* fe = static_cast<float*>(fe_work);
         int r = launch_apply_elem<NEN, NQ, float, float, false>(*mesh, static_cast<const float*>(moduli), mesh->grad32,
-                                                               vv, fe, none, nullptr, s);
+                                                               vv, fe, none, nullptr, s, 0, false);
         if (r) return r;
         return launch_kernel(k_node_gather<float>, dim3(gn), dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr,
                              mesh->node_elem, (const float*)fe, vv, static_cast<float*>(y));
@@ -1216,7 +1219,7 @@ int dfea::mg_fe_gather_cheb(const dfea_mesh_view* mesh, const void* moduli, int3
         return set_error(DFEA_ERR_INVALID, "multigrid smoothing: NULL pointer");
     if (!aligned16(moduli) || !aligned16(v) || !aligned16(fe_work))
         return set_error(DFEA_ERR_INVALID, "multigrid smoothing: moduli, v and fe_work must be 16-byte aligned");
-    if (moduli_dtype != DFEA_F64 && moduli_dtype != DFEA_F32 && moduli_dtype != DFEA_F32REF)
+    if (moduli_dtype != DFEA_F64 && moduli_dtype != DFEA_F32 && moduli_dtype != DFEA_F32REF && moduli_dtype != DFEA_F64REF)
         return set_error(DFEA_ERR_INVALID, "bad moduli dtype");
     const Mesh m = kernel_mesh(*mesh);
     const int gn = grid_for(mesh->n_nodes, kThreads, 4);
@@ -1226,9 +1229,12 @@ int dfea::mg_fe_gather_cheb(const dfea_mesh_view* mesh, const void* moduli, int3
     double* fe = static_cast<double*>(fe_work);
     rc = dispatch_element(mesh->nen, mesh->n_q, [&](auto nen_c, auto nq_c) -> int {
         constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
+        if (moduli_dtype == DFEA_F64REF)
+            return launch_apply_ref_elem<NEN, NQ, double, double, false>(*mesh, static_cast<const double*>(moduli), v, fe,
+                                                                        none, nullptr, s);
         if (moduli_dtype == DFEA_F32REF)
-            return launch_apply_ref_elem<NEN, NQ, double, false>(*mesh, static_cast<const float*>(moduli), v, fe, none,
-                                                                nullptr, s);
+            return launch_apply_ref_elem<NEN, NQ, float, double, false>(*mesh, static_cast<const float*>(moduli), v, fe,
+                                                                       none, nullptr, s);
         if (moduli_dtype == DFEA_F64)
             return launch_apply_elem<NEN, NQ, double, double, false>(*mesh, static_cast<const double*>(moduli), mesh->grad,
                                                                     v, fe, none, nullptr, s);

@@ -62,8 +62,8 @@ __device__ __forceinline__ double hat(const int32_t* X, int n_lines, int c, int 
 // ------------------------------------------------------------------------------------------
 // level 1 from the finite-element mesh: K_C = sum_e sum_q (B_q P~)^T C_q (B_q P~)
 // ------------------------------------------------------------------------------------------
-// MOD 0: FP64 physical moduli (16 per Gauss point) with the mesh gradients; 1: FP32 physical moduli; 2: FP32
-// reference-frame moduli (10 per Gauss point, DFEA_F32REF) with the reference gradients.
+// MOD 0: FP64 physical moduli (16 per Gauss point) with the mesh gradients; 1: FP32 physical moduli; 2, 3: FP32 and
+// FP64 reference-frame moduli (10 per Gauss point, DFEA_F32REF, DFEA_F64REF) with the reference gradients.
 template <int NEN, int NQ, int MOD>
 __global__ void __launch_bounds__(128)
 k_mg_galerkin_fe(Mesh m, const void* __restrict__ moduli, RefGrad<NEN, NQ> rg, const int32_t* __restrict__ node_ij,
@@ -100,13 +100,25 @@ k_mg_galerkin_fe(Mesh m, const void* __restrict__ moduli, RefGrad<NEN, NQ> rg, c
 #pragma unroll 1
                 for (int q = 0; q < NQ; ++q) {
                     double g[NEN][2], M[16];
-                    if constexpr (MOD == 2) {
-                        const float* Cf = static_cast<const float*>(moduli);
-                        const int64_t base = (int64_t)q * 10 * S;
-                        const float4 A = reinterpret_cast<const float4*>(Cf + base)[s];
-                        const float4 B = reinterpret_cast<const float4*>(Cf + base + 4 * S)[s];
-                        const float2 D = reinterpret_cast<const float2*>(Cf + base + 8 * S)[s];
-                        const double h[10] = {A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w, D.x, D.y};
+                    if constexpr (MOD >= 2) {
+                        double h[10];
+                        if constexpr (MOD == 2) {
+                            const float* Cf = static_cast<const float*>(moduli);
+                            const int64_t base = (int64_t)q * 10 * S;
+                            const float4 A = reinterpret_cast<const float4*>(Cf + base)[s];
+                            const float4 B = reinterpret_cast<const float4*>(Cf + base + 4 * S)[s];
+                            const float2 D = reinterpret_cast<const float2*>(Cf + base + 8 * S)[s];
+                            h[0] = A.x; h[1] = A.y; h[2] = A.z; h[3] = A.w; h[4] = B.x;
+                            h[5] = B.y; h[6] = B.z; h[7] = B.w; h[8] = D.x; h[9] = D.y;
+                        } else {
+                            const double2* Cd = static_cast<const double2*>(moduli) + (int64_t)(q * 5) * S + s;
+#pragma unroll
+                            for (int k = 0; k < 5; ++k) {
+                                const double2 t = Cd[k * S];
+                                h[2 * k] = t.x;
+                                h[2 * k + 1] = t.y;
+                            }
+                        }
                         // packed upper triangle: (0,0..3) (1,1..3) (2,2..3) (3,3)
                         M[0] = h[0]; M[1] = h[1]; M[2] = h[2]; M[3] = h[3];
                         M[5] = h[4]; M[6] = h[5]; M[7] = h[6];
@@ -927,6 +939,8 @@ extern "C" int dfea_mg_galerkin_fe(const dfea_mesh_view* mesh, const void* modul
             k_mg_galerkin_fe<NEN, NQ, 1><<<grid, 128, 0, s>>>(m, moduli, rg, node_ij, cell_slot, span, epc, ncy, cg);
         else if (moduli_dtype == DFEA_F32REF)
             k_mg_galerkin_fe<NEN, NQ, 2><<<grid, 128, 0, s>>>(m, moduli, rg, node_ij, cell_slot, span, epc, ncy, cg);
+        else if (moduli_dtype == DFEA_F64REF)
+            k_mg_galerkin_fe<NEN, NQ, 3><<<grid, 128, 0, s>>>(m, moduli, rg, node_ij, cell_slot, span, epc, ncy, cg);
         else
             return set_error(DFEA_ERR_INVALID, "dfea_mg_galerkin_fe: bad moduli dtype");
         return DFEA_OK;

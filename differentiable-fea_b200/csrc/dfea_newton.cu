@@ -42,8 +42,11 @@ struct Driver {
     double* uc;         // the line-search trial
 
     int residual(const double* u, double lf, double* out, double* rn) {
-        int rc = dfea_residual_mat(nw->mesh, u, nw->theta, &nw->material, nw->f, lf, out, nw->scal, nullptr,
-                                   nw->reduce_work, s);
+        int rc = nw->frame_work
+                     ? dfea_frame_residual(nw->mesh, u, nw->theta, &nw->material, nullptr, nullptr, nw->f, lf, out, nw->scal,
+                                           nullptr, nw->frame_work, s)
+                     : dfea_residual_mat(nw->mesh, u, nw->theta, &nw->material, nw->f, lf, out, nw->scal, nullptr,
+                                         nw->reduce_work, s);
         if (rc) return rc;
         if ((rc = check_cuda(cudaMemcpyAsync(nw->scal_host, nw->scal, sizeof(double), cudaMemcpyDeviceToHost, s),
                              "cudaMemcpyAsync")) ||
@@ -54,8 +57,12 @@ struct Driver {
     }
 
     int linearize(const double* u) {
-        int rc = dfea_qp_moduli_mat(nw->mesh, u, nw->theta, &nw->material, nw->moduli, nw->moduli_dtype, nw->diag,
-                                    nw->blocks, s);
+        const bool ref = nw->moduli_dtype == DFEA_F64REF || nw->moduli_dtype == DFEA_F32REF;
+        int rc = nw->frame_work && ref
+                     ? dfea_frame_moduli(nw->mesh, u, nw->theta, &nw->material, nullptr, nullptr, nw->moduli,
+                                         nw->moduli_dtype, nw->diag, nw->blocks, nw->frame_work, s)
+                     : dfea_qp_moduli_mat(nw->mesh, u, nw->theta, &nw->material, nw->moduli, nw->moduli_dtype, nw->diag,
+                                          nw->blocks, s);
         if (rc || !nw->mg) return rc;
         return dfea_mg_setup(nw->mesh, nw->mg, nw->moduli, nw->moduli_dtype, nw->diag, s);
     }

@@ -319,20 +319,21 @@ k_pcg_elem_fused(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, con
     if (last_block_sum<128, 1>(vals, site, tot) && threadIdx.x == 0) site.result[0] = tot[0];
 }
 
-template <int NEN, int NQ, typename T, bool BJ>
-__global__ void __launch_bounds__(128)
-k_pcg_elem_fused_ref(Mesh m, const float* __restrict__ C, const RefGrad<NEN, NQ> rg, const T* __restrict__ r,
+template <int NEN, int NQ, typename SD, typename T, bool BJ>
+__global__ void __launch_bounds__(FrameCfg<NEN, NQ>::NT, FrameCfg<NEN, NQ>::MINB)
+k_pcg_elem_fused_ref(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const T* __restrict__ r,
                      const T* __restrict__ d, const T* __restrict__ p, T* __restrict__ fe,
                      const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, PcgState* st, RedSite site) {
     using T2 = v2_t<T>;
-    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NT = FrameCfg<NEN, NQ>::NT;
+    __shared__ FrameShared<NEN, NQ, T> sh;
     const T2* r2 = reinterpret_cast<const T2*>(r);
     const T2* p2 = reinterpret_cast<const T2*>(p);
     T2* fe2 = reinterpret_cast<T2*>(fe);
     double curv = 0.0, pfix = 0.0;
     T beta = T(0);
-    const bool ran = apply_tiles_ref<NEN, NQ, T, true>(
-        m, 0, m.n_el, C, rg, smem, curv,
+    const bool ran = frame_product<NEN, NQ, SD, T, true>(
+        m, C, rg, sh, curv,
         [&]() -> bool {
             grid_dependency_wait();
             if (st->done) return false;
@@ -341,13 +342,21 @@ k_pcg_elem_fused_ref(Mesh m, const float* __restrict__ C, const RefGrad<NEN, NQ>
             return true;
         },
         [&](int n) { return next_direction<BJ, T>(d, n, __ldg(r2 + n), __ldg(p2 + n), beta); },
-        [&](int64_t e, const int (&node)[NEN], const int (&fix)[NEN], const T (&fx)[NEN], const T (&fy)[NEN]) {
-            fused_scatter<T, BJ, NEN>(e, m.stride, node, fix, fx, fy, fe2, inc_ptr, inc, d, r2, p2, beta, pfix);
-        });
+        [&](int a, int64_t e, T2 f) {
+            const int64_t slot = (int64_t)a * m.stride + e;
+            fe2[slot] = f;
+            const int c = __ldg(m.conn + slot);
+            if ((c & 3) && inc[inc_ptr[c >> 2]] == (int32_t)slot) {  // a fixed DOF, counted by its first slot
+                const T2 pn = next_direction<BJ, T>(d, c >> 2, __ldg(r2 + (c >> 2)), __ldg(p2 + (c >> 2)), beta);
+                if (c & 1) pfix += (double)pn.x * pn.x;
+                if (c & 2) pfix += (double)pn.y * pn.y;
+            }
+        },
+        blockIdx.x, gridDim.x);
     if (!ran) return;
-    const double vals[1] = {block_sum<128>(curv + pfix)};
+    const double vals[1] = {block_sum<NT>(curv + pfix)};
     double tot[1];
-    if (last_block_sum<128, 1>(vals, site, tot) && threadIdx.x == 0) site.result[0] = tot[0];
+    if (last_block_sum<NT, 1>(vals, site, tot) && threadIdx.x == 0) site.result[0] = tot[0];
 }
 
 template <typename T, bool BJ>
@@ -513,10 +522,10 @@ int launch_iteration(const dfea_pcg& h, cudaStream_t s, cudaGraphConditionalHand
                 opts.hit_ratio = setaside >= (long long)w.bytes ? 1.0f : (float)((double)setaside / (double)w.bytes);
             }
             if constexpr (REF) {
-                const int grid = capped(resident_grid<k_pcg_elem_fused_ref<NEN, NQ, T, BJ>, RefApplyCfg<NEN>::SMEM, 128>(mv.n_el),
+                const int grid = capped(frame_resident_grid<k_pcg_elem_fused_ref<NEN, NQ, S, T, BJ>, NEN, NQ>(mv.n_el),
                                         h.grid_cap);
-                return launch_kernel(k_pcg_elem_fused_ref<NEN, NQ, T, BJ>, dim3(grid), dim3(128), RefApplyCfg<NEN>::SMEM,
-                                     s, opts, m, reinterpret_cast<const float*>(C), ref_grad_of<NEN, NQ>(mv), (const T*)r,
+                return launch_kernel(k_pcg_elem_fused_ref<NEN, NQ, S, T, BJ>, dim3(grid), dim3(FrameCfg<NEN, NQ>::NT), 0,
+                                     s, pdl, m, C, ref_grad_of<NEN, NQ>(mv), (const T*)r,
                                      d, (const T*)p, fe, mv.node_elem_ptr, mv.node_elem, st, h.site(0, 1));
             } else {
                 using Cfg = ApplyCfg<NEN, S>;
@@ -537,7 +546,7 @@ int launch_iteration(const dfea_pcg& h, cudaStream_t s, cudaGraphConditionalHand
         rc = dispatch_element(mv.nen, mv.n_q, [&](auto nen_c, auto nq_c) -> int {
             constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
             if constexpr (REF)
-                return launch_apply_ref_elem<NEN, NQ, T, true>(mv, reinterpret_cast<const float*>(C), p, fe, h.site(0, 1),
+                return launch_apply_ref_elem<NEN, NQ, S, T, true>(mv, C, p, fe, h.site(0, 1),
                                                                &st->done, s, h.grid_cap);
             else
                 return launch_apply_elem<NEN, NQ, S, T, true>(mv, C, G, p, fe, h.site(0, 1), &st->done, s, h.grid_cap);
@@ -554,7 +563,9 @@ int launch_iteration(const dfea_pcg& h, cudaStream_t s, cudaGraphConditionalHand
         for (int c = 0; c < mv.n_colours; ++c) sites[c] = h.site(c, 1);
         rc = dispatch_element(mv.nen, mv.n_q, [&](auto nen_c, auto nq_c) -> int {
             constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
-            if constexpr (REF)
+            if constexpr (REF && std::is_same<S, double>::value)
+                return set_error(DFEA_ERR_UNSUPPORTED, "DFEA_F64REF moduli run in the gather forms");  // checked at create
+            else if constexpr (REF)
                 return launch_apply_ref_colours<NEN, NQ, T, true>(mv, reinterpret_cast<const float*>(C), p, y, sites,
                                                                   &st->done, s, h.grid_cap);
             else
@@ -579,11 +590,13 @@ int launch_iteration_any(const dfea_pcg& h, cudaStream_t s, cudaGraphConditional
     if (h.block) {  // block-Jacobi: double vectors only (checked at create)
         if (h.vec_dtype == DFEA_F64) return launch_iteration<double, double, false, true>(h, s, cond, with_cond);
         if (h.vec_dtype == DFEA_MIXED) return launch_iteration<float, double, false, true>(h, s, cond, with_cond);
+        if (h.vec_dtype == DFEA_F64REF) return launch_iteration<double, double, true, true>(h, s, cond, with_cond);
         return launch_iteration<float, double, true, true>(h, s, cond, with_cond);
     }
     if (h.vec_dtype == DFEA_F64) return launch_iteration<double, double>(h, s, cond, with_cond);
     if (h.vec_dtype == DFEA_MIXED) return launch_iteration<float, double>(h, s, cond, with_cond);
     if (h.vec_dtype == DFEA_F32REF) return launch_iteration<float, double, true>(h, s, cond, with_cond);
+    if (h.vec_dtype == DFEA_F64REF) return launch_iteration<double, double, true>(h, s, cond, with_cond);
     return launch_iteration<float, float>(h, s, cond, with_cond);
 }
 
@@ -666,7 +679,8 @@ PcgLayout layout_for(const dfea_mesh_view& mv, int32_t vec_dtype) {
 }  // namespace
 
 extern "C" int64_t dfea_pcg_work_bytes(const dfea_mesh_view* mesh, int32_t vec_dtype) {
-    if (!mesh || (vec_dtype != DFEA_F64 && vec_dtype != DFEA_F32 && vec_dtype != DFEA_MIXED && vec_dtype != DFEA_F32REF))
+    if (!mesh || (vec_dtype != DFEA_F64 && vec_dtype != DFEA_F32 && vec_dtype != DFEA_MIXED && vec_dtype != DFEA_F32REF &&
+                  vec_dtype != DFEA_F64REF))
         return -1;
     return layout_for(*mesh, vec_dtype).total;
 }
@@ -677,8 +691,11 @@ extern "C" int dfea_pcg_create(const dfea_mesh_view* mesh, const void* moduli, c
     *out = nullptr;
     int rc = validate_mesh(mesh, vec_dtype == DFEA_F32 || vec_dtype == DFEA_MIXED);
     if (rc) return rc;
-    if (vec_dtype != DFEA_F64 && vec_dtype != DFEA_F32 && vec_dtype != DFEA_MIXED && vec_dtype != DFEA_F32REF)
+    if (vec_dtype != DFEA_F64 && vec_dtype != DFEA_F32 && vec_dtype != DFEA_MIXED && vec_dtype != DFEA_F32REF &&
+        vec_dtype != DFEA_F64REF)
         return set_error(DFEA_ERR_INVALID, "bad vector dtype");
+    if (vec_dtype == DFEA_F64REF && !(use_graph & (DFEA_PCG_GATHER | DFEA_PCG_FUSED)))
+        return set_error(DFEA_ERR_UNSUPPORTED, "dfea_pcg_create: DFEA_F64REF moduli need the gather or fused form");
     if (!moduli || !diag || !b || !x || !work) return set_error(DFEA_ERR_INVALID, "dfea_pcg_create: NULL pointer");
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 255u) == 0; };
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
@@ -718,12 +735,16 @@ extern "C" int dfea_pcg_create(const dfea_mesh_view* mesh, const void* moduli, c
         constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
         if (vec_dtype == DFEA_F64) prepare_apply<NEN, NQ, double, double>();
         else if (vec_dtype == DFEA_MIXED) prepare_apply<NEN, NQ, float, double>();
-        else if (vec_dtype == DFEA_F32REF) prepare_apply_ref<NEN, NQ, double>();
+        else if (vec_dtype == DFEA_F32REF) prepare_apply_ref<NEN, NQ, float, double>();
+        else if (vec_dtype == DFEA_F64REF) prepare_apply_ref<NEN, NQ, double, double>();
         else prepare_apply<NEN, NQ, float, float>();
         if (h->fused) {  // the fused element pass of this handle's types
             if (vec_dtype == DFEA_F32REF) {
-                if (h->block) (void)resident_grid<k_pcg_elem_fused_ref<NEN, NQ, double, true>, RefApplyCfg<NEN>::SMEM, 128>(1);
-                else (void)resident_grid<k_pcg_elem_fused_ref<NEN, NQ, double, false>, RefApplyCfg<NEN>::SMEM, 128>(1);
+                if (h->block) (void)frame_resident_grid<k_pcg_elem_fused_ref<NEN, NQ, float, double, true>, NEN, NQ>(1);
+                else (void)frame_resident_grid<k_pcg_elem_fused_ref<NEN, NQ, float, double, false>, NEN, NQ>(1);
+            } else if (vec_dtype == DFEA_F64REF) {
+                if (h->block) (void)frame_resident_grid<k_pcg_elem_fused_ref<NEN, NQ, double, double, true>, NEN, NQ>(1);
+                else (void)frame_resident_grid<k_pcg_elem_fused_ref<NEN, NQ, double, double, false>, NEN, NQ>(1);
             } else if (vec_dtype == DFEA_F64) {
                 using Cfg = ApplyCfg<NEN, double>;
                 if (h->block) (void)resident_grid<k_pcg_elem_fused<NEN, NQ, double, double, true>, Cfg::SMEM, Cfg::NT>(1);
@@ -942,9 +963,10 @@ struct BatchSolve {
 };
 
 template <int NEN, int NQ>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(FrameCfg<NEN, NQ>::NT, FrameCfg<NEN, NQ>::MINB)
 k_batch_elem(const BatchSolve* __restrict__ solves, const int2* __restrict__ block_map, const RefGrad<NEN, NQ> rg) {
-    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NT = FrameCfg<NEN, NQ>::NT;
+    __shared__ FrameShared<NEN, NQ, double> sh;
     const int2 bm = block_map[blockIdx.x];
     const BatchSolve* S = solves + bm.x;
     const Mesh m = S->m;
@@ -953,8 +975,8 @@ k_batch_elem(const BatchSolve* __restrict__ solves, const int2* __restrict__ blo
     double2* fe2 = reinterpret_cast<double2*>(S->fe);
     const int64_t Sd = m.stride;
     double curv = 0.0;
-    const bool ran = apply_tiles_ref<NEN, NQ, double, true>(
-        m, 0, m.n_el, S->C, rg, smem, curv,
+    const bool ran = frame_product<NEN, NQ, float, double, true>(
+        m, S->C, rg, sh, curv,
         [&]() -> bool {
             grid_dependency_wait();
             if (st->done) return false;
@@ -962,15 +984,11 @@ k_batch_elem(const BatchSolve* __restrict__ solves, const int2* __restrict__ blo
             return true;
         },
         [&](int n) { return __ldg(p2 + n); },
-        [&](int64_t e, const int (&)[NEN], const int (&)[NEN], const double (&fx)[NEN], const double (&fy)[NEN]) {
-#pragma unroll
-            for (int a = 0; a < NEN; ++a) fe2[(int64_t)a * Sd + e] = make_double2(fx[a], fy[a]);
-        },
-        bm.y, S->elem_blocks);
+        [&](int a, int64_t e, double2 f) { fe2[(int64_t)a * Sd + e] = f; }, bm.y, S->elem_blocks);
     if (!ran) return;
-    const double vals[1] = {block_sum<128>(curv)};
+    const double vals[1] = {block_sum<NT>(curv)};
     double tot[1];
-    if (last_block_sum_in<128, 1>(vals, S->site_elem, tot, bm.y, S->elem_blocks) && threadIdx.x == 0)
+    if (last_block_sum_in<NT, 1>(vals, S->site_elem, tot, bm.y, S->elem_blocks) && threadIdx.x == 0)
         S->site_elem.result[0] = tot[0];
 }
 
@@ -1110,8 +1128,8 @@ extern "C" int dfea_batch_set(dfea_batch* b, dfea_pcg* const* solves, int32_t n,
         const int cap = h.grid_cap > 0 ? h.grid_cap : b->max_blocks;
         rc = dispatch_element(mv.nen, mv.n_q, [&](auto nen_c, auto nq_c) -> int {
             constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
-            S.elem_blocks = capped(apply_ref_elem_grid<NEN, NQ, double, true>(mv.n_el), cap);
-            (void)resident_grid<k_batch_elem<NEN, NQ>, RefApplyCfg<NEN>::SMEM, 128>(1);  // shared-memory attribute
+            S.elem_blocks = capped(apply_ref_elem_grid<NEN, NQ, float, double, true>(mv.n_el), cap);
+            (void)frame_resident_grid<k_batch_elem<NEN, NQ>, NEN, NQ>(1);
             return DFEA_OK;
         });
         if (rc) return rc;
@@ -1168,7 +1186,7 @@ extern "C" int dfea_batch_iterate(dfea_batch* b, int32_t n_iterations, int32_t* 
             const auto& ty = b->types[t];
             rc = dispatch_element(ty.nen, ty.nq, [&](auto nen_c, auto nq_c) -> int {
                 constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
-                return launch_kernel(k_batch_elem<NEN, NQ>, dim3(ty.count), dim3(128), RefApplyCfg<NEN>::SMEM, s, pdl,
+                return launch_kernel(k_batch_elem<NEN, NQ>, dim3(ty.count), dim3(FrameCfg<NEN, NQ>::NT), 0, s, pdl,
                                      (const BatchSolve*)b->d_solves, (const int2*)(b->d_map + ty.first),
                                      ref_grad_of<NEN, NQ>(ty.view));
             });

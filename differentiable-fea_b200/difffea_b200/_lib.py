@@ -16,6 +16,7 @@ DFEA_F64 = 0
 DFEA_F32 = 1
 DFEA_MIXED = 2      # PCG: FP32 moduli/gradients, FP64 Krylov vectors
 DFEA_F32REF = 3     # FP32 moduli in the element reference frame (10 per Gauss point), FP64 vectors
+DFEA_F64REF = 4     # the same in FP64
 MAX_COLOURS = 64
 
 PCG_STATUS = {0: "running", 1: "converged", 2: "max_iter", 3: "negative_curvature", 4: "zero_rhs"}
@@ -50,7 +51,7 @@ class MeshView(ctypes.Structure):
         ("colour_begin", c_i64 * (MAX_COLOURS + 1)),
         ("conn", c_vp), ("orig", c_vp), ("grad", c_vp), ("wdet", c_vp), ("grad32", c_vp), ("node_fix", c_vp),
         ("node_elem_ptr", c_vp), ("node_elem", c_vp),
-        ("jinv", c_vp), ("ref_grad", ctypes.c_double * (9 * 9 * 2)),
+        ("jinv", c_vp), ("ref_grad", ctypes.c_double * (9 * 9 * 2)), ("frame", c_vp),
     ]
 
 
@@ -85,7 +86,7 @@ class Newton(ctypes.Structure):
                 ("u_D", c_vp), ("u", c_vp), ("w", c_vp), ("uc", c_vp), ("R", c_vp), ("Rc", c_vp), ("du", c_vp),
                 ("b", c_vp), ("diag", c_vp), ("blocks", c_vp), ("moduli", c_vp), ("moduli_dtype", c_i32),
                 ("reserved", c_i32), ("reduce_work", c_vp), ("scal", c_vp), ("scal_host", c_vp), ("pcg", c_vp),
-                ("mg", ctypes.POINTER(Mg)), ("min_rtol", c_f64)]
+                ("mg", ctypes.POINTER(Mg)), ("min_rtol", c_f64), ("frame_work", c_vp)]
 
 
 class NewtonRecord(ctypes.Structure):
@@ -136,6 +137,19 @@ _PROTOS = {
     "dfea_internal_force_mat": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, ctypes.POINTER(Material), c_vp,
                                                c_vp]),
     "dfea_tangent_apply": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_i32, c_vp, c_vp, c_i32, c_vp]),
+    "dfea_mesh_frame": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, c_vp, c_vp]),
+    "dfea_frame_work_bytes": (c_i64, [ctypes.POINTER(MeshView)]),
+    "dfea_frame_moduli": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, ctypes.POINTER(Material), c_vp, c_vp, c_vp,
+                                         c_i32, c_vp, c_vp, c_vp, c_vp]),
+    "dfea_frame_residual": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, ctypes.POINTER(Material), c_vp, c_vp,
+                                           c_vp, c_f64, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "dfea_frame_internal_force": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, ctypes.POINTER(Material), c_vp,
+                                                 c_vp, c_vp, c_vp, c_vp]),
+    "dfea_frame_sensitivity": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, ctypes.POINTER(Material), c_vp, c_vp,
+                                              c_vp, c_vp]),
+    "dfea_frame_fields": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, ctypes.POINTER(Material), c_vp, c_vp, c_vp,
+                                         c_vp]),
+    "dfea_frame_push_forward": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, c_vp]),
     "dfea_gather_work_bytes": (c_i64, [ctypes.POINTER(MeshView), c_i32]),
     "dfea_tangent_apply_gather": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_i32, c_vp, c_vp, c_i32, c_vp,
                                                  c_vp]),

@@ -15,6 +15,7 @@ import warnings
 import torch
 
 from difffea_b200 import ops
+from difffea_b200.materials import device_material
 from difffea_b200.newton_krylov import pcg
 from difffea_b200.operators import _f64c, _prepare, make_AT_operator, make_preconditioner
 
@@ -64,14 +65,13 @@ def solve_adjoint(u_star, theta, params, dL_du, rtol=1e-6, max_iter=500, precond
     if on_failure not in ("warn", "raise", "ignore"):
         raise ValueError("on_failure must be 'warn', 'raise' or 'ignore'")
     b = (params["m"] * dL_du).to(torch.float64).contiguous()
-    mesh, _, _ = _prepare(u_star, theta, params)
+    mesh, _ = _prepare(u_star, theta, params)
     preconditioner = _adjoint_preconditioner(preconditioner, params, mesh)
     if preconditioner == "multigrid":
-        from difffea_b200 import _lib
         from difffea_b200.operators import make_A_operator_cuda, multigrid_for
         A = make_A_operator_cuda(u_star, theta, params)          # A^T = A: the tangent is symmetric
         mg = multigrid_for(A.mesh, params)
-        mg.setup(A.C, _lib.DFEA_F64, A.diag)
+        mg.setup(A.moduli, A.code, A.diag)
         lam = torch.empty_like(b)
         iters, status = mg.pcg(b, lam, rtol, max_iter)
     else:
@@ -86,5 +86,7 @@ def solve_adjoint(u_star, theta, params, dL_du, rtol=1e-6, max_iter=500, precond
 
 def compute_implicit_vjp(u_star, theta, params, lambda_adj):
     """dL/dtheta (n_el,) = -lambda^T dR/dtheta (theta enters linearly, so no theta dependence remains)."""
-    mesh, mid, mat = _prepare(u_star, theta, params)
-    return ops.element_sensitivity(mid, _f64c(u_star), _f64c(lambda_adj), *ops.material_args(mat))
+    mesh, mid = _prepare(u_star, theta, params)
+    if mesh.ensure_frame():
+        return ops.frame_sensitivity(mid, _f64c(u_star), _f64c(lambda_adj), *ops.frame_material(params))
+    return ops.element_sensitivity(mid, _f64c(u_star), _f64c(lambda_adj), *ops.material_args(device_material(params)))

@@ -12,6 +12,7 @@ HBM layout per element (FP64): conn 4 B x nen, orig 4 B, dN/dX 16 B x nen x n_q,
 per node: one fix-bit byte.  Rows are padded to a multiple of 32 elements.
 """
 import ctypes
+import threading
 import weakref
 
 import numpy as np
@@ -131,6 +132,10 @@ class CudaMesh:
         self.jinv = None
         self._nodes = params["nodes"]
         self._reduce_work = None
+        v.frame = None
+        self.frame = None
+        self._frame_check = None
+        self._lock = threading.RLock()       # the arrays built on demand, when several threads share the mesh
 
     # -------------------------------------------------------------------------------------------
     @property
@@ -155,6 +160,10 @@ class CudaMesh:
         Build the node -> element incidence of the gather form once: the slots of node n are the flat
         indices a * stride + e of its (element, local node) pairs, in increasing order.
         """
+        with self._lock:
+            return self._node_incidence()
+
+    def _node_incidence(self):
         if self.node_elem is None:
             S, nen, n, N, dev = self.stride, self.nen, self.n_el, self.n_nodes, self.device
             if nen * S >= 2 ** 31:
@@ -169,6 +178,35 @@ class CudaMesh:
             self.view.node_elem = self.node_elem.data_ptr()
         return self.node_elem_ptr, self.node_elem
 
+    # A Gauss point's dN/dX is taken as Jinv^T dN/dxi when the fitted Jinv reproduces it to this, relative to its
+    # largest entry: rounding leaves ~1e-15, and what is below the tolerance stays far inside FP64 parity (1e-11).
+    FRAME_TOLERANCE = 2e-13
+
+    def ensure_frame(self):
+        """
+        The FP64 frame of the mesh (Jinv of every Gauss point, fitted to the packed dN/dX) with the node incidence
+        its node passes need, built once; returns whether the frame kernels can be used.  A problem whose dN/dX is
+        not Jinv^T dN/dxi with this package's reference gradients (another quadrature, FP32 geometry) keeps the
+        kernels that read dN/dX.
+        """
+        with self._lock:
+            if self._frame_check is None:
+                if self.nen * self.stride >= 2 ** 31:                   # no 32-bit incidence
+                    self._frame_check = (float("inf"), 0.0, float("inf"))
+                    return False
+                self._node_incidence()
+                dev, S, nq = self.device, self.stride, self.n_q
+                nodes = self._nodes.detach().to(dev, torch.float64).contiguous()
+                frame = torch.empty(nq * 2 * S * 2, dtype=torch.float64, device=dev)
+                check = torch.empty(3, dtype=torch.float64, device=dev)
+                with torch.cuda.device(dev):
+                    _lib.call("dfea_mesh_frame", self.view_ref, ptr(nodes), ptr(frame), ptr(check), stream_handle())
+                self._frame_check = tuple(check.tolist())
+                if not self.n_el or self._frame_check[2] <= self.FRAME_TOLERANCE:
+                    self.frame = frame
+                    self.view.frame = frame.data_ptr()
+            return self.frame is not None
+
     def ensure_ref_frame(self):
         """
         Inverse element Jacobians Jinv = (dX/dxi)^-1 at the Gauss points, packed [n_q][2][stride] (rows of
@@ -176,24 +214,33 @@ class CudaMesh:
         Jinv^T dN/dxi with this package's quadrature; a mismatch raises instead of computing a wrong
         operator.
         """
-        if self.jinv is None:
-            dev, S, nq = self.device, self.stride, self.n_q
-            nodes = self._nodes.detach().to(dev, torch.float64).contiguous()
-            jinv = torch.empty(nq * 2 * S * 2, dtype=torch.float64, device=dev)
-            check = torch.empty(2, dtype=torch.float64, device=dev)
-            with torch.cuda.device(dev):
-                _lib.call("dfea_mesh_ref_frame", self.view_ref, ptr(nodes), ptr(jinv), ptr(check), stream_handle())
-            diff, scale = check.tolist()
-            if self.n_el and diff > 1e-9 * scale:
-                raise ValueError("dN_dX does not match this package's reference gradients and quadrature; "
-                                 "the reference-frame operator cannot be used for this problem")
-            self.jinv = jinv.view(nq, 2, S, 2)
-            self.view.jinv = self.jinv.data_ptr()
-        return self.jinv
+        with self._lock:
+            if self.jinv is None:
+                dev, S, nq = self.device, self.stride, self.n_q
+                if self.ensure_frame():
+                    jinv, (diff, scale) = self.frame, self._frame_check[:2]
+                else:
+                    nodes = self._nodes.detach().to(dev, torch.float64).contiguous()
+                    jinv = torch.empty(nq * 2 * S * 2, dtype=torch.float64, device=dev)
+                    check = torch.empty(2, dtype=torch.float64, device=dev)
+                    with torch.cuda.device(dev):
+                        _lib.call("dfea_mesh_ref_frame", self.view_ref, ptr(nodes), ptr(jinv), ptr(check),
+                                  stream_handle())
+                    diff, scale = check.tolist()
+                if self.n_el and diff > 1e-9 * scale:
+                    raise ValueError("dN_dX does not match this package's reference gradients and quadrature; "
+                                     "the reference-frame operator cannot be used for this problem")
+                self.jinv = jinv.view(nq, 2, S, 2)
+                self.view.jinv = self.jinv.data_ptr()
+            return self.jinv
 
     def moduli_numel_ref(self):
-        """FP32 entries of the reference-frame moduli (10 per Gauss point)."""
+        """Entries of the reference-frame moduli (10 per Gauss point)."""
         return self.n_q * 10 * self.stride
+
+    def frame_work(self):
+        """Scratch of one frame call (dfea_frame_*), from the caching allocator: private to the call's stream."""
+        return torch.empty(int(_lib.load().dfea_frame_work_bytes(self.view_ref)), dtype=torch.uint8, device=self.device)
 
     def reduce_work(self):
         if self._reduce_work is None:
@@ -206,7 +253,8 @@ class CudaMesh:
 
     def hbm_bytes(self):
         t = [self.conn, self.orig, self.grad, self.wdet, self.node_fix, self.perm]
-        for extra in (self.grad32, self.node_elem_ptr, self.node_elem, self.jinv):
+        for extra in (self.grad32, self.node_elem_ptr, self.node_elem, self.frame,
+                      None if self.frame is not None else self.jinv):
             if extra is not None:
                 t.append(extra)
         return sum(x.numel() * x.element_size() for x in t)

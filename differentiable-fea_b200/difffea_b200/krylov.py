@@ -30,9 +30,9 @@ class DevicePCG:
     per-node sums fused into the first vector update: 3 kernels per iteration; needs the mesh's node
     incidence, built here) or "fused" (the gather form with the direction update moved into the next
     element pass: 2 kernels per iteration).  Each form is reproducible; they agree to rounding.
-    moduli: "physical" (C with the packed dN/dX: FP64, FP32, or FP32 on FP64 vectors) or "ref" (FP32
+    moduli: "physical" (C with the packed dN/dX: FP64, FP32, or FP32 on FP64 vectors) or "ref" (FP32 or FP64
     moduli pulled back to the element reference frame, 10 per Gauss point, FP64 vectors; the product
-    reads no gradients).  max_blocks: at most this many blocks per launch (0: the whole GPU), for solves
+    reads no gradients; FP64: the gather and fused forms).  max_blocks: at most this many blocks per launch (0: the whole GPU), for solves
     that share the GPU with others; results agree with the unlimited form's to rounding.
     preconditioner: "jacobi" (diag = the (2N,) diagonal) or "block_jacobi" (diag = the (4N,) inverse 2x2
     node blocks of dfea_qp_moduli_block; FP64 vectors).
@@ -58,10 +58,12 @@ class DevicePCG:
         self.preconditioner = preconditioner
         vt = b.dtype
         if moduli == "ref":
-            # FP32 moduli in the element reference frame (10 per Gauss point): no gradients read
-            if C.dtype != torch.float32 or vt != torch.float64 or C.numel() != mesh.moduli_numel_ref():
-                raise ValueError("reference-frame moduli: FP32, 10 per Gauss point, with FP64 vectors")
-            dt = _lib.DFEA_F32REF
+            # moduli in the element reference frame (10 per Gauss point): no gradients read
+            if vt != torch.float64 or C.numel() != mesh.moduli_numel_ref():
+                raise ValueError("reference-frame moduli: 10 per Gauss point, with FP64 vectors")
+            dt = _lib.DFEA_F32REF if C.dtype == torch.float32 else _lib.DFEA_F64REF
+            if dt == _lib.DFEA_F64REF and form == "colour":
+                raise ValueError("FP64 reference-frame moduli need the gather or fused form")
         elif moduli != "physical":
             raise ValueError("moduli must be 'physical' or 'ref'")
         elif C.dtype == torch.float64:

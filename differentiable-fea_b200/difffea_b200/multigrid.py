@@ -177,7 +177,8 @@ class Multigrid:
         from the host.  Both give the same iterates.  ``bounds_every``: 0 estimates the smoother bounds by
         Lanczos at every set-up; k > 0 at the first set-up and every k-th after it, keeping the last estimates
         in between (a set-up then rebuilds the coarse operators only).  ``gather``: the level-0 products in the
-        gather form (2 launches each; the mesh's node incidence is built here) instead of one per colour."""
+        gather form (2 launches each; the mesh's node incidence is built here) instead of one per colour; a mesh
+        with a frame takes the gather form in any case."""
         g = structured_grid(params["conn"].to(mesh.device), mesh.n_nodes)
         if g is None:
             raise ValueError("preconditioner='multigrid' needs a structured mesh (a logical grid of cells)")
@@ -272,7 +273,7 @@ class Multigrid:
         h.graphs = None
         h.bounds_every, h.setups = int(bounds_every), 0
         self.fe_work = None
-        if gather:
+        if gather or mesh.ensure_frame():
             mesh.ensure_node_incidence()
             self.fe_work = torch.empty(int(_lib.load().dfea_gather_work_bytes(mesh.view_ref, _lib.DFEA_F64)),
                                        dtype=torch.uint8, device=dev)

@@ -20,7 +20,7 @@ import weakref
 
 import torch
 
-from difffea_b200 import ops
+from difffea_b200 import _lib, ops
 from difffea_b200.cuda_mesh import _require_cuda, cuda_mesh
 from difffea_b200.materials import device_material
 from difffea_b200.problem import precompute_geometry  # noqa: F401  (re-exported, as in the reference)
@@ -35,7 +35,7 @@ def _prepare(u, theta, params):
     mesh = cuda_mesh(params)
     if u.device != mesh.device:
         raise RuntimeError("u and params must be on the same device")
-    return mesh, ops.register_mesh(mesh), device_material(params)
+    return mesh, ops.register_mesh(mesh)
 
 
 def _f64c(t):
@@ -47,24 +47,28 @@ def _f64c(t):
 # ---------------------------------------------------------------------------------------------
 def global_residual(u, theta, params, load_factor=1.0):
     """R(u) = m * (R_int(u, theta) - load_factor * f), shape (2N,)."""
-    mesh, mid, mat = _prepare(u, theta, params)
-    R, _, _ = ops.residual(mid, _f64c(u), _f64c(theta), *ops.material_args(mat), _f64c(params["f"]), float(load_factor))
-    return R
+    return _residual(u, theta, params, load_factor, False)[0]
+
+
+def _residual(u, theta, params, load_factor, scalars):
+    """(R, (|R|^2, strain energy) on the device with ``scalars``)."""
+    mesh, mid = _prepare(u, theta, params)
+    u, theta, f = _f64c(u), _f64c(theta), _f64c(params["f"])
+    if mesh.ensure_frame():
+        return ops.frame_residual(mid, u, theta, *ops.frame_material(params), f, float(load_factor), scalars)
+    R, n2, W = ops.residual(mid, u, theta, *ops.material_args(device_material(params)), f, float(load_factor))
+    return R, (n2, W)
 
 
 def residual_and_norm(u, theta, params, load_factor=1.0):
     """(R, ||R||) with the norm reduced on the device in fixed order (one scalar read-back)."""
-    mesh, mid, mat = _prepare(u, theta, params)
-    R, n2, _ = ops.residual(mid, _f64c(u), _f64c(theta), *ops.material_args(mat), _f64c(params["f"]),
-                            float(load_factor))
+    R, (n2, _) = _residual(u, theta, params, load_factor, True)
     return R, float(n2) ** 0.5
 
 
 def strain_energy(u, theta, params):
     """Total strain energy sum_e sum_q w detJ psi(F), the ``strain_energy`` of compute_fields."""
-    mesh, mid, mat = _prepare(u, theta, params)
-    _, _, W = ops.residual(mid, _f64c(u), _f64c(theta), *ops.material_args(mat), _f64c(params["f"]), 0.0)
-    return W
+    return _residual(u, theta, params, 0.0, True)[1][1]
 
 
 # ---------------------------------------------------------------------------------------------
@@ -72,25 +76,36 @@ def strain_energy(u, theta, params):
 # ---------------------------------------------------------------------------------------------
 class CudaTangentOperator:
     """
-    v -> A(v) from moduli stored at the Gauss points (kernel (b)).  Holds the moduli C of its
-    linearisation point and the Jacobi diagonal computed in the same pass of kernel (a).
+    v -> A(v) from moduli stored at the Gauss points (kernel (b)).  Holds the moduli of its linearisation point
+    (``moduli``, layout ``code``: FP64 in the element reference frame where the mesh has one, else the 16 physical
+    entries) and the Jacobi diagonal computed in the same pass of kernel (a).
     """
 
-    def __init__(self, mesh, mesh_id, C, diag, precision="fp64"):
-        self.mesh, self.mesh_id, self.C, self.diag, self.precision = mesh, mesh_id, C, diag, precision
+    def __init__(self, mesh, mesh_id, moduli, diag, precision="fp64"):
+        self.mesh, self.mesh_id, self.moduli, self.diag, self.precision = mesh, mesh_id, moduli, diag, precision
+        self.code = (_lib.DFEA_F32 if moduli.dtype == torch.float32 else
+                     _lib.DFEA_F64REF if moduli.numel() == mesh.moduli_numel_ref() else _lib.DFEA_F64)
+        self._physical = None if self.code == _lib.DFEA_F64REF else moduli
         self._pcg = None
         self._pcg_diag_src = None
         self.last_status = None
 
+    @property
+    def C(self):
+        """The 16 physical moduli per Gauss point; from the reference-frame ones on first use."""
+        if self._physical is None:
+            self._physical = ops.frame_push_forward(self.mesh_id, self.moduli)
+        return self._physical
+
     def __call__(self, v):
         """A(v); FP32 moduli apply to FP32 vectors, or to FP64 vectors with FP64 arithmetic."""
-        if v.dtype != self.C.dtype and not (self.C.dtype == torch.float32 and v.dtype == torch.float64):
-            raise ValueError(f"this operator applies {self.C.dtype} vectors, got {v.dtype}")
-        return ops.tangent_apply(self.mesh_id, self.C, v.contiguous())
+        if v.dtype != self.dtype and not (self.dtype == torch.float32 and v.dtype == torch.float64):
+            raise ValueError(f"this operator applies {self.dtype} vectors, got {v.dtype}")
+        return ops.tangent_apply(self.mesh_id, self.moduli, v.contiguous())
 
     @property
     def dtype(self):
-        return self.C.dtype
+        return self.moduli.dtype
 
     def pcg_solve(self, b, diag, rtol, max_iter, preconditioner="jacobi"):
         """
@@ -98,7 +113,7 @@ class CudaTangentOperator:
         the Jacobi diagonal, or with preconditioner="block_jacobi" the (4N,) inverse node blocks.
         """
         from difffea_b200.krylov import DevicePCG
-        vt = b.dtype if self.C.dtype == torch.float32 else torch.float64   # FP32 moduli: FP64 or FP32 vectors
+        vt = b.dtype if self.dtype == torch.float32 else torch.float64   # FP32 moduli: FP64 or FP32 vectors
         if preconditioner == "block_jacobi":
             vt = torch.float64
         if (self._pcg is None or self._pcg_diag_src is not diag or self._pcg.vec_dtype != vt
@@ -109,7 +124,8 @@ class CudaTangentOperator:
             xx = torch.empty(n, dtype=vt, device=self.mesh.device)
             if self._pcg is not None:
                 self._pcg.close()
-            self._pcg = DevicePCG(self.mesh, self.C, d, bb, xx, preconditioner=preconditioner)
+            ref = dict(form="fused", moduli="ref", use_graph=2) if self.code == _lib.DFEA_F64REF else {}
+            self._pcg = DevicePCG(self.mesh, self.moduli, d, bb, xx, preconditioner=preconditioner, **ref)
             self._pcg_diag_src = diag
         self._pcg.b.copy_(b)
         iters, status = self._pcg.solve(rtol, max_iter)
@@ -130,10 +146,14 @@ def make_A_operator_cuda(u, theta, params, precision="fp64"):
     """The stored-moduli tangent operator at (u, theta); precision "fp64" or "fp32" (moduli and vectors)."""
     if precision not in ("fp64", "fp32"):
         raise ValueError("precision must be 'fp64' or 'fp32'")
-    mesh, mid, mat = _prepare(u, theta, params)
+    mesh, mid = _prepare(u, theta, params)
     if precision == "fp32":
         mesh.ensure_grad32()
-    C, diag = ops.qp_moduli(mid, _f64c(u), _f64c(theta), *ops.material_args(mat), precision == "fp32", True)
+    if precision == "fp64" and mesh.ensure_frame():
+        C, diag, _ = ops.frame_moduli(mid, _f64c(u), _f64c(theta), *ops.frame_material(params), True, False)
+    else:
+        C, diag = ops.qp_moduli(mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)),
+                                precision == "fp32", True)
     _LAST_DIAG.clear()
     _LAST_DIAG[_diag_key(u, theta, mesh)] = (weakref.ref(u), weakref.ref(theta), diag)
     return CudaTangentOperator(mesh, mid, C, diag, precision)
@@ -178,21 +198,25 @@ class CudaJacobiPreconditioner:
 
 def compute_jacobi_diagonal(u, theta, params):
     """diag(K) without forming K (kernel (a)'s element diagonals, scattered by colour), shape (2N,)."""
-    mesh, mid, mat = _prepare(u, theta, params)
+    mesh, mid = _prepare(u, theta, params)
     hit = _LAST_DIAG.get(_diag_key(u, theta, mesh))
     if hit is not None and hit[0]() is u and hit[1]() is theta:
         return hit[2]
-    return _diag_only(mesh, u, theta, mat)
+    return _preconditioner_data(mesh, mid, u, theta, params, False)[0]
 
 
-def _diag_only(mesh, u, theta, mat):
-    from difffea_b200 import _lib
+def _preconditioner_data(mesh, mid, u, theta, params, with_blocks):
+    """(diag, blocks or None) at (u, theta), without storing moduli."""
     u64, th64 = _f64c(u), _f64c(theta)
+    if mesh.ensure_frame():
+        _, diag, blocks = ops.frame_moduli(mid, u64, th64, *ops.frame_material(params), False, with_blocks)
+        return diag, blocks
     diag = torch.empty(mesh.n_dof, dtype=torch.float64, device=mesh.device)
-    empty = torch.empty(0, dtype=torch.float64, device=mesh.device)
-    torch.ops.difffea_b200.qp_moduli_out(ops.register_mesh(mesh), u64, th64, *ops.material_args(mat), empty,
-                                         _lib.DFEA_F64, diag, empty)
-    return diag
+    blocks = torch.empty(2 * mesh.n_dof if with_blocks else 0, dtype=torch.float64, device=mesh.device)
+    torch.ops.difffea_b200.qp_moduli_out(mid, u64, th64, *ops.material_args(device_material(params)),
+                                         torch.empty(0, dtype=torch.float64, device=mesh.device), _lib.DFEA_F64, diag,
+                                         blocks)
+    return diag, blocks
 
 
 def make_jacobi_preconditioner(u, theta, params):
@@ -218,15 +242,8 @@ class CudaBlockJacobiPreconditioner:
 
 def compute_block_jacobi(u, theta, params):
     """The (4N,) inverse 2x2 node blocks of the tangent at (u, theta) (kernel (a) with the coupling term)."""
-    from difffea_b200 import _lib
-    mesh, mid, mat = _prepare(u, theta, params)
-    u64, th64 = _f64c(u), _f64c(theta)
-    diag = torch.empty(mesh.n_dof, dtype=torch.float64, device=mesh.device)
-    blocks = torch.empty(2 * mesh.n_dof, dtype=torch.float64, device=mesh.device)
-    torch.ops.difffea_b200.qp_moduli_out(mid, u64, th64, *ops.material_args(mat),
-                                         torch.empty(0, dtype=torch.float64, device=mesh.device), _lib.DFEA_F64,
-                                         diag, blocks)
-    return blocks
+    mesh, mid = _prepare(u, theta, params)
+    return _preconditioner_data(mesh, mid, u, theta, params, True)[1]
 
 
 def make_block_jacobi_preconditioner(u, theta, params):
@@ -252,8 +269,7 @@ class CudaMultigridPreconditioner:
     def refresh(self):
         """Set the shared hierarchy up at this closure's linearisation again if another set-up replaced it."""
         if self.mg.generation != self.generation:
-            from difffea_b200 import _lib
-            self.mg.setup(self.A.C, _lib.DFEA_F64, self.A.diag)
+            self.mg.setup(self.A.moduli, self.A.code, self.A.diag)
             self.generation = self.mg.generation
 
     def __call__(self, r):
@@ -279,8 +295,7 @@ def multigrid_for(mesh, params):
 def make_multigrid_preconditioner(u, theta, params):
     A = make_A_operator_cuda(u, theta, params)
     mg = multigrid_for(A.mesh, params)
-    from difffea_b200 import _lib
-    mg.setup(A.C, _lib.DFEA_F64, A.diag)
+    mg.setup(A.moduli, A.code, A.diag)
     return CudaMultigridPreconditioner(mg, A)
 
 

@@ -18,6 +18,10 @@ Each op is a thin shim: it allocates its outputs through torch's caching allocat
     torch.ops.difffea_b200.mg_pcg(mg_id, C, moduli_code, b, x, rtol, max_iter) -> [iterations, status]
     torch.ops.difffea_b200.newton_solve(ws_id, theta, n_load_steps, tol, max_newton, max_cutbacks,
                                         pcg_max_iter) -> (u, [converged, load factor, Newton, CG, cut-backs])
+the same on a mesh with a frame (CudaMesh.ensure_frame), in one element pass and one node pass:
+    torch.ops.difffea_b200.frame_moduli / frame_residual / frame_internal_force / frame_sensitivity / frame_fields
+    torch.ops.difffea_b200.frame_push_forward(mesh_id, C) -> physical moduli
+    torch.ops.difffea_b200.frame_residual_out / frame_moduli_out (caller buffers)
 and three forms that write into caller buffers, for the solver's preallocated workspace:
     torch.ops.difffea_b200.residual_out(mesh_id, u, theta, model, scalable, mat_p, f, load_factor, R!, scal!, energy)
     torch.ops.difffea_b200.qp_moduli_out(mesh_id, u, theta, model, scalable, mat_p, C!, moduli_code, diag!, blocks!)
@@ -35,6 +39,7 @@ import torch
 
 from difffea_b200 import _lib
 from difffea_b200.cuda_mesh import ptr, stream_handle
+from difffea_b200.materials import device_material
 
 _MESHES = weakref.WeakValueDictionary()
 
@@ -123,6 +128,15 @@ def tangent_apply(mesh_id: int, C: torch.Tensor, v: torch.Tensor) -> torch.Tenso
     if v.device != mesh.device or not v.is_contiguous() or v.numel() != mesh.n_dof:
         raise ValueError("v must be a contiguous (2N,) tensor on the mesh's device")
     y = torch.empty_like(v)
+    if C.numel() == mesh.moduli_numel_ref():
+        # reference-frame moduli: the gather form, with its element results in scratch of this call
+        mesh.ensure_node_incidence()
+        fe = torch.empty(int(_lib.load().dfea_gather_work_bytes(mesh.view_ref, _lib.DFEA_F64)), dtype=torch.uint8,
+                         device=mesh.device)
+        code = _lib.DFEA_F64REF if C.dtype == torch.float64 else _lib.DFEA_F32REF
+        _lib.call("dfea_tangent_apply_gather", mesh.view_ref, ptr(C), code, ptr(v), ptr(y),
+                  _lib.DFEA_F32 if fp32 else _lib.DFEA_F64, ptr(fe), stream_handle())
+        return y
     dt = _lib.DFEA_F32 if fp32 else _lib.DFEA_F64
     cdt = _lib.DFEA_F32 if C.dtype == torch.float32 else _lib.DFEA_F64
     _lib.call("dfea_tangent_apply", mesh.view_ref, ptr(C), cdt, ptr(v), ptr(y), dt, stream_handle())
@@ -221,6 +235,154 @@ def internal_force(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: in
 @internal_force.register_fake
 def _(mesh_id, u, theta, model, scalable, mat_p):
     return torch.empty_like(u)
+
+
+# ---------------------------------------------------------------------------------------------
+# the same quantities on a mesh with a frame (CudaMesh.ensure_frame): one element pass and one node pass
+# ---------------------------------------------------------------------------------------------
+def frame_material(params):
+    """(model, scalable, mat_p) of a problem for the frame_* ops."""
+    return material_args(device_material(params))
+
+
+def _frame_mesh(mesh_id, u, theta=None):
+    mesh = _mesh(mesh_id)
+    _f64(u, mesh, mesh.n_dof)
+    if theta is not None:
+        _f64(theta, mesh, mesh.n_el)
+    if mesh.frame is None:
+        raise ValueError("the mesh has no frame (CudaMesh.ensure_frame)")
+    return mesh
+
+
+def _frame_args(model, scalable, mat_p):
+    return _material(model, scalable, mat_p), ptr(None), ptr(None)
+
+
+@torch.library.custom_op("difffea_b200::frame_moduli", mutates_args=(), device_types="cuda")
+def frame_moduli(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int, mat_p: list[float],
+                 with_moduli: bool, with_blocks: bool) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """FP64 reference-frame moduli (empty without with_moduli), Jacobi diagonal, inverse node blocks (or empty)."""
+    mesh = _frame_mesh(mesh_id, u, theta)
+    f64 = dict(dtype=torch.float64, device=mesh.device)
+    C = torch.empty(mesh.moduli_numel_ref() if with_moduli else 0, **f64)
+    diag = torch.empty(mesh.n_dof, **f64)
+    blocks = torch.empty(2 * mesh.n_dof if with_blocks else 0, **f64)
+    _lib.call("dfea_frame_moduli", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p),
+              ptr(C if with_moduli else None), _lib.DFEA_F64REF, ptr(diag), ptr(blocks if with_blocks else None),
+              ptr(mesh.frame_work()), stream_handle())
+    return C, diag, blocks
+
+
+@frame_moduli.register_fake
+def _(mesh_id, u, theta, model, scalable, mat_p, with_moduli, with_blocks):
+    mesh = _mesh(mesh_id)
+    return (u.new_empty(mesh.moduli_numel_ref() if with_moduli else 0), u.new_empty(mesh.n_dof),
+            u.new_empty(2 * mesh.n_dof if with_blocks else 0))
+
+
+@torch.library.custom_op("difffea_b200::frame_residual", mutates_args=(), device_types="cuda")
+def frame_residual(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int, mat_p: list[float],
+                   f: torch.Tensor, load_factor: float, scalars: bool) -> tuple[torch.Tensor, torch.Tensor]:
+    """R and, with scalars, (|R|^2, strain energy) on the device (else empty)."""
+    mesh = _frame_mesh(mesh_id, u, theta)
+    _f64(f, mesh, mesh.n_dof)
+    R = torch.empty_like(u)
+    out = torch.empty(2 if scalars else 0, dtype=torch.float64, device=mesh.device)
+    _lib.call("dfea_frame_residual", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p), ptr(f),
+              float(load_factor), ptr(R), ptr(out if scalars else None), ptr(out[1:] if scalars else None),
+              ptr(mesh.frame_work()), stream_handle())
+    return R, out
+
+
+@frame_residual.register_fake
+def _(mesh_id, u, theta, model, scalable, mat_p, f, load_factor, scalars):
+    return torch.empty_like(u), u.new_empty(2 if scalars else 0)
+
+
+@torch.library.custom_op("difffea_b200::frame_internal_force", mutates_args=(), device_types="cuda")
+def frame_internal_force(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int,
+                         mat_p: list[float]) -> torch.Tensor:
+    mesh = _frame_mesh(mesh_id, u, theta)
+    R = torch.empty_like(u)
+    _lib.call("dfea_frame_internal_force", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p),
+              ptr(R), ptr(mesh.frame_work()), stream_handle())
+    return R
+
+
+@frame_internal_force.register_fake
+def _(mesh_id, u, theta, model, scalable, mat_p):
+    return torch.empty_like(u)
+
+
+@torch.library.custom_op("difffea_b200::frame_sensitivity", mutates_args=(), device_types="cuda")
+def frame_sensitivity(mesh_id: int, u: torch.Tensor, lam: torch.Tensor, model: int, scalable: int,
+                      mat_p: list[float]) -> torch.Tensor:
+    mesh = _frame_mesh(mesh_id, u)
+    _f64(lam, mesh, mesh.n_dof)
+    g = torch.empty(mesh.n_el, dtype=torch.float64, device=mesh.device)
+    _lib.call("dfea_frame_sensitivity", mesh.view_ref, ptr(u), ptr(lam), *_frame_args(model, scalable, mat_p), ptr(g),
+              stream_handle())
+    return g
+
+
+@frame_sensitivity.register_fake
+def _(mesh_id, u, lam, model, scalable, mat_p):
+    return u.new_empty(_mesh(mesh_id).n_el)
+
+
+@torch.library.custom_op("difffea_b200::frame_fields", mutates_args=(), device_types="cuda")
+def frame_fields(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int,
+                 mat_p: list[float]) -> torch.Tensor:
+    mesh = _frame_mesh(mesh_id, u, theta)
+    out = torch.empty(7, mesh.n_el, dtype=torch.float64, device=mesh.device)
+    _lib.call("dfea_frame_fields", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p), ptr(out),
+              stream_handle())
+    return out
+
+
+@frame_fields.register_fake
+def _(mesh_id, u, theta, model, scalable, mat_p):
+    return u.new_empty(7, _mesh(mesh_id).n_el)
+
+
+@torch.library.custom_op("difffea_b200::frame_push_forward", mutates_args=(), device_types="cuda")
+def frame_push_forward(mesh_id: int, C: torch.Tensor) -> torch.Tensor:
+    """The 16 physical moduli per Gauss point (DFEA_F64 layout) of FP64 reference-frame ones."""
+    mesh = _mesh(mesh_id)
+    _f64(C, mesh, mesh.moduli_numel_ref())
+    out = torch.zeros(mesh.moduli_numel(), dtype=torch.float64, device=mesh.device)
+    _lib.call("dfea_frame_push_forward", mesh.view_ref, ptr(C), ptr(out), stream_handle())
+    return out
+
+
+@frame_push_forward.register_fake
+def _(mesh_id, C):
+    return C.new_empty(_mesh(mesh_id).moduli_numel())
+
+
+@torch.library.custom_op("difffea_b200::frame_residual_out", mutates_args=("R", "scal", "work"), device_types="cuda")
+def frame_residual_out(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int, mat_p: list[float],
+                       f: torch.Tensor, load_factor: float, R: torch.Tensor, scal: torch.Tensor, energy: bool,
+                       work: torch.Tensor) -> None:
+    """residual_out on the frame, with its scratch in ``work`` (frame_work of the mesh)."""
+    mesh = _frame_mesh(mesh_id, u, theta)
+    _f64(R, mesh, mesh.n_dof)
+    if scal.dtype != torch.float64 or scal.numel() < 2 or scal.device != mesh.device:
+        raise ValueError("scal must hold at least 2 float64 entries on the mesh's device")
+    _lib.call("dfea_frame_residual", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p), ptr(f),
+              float(load_factor), ptr(R), ptr(scal), ptr(scal[1:] if energy else None), ptr(work), stream_handle())
+
+
+@torch.library.custom_op("difffea_b200::frame_moduli_out", mutates_args=("C", "diag", "blocks", "work"),
+                         device_types="cuda")
+def frame_moduli_out(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int, mat_p: list[float],
+                     C: torch.Tensor, moduli_code: int, diag: torch.Tensor, blocks: torch.Tensor,
+                     work: torch.Tensor) -> None:
+    """Reference-frame moduli into C, the Jacobi diagonal into diag and, when not empty, the inverse node blocks."""
+    mesh = _frame_mesh(mesh_id, u, theta)
+    _lib.call("dfea_frame_moduli", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p), ptr(C),
+              int(moduli_code), ptr(diag), ptr(blocks if blocks.numel() else None), ptr(work), stream_handle())
 
 
 # ---------------------------------------------------------------------------------------------

@@ -15,6 +15,7 @@ support reactions are the internal force with no mask (every DOF) summed over th
 import torch
 
 from difffea_b200 import ops
+from difffea_b200.materials import device_material
 from difffea_b200.operators import _f64c, _prepare
 
 ELEMENT_FIELDS = ("J", "sxx", "syy", "sxy", "mises", "energy_density")
@@ -22,8 +23,10 @@ ELEMENT_FIELDS = ("J", "sxx", "syy", "sxy", "mises", "energy_density")
 
 def element_fields(u, theta, params):
     """(7, n_el) per original element: area, then the weighted means J, sxx, syy, sxy, mises, psi."""
-    mesh, mid, mat = _prepare(u, theta, params)
-    return torch.ops.difffea_b200.element_fields(mid, _f64c(u), _f64c(theta), *ops.material_args(mat))
+    mesh, mid = _prepare(u, theta, params)
+    if mesh.ensure_frame():
+        return ops.frame_fields(mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
+    return ops.element_fields(mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)))
 
 
 def compute_fields(u, theta, params) -> dict:
@@ -33,7 +36,7 @@ def compute_fields(u, theta, params) -> dict:
         per node (N,):        ux, uy, u_mag (and ux_n, uy_n, u_mag_n), and J_n ... energy_density_n
         scalars (0-d):        strain_energy, min_J
     """
-    mesh, mid, _ = _prepare(u, theta, params)
+    mesh, mid = _prepare(u, theta, params)
     el = element_fields(u, theta, params)
     nodal = torch.ops.difffea_b200.node_fields(mid, el)
     un = _f64c(u).view(mesh.n_nodes, 2)
@@ -49,8 +52,10 @@ def compute_fields(u, theta, params) -> dict:
 
 def internal_force(u, theta, params):
     """R_int(u) at every DOF, the constrained ones included (no mask, no external load)."""
-    mesh, mid, mat = _prepare(u, theta, params)
-    return torch.ops.difffea_b200.internal_force(mid, _f64c(u), _f64c(theta), *ops.material_args(mat))
+    mesh, mid = _prepare(u, theta, params)
+    if mesh.ensure_frame():
+        return ops.frame_internal_force(mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
+    return ops.internal_force(mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)))
 
 
 def support_reactions(u, theta, params) -> torch.Tensor:

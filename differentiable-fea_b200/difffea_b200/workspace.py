@@ -2,9 +2,9 @@
 Per-problem device workspace of the Newton-Krylov solver.
 
 A ``NewtonWorkspace`` keeps everything a solve touches in HBM for the whole solve: the state and
-trial vectors, the residual, the Gauss-point moduli (FP64, or for the mixed-precision form FP32 moduli
-pulled back to each element's reference frame, so that its operator reads 10 FP32 numbers per Gauss
-point and no gradients, while the Krylov vectors stay FP64), the Jacobi diagonal,
+trial vectors, the residual, the Gauss-point moduli (pulled back to each element's reference frame, so that
+the operator reads 10 numbers per Gauss point and no gradients: FP64, or FP32 for the mixed-precision form,
+whose Krylov vectors stay FP64), the Jacobi diagonal,
 and one graph-captured ``DevicePCG`` bound to them (eight iterations per graph launch, replayed until
 the solve ends: faster than the conditional-loop graph, 23 vs 28 us per iteration at 16k elements).  The solver loop
 calls the C ABI directly on these buffers (no allocation per Newton step), reading back only the
@@ -25,10 +25,13 @@ from difffea_b200.materials import device_material
 GATHER_FORM_MAX_ELEMENTS = 1_500_000
 
 
-def pcg_form_for(mesh, pcg_form="auto"):
-    """The PCG product form: "colour", "gather", "fused", or "auto" (fused below GATHER_FORM_MAX_ELEMENTS)."""
+def pcg_form_for(mesh, pcg_form="auto", moduli_code=_lib.DFEA_F64):
+    """The PCG product form: "colour", "gather", "fused", or "auto" (fused below GATHER_FORM_MAX_ELEMENTS; above it
+    colour, or gather for FP64 reference-frame moduli, which have no colour form)."""
     if pcg_form == "auto":
-        return "fused" if mesh.n_el < GATHER_FORM_MAX_ELEMENTS else "colour"
+        if mesh.n_el < GATHER_FORM_MAX_ELEMENTS:
+            return "fused"
+        return "gather" if moduli_code == _lib.DFEA_F64REF else "colour"
     if pcg_form not in ("colour", "gather", "fused"):
         raise ValueError("pcg_form must be 'auto', 'colour', 'gather' or 'fused'")
     return pcg_form
@@ -64,7 +67,15 @@ class NewtonWorkspace:
         if fp32_moduli not in ("ref", "physical"):
             raise ValueError("fp32_moduli must be 'ref' or 'physical'")
         self.moduli_kind = "ref" if (precision == "fp32" and fp32_moduli == "ref") else "physical"
-        if self.moduli_kind == "ref":
+        # with a frame the residual and the reference-frame moduli come from the frame kernels, and the FP64 operator
+        # is stored in the reference frame as well (80 B per Gauss point); the colour form and meshes without a frame
+        # keep the physical moduli
+        self.frame_work = mesh.frame_work() if mesh.ensure_frame() else None
+        if precision == "fp64" and self.frame_work is not None and (preconditioner == "multigrid" or pcg_form != "colour"):
+            self.moduli_kind = "ref"
+            self.C = torch.empty(mesh.moduli_numel_ref(), dtype=torch.float64, device=dev)
+            self.moduli_code = _lib.DFEA_F64REF
+        elif self.moduli_kind == "ref":
             mesh.ensure_ref_frame()
             self.C = torch.empty(mesh.moduli_numel_ref(), dtype=torch.float32, device=dev)
             self.moduli_code = _lib.DFEA_F32REF
@@ -89,7 +100,8 @@ class NewtonWorkspace:
             self.pcg = None
         else:
             self.pcg = DevicePCG(mesh, self.C, self.diag if self.blocks is None else self.blocks, self.b, self.du,
-                                 use_graph=use_graph, form=pcg_form_for(mesh, pcg_form), moduli=self.moduli_kind,
+                                 use_graph=use_graph, form=pcg_form_for(mesh, pcg_form, self.moduli_code),
+                                 moduli=self.moduli_kind,
                                  max_blocks=max_blocks, preconditioner=preconditioner)
         self.work = mesh.reduce_work()
         self.mesh_id = ops.register_mesh(mesh)
@@ -123,8 +135,12 @@ class NewtonWorkspace:
 
     def residual(self, u, load_factor, out, energy=False):
         """out = R(u) (FP64); returns ||R|| (and the strain energy if asked) as Python floats."""
-        torch.ops.difffea_b200.residual_out(self.mesh_id, u, self.theta, *self.mat_args, self.f, float(load_factor),
-                                            out, self.scal, bool(energy))
+        if self.frame_work is not None:
+            torch.ops.difffea_b200.frame_residual_out(self.mesh_id, u, self.theta, *self.mat_args, self.f,
+                                                      float(load_factor), out, self.scal, bool(energy), self.frame_work)
+        else:
+            torch.ops.difffea_b200.residual_out(self.mesh_id, u, self.theta, *self.mat_args, self.f, float(load_factor),
+                                                out, self.scal, bool(energy))
         self.scal_host.copy_(self.scal, non_blocking=True)
         torch.cuda.current_stream().synchronize()
         rn = float(self.scal_host[0]) ** 0.5
@@ -132,8 +148,13 @@ class NewtonWorkspace:
 
     def linearize(self, u):
         """Kernel (a): moduli C and the preconditioner at u (into the buffers the PCG graph is bound to)."""
-        torch.ops.difffea_b200.qp_moduli_out(self.mesh_id, u, self.theta, *self.mat_args, self.C, self.moduli_code,
-                                             self.diag, self.blocks if self.blocks is not None else self._empty)
+        blocks = self.blocks if self.blocks is not None else self._empty
+        if self.frame_work is not None and self.moduli_kind == "ref":
+            torch.ops.difffea_b200.frame_moduli_out(self.mesh_id, u, self.theta, *self.mat_args, self.C,
+                                                    self.moduli_code, self.diag, blocks, self.frame_work)
+        else:
+            torch.ops.difffea_b200.qp_moduli_out(self.mesh_id, u, self.theta, *self.mat_args, self.C, self.moduli_code,
+                                                 self.diag, blocks)
         if self.mg is not None:
             self.mg.setup(self.C, self.moduli_code, self.diag)
 
@@ -186,7 +207,7 @@ class NewtonWorkspace:
         for name, t in (("f", self.f), ("u_D", self.u_D), ("w", self.w), ("uc", self.uc), ("R", self.R),
                         ("Rc", self.Rc), ("du", self.du), ("b", self.b), ("diag", self.diag), ("blocks", self.blocks),
                         ("moduli", self.C), ("reduce_work", self.work), ("scal", self.scal),
-                        ("scal_host", self.scal_host)):
+                        ("scal_host", self.scal_host), ("frame_work", self.frame_work)):
             setattr(nw, name, t.data_ptr() if t is not None else None)
         nw.moduli_dtype = self.moduli_code
         if self.mg is not None:

@@ -48,6 +48,11 @@ extern "C" {
  * float2 [stride] (23 33), i.e. 10 * stride floats per q.  As a moduli dtype (dfea_qp_moduli,
  * dfea_tangent_apply[_gather] with f64 vectors) and as a PCG vec_dtype (FP64 Krylov vectors). */
 #define DFEA_F32REF 3
+/* The same moduli in FP64: 5 rows of f64 pairs per Gauss point, [n_q][5][stride][2], the entries in the order
+ * 00 01 02 03 11 12 13 22 23 33.  Written by dfea_frame_moduli, applied by dfea_tangent_apply_gather (f64 vectors),
+ * by the gather and fused PCG forms (as vec_dtype: FP64 Krylov vectors) and by the multigrid.  80 B per Gauss point
+ * and no gradients, against 128 B and 16 B per node of DFEA_F64. */
+#define DFEA_F64REF 4
 #define DFEA_MAX_NEN 9
 #define DFEA_MAX_NQ 9
 
@@ -115,6 +120,8 @@ typedef struct dfea_mesh_view {
      * ref_grad[(q * nen + a) * 2 + alpha] = dN_a/dxi_alpha (host values). */
     const double* jinv;
     double ref_grad[DFEA_MAX_NQ * DFEA_MAX_NEN * 2];
+    /* Optional: the frame of dfea_mesh_frame, [n_q][2][stride] rows of Jinv as f64 pairs (NULL if not built). */
+    const double* frame;
 } dfea_mesh_view;
 
 /* ---------------------------------------------------------------- library --------------------- */
@@ -181,6 +188,15 @@ int dfea_mesh_grad_to_f32(const dfea_mesh_view* mesh, float* grad32_out, void* s
  */
 int dfea_mesh_ref_frame(const dfea_mesh_view* mesh, const double* nodes, double* jinv_out, double* check,
                         void* stream);
+
+/*
+ * The frame of the dfea_frame_* entry points: Jinv of every Gauss point fitted to the packed gradients, so that
+ * dN/dX = Jinv^T dN/dxi holds to rounding wherever dN/dX has that form.  frame_out [n_q][2][stride][2] as jinv_out of
+ * dfea_mesh_ref_frame.  check (3 doubles): [0] and [1] as dfea_mesh_ref_frame writes them (the Jacobian of the node
+ * coordinates against dN/dX), [2] the largest fit error of a Gauss point relative to its own largest |dN/dX|: the
+ * caller sets mesh->frame when [2] is at the rounding level.  No counterpart function in the reference.
+ */
+int dfea_mesh_frame(const dfea_mesh_view* mesh, const double* nodes, double* frame_out, double* check, void* stream);
 
 /*
  * Node incidence of the gather form (the node_elem_ptr / node_elem arrays of dfea_mesh_view): ptr_out
@@ -317,6 +333,39 @@ int dfea_residual_mat(const dfea_mesh_view* mesh, const double* u, const double*
 
 /* *out (device) = sum_i x_i^2 over 2N entries, fixed-order reduction.  work as for dfea_residual. */
 int dfea_vec_norm2(const dfea_mesh_view* mesh, const double* x, double* out, void* work, void* stream);
+
+/* ---------------------------------------------------------------- frame forms ----------------- */
+
+/*
+ * The entry points above on a mesh with a frame (mesh->frame) and node incidence: the same quantities computed with
+ * 32 B of geometry per Gauss point, in one element pass and one node pass whatever the number of colours.
+ * material gives the model; its parameters come from the struct, or with mat_p and mat_scalable (device pointers,
+ * both or none: the model's parameters as f64 and their scalable flags as bytes) from device memory, which spares a
+ * caller whose problem lives on the device the copy to the host.  work: dfea_frame_work_bytes(mesh) bytes, private
+ * to the call until the stream has passed it; no initial contents are needed.
+ *   dfea_frame_moduli          dfea_qp_moduli_mat with DFEA_F64REF or DFEA_F32REF moduli (diag and blocks optional)
+ *   dfea_frame_residual        dfea_residual_mat
+ *   dfea_frame_internal_force  dfea_internal_force_mat
+ *   dfea_frame_sensitivity     dfea_element_sensitivity_mat (parameters on the device: only models all of whose
+ *                              parameters enter the energy as prefactors)
+ *   dfea_frame_fields          dfea_element_fields_mat
+ *   dfea_frame_push_forward    DFEA_F64 moduli from DFEA_F64REF ones
+ */
+int64_t dfea_frame_work_bytes(const dfea_mesh_view* mesh);
+int dfea_frame_moduli(const dfea_mesh_view* mesh, const double* u, const double* theta, const dfea_material* material,
+                      const double* mat_p, const uint8_t* mat_scalable, void* moduli, int32_t moduli_dtype, double* diag,
+                      double* blocks, void* work, void* stream);
+int dfea_frame_residual(const dfea_mesh_view* mesh, const double* u, const double* theta, const dfea_material* material,
+                        const double* mat_p, const uint8_t* mat_scalable, const double* f, double load_factor, double* R,
+                        double* out_norm2, double* out_energy, void* work, void* stream);
+int dfea_frame_internal_force(const dfea_mesh_view* mesh, const double* u, const double* theta,
+                              const dfea_material* material, const double* mat_p, const uint8_t* mat_scalable,
+                              double* R_int, void* work, void* stream);
+int dfea_frame_sensitivity(const dfea_mesh_view* mesh, const double* u, const double* lam, const dfea_material* material,
+                           const double* mat_p, const uint8_t* mat_scalable, double* g, void* stream);
+int dfea_frame_fields(const dfea_mesh_view* mesh, const double* u, const double* theta, const dfea_material* material,
+                      const double* mat_p, const uint8_t* mat_scalable, double* elem_out, void* stream);
+int dfea_frame_push_forward(const dfea_mesh_view* mesh, const double* moduli_ref, double* moduli, void* stream);
 
 /* ---------------------------------------------------------------- kernel (d) ------------------ */
 
@@ -602,6 +651,8 @@ typedef struct dfea_newton {
     dfea_mg* mg;
     double min_rtol;             /* floor of the inner tolerance: 0 (FP64 operator) or, for an FP32
                                   * operator, the accuracy it can deliver (1e-5)                     */
+    void* frame_work;            /* dfea_frame_work_bytes of scratch, or NULL: with it the residual, and
+                                  * reference-frame moduli, come from the dfea_frame_* calls          */
 } dfea_newton;
 
 typedef struct dfea_newton_record {  /* one Newton iteration, as the reference's history records     */
