@@ -34,12 +34,13 @@ buffers (krylov.DevicePCG), a multigrid hierarchy (multigrid.Multigrid), a Newto
 run them read the buffers the handle is bound to and write the tensors they declare as mutated.
 """
 import weakref
+from typing import Optional
 
 import torch
 
 from difffea_b200 import _lib
 from difffea_b200.cuda_mesh import ptr, stream_handle
-from difffea_b200.materials import device_material
+from difffea_b200.materials import device_material, get_material, material_of
 
 _MESHES = weakref.WeakValueDictionary()
 
@@ -240,9 +241,23 @@ def _(mesh_id, u, theta, model, scalable, mat_p):
 # ---------------------------------------------------------------------------------------------
 # the same quantities on a mesh with a frame (CudaMesh.ensure_frame): one element pass and one node pass
 # ---------------------------------------------------------------------------------------------
-def frame_material(params):
-    """(model, scalable, mat_p) of a problem for the frame_* ops."""
-    return material_args(device_material(params))
+def frame_material(params, linear_only=False):
+    """
+    (model, scalable, mat_p, p_dev, scalable_dev) of a problem for the frame_* ops.  A material whose parameters and
+    flags lie on the device is passed as those tensors and read by the kernels: copying it to the host first makes
+    every call wait for the GPU (six blocking reads in one linearisation).  ``linear_only``: the op looks at the flags
+    on the host unless theta may scale any parameter of the model.
+    """
+    name, p0, scalable = material_of(params)
+    mat = get_material(name)
+    n = len(mat["param_names"])
+    if (torch.is_tensor(p0) and torch.is_tensor(scalable) and p0.is_cuda
+            and p0.device == scalable.device == params["conn"].device
+            and p0.dtype == torch.float64 and scalable.dtype == torch.bool and p0.shape == scalable.shape == (n,)
+            and p0.is_contiguous() and scalable.is_contiguous()
+            and (not linear_only or name in ("neo_hookean", "mooney_rivlin", "saint_venant"))):
+        return mat["model"], 0, [], p0.detach(), scalable
+    return (*material_args(device_material(params)), None, None)
 
 
 def _frame_mesh(mesh_id, u, theta=None):
@@ -255,27 +270,32 @@ def _frame_mesh(mesh_id, u, theta=None):
     return mesh
 
 
-def _frame_args(model, scalable, mat_p):
-    return _material(model, scalable, mat_p), ptr(None), ptr(None)
+def _frame_args(mesh, model, scalable, mat_p, p_dev=None, s_dev=None):
+    for t in (p_dev, s_dev):
+        if t is not None and t.device != mesh.device:
+            raise ValueError("the material's parameters must be on the mesh's device")
+    return _material(model, scalable, mat_p), ptr(p_dev), ptr(s_dev)
 
 
 @torch.library.custom_op("difffea_b200::frame_moduli", mutates_args=(), device_types="cuda")
 def frame_moduli(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int, mat_p: list[float],
-                 with_moduli: bool, with_blocks: bool) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+                 p_dev: Optional[torch.Tensor], s_dev: Optional[torch.Tensor], with_moduli: bool,
+                 with_blocks: bool) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """FP64 reference-frame moduli (empty without with_moduli), Jacobi diagonal, inverse node blocks (or empty)."""
     mesh = _frame_mesh(mesh_id, u, theta)
     f64 = dict(dtype=torch.float64, device=mesh.device)
     C = torch.empty(mesh.moduli_numel_ref() if with_moduli else 0, **f64)
     diag = torch.empty(mesh.n_dof, **f64)
     blocks = torch.empty(2 * mesh.n_dof if with_blocks else 0, **f64)
-    _lib.call("dfea_frame_moduli", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p),
+    _lib.call("dfea_frame_moduli", mesh.view_ref, ptr(u), ptr(theta),
+              *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev),
               ptr(C if with_moduli else None), _lib.DFEA_F64REF, ptr(diag), ptr(blocks if with_blocks else None),
               ptr(mesh.frame_work()), stream_handle())
     return C, diag, blocks
 
 
 @frame_moduli.register_fake
-def _(mesh_id, u, theta, model, scalable, mat_p, with_moduli, with_blocks):
+def _(mesh_id, u, theta, model, scalable, mat_p, p_dev, s_dev, with_moduli, with_blocks):
     mesh = _mesh(mesh_id)
     return (u.new_empty(mesh.moduli_numel_ref() if with_moduli else 0), u.new_empty(mesh.n_dof),
             u.new_empty(2 * mesh.n_dof if with_blocks else 0))
@@ -283,66 +303,74 @@ def _(mesh_id, u, theta, model, scalable, mat_p, with_moduli, with_blocks):
 
 @torch.library.custom_op("difffea_b200::frame_residual", mutates_args=(), device_types="cuda")
 def frame_residual(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int, mat_p: list[float],
-                   f: torch.Tensor, load_factor: float, scalars: bool) -> tuple[torch.Tensor, torch.Tensor]:
+                   p_dev: Optional[torch.Tensor], s_dev: Optional[torch.Tensor], f: torch.Tensor,
+                   load_factor: float, scalars: bool) -> tuple[torch.Tensor, torch.Tensor]:
     """R and, with scalars, (|R|^2, strain energy) on the device (else empty)."""
     mesh = _frame_mesh(mesh_id, u, theta)
     _f64(f, mesh, mesh.n_dof)
     R = torch.empty_like(u)
     out = torch.empty(2 if scalars else 0, dtype=torch.float64, device=mesh.device)
-    _lib.call("dfea_frame_residual", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p), ptr(f),
-              float(load_factor), ptr(R), ptr(out if scalars else None), ptr(out[1:] if scalars else None),
+    _lib.call("dfea_frame_residual", mesh.view_ref, ptr(u), ptr(theta),
+              *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev), ptr(f), float(load_factor), ptr(R),
+              ptr(out if scalars else None), ptr(out[1:] if scalars else None),
               ptr(mesh.frame_work()), stream_handle())
     return R, out
 
 
 @frame_residual.register_fake
-def _(mesh_id, u, theta, model, scalable, mat_p, f, load_factor, scalars):
+def _(mesh_id, u, theta, model, scalable, mat_p, p_dev, s_dev, f, load_factor, scalars):
     return torch.empty_like(u), u.new_empty(2 if scalars else 0)
 
 
 @torch.library.custom_op("difffea_b200::frame_internal_force", mutates_args=(), device_types="cuda")
 def frame_internal_force(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int,
-                         mat_p: list[float]) -> torch.Tensor:
+                         mat_p: list[float],
+                 p_dev: Optional[torch.Tensor], s_dev: Optional[torch.Tensor]) -> torch.Tensor:
     mesh = _frame_mesh(mesh_id, u, theta)
     R = torch.empty_like(u)
-    _lib.call("dfea_frame_internal_force", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p),
+    _lib.call("dfea_frame_internal_force", mesh.view_ref, ptr(u), ptr(theta),
+              *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev),
               ptr(R), ptr(mesh.frame_work()), stream_handle())
     return R
 
 
 @frame_internal_force.register_fake
-def _(mesh_id, u, theta, model, scalable, mat_p):
+def _(mesh_id, u, theta, model, scalable, mat_p, p_dev, s_dev):
     return torch.empty_like(u)
 
 
 @torch.library.custom_op("difffea_b200::frame_sensitivity", mutates_args=(), device_types="cuda")
 def frame_sensitivity(mesh_id: int, u: torch.Tensor, lam: torch.Tensor, model: int, scalable: int,
-                      mat_p: list[float]) -> torch.Tensor:
+                      mat_p: list[float],
+                 p_dev: Optional[torch.Tensor], s_dev: Optional[torch.Tensor]) -> torch.Tensor:
     mesh = _frame_mesh(mesh_id, u)
     _f64(lam, mesh, mesh.n_dof)
     g = torch.empty(mesh.n_el, dtype=torch.float64, device=mesh.device)
-    _lib.call("dfea_frame_sensitivity", mesh.view_ref, ptr(u), ptr(lam), *_frame_args(model, scalable, mat_p), ptr(g),
+    _lib.call("dfea_frame_sensitivity", mesh.view_ref, ptr(u), ptr(lam),
+              *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev), ptr(g),
               stream_handle())
     return g
 
 
 @frame_sensitivity.register_fake
-def _(mesh_id, u, lam, model, scalable, mat_p):
+def _(mesh_id, u, lam, model, scalable, mat_p, p_dev, s_dev):
     return u.new_empty(_mesh(mesh_id).n_el)
 
 
 @torch.library.custom_op("difffea_b200::frame_fields", mutates_args=(), device_types="cuda")
 def frame_fields(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int,
-                 mat_p: list[float]) -> torch.Tensor:
+                 mat_p: list[float],
+                 p_dev: Optional[torch.Tensor], s_dev: Optional[torch.Tensor]) -> torch.Tensor:
     mesh = _frame_mesh(mesh_id, u, theta)
     out = torch.empty(7, mesh.n_el, dtype=torch.float64, device=mesh.device)
-    _lib.call("dfea_frame_fields", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p), ptr(out),
+    _lib.call("dfea_frame_fields", mesh.view_ref, ptr(u), ptr(theta),
+              *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev), ptr(out),
               stream_handle())
     return out
 
 
 @frame_fields.register_fake
-def _(mesh_id, u, theta, model, scalable, mat_p):
+def _(mesh_id, u, theta, model, scalable, mat_p, p_dev, s_dev):
     return u.new_empty(7, _mesh(mesh_id).n_el)
 
 
@@ -370,7 +398,7 @@ def frame_residual_out(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model
     _f64(R, mesh, mesh.n_dof)
     if scal.dtype != torch.float64 or scal.numel() < 2 or scal.device != mesh.device:
         raise ValueError("scal must hold at least 2 float64 entries on the mesh's device")
-    _lib.call("dfea_frame_residual", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p), ptr(f),
+    _lib.call("dfea_frame_residual", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(mesh, model, scalable, mat_p), ptr(f),
               float(load_factor), ptr(R), ptr(scal), ptr(scal[1:] if energy else None), ptr(work), stream_handle())
 
 
@@ -381,7 +409,7 @@ def frame_moduli_out(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: 
                      work: torch.Tensor) -> None:
     """Reference-frame moduli into C, the Jacobi diagonal into diag and, when not empty, the inverse node blocks."""
     mesh = _frame_mesh(mesh_id, u, theta)
-    _lib.call("dfea_frame_moduli", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(model, scalable, mat_p), ptr(C),
+    _lib.call("dfea_frame_moduli", mesh.view_ref, ptr(u), ptr(theta), *_frame_args(mesh, model, scalable, mat_p), ptr(C),
               int(moduli_code), ptr(diag), ptr(blocks if blocks.numel() else None), ptr(work), stream_handle())
 
 

@@ -95,3 +95,19 @@ def test_gradients_that_are_no_frame_keep_the_kernels_that_read_them():
     q = {**p, "dN_dX": p["dN_dX"] * noise}
     assert not cuda_mesh(q).ensure_frame() and cuda_mesh(p).ensure_frame()
     _check(q, u, v, th)
+
+
+@pytest.mark.parametrize("material,flags", [("neo_hookean", [True, False]), ("mooney_rivlin", [False, True, True]),
+                                            ("demiray", [True, False, True]),
+                                            ("fiber_reinforced", [True, False, True, False, False, False, False])])
+def test_material_read_on_the_device_is_the_host_one(material, flags):
+    """Parameters and flags as device tensors (read by the kernels) or host tensors (passed in the struct)."""
+    p, u, v, th = _problem("quad4", 9, 5, material)
+    u, lam = 0.2 * u, v
+    outs = []
+    for where in ("cuda", "cpu"):
+        q = {**p, "mat_p": p["mat_p"].to(where), "mat_scalable": torch.tensor(flags, device=where)}
+        outs.append([make_tangent_operator("cuda", u, th, q)(v), global_residual(u, th, q), internal_force(u, th, q),
+                     compute_implicit_vjp(u, th, q, lam), strain_energy(u, th, q)] + list(compute_fields(u, th, q).values()))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
