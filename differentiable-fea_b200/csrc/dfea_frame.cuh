@@ -191,10 +191,11 @@ __device__ __forceinline__ void frame_reduce(int64_t e, bool live, int q, int la
 template <typename SD> struct FrameModuli;
 template <> struct FrameModuli<double> {
     double2 h[5];
+    template <bool CACHED>
     __device__ __forceinline__ void load(const double* C, int64_t S, int q, int64_t e) {
         const double2* p = reinterpret_cast<const double2*>(C) + (int64_t)(q * 5) * S + e;
 #pragma unroll
-        for (int k = 0; k < 5; ++k) h[k] = __ldcs(p + k * S);
+        for (int k = 0; k < 5; ++k) h[k] = CACHED ? __ldg(p + k * S) : __ldcs(p + k * S);
     }
     __device__ __forceinline__ void clear() {
 #pragma unroll
@@ -213,11 +214,15 @@ template <> struct FrameModuli<double> {
 template <> struct FrameModuli<float> {
     float4 a, b;
     float2 d;
+    template <bool CACHED>
     __device__ __forceinline__ void load(const float* C, int64_t S, int q, int64_t e) {
         const float* base = C + (int64_t)q * 10 * S;
-        a = __ldcs(reinterpret_cast<const float4*>(base) + e);
-        b = __ldcs(reinterpret_cast<const float4*>(base + 4 * S) + e);
-        d = __ldcs(reinterpret_cast<const float2*>(base + 8 * S) + e);
+        const float4* pa = reinterpret_cast<const float4*>(base) + e;
+        const float4* pb = reinterpret_cast<const float4*>(base + 4 * S) + e;
+        const float2* pd = reinterpret_cast<const float2*>(base + 8 * S) + e;
+        a = CACHED ? __ldg(pa) : __ldcs(pa);
+        b = CACHED ? __ldg(pb) : __ldcs(pb);
+        d = CACHED ? __ldg(pd) : __ldcs(pd);
     }
     __device__ __forceinline__ void clear() {
         a = b = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -234,6 +239,23 @@ template <> struct FrameModuli<float> {
     }
 };
 
+// The threads that walk tiles together: a whole block, or one of several teams of a persistent block (named barrier
+// id + 1).
+struct BlockTeam {
+    static constexpr bool kCached = false;  // moduli stream through once
+    __device__ __forceinline__ int tid() const { return threadIdx.x; }
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+template <int NT>
+struct SubTeam {
+    static constexpr bool kCached = true;   // the same moduli every iteration: let L1 keep them
+    __device__ __forceinline__ int tid() const { return threadIdx.x % NT; }
+    __device__ __forceinline__ int id() const { return threadIdx.x / NT; }
+    __device__ __forceinline__ void sync() const {
+        asm volatile("bar.sync %0, %1;" ::"r"(id() + 1), "n"(NT) : "memory");
+    }
+};
+
 template <int NEN, int NQ, typename T>
 struct FrameShared {
     v2_t<T> vs[NEN][FrameCfg<NEN, NQ>::EB];
@@ -243,12 +265,13 @@ struct FrameShared {
 // All elements of the mesh by the blocks blk of nblk: gather(node) -> nodal pair (masked here), out(a, e, f)
 // receives the element results; curv accumulates G . P per thread with DOT.  `start()` runs after the first
 // tile's moduli were requested; returning false abandons the walk.
-template <int NEN, int NQ, typename SD, typename T, bool DOT, typename Start, typename Gather, typename Out>
+template <int NEN, int NQ, typename SD, typename T, bool DOT, typename Start, typename Gather, typename Out,
+          typename Team = BlockTeam>
 __device__ __forceinline__ bool frame_product(const Mesh& m, const SD* __restrict__ C, const RefGrad<NEN, NQ>& rg,
                                               FrameShared<NEN, NQ, T>& sh, double& curv, Start&& start, Gather&& gather,
-                                              Out&& out, int64_t blk, int64_t nblk) {
+                                              Out&& out, int64_t blk, int64_t nblk, Team team = Team()) {
     constexpr int EB = FrameCfg<NEN, NQ>::EB;
-    const int lane = threadIdx.x % EB, q = threadIdx.x / EB;
+    const int lane = team.tid() % EB, q = team.tid() / EB;
     const int64_t n_tiles = (m.n_el + EB - 1) / EB;
     const RefRow<NEN, T> r(rg, q);
     FrameModuli<SD> M;
@@ -258,14 +281,14 @@ __device__ __forceinline__ bool frame_product(const Mesh& m, const SD* __restric
     int64_t e = tile * EB + lane;
     bool live = tile < n_tiles && e < m.n_el;
     conn.load(m, e, live, q);
-    if (live) M.load(C, m.stride, q, e);
+    if (live) M.template load<Team::kCached>(C, m.stride, q, e);
     else M.clear();
     if (!start()) return false;
     v.template gather<true>(conn, gather);
     conn.load(m, e + nblk * EB, e + nblk * EB < m.n_el, q);
     while (tile < n_tiles) {
         v.store(sh.vs, q, lane);
-        if (NQ > 1) __syncthreads();
+        if (NQ > 1) team.sync();
         v.template gather<true>(conn, gather);  // of the next tile
         conn.load(m, e + 2 * nblk * EB, e + 2 * nblk * EB < m.n_el, q);
         T G[4], P[4];
@@ -278,7 +301,7 @@ __device__ __forceinline__ bool frame_product(const Mesh& m, const SD* __restric
         tile += nblk;
         e += nblk * EB;
         live = e < m.n_el;
-        if (live) M.load(C, m.stride, q, e);
+        if (live) M.template load<Team::kCached>(C, m.stride, q, e);
         else M.clear();
         if constexpr (NQ == 1) {
 #pragma unroll
@@ -292,7 +315,7 @@ __device__ __forceinline__ bool frame_product(const Mesh& m, const SD* __restric
                 const T r0 = r.g[a][0], r1 = r.g[a][1];
                 sh.red[q][a][lane] = make_v2<T>(P[0] * r0 + P[1] * r1, P[2] * r0 + P[3] * r1);
             }
-            __syncthreads();
+            team.sync();
             frame_reduce<NEN, NQ, T>(e_now, live_now, q, lane, sh.red, out);
         }
     }

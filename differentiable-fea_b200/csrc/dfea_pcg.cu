@@ -427,6 +427,390 @@ k_pcg_node_fused(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __r
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Cluster form: a whole solve in one launch of one thread-block cluster (at most 16 blocks).
+//
+// Small meshes are bound by the latency of an iteration, not by bytes: the launch forms pay two launches, their tails
+// and a dozen trips to L2 (14 - 17 us an iteration from 64 to 16k Q4 elements).  Here the nodes are divided over the
+// cluster's blocks and every vector lives in the shared memory of the node's owner: the element pass gathers z and p
+// from, and scatters its results to, distributed shared memory (each (element, node) slot has its own place in the
+// owner's memory, summed there in incidence order), and the two reductions of an iteration ride on the cluster's
+// hardware barriers -- each warp stores its sum into every block's table before the barrier, every warp adds the table
+// in the same order after it, so all blocks take the same branch.  Only the moduli stream from L2.
+// Microseconds an iteration, FP64, B200 (fused launch form -> this): 64 Q4 14.2 -> 2.9, 576 14.2 -> 3.7, 2,304
+// 14.1 -> 5.1, 10,000 15.4 -> 9.1, 16,384 15.4 -> 12.3; 1,800 Q9 15.9 -> 10.1; 20,000 Tri3 18.0 -> 7.8.  So wherever
+// the vectors fit the cluster's shared memory it is the faster form, and it is taken there.  Past ~10k Q4 elements the
+// FP64 chains of the element pass on 16 SMs bound it.  (A grid-wide persistent form, exchanging through L2 with polled
+// flags, took 7.7 us an iteration on one block and 13 - 18 us on many: its fences also empty L1.)
+//
+// There is no spin wait: the blocks of a cluster are scheduled together and meet at hardware barriers.  The number of
+// iterations is bounded by max_iter.
+// ------------------------------------------------------------------------------------------------
+constexpr int kClusterMax = 16;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// address of the same shared-memory location in block `rank` of the cluster
+__device__ __forceinline__ unsigned cluster_address(unsigned local, unsigned rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+    return a;
+}
+// sum over the warp, the same bits in every lane
+__device__ __forceinline__ double warp_all_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ double2 cluster_load(unsigned addr) {
+    double2 v;
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_store(unsigned addr, double2 v) {
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ void cluster_store(unsigned addr, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+
+// Shared memory of a block (byte offsets; the same in every block).  Nodes are divided in ranges of nb.
+struct ClusterLayout {
+    int nb;                                         // nodes per block
+    int x, r, p, z, d, fe, base, fix, el, table, total;  // d: 1 / diagonal, or the inverse 2 x 2 blocks (4 values)
+    int slices;  // of 32 nodes; base[s] = first fe entry of slice s, node i's j-th entry at base[i / 32] + 32 j + i % 32
+};
+
+
+// Elements of a cluster's block: of every colour its share, in order -- so that with elements and nodes both numbered
+// along the mesh a block's elements lie at its own nodes and most of its gathers stay in its own shared memory.
+struct ClusterColours {
+    int n;
+    int begin[DFEA_MAX_COLOURS + 1];
+    __host__ __device__ int lo(int c, int rank, int size) const {
+        return begin[c] + (int)((int64_t)(begin[c + 1] - begin[c]) * rank / size);
+    }
+};
+
+template <int NEN, int NQ>
+struct ClusterCfg {
+    static constexpr int TEAMS = NQ == 9 ? 2 : (NQ == 6 ? 3 : 4);  // teams (the warps of one tile) of a block
+    static constexpr int TEAM = FrameCfg<NEN, NQ>::NT;
+    static constexpr int NT = TEAM * TEAMS;
+    static constexpr int W = NT / 32;
+    static constexpr int TEAM_BYTES = TEAMS * (int)sizeof(FrameShared<NEN, NQ, double>);
+};
+
+// Element results of a node lie 32 entries apart, those of neighbouring nodes side by side (slices of 32 nodes, each as
+// deep as its busiest node): stored node by node, the element pass scattered with 8-way bank conflicts.
+// One block per rank: base[rank][s] of its slices (entries), base[rank][slices] = their total.
+__global__ void k_pcg_cluster_slices(int64_t n_nodes, int nb, int slices, const int32_t* __restrict__ inc_ptr,
+                                     int32_t* __restrict__ base) {
+    const int64_t first = (int64_t)blockIdx.x * nb;
+    int32_t* mine = base + (int64_t)blockIdx.x * (slices + 1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    for (int s = warp; s < slices; s += warps) {
+        const int i = s * 32 + lane;
+        const int64_t n = first + i;
+        int deg = (i < nb && n < n_nodes) ? inc_ptr[n + 1] - inc_ptr[n] : 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) deg = max(deg, __shfl_xor_sync(0xffffffffu, deg, o));
+        if (lane == 0) mine[s] = 32 * deg;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int32_t at = 0;
+        for (int s = 0; s < slices; ++s) {
+            const int32_t n = mine[s];
+            mine[s] = at;
+            at += n;
+        }
+        mine[slices] = at;
+    }
+}
+
+// map[slot] = (rank << 18 | local << 2 | fix bits, rank << 18 | entry in the owner's fe) of every (a, e) slot
+__global__ void __launch_bounds__(kThreads)
+k_pcg_cluster_map(Mesh m, int nb, int slices, const int32_t* __restrict__ base, const int32_t* __restrict__ inc_ptr,
+                  const int32_t* __restrict__ inc, int2* __restrict__ map) {
+    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < m.n_nodes; n += (int64_t)gridDim.x * blockDim.x) {
+        const int rank = (int)(n / nb), i = (int)(n - (int64_t)rank * nb), fix = m.node_fix[n];
+        int at = base[(int64_t)rank * (slices + 1) + i / 32] + i % 32;
+        for (int j = inc_ptr[n]; j < inc_ptr[n + 1]; ++j, at += 32)
+            map[inc[j]] = make_int2(rank << 18 | i << 2 | fix, rank << 18 | at);
+    }
+}
+
+template <int NEN, int NQ, typename SD, bool BJ>
+__global__ void __launch_bounds__(ClusterCfg<NEN, NQ>::NT, 1)
+k_pcg_cluster(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const int2* __restrict__ map,
+              const double* __restrict__ b, const double* __restrict__ diag, double* __restrict__ x_out,
+              const int32_t* __restrict__ slice_base, PcgState* __restrict__ st, ClusterLayout L, ClusterColours colours,
+              double rtol, int max_iter) {
+    using Cfg = ClusterCfg<NEN, NQ>;
+    constexpr int NT = Cfg::NT, W = Cfg::W, EB = FrameCfg<NEN, NQ>::EB, GA = ConnRow<NEN, NQ>::GA;
+    extern __shared__ __align__(16) unsigned char cluster_smem[];
+    const SubTeam<Cfg::TEAM> team;
+    FrameShared<NEN, NQ, double>& sh = reinterpret_cast<FrameShared<NEN, NQ, double>*>(cluster_smem)[team.id()];
+    double2* xs = reinterpret_cast<double2*>(cluster_smem + L.x);
+    double2* rs = reinterpret_cast<double2*>(cluster_smem + L.r);
+    double2* ps = reinterpret_cast<double2*>(cluster_smem + L.p);
+    double2* zs = reinterpret_cast<double2*>(cluster_smem + L.z);
+    double* ds = reinterpret_cast<double*>(cluster_smem + L.d);
+    double2* fes = reinterpret_cast<double2*>(cluster_smem + L.fe);
+    int* base = reinterpret_cast<int*>(cluster_smem + L.base);
+    unsigned char* fixs = cluster_smem + L.fix;
+    int* els = reinterpret_cast<int*>(cluster_smem + L.el);
+    double* table = reinterpret_cast<double*>(cluster_smem + L.table);  // [2][2][kClusterMax * W]
+    const unsigned smem0 = (unsigned)__cvta_generic_to_shared(cluster_smem);
+    const unsigned rank = cluster_rank();
+    const int size = gridDim.x;  // the grid is the cluster
+    const int lane32 = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned turn = 0;
+
+    // sums over the cluster, the same bits in every thread; also the barrier after each pass
+    auto exchange = [&](auto two, double v0, double v1, double& t0, double& t1) {
+        constexpr bool TWO = decltype(two)::value;
+        v0 = warp_all_sum(v0);
+        if (TWO) v1 = warp_all_sum(v1);
+        double* tab = table + (turn & 1u) * 2 * kClusterMax * W;
+        const unsigned here = (unsigned)__cvta_generic_to_shared(tab + rank * W + warp);
+        if (lane32 < size) {
+            const unsigned to = cluster_address(here, lane32);
+            cluster_store(to, v0);
+            if (TWO) cluster_store(to + kClusterMax * W * 8, v1);
+        }
+        ++turn;
+        __syncwarp();
+        cluster_barrier();
+        double a0 = 0.0, a1 = 0.0;
+        for (int i = lane32; i < size * W; i += 32) {
+            a0 += tab[i];
+            if (TWO) a1 += tab[kClusterMax * W + i];
+        }
+        t0 = warp_all_sum(a0);
+        if (TWO) t1 = warp_all_sum(a1);
+    };
+
+    const int64_t node0 = (int64_t)rank * L.nb;
+    const int n_own = (int)(node0 >= m.n_nodes ? 0 : (m.n_nodes - node0 < L.nb ? m.n_nodes - node0 : L.nb));
+    double rz = 0.0, bb = 0.0;
+    for (int i = threadIdx.x; i < n_own; i += NT) {
+        const int64_t n = node0 + i;
+        const double2 bn = reinterpret_cast<const double2*>(b)[n];
+        const double2 zn = precond<BJ, double>(diag, n, bn);
+        if constexpr (BJ) {
+            reinterpret_cast<double2*>(ds)[2 * i] = reinterpret_cast<const double2*>(diag)[2 * n];
+            reinterpret_cast<double2*>(ds)[2 * i + 1] = reinterpret_cast<const double2*>(diag)[2 * n + 1];
+        } else {
+            const double2 dn = reinterpret_cast<const double2*>(diag)[n];
+            reinterpret_cast<double2*>(ds)[i] = make_double2(1.0 / dn.x, 1.0 / dn.y);
+        }
+        xs[i] = make_double2(0.0, 0.0);
+        rs[i] = bn;
+        zs[i] = zn;
+        ps[i] = make_double2(0.0, 0.0);
+        fixs[i] = m.node_fix[n];
+        rz += bn.x * zn.x + bn.y * zn.y;
+        bb += bn.x * bn.x + bn.y * bn.y;
+    }
+    const int32_t* my_base = slice_base + (int64_t)rank * (L.slices + 1);
+    for (int i = threadIdx.x; i <= L.slices; i += NT) base[i] = my_base[i];
+    for (int i = threadIdx.x; i < my_base[L.slices]; i += NT) fes[i] = make_double2(0.0, 0.0);  // unused entries stay zero
+    int n_els = 0;
+    for (int c = 0; c < colours.n; ++c) {
+        const int lo = colours.lo(c, rank, size), hi = colours.lo(c, rank + 1, size);
+        for (int i = lo + threadIdx.x; i < hi; i += NT) els[n_els + i - lo] = i;
+        n_els += hi - lo;
+    }
+    int status = DFEA_PCG_RUNNING, iters = 0;
+    double rr = 0.0, curv = 0.0, beta = 0.0;
+    cluster_barrier();  // every block has started: its shared memory may be written from here on
+    exchange(std::true_type{}, rz, bb, rz, bb);
+    const double norm_b = sqrt(bb);
+    if (norm_b == 0.0) status = DFEA_PCG_ZERO_RHS;
+
+    // this thread's share of the element pass: Gauss point q of lane's element in the tiles of its team.  The slots of the next two tiles and the moduli of the next are in
+    // flight, around the end of the pass as well: they do not change from iteration to iteration.
+    const int q = team.tid() / EB, lane = team.tid() % EB;
+    constexpr int step = Cfg::TEAMS * EB;
+    const int i_first = team.id() * EB + lane;
+    auto element = [&](int i) -> int { return i < n_els ? els[i] : -1; };
+    const RefRow<NEN, double> row(rg, q);
+    FrameModuli<SD> M;
+    int2 s0[GA], s1[GA];
+    auto load_slots = [&](int e, int2 (&s)[GA]) {
+#pragma unroll
+        for (int i = 0; i < GA; ++i) {
+            const int a = i * NQ + q;
+            s[i] = (a < NEN && e >= 0) ? __ldg(map + (int64_t)a * m.stride + e) : make_int2(-1, -1);
+        }
+    };
+    auto load_moduli = [&](int e) {
+        if (e >= 0) M.template load<true>(C, m.stride, q, e);
+        else M.clear();
+    };
+    load_slots(element(i_first), s0);
+    load_slots(element(i_first + step), s1);
+    load_moduli(element(i_first));
+
+    for (int k = 0; status == DFEA_PCG_RUNNING; ++k) {
+        double c = 0.0;
+        // z and p of the next tile's nodes; combined when they go to shared memory, a tile later
+        double2 zn[GA], pn[GA];
+        auto gather = [&](const int2 (&s)[GA]) {
+#pragma unroll
+            for (int i = 0; i < GA; ++i) {
+                zn[i] = pn[i] = make_double2(0.0, 0.0);
+                if (s[i].x < 0) continue;
+                const unsigned who = (unsigned)s[i].x >> 18;
+                const int at = (s[i].x & 0x3ffff) >> 2;
+                if (who == rank) {
+                    zn[i] = zs[at];
+                    pn[i] = ps[at];
+                } else {
+                    zn[i] = cluster_load(cluster_address(smem0 + L.z + at * 16, who));
+                    pn[i] = cluster_load(cluster_address(smem0 + L.p + at * 16, who));
+                }
+            }
+        };
+        gather(s0);
+        for (int tile = team.id() * EB; tile < n_els; tile += step) {
+#pragma unroll
+            for (int i = 0; i < GA; ++i)
+                if (i * NQ + q < NEN)
+                    sh.vs[i * NQ + q][lane] = make_double2((s0[i].x & 1) ? 0.0 : zn[i].x + beta * pn[i].x,
+                                                           (s0[i].x & 2) ? 0.0 : zn[i].y + beta * pn[i].y);
+            if (NQ > 1) team.sync();
+            int2 now[GA];
+#pragma unroll
+            for (int i = 0; i < GA; ++i) {
+                now[i] = s0[i];
+                s0[i] = s1[i];
+            }
+            const bool more = tile + step < n_els;
+            if (more) {
+                gather(s0);
+                load_slots(element(tile + lane + 2 * step), s1);
+            }
+            double G[4], P[4];
+            frame_gradient<NEN, NQ, double>(row, lane, sh.vs, G);
+            M.apply(G, P);
+            c += G[0] * P[0] + G[1] * P[1] + G[2] * P[2] + G[3] * P[3];
+            load_moduli(element(more ? tile + lane + step : i_first));
+            auto put = [&](const int2& s, double2 f) {
+                if (s.y < 0) return;
+                const unsigned who = (unsigned)s.y >> 18;
+                if (who == rank) fes[s.y & 0x3ffff] = f;
+                else cluster_store(cluster_address(smem0 + L.fe + (s.y & 0x3ffff) * 16, who), f);
+            };
+            if constexpr (NQ == 1) {
+#pragma unroll
+                for (int a = 0; a < NEN; ++a)
+                    put(now[a], make_double2(P[0] * row.g[a][0] + P[1] * row.g[a][1], P[2] * row.g[a][0] + P[3] * row.g[a][1]));
+            } else {
+#pragma unroll
+                for (int a = 0; a < NEN; ++a)
+                    sh.red[q][a][lane] = make_double2(P[0] * row.g[a][0] + P[1] * row.g[a][1], P[2] * row.g[a][0] + P[3] * row.g[a][1]);
+                team.sync();
+                if (q < NEN) {
+                    double2 f = sh.red[0][q][lane];
+#pragma unroll
+                    for (int g = 1; g < NQ; ++g) {
+                        const double2 t = sh.red[g][q][lane];
+                        f.x += t.x;
+                        f.y += t.y;
+                    }
+                    put(now[0], f);
+                }
+            }
+        }
+        load_slots(element(i_first), s0);
+        load_slots(element(i_first + step), s1);
+        for (int i = threadIdx.x; i < n_own; i += NT) {  // the identity rows' part of p.Ap
+            const int fix = fixs[i];
+            if (fix) {
+                const double px = zs[i].x + beta * ps[i].x, py = zs[i].y + beta * ps[i].y;
+                if (fix & 1) c += px * px;
+                if (fix & 2) c += py * py;
+            }
+        }
+        double unused;
+        exchange(std::false_type{}, c, 0.0, curv, unused);
+        if (curv <= 0.0) {
+            // not SPD along p: return z at k = 0 and x otherwise (newton_krylov.py:69-70)
+            if (k == 0)
+                for (int i = threadIdx.x; i < n_own; i += NT) xs[i] = zs[i];
+            iters = k;
+            status = DFEA_PCG_NEG_CURV;
+            break;
+        }
+        const double a = rz / curv;
+        double s_rr = 0.0, s_rz = 0.0;
+        for (int i = threadIdx.x; i < n_own; i += NT) {
+            const int fix = fixs[i];
+            const double2 zn = zs[i], po = ps[i];
+            const double2 pn = make_double2(zn.x + beta * po.x, zn.y + beta * po.y);
+            double2 f = make_double2(0.0, 0.0);
+            const int j1 = base[(i >> 5) + 1];
+#pragma unroll 4
+            for (int j = base[i >> 5] + (i & 31); j < j1; j += 32) {
+                const double2 t = fes[j];
+                f.x += t.x;
+                f.y += t.y;
+            }
+            const double2 yn = make_double2((fix & 1) ? pn.x : f.x, (fix & 2) ? pn.y : f.y);
+            double2 xn = xs[i], rn = rs[i];
+            xn.x += a * pn.x;
+            xn.y += a * pn.y;
+            rn.x -= a * yn.x;
+            rn.y -= a * yn.y;
+            double2 zw;
+            if constexpr (BJ) {
+                zw = precond<true, double>(ds, i, rn);
+            } else {
+                const double2 dn = reinterpret_cast<const double2*>(ds)[i];
+                zw = make_double2(rn.x * dn.x, rn.y * dn.y);
+            }
+            xs[i] = xn;
+            rs[i] = rn;
+            ps[i] = pn;
+            zs[i] = zw;
+            s_rr += rn.x * rn.x + rn.y * rn.y;
+            s_rz += rn.x * zw.x + rn.y * zw.y;
+        }
+        double rz_new;
+        exchange(std::true_type{}, s_rr, s_rz, rr, rz_new);
+        beta = rz_new / rz;  // beside the square root: both chains are long
+        if (sqrt(rr) <= rtol * norm_b) {  // newton_krylov.py:77-79
+            iters = k + 1;
+            status = DFEA_PCG_CONVERGED;
+        } else {
+            rz = rz_new;
+            if (k + 1 >= max_iter) {
+                iters = max_iter;
+                status = DFEA_PCG_MAX_ITER;
+            }
+        }
+    }
+    for (int i = threadIdx.x; i < n_own; i += NT) reinterpret_cast<double2*>(x_out)[node0 + i] = xs[i];
+    if (rank == 0 && threadIdx.x == 0) {
+        st->rr = rr;
+        st->rz = rz;
+        st->norm_b = norm_b;
+        st->curv = curv;
+        st->iters = iters;
+        st->k = iters;
+        st->done = status;
+    }
+}
+
 __global__ void k_pcg_cond(PcgState* st, cudaGraphConditionalHandle h) {
     if (threadIdx.x != 0) return;
     const int g = ++st->guard;
@@ -455,6 +839,12 @@ struct dfea_pcg {
     int grid_cap = 0;                // most blocks per launch (0: as many as the GPU holds)
     bool block = false;              // nodal block-Jacobi: diag holds the inverse 2x2 blocks (4N doubles)
     bool fused = false;              // fused gather form: 2 kernels per iteration
+    bool clustered = false;          // the whole solve in one launch of a thread-block cluster
+    int cluster_blocks = 0;
+    ClusterLayout cluster{};
+    // the cluster form's arrays, in room that the launch forms use for fe and the vectors
+    int2* slot_map() const { return reinterpret_cast<int2*>(work + layout.off_fe); }
+    int32_t* slice_base() const { return reinterpret_cast<int32_t*>(work + layout.off_r); }
     cudaStream_t capture_stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -600,6 +990,139 @@ int launch_iteration_any(const dfea_pcg& h, cudaStream_t s, cudaGraphConditional
     return launch_iteration<float, float>(h, s, cond, with_cond);
 }
 
+template <auto Kernel>
+int cluster_configure() {
+    static std::once_flag once[64];
+    static int result[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    std::call_once(once[dev], [dev] {
+        int most = 0;
+        int rc = check_cuda(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
+        cudaFuncAttributes fa;
+        if (!rc) rc = check_cuda(cudaFuncGetAttributes(&fa, Kernel), "cudaFuncGetAttributes");
+        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                      most - (int)fa.sharedSizeBytes), "cudaFuncSetAttribute");
+        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "cudaFuncSetAttribute");
+        result[dev] = rc;
+    });
+    return result[dev];
+}
+
+constexpr int kClusterSmem = 220 * 1024;  // dynamic shared memory a block may take (of 227 KB)
+
+// The cluster of a mesh: blocks (a power of two, every team with at least a tile) and shared memory, or 0 blocks where
+// the mesh does not fit.  max_slots(blocks, nb, slices): the most fe entries of a block's node range.
+template <int NEN, int NQ, typename MaxSlots>
+int cluster_layout(const dfea_mesh_view& mv, bool block_jacobi, ClusterLayout* out, MaxSlots&& max_slots) {
+    using Cfg = ClusterCfg<NEN, NQ>;
+    const int64_t tiles = (mv.n_el + FrameCfg<NEN, NQ>::EB - 1) / FrameCfg<NEN, NQ>::EB;
+    int blocks = 1;
+    while (blocks < kClusterMax && (int64_t)blocks * Cfg::TEAMS < tiles) blocks *= 2;
+    const int64_t nb = (mv.n_nodes + blocks - 1) / blocks;
+    if (nb >= (1 << 16) || 96 * nb > kClusterSmem) return 0;  // five vectors and an entry per node at the least
+    const int slices = (int)((nb + 31) / 32);
+    const int64_t slots = max_slots(blocks, nb, slices);
+    if (slots >= (1 << 18)) return 0;
+    int64_t at = (Cfg::TEAM_BYTES + 15) / 16 * 16;
+    auto take = [&](int64_t bytes) {
+        const int64_t o = at;
+        at += (bytes + 15) / 16 * 16;
+        return (int)(o < (int64_t(1) << 30) ? o : (int64_t(1) << 30));
+    };
+    ClusterLayout L;
+    L.nb = (int)nb;
+    L.x = take(16 * nb);
+    L.r = take(16 * nb);
+    L.p = take(16 * nb);
+    L.z = take(16 * nb);
+    L.d = take((block_jacobi ? 32 : 16) * nb);
+    L.fe = take(16 * slots);
+    L.base = take(4 * (slices + 1));
+    L.slices = slices;
+    L.fix = take(nb);
+    L.el = take(4 * (mv.n_el / blocks + mv.n_colours + 1));
+    L.table = take(2 * 2 * kClusterMax * Cfg::W * 8);
+    if (at > kClusterSmem) return 0;
+    L.total = (int)at;
+    *out = L;
+    return blocks;
+}
+
+template <typename SD, bool BJ>
+int launch_cluster(const dfea_pcg& h, cudaStream_t s, double rtol, int max_iter) {
+    const dfea_mesh_view& mv = h.mesh;
+    const Mesh m = kernel_mesh(mv);
+    PcgState* st = h.state();
+    ClusterColours colours;
+    colours.n = mv.n_colours;
+    for (int c = 0; c <= mv.n_colours; ++c) colours.begin[c] = (int)mv.colour_begin[c];
+    k_pcg_reset<<<1, 128, 0, s>>>(st);
+    int rc = dispatch_element(mv.nen, mv.n_q, [&](auto nen_c, auto nq_c) -> int {
+        constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
+        constexpr auto kernel = k_pcg_cluster<NEN, NQ, SD, BJ>;
+        int rc2 = cluster_configure<kernel>();
+        if (rc2) return rc2;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = h.cluster_blocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(h.cluster_blocks);
+        cfg.blockDim = dim3(ClusterCfg<NEN, NQ>::NT);
+        cfg.dynamicSmemBytes = h.cluster.total;
+        cfg.stream = s;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return check_cuda(cudaLaunchKernelEx(&cfg, kernel, m, static_cast<const SD*>(h.moduli), ref_grad_of<NEN, NQ>(mv),
+                                             (const int2*)h.slot_map(),
+                                             static_cast<const double*>(h.b), static_cast<const double*>(h.diag),
+                                             static_cast<double*>(h.x), (const int32_t*)h.slice_base(), st, h.cluster, colours, rtol, max_iter),
+                          "cudaLaunchKernelEx(cluster PCG)");
+    });
+    if (rc) return rc;
+    note_launches(2);
+    return launch_check("cluster PCG");
+}
+
+int launch_cluster_any(const dfea_pcg& h, cudaStream_t s, double rtol, int max_iter) {
+    if (h.vec_dtype == DFEA_F64REF)
+        return h.block ? launch_cluster<double, true>(h, s, rtol, max_iter) : launch_cluster<double, false>(h, s, rtol, max_iter);
+    return h.block ? launch_cluster<float, true>(h, s, rtol, max_iter) : launch_cluster<float, false>(h, s, rtol, max_iter);
+}
+
+// Lay the cluster out (exact entry counts of the node ranges, read once) and write the slot map of the handle.
+int prepare_cluster(dfea_pcg* h) {
+    const dfea_mesh_view& mv = h->mesh;
+    cudaStream_t s = cudaStreamPerThread;
+    int rc = DFEA_OK;
+    h->cluster_blocks = dispatch_element(mv.nen, mv.n_q, [&](auto nen_c, auto nq_c) -> int {
+        constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
+        return cluster_layout<NEN, NQ>(mv, h->block, &h->cluster, [&](int blocks, int64_t nb, int slices) -> int64_t {
+            k_pcg_cluster_slices<<<blocks, 256, 0, s>>>(mv.n_nodes, (int)nb, slices, mv.node_elem_ptr, h->slice_base());
+            note_launches(1);
+            int32_t total[kClusterMax];
+            if ((rc = launch_check("cluster PCG slices")) ||
+                (rc = check_cuda(cudaMemcpy2DAsync(total, sizeof(int32_t), h->slice_base() + slices,
+                                                   (slices + 1) * sizeof(int32_t), sizeof(int32_t), blocks,
+                                                   cudaMemcpyDeviceToHost, s), "cudaMemcpy2DAsync")) ||
+                (rc = check_cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize")))
+                return 0;
+            int64_t most = 0;
+            for (int i = 0; i < blocks; ++i) most = total[i] > most ? total[i] : most;
+            return most;
+        });
+    });
+    if (rc) return rc;
+    if (h->cluster_blocks == 0)
+        return set_error(DFEA_ERR_UNSUPPORTED, "dfea_pcg_create: the mesh does not fit the shared memory of a cluster");
+    k_pcg_cluster_map<<<grid_for(mv.n_nodes, kThreads, 8), kThreads, 0, s>>>(
+        kernel_mesh(mv), h->cluster.nb, h->cluster.slices, h->slice_base(), mv.node_elem_ptr, mv.node_elem, h->slot_map());
+    note_launches(1);
+    if ((rc = launch_check("cluster PCG map"))) return rc;
+    return check_cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+}
+
 template <typename T, bool BJ = false>
 int launch_setup(const dfea_pcg& h, cudaStream_t s, double rtol, int max_iter) {
     const dfea_mesh_view& mv = h.mesh;
@@ -694,7 +1217,7 @@ extern "C" int dfea_pcg_create(const dfea_mesh_view* mesh, const void* moduli, c
     if (vec_dtype != DFEA_F64 && vec_dtype != DFEA_F32 && vec_dtype != DFEA_MIXED && vec_dtype != DFEA_F32REF &&
         vec_dtype != DFEA_F64REF)
         return set_error(DFEA_ERR_INVALID, "bad vector dtype");
-    if (vec_dtype == DFEA_F64REF && !(use_graph & (DFEA_PCG_GATHER | DFEA_PCG_FUSED)))
+    if (vec_dtype == DFEA_F64REF && !(use_graph & (DFEA_PCG_GATHER | DFEA_PCG_FUSED | DFEA_PCG_CLUSTER)))
         return set_error(DFEA_ERR_UNSUPPORTED, "dfea_pcg_create: DFEA_F64REF moduli need the gather or fused form");
     if (!moduli || !diag || !b || !x || !work) return set_error(DFEA_ERR_INVALID, "dfea_pcg_create: NULL pointer");
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 255u) == 0; };
@@ -717,9 +1240,16 @@ extern "C" int dfea_pcg_create(const dfea_mesh_view* mesh, const void* moduli, c
     h->gather = (use_graph & DFEA_PCG_GATHER) != 0;
     h->block = (use_graph & DFEA_PCG_BLOCK_JACOBI) != 0;
     h->fused = (use_graph & DFEA_PCG_FUSED) != 0;
-    if (h->fused) h->gather = true;
+    h->clustered = (use_graph & DFEA_PCG_CLUSTER) != 0;
+    // beside a launch form, the cluster form is taken where the mesh fits it
+    const bool cluster_optional = h->clustered && (use_graph & (DFEA_PCG_GATHER | DFEA_PCG_FUSED)) != 0;
+    if (h->fused || h->clustered) h->gather = true;
+    if (h->clustered && vec_dtype != DFEA_F64REF && vec_dtype != DFEA_F32REF) {
+        delete h;
+        return set_error(DFEA_ERR_UNSUPPORTED, "dfea_pcg_create: the cluster form takes reference-frame moduli");
+    }
     h->grid_cap = (int)((uint32_t)use_graph >> 8);
-    use_graph &= 0xff & ~(DFEA_PCG_GATHER | DFEA_PCG_BLOCK_JACOBI | DFEA_PCG_FUSED);
+    use_graph &= 0xff & ~(DFEA_PCG_GATHER | DFEA_PCG_BLOCK_JACOBI | DFEA_PCG_FUSED | DFEA_PCG_CLUSTER);
     if (h->block && vec_dtype == DFEA_F32) {
         delete h;
         return set_error(DFEA_ERR_UNSUPPORTED, "dfea_pcg_create: block-Jacobi needs f64 Krylov vectors");
@@ -728,6 +1258,18 @@ extern "C" int dfea_pcg_create(const dfea_mesh_view* mesh, const void* moduli, c
     if (h->gather && h->layout.off_fe == h->layout.total) {
         delete h;
         return set_error(DFEA_ERR_INVALID, "dfea_pcg_create: the gather form needs the mesh's node incidence");
+    }
+    if (h->clustered) {  // captures nothing, and every solve resets the state it uses
+        rc = prepare_cluster(h);
+        if (!rc) {
+            *out = h;
+            return DFEA_OK;
+        }
+        if (rc != DFEA_ERR_UNSUPPORTED || !cluster_optional) {
+            release(h);
+            return rc;
+        }
+        h->clustered = false;
     }
     // device queries and kernel attributes are set up before any stream capture
     (void)device_sm_count();
@@ -789,6 +1331,15 @@ extern "C" int dfea_pcg_solve(dfea_pcg* h, double rtol, int32_t max_iter, int32_
     if (max_iter < 1 || max_iter > 100000000) return set_error(DFEA_ERR_INVALID, "max_iter %d out of [1, 1e8]", max_iter);
     if (!(rtol >= 0.0)) return set_error(DFEA_ERR_INVALID, "rtol must be >= 0");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (h->clustered) {
+        int rcc = launch_cluster_any(*h, s, rtol, max_iter);
+        if (rcc || (rcc = read_to_host(h->host_status, &h->state()->done, 2 * sizeof(int32_t), s))) return rcc;
+        if (h->host_status[0] == DFEA_PCG_RUNNING)
+            return set_error(DFEA_ERR_INVALID, "PCG ended without a status (internal error)");
+        if (status) *status = h->host_status[0];
+        if (iters) *iters = h->host_status[1];
+        return DFEA_OK;
+    }
     int rc = (h->vec_dtype == DFEA_F32) ? launch_setup<float>(*h, s, rtol, max_iter)
              : h->block                 ? launch_setup<double, true>(*h, s, rtol, max_iter)
                                         : launch_setup<double>(*h, s, rtol, max_iter);
@@ -830,6 +1381,8 @@ extern "C" int dfea_pcg_solve(dfea_pcg* h, double rtol, int32_t max_iter, int32_
     if (iters) *iters = h->host_status[1];
     return DFEA_OK;
 }
+
+extern "C" int dfea_pcg_clustered(const dfea_pcg* h) { return h && h->clustered ? 1 : 0; }
 
 extern "C" int dfea_pcg_destroy(dfea_pcg* h) {
     if (h) release(h);
@@ -1088,7 +1641,7 @@ extern "C" int dfea_batch_destroy(dfea_batch* b) {
 
 extern "C" int dfea_batch_start(dfea_batch* b, dfea_pcg* h, double rtol, int32_t max_iter, void* stream) {
     if (!b || !h) return set_error(DFEA_ERR_INVALID, "dfea_batch_start: NULL pointer");
-    if (!h->gather || h->fused || h->block || h->vec_dtype != DFEA_F32REF)
+    if (!h->gather || h->fused || h->clustered || h->block || h->vec_dtype != DFEA_F32REF)
         return set_error(DFEA_ERR_UNSUPPORTED,
                          "dfea_batch_start: batched solves need the gather form, Jacobi and DFEA_F32REF moduli");
     if (max_iter < 1 || max_iter > 100000000) return set_error(DFEA_ERR_INVALID, "max_iter %d out of [1, 1e8]", max_iter);
@@ -1108,7 +1661,7 @@ extern "C" int dfea_batch_set(dfea_batch* b, dfea_pcg* const* solves, int32_t n,
     int entries = 0;
     for (int i = 0; i < n; ++i) {
         const dfea_pcg& h = *solves[i];
-        if (!h.gather || h.fused || h.block || h.vec_dtype != DFEA_F32REF)
+        if (!h.gather || h.fused || h.clustered || h.block || h.vec_dtype != DFEA_F32REF)
             return set_error(DFEA_ERR_UNSUPPORTED, "dfea_batch_set: solve %d is not in the batched configuration", i);
         const dfea_mesh_view& mv = h.mesh;
         BatchSolve& S = b->h_solves[i];

@@ -23,6 +23,7 @@ PCG_STATUS = {0: "running", 1: "converged", 2: "max_iter", 3: "negative_curvatur
 DFEA_PCG_GATHER = 16  # dfea_pcg_create flag: gather form of the product
 DFEA_PCG_BLOCK_JACOBI = 32  # dfea_pcg_create flag: nodal block-Jacobi (diag = inverse 2x2 blocks, 4N)
 DFEA_PCG_FUSED = 64  # dfea_pcg_create flag: fused gather form (2 kernels per iteration)
+DFEA_PCG_CLUSTER = 128  # dfea_pcg_create flag: the whole solve in one launch
 
 
 def pcg_max_blocks(n):
@@ -191,6 +192,7 @@ _PROTOS = {
     "dfea_pcg_create": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, c_vp, c_vp, c_i32, c_vp, c_i32,
                                        ctypes.POINTER(c_vp)]),
     "dfea_pcg_solve": (ctypes.c_int, [c_vp, c_f64, c_i32, ctypes.POINTER(c_i32), ctypes.POINTER(c_i32), c_vp]),
+    "dfea_pcg_clustered": (ctypes.c_int, [c_vp]),
     "dfea_pcg_destroy": (ctypes.c_int, [c_vp]),
     "dfea_pcg_solve_noalloc": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, c_vp, c_vp, c_i32, c_f64, c_i32,
                                               ctypes.POINTER(c_i32), ctypes.POINTER(c_i32), c_vp]),

@@ -29,24 +29,32 @@ class DevicePCG:
     form: "colour" (one launch per colour, scatter by read-modify-write) or "gather" (one element pass,
     per-node sums fused into the first vector update: 3 kernels per iteration; needs the mesh's node
     incidence, built here) or "fused" (the gather form with the direction update moved into the next
-    element pass: 2 kernels per iteration).  Each form is reproducible; they agree to rounding.
+    element pass: 2 kernels per iteration) or "cluster" (the whole solve in one launch of a thread-block cluster,
+    its vectors in distributed shared memory; reference-frame moduli, meshes that fit).  Each form is reproducible; they agree to rounding.
     moduli: "physical" (C with the packed dN/dX: FP64, FP32, or FP32 on FP64 vectors) or "ref" (FP32 or FP64
     moduli pulled back to the element reference frame, 10 per Gauss point, FP64 vectors; the product
     reads no gradients; FP64: the gather and fused forms).  max_blocks: at most this many blocks per launch (0: the whole GPU), for solves
     that share the GPU with others; results agree with the unlimited form's to rounding.
+    cluster: take the cluster form instead of ``form`` (gather or fused, reference-frame moduli) where the mesh fits.
     preconditioner: "jacobi" (diag = the (2N,) diagonal) or "block_jacobi" (diag = the (4N,) inverse 2x2
     node blocks of dfea_qp_moduli_block; FP64 vectors).
     """
 
     def __init__(self, mesh, C, diag, b, x, use_graph=True, form="colour", moduli="physical", max_blocks=0,
-                 preconditioner="jacobi"):
+                 preconditioner="jacobi", cluster=False):
         use_graph = int(use_graph) if os.environ.get("DFEA_PCG_GRAPH", "1") != "0" else 0
-        if form not in ("colour", "gather", "fused"):
-            raise ValueError("form must be 'colour', 'gather' or 'fused'")
-        flags = 0
-        if form in ("gather", "fused"):
+        if form not in ("colour", "gather", "fused", "cluster"):
+            raise ValueError("form must be 'colour', 'gather', 'fused' or 'cluster'")
+        cluster = cluster and form != "colour" and moduli == "ref"
+        if form == "cluster":
+            if moduli != "ref":
+                raise ValueError("the cluster form needs reference-frame moduli")
+            use_graph = 0
+        flags = _lib.DFEA_PCG_CLUSTER if cluster else 0
+        if form != "colour":
             mesh.ensure_node_incidence()
-            flags = _lib.DFEA_PCG_GATHER | (_lib.DFEA_PCG_FUSED if form == "fused" else 0)
+            flags |= {"gather": _lib.DFEA_PCG_GATHER, "fused": _lib.DFEA_PCG_GATHER | _lib.DFEA_PCG_FUSED,
+                      "cluster": _lib.DFEA_PCG_CLUSTER}[form]
         flags |= _lib.pcg_max_blocks(max_blocks)
         if preconditioner == "block_jacobi":
             # diag holds the inverse 2x2 node blocks (4N doubles) of dfea_qp_moduli_block
@@ -97,7 +105,8 @@ class DevicePCG:
                                                  ptr(self.work), flags, ctypes.byref(self._h))
             _lib.check(rc, "dfea_pcg_create")
         self.use_graph = use_graph
-        self.form = form
+        self.clustered = bool(_lib.load().dfea_pcg_clustered(self._h))
+        self.form = "cluster" if self.clustered else form
         self.last_status = None
         self.id = ops.register_handle(self)
 
@@ -138,6 +147,8 @@ class BatchExecutor:
     stream; the call returns when that solve has ended (its ``x`` is then final).  New solves join at
     the next round.  Each solve's iterates are bitwise those of ``pcg.solve`` alone (same block cap).
     Handles must be in the serving configuration: gather form, Jacobi, reference-frame FP32 moduli.
+    A handle in the cluster form is a launch of a few blocks by itself: its solve runs on the caller's stream, beside
+    the others in flight.
     """
 
     def __init__(self, device, capacity=64, max_blocks=64, iterations_per_check=8):
@@ -152,12 +163,23 @@ class BatchExecutor:
             self.stream = torch.cuda.Stream(self.device)
         self._q = queue.Queue()
         self._failure = ""
+        self._lock = threading.Lock()
+        self._beside = 0                 # cluster-form solves in flight
         self.rounds = 0
         self.peak_batch = 0
         self._thread = threading.Thread(target=self._loop, daemon=True)
         self._thread.start()
 
     def solve(self, pcg, rtol, max_iter):
+        if pcg.clustered:
+            with self._lock:
+                self._beside += 1
+                self.peak_batch = max(self.peak_batch, self._beside)
+            try:
+                return pcg.solve(rtol, max_iter)
+            finally:
+                with self._lock:
+                    self._beside -= 1
         ev = torch.cuda.Event()
         ev.record(torch.cuda.current_stream(self.device))
         t = _Ticket(pcg, float(rtol), int(max_iter), ev)

@@ -124,7 +124,7 @@ class CudaTangentOperator:
             xx = torch.empty(n, dtype=vt, device=self.mesh.device)
             if self._pcg is not None:
                 self._pcg.close()
-            ref = dict(form="fused", moduli="ref", use_graph=2) if self.code == _lib.DFEA_F64REF else {}
+            ref = dict(form="fused", moduli="ref", use_graph=2, cluster=True) if self.code == _lib.DFEA_F64REF else {}
             self._pcg = DevicePCG(self.mesh, self.moduli, d, bb, xx, preconditioner=preconditioner, **ref)
             self._pcg_diag_src = diag
         self._pcg.b.copy_(b)

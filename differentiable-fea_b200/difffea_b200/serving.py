@@ -390,7 +390,8 @@ def solve_request(req, device, precision="fp32", n_load_steps=1, tol_rel=1e-10, 
     Build (or copy from ``host_params``) and solve one request on the current stream; returns
     (u on device, info).  ``pcg_graph`` is the PCG launch form (2: unrolled graph, the default for
     a request solved alone; 1: conditional-loop graph; 0: direct launches, the serving engine's default); ``pcg_form`` the product form inside
-    it ("auto", "colour" or "gather", see DevicePCG and workspace.pcg_form_for); ``fp32_moduli`` the FP32
+    it ("auto", "colour" or "gather", see DevicePCG and workspace.pcg_form_for) of a mesh too large for the cluster
+    form, which solves the smaller ones in one launch; ``fp32_moduli`` the FP32
     operator's moduli ("ref": reference frame, no gradients read; "physical"); ``max_blocks`` the most blocks
     per PCG launch (0: the whole GPU); ``preconditioner`` "jacobi", "block_jacobi", "multigrid" or "auto"
     (``preconditioner_for``); ``batch`` a ``BatchExecutor`` that runs the PCG solves of all slots together;
@@ -418,7 +419,7 @@ def solve_request(req, device, precision="fp32", n_load_steps=1, tol_rel=1e-10, 
             p = request_problem(req, device, build_on_device=True)
         ws = NewtonWorkspace(p, precision, use_graph=pcg_graph, pcg_form=pcg_form, fp32_moduli=fp32_moduli,
                              max_blocks=max_blocks, preconditioner=preconditioner, batch=batch, mg_graphs=mg_graphs,
-                             mg_bounds_every=mg_bounds_every, mg_gather=mg_gather)
+                             mg_bounds_every=mg_bounds_every, mg_gather=mg_gather, cluster=True)
     th = torch.ones(p["conn"].shape[0], dtype=torch.float64, device=device)
     tol = tol_rel * float(torch.linalg.vector_norm(p["f"]))
     if batch is not None:

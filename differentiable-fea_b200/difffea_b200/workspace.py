@@ -18,10 +18,10 @@ from difffea_b200.krylov import DevicePCG
 from difffea_b200.materials import device_material
 
 
-# Below this many elements the fused gather form of the PCG iteration (2 kernels) is faster than the
-# colour form (n_colours + 2 kernels); above it the colour form's lower traffic wins (measured on B200,
-# FP64, per iteration: 23.0 vs 40.2 us at 16k Q4 elements, 27.5 vs 46.5 at 40k, 171 vs 174 at 640k,
-# 608 vs 550 at 2.56M).
+# Launch forms for meshes too large for the cluster form.  Physical moduli: below this many elements the fused gather
+# form of the PCG iteration (2 kernels) is faster than the colour form (n_colours + 2 kernels); above it the colour
+# form's lower traffic wins (measured on B200, FP64, per iteration: 23.0 vs 40.2 us at 16k Q4 elements, 27.5 vs 46.5 at
+# 40k, 171 vs 174 at 640k, 608 vs 550 at 2.56M).  Reference-frame moduli: fused, 54 us at 262k, 135 us at 655k.
 GATHER_FORM_MAX_ELEMENTS = 1_500_000
 
 
@@ -39,7 +39,8 @@ def pcg_form_for(mesh, pcg_form="auto", moduli_code=_lib.DFEA_F64):
 
 class NewtonWorkspace:
     def __init__(self, params, precision="fp64", use_graph=2, pcg_form="auto", fp32_moduli="ref", max_blocks=0,
-                 preconditioner="jacobi", batch=None, mg_graphs=True, mg_bounds_every=0, mg_gather=False):
+                 preconditioner="jacobi", batch=None, mg_graphs=True, mg_bounds_every=0, mg_gather=False, cluster=None):
+        """``cluster``: solve in the cluster form of DevicePCG where the mesh fits it; None: with pcg_form "auto"."""
         if precision not in ("fp64", "fp32"):
             raise ValueError("precision must be 'fp64' or 'fp32' (FP32 moduli and PCG, FP64 Newton)")
         if preconditioner not in ("jacobi", "block_jacobi", "multigrid"):
@@ -101,8 +102,8 @@ class NewtonWorkspace:
         else:
             self.pcg = DevicePCG(mesh, self.C, self.diag if self.blocks is None else self.blocks, self.b, self.du,
                                  use_graph=use_graph, form=pcg_form_for(mesh, pcg_form, self.moduli_code),
-                                 moduli=self.moduli_kind,
-                                 max_blocks=max_blocks, preconditioner=preconditioner)
+                                 moduli=self.moduli_kind, max_blocks=max_blocks, preconditioner=preconditioner,
+                                 cluster=pcg_form == "auto" if cluster is None else cluster)
         self.work = mesh.reduce_work()
         self.mesh_id = ops.register_mesh(mesh)
         self.mat_args = ops.material_args(self.material)

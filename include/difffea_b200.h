@@ -70,6 +70,11 @@ extern "C" {
                                   * inverse 2x2 blocks of dfea_qp_moduli_block (4N f64) */
 #define DFEA_PCG_FUSED 64      /* dfea_pcg_create flag: fused gather form, 2 kernels per iteration
                                 * (implies DFEA_PCG_GATHER) */
+#define DFEA_PCG_CLUSTER 128   /* dfea_pcg_create flag: the whole solve in one launch of a thread-block cluster with
+                                * its vectors in distributed shared memory (DFEA_F32REF or DFEA_F64REF moduli, node
+                                * incidence; no block cap).  Alone: DFEA_ERR_UNSUPPORTED for a mesh that does not
+                                * fit; beside DFEA_PCG_GATHER or _FUSED: taken where the mesh fits, else that form.
+                                * The creation reads the mesh's incidence, which has to be complete by then. */
 /* dfea_pcg_create option: at most n blocks per launch (n < 2^23; 0 = as many as the GPU holds at
  * once).  For solves that share the GPU with solves on other streams. */
 #define DFEA_PCG_MAX_BLOCKS(n) ((int32_t)(n) << 8)
@@ -570,6 +575,8 @@ int dfea_pcg_solve(dfea_pcg* pcg, double rtol, int32_t max_iter, int32_t* iters,
                    void* stream);
 
 /* Release the graph and the handle (not the bound buffers). */
+/* 1 if the handle solves in the cluster form (DFEA_PCG_CLUSTER, and the mesh fits), else 0. */
+int dfea_pcg_clustered(const dfea_pcg* h);
 int dfea_pcg_destroy(dfea_pcg* pcg);
 
 /*
