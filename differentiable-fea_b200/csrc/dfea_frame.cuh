@@ -239,23 +239,6 @@ template <> struct FrameModuli<float> {
     }
 };
 
-// The threads that walk tiles together: a whole block, or one of several teams of a persistent block (named barrier
-// id + 1).
-struct BlockTeam {
-    static constexpr bool kCached = false;  // moduli stream through once
-    __device__ __forceinline__ int tid() const { return threadIdx.x; }
-    __device__ __forceinline__ void sync() const { __syncthreads(); }
-};
-template <int NT>
-struct SubTeam {
-    static constexpr bool kCached = true;   // the same moduli every iteration: let L1 keep them
-    __device__ __forceinline__ int tid() const { return threadIdx.x % NT; }
-    __device__ __forceinline__ int id() const { return threadIdx.x / NT; }
-    __device__ __forceinline__ void sync() const {
-        asm volatile("bar.sync %0, %1;" ::"r"(id() + 1), "n"(NT) : "memory");
-    }
-};
-
 template <int NEN, int NQ, typename T>
 struct FrameShared {
     v2_t<T> vs[NEN][FrameCfg<NEN, NQ>::EB];
@@ -265,13 +248,12 @@ struct FrameShared {
 // All elements of the mesh by the blocks blk of nblk: gather(node) -> nodal pair (masked here), out(a, e, f)
 // receives the element results; curv accumulates G . P per thread with DOT.  `start()` runs after the first
 // tile's moduli were requested; returning false abandons the walk.
-template <int NEN, int NQ, typename SD, typename T, bool DOT, typename Start, typename Gather, typename Out,
-          typename Team = BlockTeam>
+template <int NEN, int NQ, typename SD, typename T, bool DOT, typename Start, typename Gather, typename Out>
 __device__ __forceinline__ bool frame_product(const Mesh& m, const SD* __restrict__ C, const RefGrad<NEN, NQ>& rg,
                                               FrameShared<NEN, NQ, T>& sh, double& curv, Start&& start, Gather&& gather,
-                                              Out&& out, int64_t blk, int64_t nblk, Team team = Team()) {
+                                              Out&& out, int64_t blk, int64_t nblk) {
     constexpr int EB = FrameCfg<NEN, NQ>::EB;
-    const int lane = team.tid() % EB, q = team.tid() / EB;
+    const int lane = threadIdx.x % EB, q = threadIdx.x / EB;
     const int64_t n_tiles = (m.n_el + EB - 1) / EB;
     const RefRow<NEN, T> r(rg, q);
     FrameModuli<SD> M;
@@ -281,14 +263,14 @@ __device__ __forceinline__ bool frame_product(const Mesh& m, const SD* __restric
     int64_t e = tile * EB + lane;
     bool live = tile < n_tiles && e < m.n_el;
     conn.load(m, e, live, q);
-    if (live) M.template load<Team::kCached>(C, m.stride, q, e);
+    if (live) M.template load<false>(C, m.stride, q, e);
     else M.clear();
     if (!start()) return false;
     v.template gather<true>(conn, gather);
     conn.load(m, e + nblk * EB, e + nblk * EB < m.n_el, q);
     while (tile < n_tiles) {
         v.store(sh.vs, q, lane);
-        if (NQ > 1) team.sync();
+        if (NQ > 1) __syncthreads();
         v.template gather<true>(conn, gather);  // of the next tile
         conn.load(m, e + 2 * nblk * EB, e + 2 * nblk * EB < m.n_el, q);
         T G[4], P[4];
@@ -301,7 +283,7 @@ __device__ __forceinline__ bool frame_product(const Mesh& m, const SD* __restric
         tile += nblk;
         e += nblk * EB;
         live = e < m.n_el;
-        if (live) M.template load<Team::kCached>(C, m.stride, q, e);
+        if (live) M.template load<false>(C, m.stride, q, e);
         else M.clear();
         if constexpr (NQ == 1) {
 #pragma unroll
@@ -315,7 +297,7 @@ __device__ __forceinline__ bool frame_product(const Mesh& m, const SD* __restric
                 const T r0 = r.g[a][0], r1 = r.g[a][1];
                 sh.red[q][a][lane] = make_v2<T>(P[0] * r0 + P[1] * r1, P[2] * r0 + P[3] * r1);
             }
-            team.sync();
+            __syncthreads();
             frame_reduce<NEN, NQ, T>(e_now, live_now, q, lane, sh.red, out);
         }
     }

@@ -437,10 +437,11 @@ k_pcg_node_fused(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __r
 // owner's memory, summed there in incidence order), and the two reductions of an iteration ride on the cluster's
 // hardware barriers -- each warp stores its sum into every block's table before the barrier, every warp adds the table
 // in the same order after it, so all blocks take the same branch.  Only the moduli stream from L2.
-// Microseconds an iteration, FP64, B200 (fused launch form -> this): 64 Q4 14.2 -> 2.9, 576 14.2 -> 3.7, 2,304
-// 14.1 -> 5.1, 10,000 15.4 -> 9.1, 16,384 15.4 -> 12.3; 1,800 Q9 15.9 -> 10.1; 20,000 Tri3 18.0 -> 7.8.  So wherever
-// the vectors fit the cluster's shared memory it is the faster form, and it is taken there.  Past ~10k Q4 elements the
-// FP64 chains of the element pass on 16 SMs bound it.  (A grid-wide persistent form, exchanging through L2 with polled
+// Microseconds an iteration, FP64, B200 (fused launch form -> this): 64 Q4 14.0 -> 3.0, 576 15.4 -> 3.7, 2,304
+// 15.5 -> 5.1, 10,000 16.2 -> 7.9, 16,384 15.6 -> 10.1; 1,800 Q9 15.5 -> 7.7, 5,000 17.1 -> 10.9; 4,800 Tri6
+// 16.8 -> 8.9; 20,000 Tri3 17.6 -> 7.9.  So wherever the vectors fit the cluster's shared memory it is the faster form,
+// and it is taken there.  Past ~5k Q4 elements the element pass on 16 SMs (its FP64 chains) bounds it, below that the
+// two exchanges.  (A grid-wide persistent form, exchanging through L2 with polled
 // flags, took 7.7 us an iteration on one block and 13 - 18 us on many: its fences also empty L1.)
 //
 // There is no spin wait: the blocks of a cluster are scheduled together and meet at hardware barriers.  The number of
@@ -498,14 +499,25 @@ struct ClusterColours {
     }
 };
 
-template <int NEN, int NQ>
+// The element pass of a block, two ways.  SPLIT: teams of NQ warps on tiles of 32 elements, a warp per Gauss point, sums
+// through shared memory -- the shorter chain, while a block's elements are about one round of its teams.  Else one
+// thread per element, its Gauss points independent chains and the reference gradients constants of the unrolled loop:
+// no barriers, so more elements per block cost less.  Microseconds an iteration, FP64 (split / per element): 64 Q4
+// 3.0 / 4.1, 576 3.7 / 5.6, 2,304 5.1 / 5.7, 10,000 9.1 / 7.9, 16,384 12.3 / 10.1; 576 Q9 6.1 / 7.9, 1,800 10.1 / 7.7.
+template <int NEN, int NQ, bool SPLIT>
 struct ClusterCfg {
-    static constexpr int TEAMS = NQ == 9 ? 2 : (NQ == 6 ? 3 : 4);  // teams (the warps of one tile) of a block
-    static constexpr int TEAM = FrameCfg<NEN, NQ>::NT;
-    static constexpr int NT = TEAM * TEAMS;
+    static constexpr int TEAMS = NQ == 9 ? 2 : (NQ == 6 ? 3 : 4);
+    static constexpr int TEAM = 32 * NQ;
+    static constexpr int NT = SPLIT ? TEAM * TEAMS : (NEN <= 4 ? 640 : (NEN == 6 ? 512 : 384));  // 96 - 168 registers
     static constexpr int W = NT / 32;
-    static constexpr int TEAM_BYTES = TEAMS * (int)sizeof(FrameShared<NEN, NQ, double>);
+    static constexpr int TEAM_BYTES = SPLIT ? TEAMS * (int)sizeof(FrameShared<NEN, NQ, double>) : 0;
 };
+
+// SPLIT up to a round and a quarter of 16 blocks' teams
+template <int NEN, int NQ>
+bool cluster_split(int64_t n_el) {
+    return NQ > 1 && n_el <= (int64_t)kClusterMax * ClusterCfg<NEN, NQ, true>::TEAMS * 32 * 5 / 4;
+}
 
 // Element results of a node lie 32 entries apart, those of neighbouring nodes side by side (slices of 32 nodes, each as
 // deep as its busiest node): stored node by node, the element pass scattered with 8-way bank conflicts.
@@ -547,17 +559,15 @@ k_pcg_cluster_map(Mesh m, int nb, int slices, const int32_t* __restrict__ base, 
     }
 }
 
-template <int NEN, int NQ, typename SD, bool BJ>
-__global__ void __launch_bounds__(ClusterCfg<NEN, NQ>::NT, 1)
+template <int NEN, int NQ, typename SD, bool BJ, bool SPLIT>
+__global__ void __launch_bounds__(ClusterCfg<NEN, NQ, SPLIT>::NT, 1)
 k_pcg_cluster(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const int2* __restrict__ map,
               const double* __restrict__ b, const double* __restrict__ diag, double* __restrict__ x_out,
               const int32_t* __restrict__ slice_base, PcgState* __restrict__ st, ClusterLayout L, ClusterColours colours,
               double rtol, int max_iter) {
-    using Cfg = ClusterCfg<NEN, NQ>;
-    constexpr int NT = Cfg::NT, W = Cfg::W, EB = FrameCfg<NEN, NQ>::EB, GA = ConnRow<NEN, NQ>::GA;
+    using Cfg = ClusterCfg<NEN, NQ, SPLIT>;
+    constexpr int NT = Cfg::NT, W = Cfg::W;
     extern __shared__ __align__(16) unsigned char cluster_smem[];
-    const SubTeam<Cfg::TEAM> team;
-    FrameShared<NEN, NQ, double>& sh = reinterpret_cast<FrameShared<NEN, NQ, double>*>(cluster_smem)[team.id()];
     double2* xs = reinterpret_cast<double2*>(cluster_smem + L.x);
     double2* rs = reinterpret_cast<double2*>(cluster_smem + L.r);
     double2* ps = reinterpret_cast<double2*>(cluster_smem + L.p);
@@ -636,103 +646,138 @@ k_pcg_cluster(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const
     const double norm_b = sqrt(bb);
     if (norm_b == 0.0) status = DFEA_PCG_ZERO_RHS;
 
-    // this thread's share of the element pass: Gauss point q of lane's element in the tiles of its team.  The slots of the next two tiles and the moduli of the next are in
-    // flight, around the end of the pass as well: they do not change from iteration to iteration.
-    const int q = team.tid() / EB, lane = team.tid() % EB;
-    constexpr int step = Cfg::TEAMS * EB;
-    const int i_first = team.id() * EB + lane;
-    auto element = [&](int i) -> int { return i < n_els ? els[i] : -1; };
-    const RefRow<NEN, double> row(rg, q);
-    FrameModuli<SD> M;
-    int2 s0[GA], s1[GA];
-    auto load_slots = [&](int e, int2 (&s)[GA]) {
-#pragma unroll
-        for (int i = 0; i < GA; ++i) {
-            const int a = i * NQ + q;
-            s[i] = (a < NEN && e >= 0) ? __ldg(map + (int64_t)a * m.stride + e) : make_int2(-1, -1);
+    // z and p at a node, from its owner
+    auto fetch = [&](int word, double2& zn, double2& pn) {
+        const unsigned who = (unsigned)word >> 18;
+        const int at = (word & 0x3ffff) >> 2;
+        if (who == rank) {
+            zn = zs[at];
+            pn = ps[at];
+        } else {
+            zn = cluster_load(cluster_address(smem0 + L.z + at * 16, who));
+            pn = cluster_load(cluster_address(smem0 + L.p + at * 16, who));
         }
     };
-    auto load_moduli = [&](int e) {
-        if (e >= 0) M.template load<true>(C, m.stride, q, e);
-        else M.clear();
+    auto put = [&](int word, double2 f) {
+        const unsigned who = (unsigned)word >> 18;
+        const int at = word & 0x3ffff;
+        if (who == rank) fes[at] = f;
+        else cluster_store(cluster_address(smem0 + L.fe + at * 16, who), f);
     };
-    load_slots(element(i_first), s0);
-    load_slots(element(i_first + step), s1);
-    load_moduli(element(i_first));
+    // Slots and moduli of the first tile (or element) stay in flight around the end of the pass: they do not change from
+    // iteration to iteration.
+    constexpr bool KEEP = NEN <= 4;  // per element: the slots too, where registers allow
+    constexpr int NS = SPLIT ? 1 : NEN;
+    const int team = threadIdx.x / Cfg::TEAM, q = (threadIdx.x % Cfg::TEAM) / 32;       // SPLIT
+    const int i_first = SPLIT ? team * 32 + lane32 : threadIdx.x;
+    constexpr int step = SPLIT ? Cfg::TEAMS * 32 : NT;
+    FrameModuli<SD> M;
+    int2 s[NS], s_next = make_int2(-1, -1);
+    auto element = [&](int i) -> int { return i < n_els ? els[i] : -1; };
+    auto load_slot = [&](int a, int e) { return e >= 0 ? __ldg(map + (int64_t)a * m.stride + e) : make_int2(-1, -1); };
+    auto load_first = [&]() {
+        const int e = element(i_first);
+        if constexpr (SPLIT) {
+            s[0] = load_slot(q < NEN ? q : 0, q < NEN ? e : -1);
+            s_next = load_slot(q < NEN ? q : 0, q < NEN ? element(i_first + step) : -1);
+            if (e >= 0) M.template load<true>(C, m.stride, q, e);
+            else M.clear();
+        } else if (e >= 0) {
+            if (KEEP) {
+#pragma unroll
+                for (int a = 0; a < NS; ++a) s[a] = load_slot(a, e);
+            }
+            M.template load<true>(C, m.stride, 0, e);
+        }
+    };
+    load_first();
 
     for (int k = 0; status == DFEA_PCG_RUNNING; ++k) {
         double c = 0.0;
-        // z and p of the next tile's nodes; combined when they go to shared memory, a tile later
-        double2 zn[GA], pn[GA];
-        auto gather = [&](const int2 (&s)[GA]) {
-#pragma unroll
-            for (int i = 0; i < GA; ++i) {
-                zn[i] = pn[i] = make_double2(0.0, 0.0);
-                if (s[i].x < 0) continue;
-                const unsigned who = (unsigned)s[i].x >> 18;
-                const int at = (s[i].x & 0x3ffff) >> 2;
-                if (who == rank) {
-                    zn[i] = zs[at];
-                    pn[i] = ps[at];
-                } else {
-                    zn[i] = cluster_load(cluster_address(smem0 + L.z + at * 16, who));
-                    pn[i] = cluster_load(cluster_address(smem0 + L.p + at * 16, who));
+        if constexpr (SPLIT) {
+            FrameShared<NEN, NQ, double>& sh = reinterpret_cast<FrameShared<NEN, NQ, double>*>(cluster_smem)[team];
+            const RefRow<NEN, double> row(rg, q);
+            auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(Cfg::TEAM) : "memory"); };
+            // z and p of the next tile's nodes; combined when they go to shared memory, a tile later
+            double2 zn = make_double2(0.0, 0.0), pn = zn;
+            if (s[0].x >= 0) fetch(s[0].x, zn, pn);
+            for (int tile = team * 32; tile < n_els; tile += step) {
+                if (q < NEN)
+                    sh.vs[q][lane32] = make_double2((s[0].x & 1) ? 0.0 : zn.x + beta * pn.x, (s[0].x & 2) ? 0.0 : zn.y + beta * pn.y);
+                team_sync();
+                const int to = s[0].y;
+                const bool more = tile + step < n_els;
+                if (more) {
+                    s[0] = s_next;
+                    zn = pn = make_double2(0.0, 0.0);
+                    if (s[0].x >= 0) fetch(s[0].x, zn, pn);
+                    s_next = load_slot(q < NEN ? q : 0, q < NEN ? element(tile + lane32 + 2 * step) : -1);
                 }
-            }
-        };
-        gather(s0);
-        for (int tile = team.id() * EB; tile < n_els; tile += step) {
-#pragma unroll
-            for (int i = 0; i < GA; ++i)
-                if (i * NQ + q < NEN)
-                    sh.vs[i * NQ + q][lane] = make_double2((s0[i].x & 1) ? 0.0 : zn[i].x + beta * pn[i].x,
-                                                           (s0[i].x & 2) ? 0.0 : zn[i].y + beta * pn[i].y);
-            if (NQ > 1) team.sync();
-            int2 now[GA];
-#pragma unroll
-            for (int i = 0; i < GA; ++i) {
-                now[i] = s0[i];
-                s0[i] = s1[i];
-            }
-            const bool more = tile + step < n_els;
-            if (more) {
-                gather(s0);
-                load_slots(element(tile + lane + 2 * step), s1);
-            }
-            double G[4], P[4];
-            frame_gradient<NEN, NQ, double>(row, lane, sh.vs, G);
-            M.apply(G, P);
-            c += G[0] * P[0] + G[1] * P[1] + G[2] * P[2] + G[3] * P[3];
-            load_moduli(element(more ? tile + lane + step : i_first));
-            auto put = [&](const int2& s, double2 f) {
-                if (s.y < 0) return;
-                const unsigned who = (unsigned)s.y >> 18;
-                if (who == rank) fes[s.y & 0x3ffff] = f;
-                else cluster_store(cluster_address(smem0 + L.fe + (s.y & 0x3ffff) * 16, who), f);
-            };
-            if constexpr (NQ == 1) {
+                double G[4], P[4];
+                frame_gradient<NEN, NQ, double>(row, lane32, sh.vs, G);
+                M.apply(G, P);
+                c += G[0] * P[0] + G[1] * P[1] + G[2] * P[2] + G[3] * P[3];
+                if (more) {
+                    const int e = element(tile + lane32 + step);
+                    if (e >= 0) M.template load<true>(C, m.stride, q, e);
+                    else M.clear();
+                }
 #pragma unroll
                 for (int a = 0; a < NEN; ++a)
-                    put(now[a], make_double2(P[0] * row.g[a][0] + P[1] * row.g[a][1], P[2] * row.g[a][0] + P[3] * row.g[a][1]));
-            } else {
-#pragma unroll
-                for (int a = 0; a < NEN; ++a)
-                    sh.red[q][a][lane] = make_double2(P[0] * row.g[a][0] + P[1] * row.g[a][1], P[2] * row.g[a][0] + P[3] * row.g[a][1]);
-                team.sync();
-                if (q < NEN) {
-                    double2 f = sh.red[0][q][lane];
+                    sh.red[q][a][lane32] = make_double2(P[0] * row.g[a][0] + P[1] * row.g[a][1], P[2] * row.g[a][0] + P[3] * row.g[a][1]);
+                team_sync();
+                if (q < NEN && to >= 0) {
+                    double2 f = sh.red[0][q][lane32];
 #pragma unroll
                     for (int g = 1; g < NQ; ++g) {
-                        const double2 t = sh.red[g][q][lane];
+                        const double2 t = sh.red[g][q][lane32];
                         f.x += t.x;
                         f.y += t.y;
                     }
-                    put(now[0], f);
+                    put(to, f);
                 }
             }
+        } else {
+            for (int i = threadIdx.x; i < n_els; i += NT) {
+                const int e = els[i];
+                if (!KEEP || i >= NT) {
+#pragma unroll
+                    for (int a = 0; a < NS; ++a) s[a] = load_slot(a, e);
+                }
+                if (i >= NT) M.template load<true>(C, m.stride, 0, e);
+                double2 v[NS], f[NS];
+#pragma unroll
+                for (int a = 0; a < NS; ++a) {
+                    double2 zn, pn;
+                    fetch(s[a].x, zn, pn);
+                    v[a] = make_double2((s[a].x & 1) ? 0.0 : zn.x + beta * pn.x, (s[a].x & 2) ? 0.0 : zn.y + beta * pn.y);
+                    f[a] = make_double2(0.0, 0.0);
+                }
+#pragma unroll(NQ > 4 ? 1 : NQ)
+                for (int g = 0; g < NQ; ++g) {
+                    const FrameModuli<SD> now = M;
+                    if (g + 1 < NQ) M.template load<true>(C, m.stride, g + 1, e);
+                    double G[4] = {0.0, 0.0, 0.0, 0.0}, P[4];
+#pragma unroll
+                    for (int a = 0; a < NS; ++a) {
+                        G[0] += v[a].x * rg.g[g][a][0];
+                        G[1] += v[a].x * rg.g[g][a][1];
+                        G[2] += v[a].y * rg.g[g][a][0];
+                        G[3] += v[a].y * rg.g[g][a][1];
+                    }
+                    now.apply(G, P);
+                    c += G[0] * P[0] + G[1] * P[1] + G[2] * P[2] + G[3] * P[3];
+#pragma unroll
+                    for (int a = 0; a < NS; ++a) {
+                        f[a].x += P[0] * rg.g[g][a][0] + P[1] * rg.g[g][a][1];
+                        f[a].y += P[2] * rg.g[g][a][0] + P[3] * rg.g[g][a][1];
+                    }
+                }
+#pragma unroll
+                for (int a = 0; a < NS; ++a) put(s[a].y, f[a]);
+            }
         }
-        load_slots(element(i_first), s0);
-        load_slots(element(i_first + step), s1);
+        load_first();
         for (int i = threadIdx.x; i < n_own; i += NT) {  // the identity rows' part of p.Ap
             const int fix = fixs[i];
             if (fix) {
@@ -1011,14 +1056,13 @@ int cluster_configure() {
 
 constexpr int kClusterSmem = 220 * 1024;  // dynamic shared memory a block may take (of 227 KB)
 
-// The cluster of a mesh: blocks (a power of two, every team with at least a tile) and shared memory, or 0 blocks where
+// The cluster of a mesh: blocks (a power of two) and shared memory, or 0 blocks where
 // the mesh does not fit.  max_slots(blocks, nb, slices): the most fe entries of a block's node range.
-template <int NEN, int NQ, typename MaxSlots>
+template <int NEN, int NQ, bool SPLIT, typename MaxSlots>
 int cluster_layout(const dfea_mesh_view& mv, bool block_jacobi, ClusterLayout* out, MaxSlots&& max_slots) {
-    using Cfg = ClusterCfg<NEN, NQ>;
-    const int64_t tiles = (mv.n_el + FrameCfg<NEN, NQ>::EB - 1) / FrameCfg<NEN, NQ>::EB;
+    using Cfg = ClusterCfg<NEN, NQ, SPLIT>;
     int blocks = 1;
-    while (blocks < kClusterMax && (int64_t)blocks * Cfg::TEAMS < tiles) blocks *= 2;
+    while (blocks < kClusterMax && (int64_t)blocks * Cfg::TEAMS * 32 < mv.n_el) blocks *= 2;
     const int64_t nb = (mv.n_nodes + blocks - 1) / blocks;
     if (nb >= (1 << 16) || 96 * nb > kClusterSmem) return 0;  // five vectors and an entry per node at the least
     const int slices = (int)((nb + 31) / 32);
@@ -1058,27 +1102,33 @@ int launch_cluster(const dfea_pcg& h, cudaStream_t s, double rtol, int max_iter)
     colours.n = mv.n_colours;
     for (int c = 0; c <= mv.n_colours; ++c) colours.begin[c] = (int)mv.colour_begin[c];
     k_pcg_reset<<<1, 128, 0, s>>>(st);
-    int rc = dispatch_element(mv.nen, mv.n_q, [&](auto nen_c, auto nq_c) -> int {
+    const int rc = dispatch_element(mv.nen, mv.n_q, [&](auto nen_c, auto nq_c) -> int {
         constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
-        constexpr auto kernel = k_pcg_cluster<NEN, NQ, SD, BJ>;
-        int rc2 = cluster_configure<kernel>();
-        if (rc2) return rc2;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = h.cluster_blocks;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(h.cluster_blocks);
-        cfg.blockDim = dim3(ClusterCfg<NEN, NQ>::NT);
-        cfg.dynamicSmemBytes = h.cluster.total;
-        cfg.stream = s;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        return check_cuda(cudaLaunchKernelEx(&cfg, kernel, m, static_cast<const SD*>(h.moduli), ref_grad_of<NEN, NQ>(mv),
-                                             (const int2*)h.slot_map(),
-                                             static_cast<const double*>(h.b), static_cast<const double*>(h.diag),
-                                             static_cast<double*>(h.x), (const int32_t*)h.slice_base(), st, h.cluster, colours, rtol, max_iter),
-                          "cudaLaunchKernelEx(cluster PCG)");
+        const auto launch = [&](auto split_c) -> int {
+            constexpr bool SPLIT = decltype(split_c)::value;
+            constexpr auto kernel = k_pcg_cluster<NEN, NQ, SD, BJ, SPLIT>;
+            const int rc2 = cluster_configure<kernel>();
+            if (rc2) return rc2;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = h.cluster_blocks;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(h.cluster_blocks);
+            cfg.blockDim = dim3(ClusterCfg<NEN, NQ, SPLIT>::NT);
+            cfg.dynamicSmemBytes = h.cluster.total;
+            cfg.stream = s;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            return check_cuda(cudaLaunchKernelEx(&cfg, kernel, m, static_cast<const SD*>(h.moduli), ref_grad_of<NEN, NQ>(mv),
+                                                 (const int2*)h.slot_map(), static_cast<const double*>(h.b),
+                                                 static_cast<const double*>(h.diag), static_cast<double*>(h.x),
+                                                 (const int32_t*)h.slice_base(), st, h.cluster, colours, rtol, max_iter),
+                              "cudaLaunchKernelEx(cluster PCG)");
+        };
+        if constexpr (NQ > 1)
+            if (cluster_split<NEN, NQ>(mv.n_el)) return launch(std::true_type{});
+        return launch(std::false_type{});
     });
     if (rc) return rc;
     note_launches(2);
@@ -1098,7 +1148,7 @@ int prepare_cluster(dfea_pcg* h) {
     int rc = DFEA_OK;
     h->cluster_blocks = dispatch_element(mv.nen, mv.n_q, [&](auto nen_c, auto nq_c) -> int {
         constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
-        return cluster_layout<NEN, NQ>(mv, h->block, &h->cluster, [&](int blocks, int64_t nb, int slices) -> int64_t {
+        const auto max_slots = [&](int blocks, int64_t nb, int slices) -> int64_t {
             k_pcg_cluster_slices<<<blocks, 256, 0, s>>>(mv.n_nodes, (int)nb, slices, mv.node_elem_ptr, h->slice_base());
             note_launches(1);
             int32_t total[kClusterMax];
@@ -1111,7 +1161,9 @@ int prepare_cluster(dfea_pcg* h) {
             int64_t most = 0;
             for (int i = 0; i < blocks; ++i) most = total[i] > most ? total[i] : most;
             return most;
-        });
+        };
+        return cluster_split<NEN, NQ>(mv.n_el) ? cluster_layout<NEN, NQ, true>(mv, h->block, &h->cluster, max_slots)
+                                               : cluster_layout<NEN, NQ, false>(mv, h->block, &h->cluster, max_slots);
     });
     if (rc) return rc;
     if (h->cluster_blocks == 0)
