@@ -17,6 +17,7 @@
 #include <new>
 #include <utility>
 
+#include "dfea_cluster.cuh"
 #include "dfea_common.cuh"
 
 namespace dfea {
@@ -31,10 +32,16 @@ struct MgGrid {
     const int32_t* cell_y;
     double* K;
     uint8_t* fix;
+    double* S;  // node stencils (k_mg_stencil), or NULL: products from the element matrices
 };
 
-static MgGrid mg_grid(const dfea_mg_grid& g) {
-    return MgGrid{g.gx, g.gy, g.line_x, g.line_y, g.cell_x, g.cell_y, g.K, g.fix};
+static MgGrid mg_grid(const dfea_mg_grid& g, double* stencil = nullptr) {
+    return MgGrid{g.gx, g.gy, g.line_x, g.line_y, g.cell_x, g.cell_y, g.K, g.fix, stencil};
+}
+
+// num / den for the integers of the grid maps: lines are 1 or 2 apart, so the quotient is exact without a division
+__device__ __forceinline__ double frac(int num, int den) {
+    return den == 1 ? (double)num : (den == 2 ? 0.5 * num : (double)num / (double)den);
 }
 
 static int validate_grid(const dfea_mg_grid* g, bool coarse, const char* what) {
@@ -52,11 +59,11 @@ __device__ __forceinline__ double hat(const int32_t* X, int n_lines, int c, int 
     if (i < xc) {
         if (c == 0) return 0.0;
         const int xl = X[c - 1];
-        return i <= xl ? 0.0 : (double)(i - xl) / (double)(xc - xl);
+        return i <= xl ? 0.0 : frac(i - xl, xc - xl);
     }
     if (c == n_lines - 1) return 0.0;
     const int xr = X[c + 1];
-    return i >= xr ? 0.0 : (double)(xr - i) / (double)(xr - xc);
+    return i >= xr ? 0.0 : frac(xr - i, xr - xc);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -89,8 +96,7 @@ k_mg_galerkin_fe(Mesh m, const void* __restrict__ moduli, RefGrad<NEN, NQ> rg, c
                     const int c = m.conn[a * S + s];
                     const int n = c >> 2;
                     fix[a] = c & 3;
-                    const double wx1 = (double)(node_ij[2 * n] - x0) / (double)(x1 - x0);
-                    const double wy1 = (double)(node_ij[2 * n + 1] - y0) / (double)(y1 - y0);
+                    const double wx1 = frac(node_ij[2 * n] - x0, x1 - x0), wy1 = frac(node_ij[2 * n + 1] - y0, y1 - y0);
                     const double wx0 = 1.0 - wx1, wy0 = 1.0 - wy1;
                     P[a][0] = wx0 * wy0;
                     P[a][1] = wx1 * wy0;
@@ -192,58 +198,129 @@ k_mg_galerkin_fe(Mesh m, const void* __restrict__ moduli, RefGrad<NEN, NQ> rg, c
 // ------------------------------------------------------------------------------------------
 // level l + 1 from level l: K_C = sum_{fine cells c in C} P_c^T K_c P_c
 // ------------------------------------------------------------------------------------------
+// One thread per coarse cell and column of its matrix (cells fastest): a level of a few hundred cells fills more of
+// the chip than with a thread per cell (26 us a level on the serving meshes, whatever its size), in the same order.
 __global__ void __launch_bounds__(128) k_mg_galerkin(MgGrid fg, MgGrid cg) {
     const int n_cells = cg.gx * cg.gy, nf_cells = fg.gx * fg.gy;
-    for (int C = blockIdx.x * blockDim.x + threadIdx.x; C < n_cells; C += gridDim.x * blockDim.x) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 8 * n_cells; t += gridDim.x * blockDim.x) {
+        const int col = t / n_cells, C = t - col * n_cells, kc = col & 1, bc = col >> 1;
         const int CX = C / cg.gy, CY = C % cg.gy;
         const int x0 = cg.line_x[CX], x1 = cg.line_x[CX + 1], y0 = cg.line_y[CY], y1 = cg.line_y[CY + 1];
-        double K[64];
+        double K[8];
 #pragma unroll
-        for (int k = 0; k < 64; ++k) K[k] = 0.0;
+        for (int k = 0; k < 8; ++k) K[k] = 0.0;
 #pragma unroll 1
         for (int fx = x0; fx < x1; ++fx) {
 #pragma unroll 1
             for (int fy = y0; fy < y1; ++fy) {
                 const int fc = fx * fg.gy + fy;
                 // P[a][b]: weight of coarse corner b at fine corner a (corners (0,0) (1,0) (1,1) (0,1))
-                double P[4][4];
+                double P[4][4], Pc[4];
 #pragma unroll
                 for (int a = 0; a < 4; ++a) {
                     const int i = fx + ((a == 1 || a == 2) ? 1 : 0), j = fy + ((a >= 2) ? 1 : 0);
-                    const double wx1 = (double)(i - x0) / (double)(x1 - x0), wy1 = (double)(j - y0) / (double)(y1 - y0);
+                    const double wx1 = frac(i - x0, x1 - x0), wy1 = frac(j - y0, y1 - y0);
                     const double wx0 = 1.0 - wx1, wy0 = 1.0 - wy1;
                     P[a][0] = wx0 * wy0;
                     P[a][1] = wx1 * wy0;
                     P[a][2] = wx1 * wy1;
                     P[a][3] = wx0 * wy1;
+                    Pc[a] = bc == 0 ? P[a][0] : bc == 1 ? P[a][1] : bc == 2 ? P[a][2] : P[a][3];
                 }
-                // T = K_c P (8 x 8), then K += P^T T; P acts on both components alike
-#pragma unroll 1
-                for (int col = 0; col < 8; ++col) {
-                    const int b = col >> 1, k = col & 1;
-                    double t[8];
+                // t = column of K_c P, then K += P^T t; P acts on both components alike
+                double tc[8];
 #pragma unroll
-                    for (int row = 0; row < 8; ++row) {
+                for (int row = 0; row < 8; ++row) {
+                    double acc = 0.0;
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) acc += fg.K[(int64_t)(row * 8 + 2 * a + kc) * nf_cells + fc] * Pc[a];
+                    tc[row] = acc;
+                }
+#pragma unroll
+                for (int bb = 0; bb < 4; ++bb)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
                         double acc = 0.0;
 #pragma unroll
-                        for (int a = 0; a < 4; ++a) acc += fg.K[(int64_t)(row * 8 + 2 * a + k) * nf_cells + fc] * P[a][b];
-                        t[row] = acc;
+                        for (int a = 0; a < 4; ++a) acc += P[a][bb] * tc[2 * a + i];
+                        K[2 * bb + i] += acc;
                     }
-#pragma unroll
-                    for (int bb = 0; bb < 4; ++bb)
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            double acc = 0.0;
-#pragma unroll
-                            for (int a = 0; a < 4; ++a) acc += P[a][bb] * t[2 * a + i];
-                            K[(2 * bb + i) * 8 + col] += acc;
-                        }
-                }
             }
         }
 #pragma unroll
-        for (int k = 0; k < 64; ++k) cg.K[(int64_t)k * n_cells + C] = K[k];
+        for (int r = 0; r < 8; ++r) cg.K[(int64_t)(r * 8 + col) * n_cells + C] = K[r];
     }
+}
+
+// ------------------------------------------------------------------------------------------
+// node stencils: the rows of a coarse operator as the 2 x 2 blocks of a node with itself and its eight neighbours
+// ------------------------------------------------------------------------------------------
+// Block of node n = (I, J) with node (I + di, J + dj), both rows r and columns c as c4[2 r + c], summed over the cells
+// that hold both nodes in cell order; the identity of a fixed DOF on the diagonal.
+__device__ __forceinline__ void mg_stencil_block(const MgGrid& g, int I, int J, int di, int dj, double (&c4)[4]) {
+    const int n_cells = g.gx * g.gy;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c4[k] = 0.0;
+#pragma unroll
+    for (int cx = -1; cx <= 0; ++cx)
+#pragma unroll
+        for (int cy = -1; cy <= 0; ++cy) {
+            const int CX = I + cx, CY = J + cy;
+            const int ai = -cx, aj = -cy, bi = di - cx, bj = dj - cy;  // corners of the two nodes in the cell
+            if (bi < 0 || bi > 1 || bj < 0 || bj > 1 || CX < 0 || CY < 0 || CX >= g.gx || CY >= g.gy) continue;
+            const int a = aj ? (ai ? 2 : 3) : ai, b = bj ? (bi ? 2 : 3) : bi;
+            const int c = CX * g.gy + CY;
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) c4[2 * r + q] += g.K[(int64_t)((2 * a + r) * 8 + 2 * b + q) * n_cells + c];
+        }
+    if (di == 0 && dj == 0) {
+        const int f = g.fix[I * (g.gy + 1) + J];
+        if (f & 1) c4[0] += 1.0;
+        if (f & 2) c4[3] += 1.0;
+    }
+}
+
+// S[(4 m + k) N + n], m = 3 (di + 1) + dj + 1: 36 numbers a node where the cells around it hold 64, and no identity or
+// grid-edge cases left in the products.  diag: the operator's diagonal.  One thread per node and neighbour.
+__global__ void __launch_bounds__(256) k_mg_stencil(MgGrid g, double* __restrict__ diag) {
+    const int N = (g.gx + 1) * (g.gy + 1), ny = g.gy + 1;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 9 * N; t += gridDim.x * blockDim.x) {
+        const int m = t / N, n = t - m * N;
+        const int di = m / 3 - 1, dj = m % 3 - 1;
+        double c4[4];
+        mg_stencil_block(g, n / ny, n % ny, di, dj, c4);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) g.S[(int64_t)(4 * m + k) * N + n] = c4[k];
+        if (m == 4) reinterpret_cast<double2*>(diag)[n] = make_double2(c4[0], c4[3]);
+    }
+}
+
+// The product's row at node n from its stencil: load(id) v at a neighbour, entry(4 m + k) of the stencil.  A neighbour
+// past the grid's edge has a zero block: the node's own value stands in, so all nine loads are issued before the sums.
+template <typename Load, typename Entry>
+__device__ __forceinline__ double2 mg_stencil_row(const MgGrid& g, Load&& load, Entry&& entry, int n) {
+    const int ny = g.gy + 1, I = n / ny, J = n - I * ny;
+    double2 v[9];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) {
+        const int i = I + m / 3 - 1, j = J + m % 3 - 1;
+        const bool in = i >= 0 && i <= g.gx && j >= 0 && j <= g.gy;
+        v[m] = load(in ? n + (m / 3 - 1) * ny + m % 3 - 1 : n);
+    }
+    double2 y[3];  // a sum per grid line: three short chains
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        y[i] = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int m = 3 * i + j;
+            y[i].x += entry(4 * m) * v[m].x + entry(4 * m + 1) * v[m].y;
+            y[i].y += entry(4 * m + 2) * v[m].x + entry(4 * m + 3) * v[m].y;
+        }
+    }
+    return make_double2(y[0].x + y[1].x + y[2].x, y[0].y + y[1].y + y[2].y);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -257,19 +334,47 @@ __device__ __forceinline__ int fine_node(const int32_t* gnode, int fgy, int i, i
 
 // rc = P~^T r (masked at fixed fine DOFs); with fix_out, also the coarse fix bits (a coarse DOF is fixed
 // when every fine DOF it interpolates to is fixed)
-// coarse node n of the restriction r_c = P~^T r (and the coarse fixed-DOF bits); the kernels below and the
-// one-block tail of the V-cycle share these per-node functions, whose pointers carry no __restrict__ because
-// the tail reads in one phase what it wrote in the previous one
-__device__ __forceinline__ void mg_restrict_node(const MgGrid& fg, const MgGrid& cg, const int32_t* gnode,
-                                                 const uint8_t* ffix, const double* r, double* rc, uint8_t* fix_out,
-                                                 int n) {
+// coarse node n of the restriction r_c = P~^T r (and the coarse fixed-DOF bits); load(id): r at a fine node.  The
+// kernels below and the cluster tail of the V-cycle share these per-node functions.
+template <bool SUM, typename Load>
+__device__ __forceinline__ double2 mg_restrict_sum(const MgGrid& fg, const MgGrid& cg, const int32_t* gnode,
+                                                   const uint8_t* ffix, Load&& load, int n, int* fixed) {
     const int nx = cg.gx + 1, ny = cg.gy + 1;
-    const double2* r2 = reinterpret_cast<const double2*>(r);
     const int I = n / ny, J = n % ny;
-    const int ilo = I > 0 ? cg.line_x[I - 1] + 1 : cg.line_x[I], ihi = I < cg.gx ? cg.line_x[I + 1] - 1 : cg.line_x[I];
-    const int jlo = J > 0 ? cg.line_y[J - 1] + 1 : cg.line_y[J], jhi = J < cg.gy ? cg.line_y[J + 1] - 1 : cg.line_y[J];
+    const int xc = cg.line_x[I], xl = I > 0 ? cg.line_x[I - 1] : xc, xr = I < cg.gx ? cg.line_x[I + 1] : xc;
+    const int yc = cg.line_y[J], yl = J > 0 ? cg.line_y[J - 1] : yc, yr = J < cg.gy ? cg.line_y[J + 1] : yc;
     double ax = 0.0, ay = 0.0;
     int free_bits = 0;
+    if (xc - xl <= 2 && xr - xc <= 2 && yc - yl <= 2 && yr - yc <= 2) {
+        // lines one or two apart: the node itself and the fine lines halfway to its neighbours, all loads first
+        int id[9], f[9];
+        double2 t[9];
+        double w[9];
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {
+            const int a = m / 3 - 1, b = m % 3 - 1;
+            const bool in = (a == 0 || (a < 0 ? xc - xl == 2 : xr - xc == 2)) && (b == 0 || (b < 0 ? yc - yl == 2 : yr - yc == 2));
+            w[m] = in ? (a == 0 ? 1.0 : 0.5) * (b == 0 ? 1.0 : 0.5) : 0.0;
+            id[m] = fine_node(gnode, fg.gy, in ? xc + a : xc, in ? yc + b : yc);
+        }
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {
+            const bool there = id[m] >= 0;
+            f[m] = there ? ffix[id[m]] : 3;
+            t[m] = SUM && there ? load(id[m]) : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {
+            if (w[m] == 0.0 || id[m] < 0) continue;
+            if (SUM && !(f[m] & 1)) ax += w[m] * t[m].x;
+            if (SUM && !(f[m] & 2)) ay += w[m] * t[m].y;
+            free_bits |= (~f[m]) & 3;
+        }
+        if (fixed) *fixed = (~free_bits) & 3;
+        return make_double2(ax, ay);
+    }
+    const int ilo = I > 0 ? xl + 1 : xc, ihi = I < cg.gx ? xr - 1 : xc;
+    const int jlo = J > 0 ? yl + 1 : yc, jhi = J < cg.gy ? yr - 1 : yc;
     for (int i = ilo; i <= ihi; ++i) {
         const double wx = hat(cg.line_x, nx, I, i);
         for (int j = jlo; j <= jhi; ++j) {
@@ -277,31 +382,37 @@ __device__ __forceinline__ void mg_restrict_node(const MgGrid& fg, const MgGrid&
             if (id < 0) continue;
             const double w = wx * hat(cg.line_y, ny, J, j);
             const int f = ffix[id];
-            if (r) {
-                const double2 t = r2[id];
+            if (SUM) {
+                const double2 t = load(id);
                 if (!(f & 1)) ax += w * t.x;
                 if (!(f & 2)) ay += w * t.y;
             }
             if (w > 0.0) free_bits |= (~f) & 3;
         }
     }
-    if (rc) reinterpret_cast<double2*>(rc)[n] = make_double2(ax, ay);
-    if (fix_out) fix_out[n] = (uint8_t)((~free_bits) & 3);
+    if (fixed) *fixed = (~free_bits) & 3;
+    return make_double2(ax, ay);
 }
 
 __global__ void k_mg_restrict(MgGrid fg, MgGrid cg, const int32_t* __restrict__ gnode, const uint8_t* __restrict__ ffix,
                               const double* __restrict__ r, double* __restrict__ rc, uint8_t* __restrict__ fix_out) {
     const int n_nodes = (cg.gx + 1) * (cg.gy + 1);
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < n_nodes; n += gridDim.x * blockDim.x)
-        mg_restrict_node(fg, cg, gnode, ffix, r, rc, fix_out, n);
+    const double2* r2 = reinterpret_cast<const double2*>(r);
+    const auto load = [&](int id) { return r2[id]; };
+    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < n_nodes; n += gridDim.x * blockDim.x) {
+        int fixed;
+        const double2 t = r ? mg_restrict_sum<true>(fg, cg, gnode, ffix, load, n, &fixed)
+                            : mg_restrict_sum<false>(fg, cg, gnode, ffix, load, n, &fixed);
+        if (rc) reinterpret_cast<double2*>(rc)[n] = t;
+        if (fix_out) fix_out[n] = (uint8_t)fixed;
+    }
 }
 
-// x += P~ ec (x untouched at fixed fine DOFs) at fine grid node n
+// x += P~ ec (x untouched at fixed fine DOFs) at fine grid node n; load(c): ec at a coarse node, x(id): the fine value
+template <typename Load, typename X>
 __device__ __forceinline__ void mg_prolong_node(const MgGrid& fg, const MgGrid& cg, const int32_t* gnode,
-                                                const uint8_t* ffix, const double* ec, double* x, int n) {
+                                                const uint8_t* ffix, Load&& load, X&& x, int n) {
     const int fny = fg.gy + 1, cny = cg.gy + 1;
-    const double2* e2 = reinterpret_cast<const double2*>(ec);
-    double2* x2 = reinterpret_cast<double2*>(x);
     const int i = n / fny, j = n % fny;
     const int id = gnode ? gnode[n] : n;
     if (id < 0) return;
@@ -309,31 +420,34 @@ __device__ __forceinline__ void mg_prolong_node(const MgGrid& fg, const MgGrid& 
     if ((f & 3) == 3) return;
     const int CX = cg.cell_x[i], CY = cg.cell_y[j];
     const int x0 = cg.line_x[CX], x1 = cg.line_x[CX + 1], y0 = cg.line_y[CY], y1 = cg.line_y[CY + 1];
-    const double wx1 = (double)(i - x0) / (double)(x1 - x0), wy1 = (double)(j - y0) / (double)(y1 - y0);
+    const double wx1 = frac(i - x0, x1 - x0), wy1 = frac(j - y0, y1 - y0);
     const double wx0 = 1.0 - wx1, wy0 = 1.0 - wy1;
-    const double2 e00 = e2[CX * cny + CY], e10 = e2[(CX + 1) * cny + CY];
-    const double2 e11 = e2[(CX + 1) * cny + CY + 1], e01 = e2[CX * cny + CY + 1];
-    double2 t = x2[id];
+    const double2 e00 = load(CX * cny + CY), e10 = load((CX + 1) * cny + CY);
+    const double2 e11 = load((CX + 1) * cny + CY + 1), e01 = load(CX * cny + CY + 1);
+    double2& t = x(id);
     if (!(f & 1)) t.x += wx0 * wy0 * e00.x + wx1 * wy0 * e10.x + wx1 * wy1 * e11.x + wx0 * wy1 * e01.x;
     if (!(f & 2)) t.y += wx0 * wy0 * e00.y + wx1 * wy0 * e10.y + wx1 * wy1 * e11.y + wx0 * wy1 * e01.y;
-    x2[id] = t;
 }
 
 __global__ void k_mg_prolong_add(MgGrid fg, MgGrid cg, const int32_t* __restrict__ gnode, const uint8_t* __restrict__ ffix,
                                  const double* __restrict__ ec, double* __restrict__ x) {
     const int n_nodes = (fg.gx + 1) * (fg.gy + 1);
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < n_nodes; n += gridDim.x * blockDim.x)
-        mg_prolong_node(fg, cg, gnode, ffix, ec, x, n);
+        mg_prolong_node(fg, cg, gnode, ffix, [&](int c) { return reinterpret_cast<const double2*>(ec)[c]; },
+                        [&](int id) -> double2& { return reinterpret_cast<double2*>(x)[id]; }, n);
 }
 
 // ------------------------------------------------------------------------------------------
 // coarse-level operator: y = K v + (I - M) v (K has zero rows and columns at fixed DOFs); DIAG: diag(A)
 // ------------------------------------------------------------------------------------------
-// row of node n = I * ny + J (both DOFs); the standalone product and the fused smoothing steps below share it,
-// so they compute the same sums in the same order
+// row of node n = I * ny + J (both DOFs): from the stencil, or from the element matrices of the cells around the node
 template <bool DIAG>
 __device__ __forceinline__ double2 mg_node_row(const MgGrid& g, const double2* v2, int n) {
     const int ny = g.gy + 1, n_cells = g.gx * g.gy;
+    if (!DIAG && g.S != nullptr) {
+        const int64_t N = (int64_t)(g.gx + 1) * ny;
+        return mg_stencil_row(g, [&](int i) { return v2[i]; }, [&](int k) { return g.S[k * N + n]; }, n);
+    }
     const int I = n / ny, J = n % ny;
     double y0 = 0.0, y1 = 0.0;
 #pragma unroll
@@ -641,110 +755,122 @@ static int mg_lanczos_step1(int64_t n, double* p, const double* q, double* r, do
 }
 
 // ------------------------------------------------------------------------------------------
-// Lanczos of the small levels in one block (levels of at most kMgTailNodes nodes, each smoothed level's
-// start and all its steps).  The dot products reproduce dfea_mg_dot inside the block: nb = mg_dot_blocks(n)
-// virtual blocks of kMgDotThreads threads with the same grid-stride accumulation, the same warp and block
-// trees, then the final block's tree over the nb partials, so the coefficients, the bounds and every later
-// iterate are bitwise those of the separate launches.
+// the small levels in distributed shared memory
 // ------------------------------------------------------------------------------------------
-constexpr int kMgTailLanczosThreads = 2 * kMgDotThreads;
+// Levels of at most kMgTailNodes nodes are worked on by thread-block clusters: the nodes of a level are divided over the
+// cluster's blocks in ranges, its vectors, its rows (node stencils) and its 1 / D lie in the owners' shared memory, and
+// cluster barriers separate the phases.  What bounds a phase is latency: a gather through distributed shared memory, two
+// chains of multiply-adds, a barrier: 1.7 us.  (A launch per phase costs 5 - 6 us; one block alone streams the rows
+// through one SM; rows read from L2, divisions by D and neighbours loaded one after the other left a phase at 4 us.)
+// The tail of a 128 x 128 Q9 cycle (levels of 4,225 nodes down to 25): 100 us in one block, plus 44 us of launches for
+// the 4,225-node level, -> 54 us; the Lanczos estimates of these levels 247 -> 51 us, the clusters side by side.
+constexpr int kMgTailNodes = 6000;
+constexpr int kMgClusterThreads = 512;
+constexpr int kMgClusterWarps = kMgClusterThreads / 32;
+
+// a level's vector: entry n at place n % nb of block n / nb (n below 2^22: the quotient by a float reciprocal is exact)
+struct ClusterVec {
+    double2* mine;  // this block's range
+    unsigned here;  // its shared address, the same in every block
+    int nb;
+    float inv_nb;
+    __device__ __forceinline__ ClusterVec(unsigned char* smem, int offset, int nb_)
+        : mine(reinterpret_cast<double2*>(smem + offset)), here((unsigned)__cvta_generic_to_shared(smem + offset)), nb(nb_),
+          inv_nb(1.0f / (float)nb_) {}
+    __device__ __forceinline__ double2 operator()(int n) const {
+        const int who = (int)(((float)n + 0.5f) * inv_nb), at = n - who * nb;
+        return cluster_load(cluster_address(here + at * 16, who));
+    }
+};
+
+// the stencils of this block's nodes to shared memory, rows[entry][node]
+__device__ __forceinline__ void load_rows(const MgGrid& g, double* rows, int nb, int first, int n_own, int n_nodes) {
+    for (int t = threadIdx.x; t < 36 * n_own; t += kMgClusterThreads) {
+        const int e = t / n_own, i = t - e * n_own;
+        rows[e * nb + i] = __ldg(g.S + (int64_t)e * n_nodes + first + i);
+    }
+}
 
 struct MgLanczosLevel {
     MgGrid grid;
-    int n;                       // DOFs
+    int n_nodes, nb;             // nodes, nodes per block
     const double* diag;
-    double *r, *z, *p, *q;       // the level's r, d, x and q buffers
     double* s;                   // [p.Ap, r.z, -, beta]
     double* hist;                // (alpha_k, beta_k) per step
 };
 
 struct MgLanczosTail {
-    int n_levels, steps;
+    int steps, size;             // blocks of a level's cluster
     MgLanczosLevel lv[DFEA_MG_MAX_LEVELS];
 };
 
-// x.y, returned to every thread; every thread of the block calls it
-__device__ double tail_dot(int n, const double* x, const double* y) {
-    constexpr int NW = kMgDotThreads / 32;
-    __shared__ double warp_part[kMgTailLanczosThreads / 32];
-    __shared__ double block_part[kMgDotBlocks];
-    __shared__ double result;
-    const int half = threadIdx.x / kMgDotThreads, vt = threadIdx.x % kMgDotThreads;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nb = mg_dot_blocks(n);
-    for (int vb0 = 0; vb0 < nb; vb0 += 2) {
-        const int vb = vb0 + half;
+// Lanczos of the small smoothed levels, one cluster per level side by side: r = sin(i + 1), z = r / D, p = z, then the
+// CG steps of the separate launches (their sums in the cluster's order)
+__global__ void __launch_bounds__(kMgClusterThreads, 1) k_mg_tail_lanczos(const __grid_constant__ MgLanczosTail T) {
+    constexpr int NT = kMgClusterThreads;
+    extern __shared__ __align__(16) unsigned char mg_smem[];
+    __shared__ double table[ClusterExchange<kMgClusterWarps>::kDoubles];
+    const unsigned rank = cluster_rank();
+    const MgLanczosLevel& L = T.lv[blockIdx.x / T.size];
+    ClusterExchange<kMgClusterWarps> sums(table, rank, T.size);
+    const ClusterVec p(mg_smem, 0, L.nb);
+    double2* r = p.mine + L.nb;
+    double2* z = p.mine + 2 * L.nb;
+    double2* q = p.mine + 3 * L.nb;
+    double* rows = reinterpret_cast<double*>(q + L.nb);
+    const int first = rank * L.nb, n_own = min(L.nb, max(0, L.n_nodes - first));
+    load_rows(L.grid, rows, L.nb, first, n_own, L.n_nodes);
+    const double2* diag2 = reinterpret_cast<const double2*>(L.diag) + first;
+    double rz = 0.0;
+    for (int i = threadIdx.x; i < n_own; i += NT) {
+        const double2 rn = make_double2(sin((double)(2 * (first + i) + 1)), sin((double)(2 * (first + i) + 2)));
+        const double2 D = diag2[i], zn = make_double2(rn.x / D.x, rn.y / D.y);
+        r[i] = rn;
+        z[i] = zn;
+        p.mine[i] = zn;
+        rz += rn.x * zn.x + rn.y * zn.y;
+    }
+    cluster_barrier();  // every block has started
+    rz = sums.one(rz);
+    if (rank == 0 && threadIdx.x == 0) L.s[1] = rz;
+    for (int k = 0; k < T.steps; ++k) {
         double a = 0.0;
-        if (vb < nb)
-            for (int64_t i = vb * (int64_t)kMgDotThreads + vt; i < n; i += (int64_t)nb * kMgDotThreads) a += x[i] * y[i];
-        a = warp_sum(a);
-        if (lane == 0) warp_part[warp] = a;
-        __syncthreads();
-        if (warp % NW == 0) {
-            double r = (lane < NW) ? warp_part[warp + lane] : 0.0;
-            r = warp_sum(r);
-            if (lane == 0 && vb < nb) block_part[vb] = r;
+        for (int i = threadIdx.x; i < n_own; i += NT) {
+            const double2 qn = mg_stencil_row(L.grid, p, [&](int e) { return rows[e * L.nb + i]; }, first + i);
+            q[i] = qn;
+            a += p.mine[i].x * qn.x + p.mine[i].y * qn.y;
         }
-        __syncthreads();
-    }
-    if (threadIdx.x < kMgDotThreads) {
-        double a = 0.0;
-        for (int b = threadIdx.x; b < nb; b += kMgDotThreads) a += block_part[b];
-        a = warp_sum(a);
-        if (lane == 0) warp_part[warp] = a;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        double r = (lane < NW) ? warp_part[lane] : 0.0;
-        r = warp_sum(r);
-        if (lane == 0) result = r;
-    }
-    __syncthreads();
-    const double out = result;
-    __syncthreads();
-    return out;
-}
-
-__global__ void __launch_bounds__(kMgTailLanczosThreads) k_mg_tail_lanczos(const __grid_constant__ MgLanczosTail T) {
-    for (int l = 0; l < T.n_levels; ++l) {
-        const MgLanczosLevel& L = T.lv[l];
-        const int n_nodes = L.n / 2;
-        // start: r = sin(i + 1), z = r / D, p = z, s[1] = r.z
-        for (int i = threadIdx.x; i < L.n; i += blockDim.x) {
-            const double ri = sin((double)(i + 1));
-            L.r[i] = ri;
-            const double zi = ri / L.diag[i];
-            L.z[i] = zi;
-            L.p[i] = zi;
+        const double pq = sums.one(a);
+        const double alpha = rz / pq;
+        a = 0.0;
+        for (int i = threadIdx.x; i < n_own; i += NT) {
+            const double2 qn = q[i], D = diag2[i];
+            double2 rn = r[i];
+            rn.x -= alpha * qn.x;
+            rn.y -= alpha * qn.y;
+            const double2 zn = make_double2(rn.x / D.x, rn.y / D.y);
+            r[i] = rn;
+            z[i] = zn;
+            a += rn.x * zn.x + rn.y * zn.y;
         }
-        __syncthreads();
-        double rz = tail_dot(L.n, L.r, L.z);
-        if (threadIdx.x == 0) L.s[1] = rz;
-        for (int k = 0; k < T.steps; ++k) {
-            for (int n = threadIdx.x; n < n_nodes; n += blockDim.x)
-                reinterpret_cast<double2*>(L.q)[n] = mg_node_row<false>(L.grid, reinterpret_cast<const double2*>(L.p), n);
-            __syncthreads();
-            const double pq = tail_dot(L.n, L.p, L.q);
-            const double alpha = rz / pq;
-            for (int i = threadIdx.x; i < L.n; i += blockDim.x) {
-                const double ri = L.r[i] - alpha * L.q[i];
-                L.r[i] = ri;
-                L.z[i] = ri / L.diag[i];
-            }
-            __syncthreads();
-            const double rz_new = tail_dot(L.n, L.r, L.z);
-            const double beta = rz_new / rz;
-            if (threadIdx.x == 0) {
-                L.hist[2 * k] = alpha;
-                L.hist[2 * k + 1] = beta;
-                L.s[0] = pq;
-                L.s[1] = rz_new;
-                L.s[3] = beta;
-            }
-            rz = rz_new;
-            for (int i = threadIdx.x; i < L.n; i += blockDim.x) L.p[i] = L.z[i] + beta * L.p[i];
-            __syncthreads();
+        const double rz_new = sums.one(a);
+        const double beta = rz_new / rz;
+        if (rank == 0 && threadIdx.x == 0) {
+            L.hist[2 * k] = alpha;
+            L.hist[2 * k + 1] = beta;
+            L.s[0] = pq;
+            L.s[1] = rz_new;
+            L.s[3] = beta;
         }
+        rz = rz_new;
+        for (int i = threadIdx.x; i < n_own; i += NT) {
+            const double2 zn = z[i];
+            double2 pn = p.mine[i];
+            pn.x = zn.x + beta * pn.x;
+            pn.y = zn.y + beta * pn.y;
+            p.mine[i] = pn;
+        }
+        cluster_barrier();
     }
 }
 
@@ -752,18 +878,78 @@ __global__ void __launch_bounds__(kMgTailLanczosThreads) k_mg_tail_lanczos(const
 // coarsest level: dense A (assembled in cell order), inverted by Gauss-Jordan (A is SPD: no pivoting)
 // ------------------------------------------------------------------------------------------
 constexpr int kMgDenseMax = 256;     // DOFs
-constexpr int kMgDenseShared = 112;  // up to this many DOFs A, Ainv and the pivot column live in shared memory
+constexpr int kMgDenseShared = 112;  // up to this many DOFs the matrix is inverted in registers
 
-// SHARED: A and Ainv in dynamic shared memory (copied to Ainv_out at the end), else in global memory
-template <bool SHARED>
-__global__ void __launch_bounds__(1024) k_mg_dense_inverse(MgGrid g, double* __restrict__ A_glob, double* __restrict__ Ainv_out) {
-    extern __shared__ double dense_sm[];
+// n <= kMgDenseShared: in-place Gauss-Jordan with the matrix in registers (a thread holds rows ti + 16 r, columns
+// tj + 32 q), the pivot row and column of a step through shared memory, one barrier per step.  (The matrix in shared
+// memory, assembled cell after cell, took 70 us for 50 DOFs and 115 us for 90.)
+template <int R, int Q>
+__global__ void __launch_bounds__(512) k_mg_dense_inverse_small(MgGrid g, double* __restrict__ Ainv_out) {
+    __shared__ double row[2][32 * Q], col[2][16 * R];
+    const int ny = g.gy + 1, n = 2 * (g.gx + 1) * ny;
+    const int ti = threadIdx.x >> 5, tj = threadIdx.x & 31;
+    double a[R][Q];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int i = ti + 16 * r, j = tj + 32 * q;
+            a[r][q] = 0.0;
+            if (i < n && j < n) {
+                const int ni = i >> 1, nj = j >> 1, I = ni / ny, J = ni % ny, di = nj / ny - I, dj = nj % ny - J;
+                if (di >= -1 && di <= 1 && dj >= -1 && dj <= 1) {
+                    double c4[4];
+                    mg_stencil_block(g, I, J, di, dj, c4);
+                    a[r][q] = (i & 1) ? ((j & 1) ? c4[3] : c4[2]) : ((j & 1) ? c4[1] : c4[0]);
+                }
+            }
+        }
+#pragma unroll
+    for (int kr = 0; kr < R; ++kr) {  // step k = 16 kr + kk: the pivot's register indices are constants
+        for (int kk = 0; kk < 16 && 16 * kr + kk < n; ++kk) {
+            const int k = 16 * kr + kk;
+            double *rk = row[k & 1], *ck = col[k & 1];
+            // publish pivot row and column and clear them: a_ij - c_i s_j then holds for every entry, with c_k = -1
+            if (ti == kk) {
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    rk[tj + 32 * q] = a[kr][q];
+                    if (tj + 32 * q != k) a[kr][q] = 0.0;
+                }
+            }
+            if (tj == (k & 31)) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    ck[ti + 16 * r] = ti + 16 * r == k ? -1.0 : a[r][kr / 2];
+                    a[r][kr / 2] = 0.0;
+                }
+            }
+            __syncthreads();  // the next step writes the other buffers
+            const double p = 1.0 / rk[k];
+            double s[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) s[q] = tj + 32 * q == k ? p : rk[tj + 32 * q] * p;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const double c = ck[ti + 16 * r];
+#pragma unroll
+                for (int q = 0; q < Q; ++q) a[r][q] -= c * s[q];
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int i = ti + 16 * r, j = tj + 32 * q;
+            if (i < n && j < n) Ainv_out[i * n + j] = a[r][q];
+        }
+}
+
+// larger: A and Ainv in global memory
+__global__ void __launch_bounds__(1024) k_mg_dense_inverse(MgGrid g, double* __restrict__ A, double* __restrict__ Ainv) {
     const int ny = g.gy + 1, nn = (g.gx + 1) * ny, n = 2 * nn, n_cells = g.gx * g.gy;
-    double* A = SHARED ? dense_sm : A_glob;
-    double* Ainv = SHARED ? dense_sm + n * n : Ainv_out;
-    double* fcol = SHARED ? dense_sm + 2 * n * n : nullptr;
-    __shared__ double fcol_glob[SHARED ? 1 : 2 * kMgDenseMax];
-    if (!SHARED) fcol = fcol_glob;
+    __shared__ double fcol[kMgDenseMax];
     for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
         A[k] = 0.0;
         Ainv[k] = (k / n == k % n) ? 1.0 : 0.0;
@@ -801,8 +987,6 @@ __global__ void __launch_bounds__(1024) k_mg_dense_inverse(MgGrid g, double* __r
         }
         __syncthreads();
     }
-    if (SHARED)
-        for (int t = threadIdx.x; t < n * n; t += blockDim.x) Ainv_out[t] = Ainv[t];
 }
 
 // x = Ainv b, one warp per row
@@ -821,21 +1005,17 @@ __global__ void k_mg_dense_solve(int n, const double* __restrict__ Ainv, const d
 }
 
 // ------------------------------------------------------------------------------------------
-// the coarse tail of a V-cycle in one block: levels t .. L-1 are small enough that a launch per smoothing
-// step costs more than the step, so one block runs the restriction from level t - 1, the smoothing of
-// every tail level, the coarsest solve and the prolongation back to level t - 1, with a block barrier
-// between phases.  Each phase calls the per-node function of the kernel it replaces, so the result is
-// bitwise that of the separate launches.
+// the coarse tail of a V-cycle in one cluster: levels t .. L-1 are small enough that a launch per smoothing step costs
+// more than the step, so one launch runs the restriction from level t - 1, the smoothing of every tail level, the
+// coarsest solve and the prolongation back to level t - 1, with a cluster barrier between phases.  Each phase computes
+// the per-node expressions of the kernel it replaces.
 // ------------------------------------------------------------------------------------------
-constexpr int kMgTailThreads = 1024;
-constexpr int kMgTailNodes = 1536;   // levels of at most this many nodes run in the tail
-
 struct MgTailLevel {
     MgGrid grid;
-    int n;                       // DOFs
+    int n_nodes, nb;             // nodes, nodes per block
+    int vec;                     // byte offset in shared memory: vectors b, x, r, d, q, 1 / D (nb pairs each), rows
     const double* diag;
     const double* coef;          // [scale, (c1, c2) per step]
-    double *b, *x, *r, *d, *q;
 };
 
 struct MgTail {
@@ -849,62 +1029,171 @@ struct MgTail {
     MgTailLevel lv[DFEA_MG_MAX_LEVELS];
 };
 
-__device__ __forceinline__ void tail_smooth(const MgTailLevel& L, int degree) {
-    const int n_nodes = L.n / 2;
-    double *d_in = L.d, *d_out = L.q;
-    for (int k = 1; k <= degree; ++k) {
-        const int last = k == degree ? 1 : 0;
-        const double c1 = last ? 0.0 : L.coef[1 + 2 * (k - 1)], c2 = last ? 0.0 : L.coef[2 + 2 * (k - 1)];
-        for (int n = threadIdx.x; n < n_nodes; n += blockDim.x)
-            mg_cheb_apply_step_node(L.grid, L.x, L.r, d_in, d_out, L.diag, c1, c2, last, n);
-        __syncthreads();
-        double* t = d_in;
-        d_in = d_out;
-        d_out = t;
-    }
-}
+__global__ void __launch_bounds__(kMgClusterThreads, 1) k_mg_tail(const __grid_constant__ MgTail T) {
+    constexpr int NT = kMgClusterThreads;
+    extern __shared__ __align__(16) unsigned char mg_smem[];
+    __shared__ double b_all[kMgDenseMax];
+    const unsigned rank = cluster_rank();
+    const int size = gridDim.x, last = T.n_levels - 1;  // the grid is the cluster
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto vec = [&](const MgTailLevel& L, int k) { return ClusterVec(mg_smem, L.vec + k * L.nb * 16, L.nb); };
+    auto owned = [&](const MgTailLevel& L) { return min(L.nb, max(0, L.n_nodes - (int)rank * L.nb)); };
+    enum { VB, VX, VR, VD, VQ, VI, VROWS };
+    auto rows_of = [&](const MgTailLevel& L) { return reinterpret_cast<double*>(mg_smem + L.vec + VROWS * L.nb * 16); };
 
-__global__ void __launch_bounds__(kMgTailThreads) k_mg_tail(const __grid_constant__ MgTail T) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-    const int last = T.n_levels - 1;
+    auto smooth = [&](const MgTailLevel& L) {
+        const int first = rank * L.nb, n_own = owned(L);
+        double2 *x = vec(L, VX).mine, *r = vec(L, VR).mine;
+        const double2* inv = vec(L, VI).mine;
+        const double* rows = rows_of(L);
+        int in = VD, out = VQ;
+        for (int k = 1; k <= T.degree; ++k) {
+            const bool more = k < T.degree;
+            const double c1 = more ? L.coef[1 + 2 * (k - 1)] : 0.0, c2 = more ? L.coef[2 + 2 * (k - 1)] : 0.0;
+            const ClusterVec d = vec(L, in);
+            double2* d_out = vec(L, out).mine;
+            for (int i = threadIdx.x; i < n_own; i += NT) {
+                const double2 q = mg_stencil_row(L.grid, d, [&](int e) { return rows[e * L.nb + i]; }, first + i);
+                const double2 dn = d.mine[i], I = inv[i];
+                double2 xn = x[i];
+                xn.x += dn.x;
+                xn.y += dn.y;
+                x[i] = xn;
+                const double r0 = r[i].x - q.x, r1 = r[i].y - q.y;
+                r[i] = make_double2(r0, r1);
+                if (more) d_out[i] = make_double2(c1 * dn.x + c2 * r0 * I.x, c1 * dn.y + c2 * r1 * I.y);
+            }
+            cluster_barrier();
+            const int t = in;
+            in = out;
+            out = t;
+        }
+    };
+
+    for (int l = 0; l < last; ++l) {
+        const MgTailLevel& L = T.lv[l];
+        const int first = rank * L.nb, n_own = owned(L);
+        load_rows(L.grid, rows_of(L), L.nb, first, n_own, L.n_nodes);
+        double2* inv = vec(L, VI).mine;
+        for (int i = threadIdx.x; i < n_own; i += NT) {
+            const double2 D = reinterpret_cast<const double2*>(L.diag)[first + i];
+            inv[i] = make_double2(1.0 / D.x, 1.0 / D.y);
+        }
+    }
+    cluster_barrier();  // every block has started, its rows are loaded
     for (int l = 0; l <= last; ++l) {
         const MgTailLevel& L = T.lv[l];
-        const MgGrid& fg = l == 0 ? T.fine : T.lv[l - 1].grid;
-        const int32_t* gn = l == 0 ? T.gnode : nullptr;
-        const uint8_t* ffix = l == 0 ? T.ffix : T.lv[l - 1].grid.fix;
-        const double* r = l == 0 ? T.r_fine : T.lv[l - 1].r;
-        for (int n = threadIdx.x; n < L.n / 2; n += blockDim.x) mg_restrict_node(fg, L.grid, gn, ffix, r, L.b, nullptr, n);
-        __syncthreads();
-        if (l == last) break;
-        const double s = L.coef[0];
-        for (int i = threadIdx.x; i < L.n; i += blockDim.x) {
-            const double bi = L.b[i];
-            L.r[i] = bi;
-            L.x[i] = 0.0;
-            L.d[i] = s * bi / L.diag[i];
+        const int first = rank * L.nb, n_own = owned(L);
+        double2 *b = vec(L, VB).mine, *x = vec(L, VX).mine, *r = vec(L, VR).mine, *d = vec(L, VD).mine;
+        const double2* inv = vec(L, VI).mine;
+        const double s = l < last ? L.coef[0] : 0.0;
+        for (int i = threadIdx.x; i < n_own; i += NT) {
+            double2 bn;
+            if (l == 0) {
+                const double2* r2 = reinterpret_cast<const double2*>(T.r_fine);
+                bn = mg_restrict_sum<true>(T.fine, L.grid, T.gnode, T.ffix, [&](int id) { return r2[id]; }, first + i, nullptr);
+            } else {
+                const MgTailLevel& F = T.lv[l - 1];
+                bn = mg_restrict_sum<true>(F.grid, L.grid, nullptr, F.grid.fix, vec(F, VR), first + i, nullptr);
+            }
+            b[i] = bn;
+            if (l < last) {
+                r[i] = bn;
+                x[i] = make_double2(0.0, 0.0);
+                d[i] = make_double2(s * bn.x * inv[i].x, s * bn.y * inv[i].y);
+            }
+        }
+        cluster_barrier();
+        if (l < last) smooth(L);
+    }
+    {
+        const MgTailLevel& C = T.lv[last];
+        const ClusterVec b = vec(C, VB);
+        for (int n = threadIdx.x; n < C.n_nodes; n += NT) {
+            const double2 t = b(n);
+            b_all[2 * n] = t.x;
+            b_all[2 * n + 1] = t.y;
         }
         __syncthreads();
-        tail_smooth(L, T.degree);
+        const unsigned x_here = vec(C, VX).here;
+        const int n = 2 * C.n_nodes;
+        for (int row = rank * (NT / 32) + warp; row < n; row += size * (NT / 32)) {
+            double s = 0.0;
+            for (int j = lane; j < n; j += 32) s += T.Ainv[(int64_t)row * n + j] * b_all[j];
+            s = warp_sum(s);
+            if (lane == 0) cluster_store(cluster_address(x_here + (row / 2 % C.nb) * 16 + (row & 1) * 8, row / 2 / C.nb), s);
+        }
+        cluster_barrier();
     }
-    const MgTailLevel& C = T.lv[last];
-    for (int r = warp; r < C.n; r += n_warps) mg_dense_row(C.n, T.Ainv, C.b, C.x, r, lane);
-    __syncthreads();
     for (int l = last; l >= 0; --l) {
         const MgTailLevel& L = T.lv[l];
-        const MgGrid& fg = l == 0 ? T.fine : T.lv[l - 1].grid;
-        const int32_t* gn = l == 0 ? T.gnode : nullptr;
-        const uint8_t* ffix = l == 0 ? T.ffix : T.lv[l - 1].grid.fix;
-        double* xf = l == 0 ? T.x_fine : T.lv[l - 1].x;
-        const int fine_nodes = (fg.gx + 1) * (fg.gy + 1);
-        for (int n = threadIdx.x; n < fine_nodes; n += blockDim.x) mg_prolong_node(fg, L.grid, gn, ffix, L.x, xf, n);
-        __syncthreads();
-        if (l == 0) break;
+        const ClusterVec ec = vec(L, VX);
+        if (l == 0) {
+            const int fine_nodes = (T.fine.gx + 1) * (T.fine.gy + 1);
+            for (int n = rank * NT + threadIdx.x; n < fine_nodes; n += size * NT)
+                mg_prolong_node(T.fine, L.grid, T.gnode, T.ffix, ec,
+                                [&](int id) -> double2& { return reinterpret_cast<double2*>(T.x_fine)[id]; }, n);
+            break;
+        }
         const MgTailLevel& F = T.lv[l - 1];
+        const int first = rank * F.nb, n_own = owned(F);
+        const ClusterVec x = vec(F, VX);
+        double2 *b = vec(F, VB).mine, *r = vec(F, VR).mine, *d = vec(F, VD).mine;
+        for (int i = threadIdx.x; i < n_own; i += NT)
+            mg_prolong_node(F.grid, L.grid, nullptr, F.grid.fix, ec, [&](int id) -> double2& { return x.mine[id - first]; }, first + i);
+        cluster_barrier();
         const double s = F.coef[0];
-        for (int n = threadIdx.x; n < F.n / 2; n += blockDim.x) mg_residual_restart_node(F.grid, F.b, F.x, F.diag, s, F.r, F.d, n);
-        __syncthreads();
-        tail_smooth(F, T.degree);
+        const double2* inv = vec(F, VI).mine;
+        const double* rows = rows_of(F);
+        for (int i = threadIdx.x; i < n_own; i += NT) {
+            const double2 q = mg_stencil_row(F.grid, x, [&](int e) { return rows[e * F.nb + i]; }, first + i);
+            const double r0 = b[i].x - q.x, r1 = b[i].y - q.y;
+            r[i] = make_double2(r0, r1);
+            d[i] = make_double2(s * r0 * inv[i].x, s * r1 * inv[i].y);
+        }
+        cluster_barrier();
+        smooth(F);
     }
+    cluster_barrier();  // no block leaves while another may read its shared memory
+}
+
+// A launch of clusters of `size` blocks (a power of two of at most kClusterMax).
+template <auto Kernel, typename... Args>
+static int launch_clusters(int n_clusters, int size, size_t smem, cudaStream_t s, const Args&... args) {
+    static std::once_flag once[64];
+    static int result[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    std::call_once(once[dev], [dev] {
+        int most = 0;
+        int rc = check_cuda(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
+        cudaFuncAttributes fa;
+        if (!rc) rc = check_cuda(cudaFuncGetAttributes(&fa, Kernel), "cudaFuncGetAttributes");
+        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                      most - (int)fa.sharedSizeBytes), "cudaFuncSetAttribute");
+        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "cudaFuncSetAttribute");
+        result[dev] = rc;
+    });
+    if (result[dev]) return result[dev];
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n_clusters * size);
+    cfg.blockDim = dim3(kMgClusterThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return check_cuda(cudaLaunchKernelEx(&cfg, Kernel, args...), "cudaLaunchKernelEx");
+}
+
+// blocks for a largest level of n nodes: about 64 nodes a block, 16 blocks at the most
+static int mg_cluster_size(int64_t n_nodes) {
+    int size = 1;
+    while (size < kClusterMax && (int64_t)size * 64 < n_nodes) size *= 2;
+    return size;
 }
 
 }  // namespace dfea
@@ -956,7 +1245,7 @@ extern "C" int dfea_mg_galerkin(const dfea_mg_grid* fine, const dfea_mg_grid* co
         return rc;
     if (!fine->K || !coarse->K) return set_error(DFEA_ERR_INVALID, "dfea_mg_galerkin: NULL element matrices");
     const int n_cells = coarse->gx * coarse->gy;
-    k_mg_galerkin<<<grid_for(n_cells, 128, 8), 128, 0, static_cast<cudaStream_t>(stream)>>>(mg_grid(*fine), mg_grid(*coarse));
+    k_mg_galerkin<<<grid_for(8 * (int64_t)n_cells, 128, 8), 128, 0, static_cast<cudaStream_t>(stream)>>>(mg_grid(*fine), mg_grid(*coarse));
     note_launches(1);
     return launch_check("dfea_mg_galerkin");
 }
@@ -1038,29 +1327,16 @@ extern "C" int dfea_mg_dense_inverse(const dfea_mg_grid* grid, double* work, dou
     if (n > kMgDenseMax) return set_error(DFEA_ERR_INVALID, "dfea_mg_dense_inverse: %d DOFs exceed %d", n, kMgDenseMax);
     if (!grid->K || !grid->fix || !work || !Ainv) return set_error(DFEA_ERR_INVALID, "dfea_mg_dense_inverse: NULL pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (n <= kMgDenseShared) {
-        const size_t smem = (size_t)(2 * n * n + n) * sizeof(double);
-        // the shared-memory opt-in is a property of the function on each device: set once per device
-        // ordinal (a bit per device, set under a mutex so that concurrent first set-ups are safe)
-        static std::mutex attr_mutex;
-        static unsigned long long attr_set = 0ull;
-        int dev = 0;
-        if ((rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice"))) return rc;
-        if (dev < 0 || dev >= 64) return set_error(DFEA_ERR_INVALID, "dfea_mg_dense_inverse: device ordinal %d", dev);
-        {
-            std::lock_guard<std::mutex> lock(attr_mutex);
-            if (!(attr_set & (1ull << dev))) {
-                rc = check_cuda(cudaFuncSetAttribute(k_mg_dense_inverse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)((2 * kMgDenseShared * kMgDenseShared + kMgDenseShared) * sizeof(double))),
-                                "cudaFuncSetAttribute");
-                if (rc) return rc;
-                attr_set |= 1ull << dev;
-            }
-        }
-        k_mg_dense_inverse<true><<<1, 1024, smem, st>>>(mg_grid(*grid), work, Ainv);
-    } else {
-        k_mg_dense_inverse<false><<<1, 1024, 0, st>>>(mg_grid(*grid), work, Ainv);
-    }
+    if (n <= 32)
+        k_mg_dense_inverse_small<2, 1><<<1, 512, 0, st>>>(mg_grid(*grid), Ainv);
+    else if (n <= 64)
+        k_mg_dense_inverse_small<4, 2><<<1, 512, 0, st>>>(mg_grid(*grid), Ainv);
+    else if (n <= 96)
+        k_mg_dense_inverse_small<6, 3><<<1, 512, 0, st>>>(mg_grid(*grid), Ainv);
+    else if (n <= kMgDenseShared)
+        k_mg_dense_inverse_small<7, 4><<<1, 512, 0, st>>>(mg_grid(*grid), Ainv);
+    else
+        k_mg_dense_inverse<<<1, 1024, 0, st>>>(mg_grid(*grid), work, Ainv);
     note_launches(1);
     return launch_check("dfea_mg_dense_inverse");
 }
@@ -1158,6 +1434,15 @@ static double ritz_max(const double* hist, int steps) {
     return tridiag_max_eig(a, e, m);
 }
 
+// the stencils of level l >= 1 in mg->stencil (36 numbers a node, level after level), or NULL
+static double* stencil_of(const dfea_mg* mg, int l) {
+    if (!mg->stencil || l < 1) return nullptr;
+    double* s = mg->stencil;
+    for (int k = 1; k < l; ++k) s += 36 * (mg->level[k].n / 2);
+    return s;
+}
+static MgGrid level_grid(const dfea_mg* mg, int l) { return mg_grid(mg->level[l].grid, stencil_of(mg, l)); }
+
 static void transfer_args(const dfea_mesh_view* mesh, const dfea_mg* mg, int l, const int32_t** gnode,
                           const uint8_t** ffix) {
     *gnode = l == 0 ? mg->gnode : nullptr;
@@ -1175,7 +1460,10 @@ static int mg_apply(const dfea_mesh_view* mesh, const dfea_mg* mg, const void* m
         return fe_gather(mesh, mg)
                    ? dfea_tangent_apply_gather(mesh, moduli, code, v, y, DFEA_F64, mg->fe_work, s)
                    : dfea_tangent_apply(mesh, moduli, code, v, y, DFEA_F64, s);
-    return dfea_mg_apply(&mg->level[l].grid, v, y, s);
+    const int n_nodes = (int)(mg->level[l].n / 2);
+    k_mg_apply<false><<<grid_for(n_nodes, 256, 8), 256, 0, s>>>(level_grid(mg, l), v, y);
+    note_launches(1);
+    return launch_check("multigrid product");
 }
 
 // the Chebyshev steps of one smoothing pass at level l, from the first direction in lv.d; on coarse levels
@@ -1200,7 +1488,7 @@ static int mg_cheb_steps(const dfea_mesh_view* mesh, const dfea_mg* mg, const vo
             continue;
         }
         const int n_nodes = (lv.grid.gx + 1) * (lv.grid.gy + 1);
-        k_mg_cheb_apply_step<<<grid_for(n_nodes, 256, 8), 256, 0, s>>>(mg_grid(lv.grid), x, r, d_in, d_out, lv.diag, c, last);
+        k_mg_cheb_apply_step<<<grid_for(n_nodes, 256, 8), 256, 0, s>>>(level_grid(mg, l), x, r, d_in, d_out, lv.diag, c, last);
         note_launches(1);
         rc = launch_check("dfea_mg_vcycle: smoothing step");
         std::swap(d_in, d_out);
@@ -1210,6 +1498,7 @@ static int mg_cheb_steps(const dfea_mesh_view* mesh, const dfea_mg* mg, const vo
 
 // first level (>= 1) of the one-block tail: levels shrink, so every level from it on is small enough
 static int tail_start(const dfea_mg* mg) {
+    if (!mg->stencil) return mg->n_levels;
     for (int l = 1; l < mg->n_levels; ++l)
         if (mg->level[l].n / 2 <= kMgTailNodes) return l;
     return mg->n_levels;
@@ -1226,12 +1515,16 @@ static int launch_tail(const dfea_mesh_view* mesh, const dfea_mg* mg, int l, dou
     T.Ainv = mg->Ainv;
     T.n_levels = mg->n_levels - (l + 1);
     T.degree = mg->degree;
+    const int size = mg_cluster_size(mg->level[l + 1].n / 2);
+    int at = 0;
     for (int k = 0; k < T.n_levels; ++k) {
         const dfea_mg_level& c = mg->level[l + 1 + k];
-        T.lv[k] = MgTailLevel{mg_grid(c.grid), (int)c.n, c.diag, mg->coef + (int64_t)(l + 1 + k) * 2 * DFEA_MG_MAX_DEGREE,
-                              c.b, c.x, c.r, c.d, c.q};
+        const int n_nodes = (int)(c.n / 2), nb = (n_nodes + size - 1) / size;
+        T.lv[k] = MgTailLevel{level_grid(mg, l + 1 + k), n_nodes, nb, at, c.diag, mg->coef + (int64_t)(l + 1 + k) * 2 * DFEA_MG_MAX_DEGREE};
+        at += (6 * 16 + 36 * 8) * nb;
     }
-    k_mg_tail<<<1, kMgTailThreads, 0, s>>>(T);
+    const int rc = launch_clusters<k_mg_tail>(1, size, at, s, T);
+    if (rc) return rc;
     note_launches(1);
     return launch_check("dfea_mg_vcycle: coarse tail");
 }
@@ -1268,7 +1561,7 @@ static int mg_vcycle(const dfea_mesh_view* mesh, const dfea_mg* mg, const void* 
         k_mg_cheb_restart<<<grid_for(lv.n, kThreads, 8), kThreads, 0, s>>>(lv.n, b, lv.q, lv.diag, scale, lv.r, lv.d);
     } else {
         const int n_nodes = (lv.grid.gx + 1) * (lv.grid.gy + 1);
-        k_mg_residual_restart<<<grid_for(n_nodes, 256, 8), 256, 0, s>>>(mg_grid(lv.grid), b, x, lv.diag, scale, lv.r, lv.d);
+        k_mg_residual_restart<<<grid_for(n_nodes, 256, 8), 256, 0, s>>>(level_grid(mg, l), b, x, lv.diag, scale, lv.r, lv.d);
     }
     note_launches(1);
     if ((rc = launch_check("dfea_mg_vcycle: residual"))) return rc;
@@ -1375,22 +1668,33 @@ static int setup_device_part(const dfea_mesh_view* mesh, const dfea_mg* mg, cons
         rc = l == 1 ? dfea_mg_galerkin_fe(mesh, moduli, moduli_dtype, mg->node_ij, mg->cell_slot, mg->span,
                                           &mg->level[0].grid, &mg->level[1].grid, s)
                     : dfea_mg_galerkin(&mg->level[l - 1].grid, &mg->level[l].grid, s);
-        if (rc || (rc = dfea_mg_diag(&mg->level[l].grid, mg->level[l].diag, s))) return rc;
+        if (rc) return rc;
+        if (mg->stencil) {
+            k_mg_stencil<<<grid_for(9 * (mg->level[l].n / 2), 256, 8), 256, 0, s>>>(level_grid(mg, l), mg->level[l].diag);
+            note_launches(1);
+            rc = launch_check("dfea_mg_setup: stencils");
+        } else {
+            rc = dfea_mg_diag(&mg->level[l].grid, mg->level[l].diag, s);
+        }
+        if (rc) return rc;
     }
     if ((rc = dfea_mg_dense_inverse(&mg->level[L - 1].grid, mg->dense_work, mg->Ainv, s))) return rc;
     if (!lanczos) return DFEA_OK;
-    // Lanczos on every smoothed level (p in x, z in d): the small levels in one block, the others in lockstep
+    // Lanczos on every smoothed level (p in x, z in d): one cluster per small level, the others in lockstep
     const int t = tail_start(mg) < L - 1 ? tail_start(mg) : L - 1;
     if (t < L - 1) {
         MgLanczosTail T = {};
-        T.n_levels = L - 1 - t;
         T.steps = mg->lanczos_steps;
-        for (int k = 0; k < T.n_levels; ++k) {
+        T.size = mg_cluster_size(mg->level[t].n / 2);
+        int most = 0;
+        for (int k = 0; k < L - 1 - t; ++k) {
             const dfea_mg_level& lv = mg->level[t + k];
-            T.lv[k] = MgLanczosLevel{mg_grid(lv.grid), (int)lv.n, lv.diag, lv.r, lv.d, lv.x, lv.q, mg->lscal + 4 * (t + k),
+            const int n_nodes = (int)(lv.n / 2), nb = (n_nodes + T.size - 1) / T.size;
+            T.lv[k] = MgLanczosLevel{level_grid(mg, t + k), n_nodes, nb, lv.diag, mg->lscal + 4 * (t + k),
                                      mg->lhist + (int64_t)2 * mg->lanczos_steps * (t + k)};
+            most = nb > most ? nb : most;
         }
-        k_mg_tail_lanczos<<<1, kMgTailLanczosThreads, 0, s>>>(T);
+        if ((rc = launch_clusters<k_mg_tail_lanczos>(L - 1 - t, T.size, (size_t)(4 * 16 + 36 * 8) * most, s, T))) return rc;
         note_launches(1);
         if ((rc = launch_check("dfea_mg_setup: Lanczos of the small levels"))) return rc;
     }

@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "dfea_apply.cuh"
+#include "dfea_cluster.cuh"
 #include "dfea_common.cuh"
 
 namespace dfea {
@@ -447,40 +448,6 @@ k_pcg_node_fused(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __r
 // There is no spin wait: the blocks of a cluster are scheduled together and meet at hardware barriers.  The number of
 // iterations is bounded by max_iter.
 // ------------------------------------------------------------------------------------------------
-constexpr int kClusterMax = 16;
-
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// address of the same shared-memory location in block `rank` of the cluster
-__device__ __forceinline__ unsigned cluster_address(unsigned local, unsigned rank) {
-    unsigned a;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
-    return a;
-}
-// sum over the warp, the same bits in every lane
-__device__ __forceinline__ double warp_all_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ double2 cluster_load(unsigned addr) {
-    double2 v;
-    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ void cluster_store(unsigned addr, double2 v) {
-    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.x), "d"(v.y) : "memory");
-}
-__device__ __forceinline__ void cluster_store(unsigned addr, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
-}
-
 // Shared memory of a block (byte offsets; the same in every block).  Nodes are divided in ranges of nb.
 struct ClusterLayout {
     int nb;                                         // nodes per block
@@ -581,32 +548,8 @@ k_pcg_cluster(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const
     const unsigned smem0 = (unsigned)__cvta_generic_to_shared(cluster_smem);
     const unsigned rank = cluster_rank();
     const int size = gridDim.x;  // the grid is the cluster
-    const int lane32 = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned turn = 0;
-
-    // sums over the cluster, the same bits in every thread; also the barrier after each pass
-    auto exchange = [&](auto two, double v0, double v1, double& t0, double& t1) {
-        constexpr bool TWO = decltype(two)::value;
-        v0 = warp_all_sum(v0);
-        if (TWO) v1 = warp_all_sum(v1);
-        double* tab = table + (turn & 1u) * 2 * kClusterMax * W;
-        const unsigned here = (unsigned)__cvta_generic_to_shared(tab + rank * W + warp);
-        if (lane32 < size) {
-            const unsigned to = cluster_address(here, lane32);
-            cluster_store(to, v0);
-            if (TWO) cluster_store(to + kClusterMax * W * 8, v1);
-        }
-        ++turn;
-        __syncwarp();
-        cluster_barrier();
-        double a0 = 0.0, a1 = 0.0;
-        for (int i = lane32; i < size * W; i += 32) {
-            a0 += tab[i];
-            if (TWO) a1 += tab[kClusterMax * W + i];
-        }
-        t0 = warp_all_sum(a0);
-        if (TWO) t1 = warp_all_sum(a1);
-    };
+    const int lane32 = threadIdx.x & 31;
+    ClusterExchange<W> sums(table, rank, size);
 
     const int64_t node0 = (int64_t)rank * L.nb;
     const int n_own = (int)(node0 >= m.n_nodes ? 0 : (m.n_nodes - node0 < L.nb ? m.n_nodes - node0 : L.nb));
@@ -642,7 +585,7 @@ k_pcg_cluster(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const
     int status = DFEA_PCG_RUNNING, iters = 0;
     double rr = 0.0, curv = 0.0, beta = 0.0;
     cluster_barrier();  // every block has started: its shared memory may be written from here on
-    exchange(std::true_type{}, rz, bb, rz, bb);
+    sums.two(rz, bb, rz, bb);
     const double norm_b = sqrt(bb);
     if (norm_b == 0.0) status = DFEA_PCG_ZERO_RHS;
 
@@ -786,8 +729,7 @@ k_pcg_cluster(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const
                 if (fix & 2) c += py * py;
             }
         }
-        double unused;
-        exchange(std::false_type{}, c, 0.0, curv, unused);
+        curv = sums.one(c);
         if (curv <= 0.0) {
             // not SPD along p: return z at k = 0 and x otherwise (newton_krylov.py:69-70)
             if (k == 0)
@@ -831,7 +773,7 @@ k_pcg_cluster(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const
             s_rz += rn.x * zw.x + rn.y * zw.y;
         }
         double rz_new;
-        exchange(std::true_type{}, s_rr, s_rz, rr, rz_new);
+        sums.two(s_rr, s_rz, rr, rz_new);
         beta = rz_new / rz;  // beside the square root: both chains are long
         if (sqrt(rr) <= rtol * norm_b) {  // newton_krylov.py:77-79
             iters = k + 1;

@@ -242,6 +242,7 @@ class Multigrid:
                 fa.add((l, name), lv.n)
             if l > 0:
                 fa.add((l, "K"), 64 * lv.gx * lv.gy)
+        fa.add("stencil", 36 * sum(lv.n_nodes for lv in self.levels[1:]))
         self._f64 = torch.empty(fa.size, dtype=torch.float64, device=dev)
         self._f64[:zero_end].zero_()
         ba = _Arena(1)
@@ -266,7 +267,7 @@ class Multigrid:
             dst.n = lv.n
             for name in ("diag", "b", "x", "r", "d", "q"):
                 setattr(dst, name, fptr((l, name)))
-        for name in ("Ainv", "dense_work", "coef", "lscal", "lhist", "dot_work", "scal"):
+        for name in ("Ainv", "dense_work", "coef", "lscal", "lhist", "dot_work", "scal", "stencil"):
             setattr(h, name, fptr(name))
         h.pcg = fptr("pcg")
         h.pcg_state = fptr("pcg_state") if graphs else None

@@ -151,7 +151,8 @@ def hbm_estimate(req, precision="fp32", preconditioner="jacobi"):
         # the grid inference's int64 temporaries (connectivity built per candidate numbering, grid maps)
         per_el += 8 * nen + 96
         per_node += 96
-        return int(1.1 * (E * per_el + N * per_node + cells1 * 512 * 4 / 3) + 4 * 2 ** 20)
+        # + the node stencils of the coarse levels, 288 B per node
+        return int(1.1 * (E * per_el + N * per_node + cells1 * (512 + 288) * 4 / 3) + 4 * 2 ** 20)
     return int(E * per_el + N * per_node + 4 * 2 ** 20)  # + reduction scratch and PCG state
 
 

@@ -513,6 +513,11 @@ typedef struct dfea_mg {
      * its node incidence, every level-0 product of the hierarchy runs in the gather form (an element pass and
      * the node sums: 2 launches) instead of one launch per colour; NULL: the colour form. */
     void* fe_work;
+    /* Optional: 36 doubles per node of every coarse level (levels 1 .. n_levels - 1, one after the other), where the
+     * set-up keeps the operators as node stencils; with it the coarse products read 288 B per node and the small
+     * levels of a cycle and of the Lanczos estimates run in thread-block clusters.  NULL: products from the element
+     * matrices, a launch per step. */
+    double* stencil;
 } dfea_mg;
 
 /* Set-up at a linearisation: coarse operators from the moduli, coarsest inverse, Lanczos estimates,
