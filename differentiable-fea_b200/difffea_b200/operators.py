@@ -149,6 +149,8 @@ def make_A_operator_cuda(u, theta, params, precision="fp64"):
     mesh, mid = _prepare(u, theta, params)
     if precision == "fp32":
         mesh.ensure_grad32()
+        if mesh.nen * mesh.stride < 2 ** 31:
+            mesh.ensure_node_incidence()
     if precision == "fp64" and mesh.ensure_frame():
         C, diag, _ = ops.frame_moduli(mid, _f64c(u), _f64c(theta), *ops.frame_material(params), True, False)
     else:

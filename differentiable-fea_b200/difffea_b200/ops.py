@@ -140,6 +140,10 @@ def tangent_apply(mesh_id: int, C: torch.Tensor, v: torch.Tensor) -> torch.Tenso
         return y
     dt = _lib.DFEA_F32 if fp32 else _lib.DFEA_F64
     cdt = _lib.DFEA_F32 if C.dtype == torch.float32 else _lib.DFEA_F64
+    if mesh.node_elem is not None and mesh.n_el < mesh.GATHER_MAX_ELEMENTS:
+        fe = torch.empty(int(_lib.load().dfea_gather_work_bytes(mesh.view_ref, dt)), dtype=torch.uint8, device=mesh.device)
+        _lib.call("dfea_tangent_apply_gather", mesh.view_ref, ptr(C), cdt, ptr(v), ptr(y), dt, ptr(fe), stream_handle())
+        return y
     _lib.call("dfea_tangent_apply", mesh.view_ref, ptr(C), cdt, ptr(v), ptr(y), dt, stream_handle())
     return y
 
