@@ -360,6 +360,29 @@ k_frame_residual(Mesh m, const double* __restrict__ frame, RefGrad<NEN, NQ> rg, 
     }
 }
 
+// The internal force summed over the fixed DOFs (support reactions), without storing it
+__global__ void __launch_bounds__(kThreads)
+k_frame_node_reactions(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
+                       const double* __restrict__ fe, const uint8_t* __restrict__ fixed, RedSite site, double* __restrict__ out) {
+    grid_dependency_wait();
+    grid_dependents_launch();
+    const double2* fe2 = reinterpret_cast<const double2*>(fe);
+    double rx = 0.0, ry = 0.0;
+    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < m.n_nodes; n += (int64_t)gridDim.x * blockDim.x) {
+        const bool fx = fixed[2 * n], fy = fixed[2 * n + 1];
+        if (!fx && !fy) continue;
+        const double2 s = node_sum<double>(inc_ptr, inc, fe2, n);
+        if (fx) rx += s.x;
+        if (fy) ry += s.y;
+    }
+    const double vals[2] = {block_sum<kThreads>(rx), block_sum<kThreads>(ry)};
+    double tot[2];
+    if (last_block_sum<kThreads, 2>(vals, site, tot) && threadIdx.x == 0) {
+        out[0] = tot[0];
+        out[1] = tot[1];
+    }
+}
+
 // MASK: R = m (sum - lf f); else the unmasked sum.  NORM: |R|^2 into out_norm2 and the energy partials of the
 // element pass (n_part of them) into out_energy by the last block.
 template <bool MASK, bool NORM>
@@ -480,8 +503,9 @@ k_frame_sensitivity(Mesh m, const double* __restrict__ frame, RefGrad<NEN, NQ> r
 template <int NEN, int NQ, bool GEN>
 __global__ void __launch_bounds__(FrameCfg<NEN, NQ>::NT, GEN ? 1 : FrameCfg<NEN, NQ>::MINB)
 k_frame_fields(Mesh m, const double* __restrict__ frame, RefGrad<NEN, NQ> rg, const double* __restrict__ u,
-               const double* __restrict__ theta, MatArg mat, double* __restrict__ out) {
-    constexpr int EB = FrameCfg<NEN, NQ>::EB;
+               const double* __restrict__ theta, MatArg mat, double* __restrict__ out, double* __restrict__ part) {
+    constexpr int EB = FrameCfg<NEN, NQ>::EB, NT = FrameCfg<NEN, NQ>::NT;
+    double energy = 0.0, min_J = INFINITY;  // of this block's elements: sum of psi area, smallest mean J (a NaN wins)
     __shared__ double2 us[NEN][EB];
     __shared__ double red[NQ][7][EB];
     const int lane = threadIdx.x % EB, q = threadIdx.x / EB;
@@ -560,8 +584,66 @@ k_frame_fields(Mesh m, const double* __restrict__ frame, RefGrad<NEN, NQ> rg, co
             out[4 * n_el + oe] = c;
             out[5 * n_el + oe] = mises;
             out[6 * n_el + oe] = mpsi;
+            energy += mpsi * area;
+            if (mJ < min_J || mJ != mJ) min_J = (min_J != min_J) ? min_J : mJ;
         }
         __syncthreads();
+    }
+    if (part != nullptr) {
+        const double E = block_sum<NT>(energy);
+        __shared__ double mins[NT / 32];
+        auto take = [](double a, double b) { return (b < a || b != b) ? ((a != a) ? a : b) : a; };
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) min_J = take(min_J, __shfl_down_sync(0xffffffffu, min_J, o));
+        if ((threadIdx.x & 31) == 0) mins[threadIdx.x >> 5] = min_J;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < NT / 32; ++w) min_J = take(min_J, mins[w]);
+            part[blockIdx.x] = E;
+            part[kMaxBlocks + blockIdx.x] = min_J;
+        }
+    }
+}
+
+// nodal post-processing: the means of the six element rows over a node's elements (incidence order) and |u|, rows
+// 0 .. 6 of out; block 0 adds the element pass's energy partials and takes its smallest J
+__global__ void __launch_bounds__(kThreads)
+k_frame_node_fields(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
+                    const double* __restrict__ elem, const double* __restrict__ u, double* __restrict__ out,
+                    const double* __restrict__ part, int n_part, double* __restrict__ scal) {
+    grid_dependency_wait();
+    grid_dependents_launch();
+    const int64_t S = m.stride, n_el = m.n_el, N = m.n_nodes;
+    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x) {
+        double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        const int j0 = inc_ptr[n], j1 = inc_ptr[n + 1];
+        for (int j = j0; j < j1; ++j) {
+            const int64_t oe = m.orig[inc[j] % S];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) acc[k] += elem[(k + 1) * n_el + oe];
+        }
+        const double cnt = (j1 > j0) ? (double)(j1 - j0) : 1.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) out[k * N + n] = acc[k] / cnt;
+        const double2 un = reinterpret_cast<const double2*>(u)[n];
+        out[6 * N + n] = sqrt(un.x * un.x + un.y * un.y);
+    }
+    if (blockIdx.x == 0) {
+        double E = 0.0, low = INFINITY;
+        auto take = [](double a, double b) { return (b < a || b != b) ? ((a != a) ? a : b) : a; };
+        for (int i = threadIdx.x; i < n_part; i += kThreads) {
+            E += part[i];
+            low = take(low, part[kMaxBlocks + i]);
+        }
+        E = block_sum<kThreads>(E);
+        __shared__ double lows[kThreads];
+        lows[threadIdx.x] = low;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int i = 1; i < kThreads; ++i) low = take(low, lows[i]);
+            scal[0] = E;
+            scal[1] = low;
+        }
     }
 }
 
@@ -607,7 +689,7 @@ struct FrameWork {
     unsigned* ticket;
     static int64_t up(int64_t x) { return (x + 255) / 256 * 256; }
     static int64_t bytes(const dfea_mesh_view& v) {
-        return up((int64_t)v.nen * v.stride * 16) + up((int64_t)v.nen * v.stride * 8) + 2 * kMaxBlocks * 8 + 256;
+        return up((int64_t)v.nen * v.stride * 16) + up((int64_t)v.nen * v.stride * 8) + 3 * kMaxBlocks * 8 + 256;
     }
     FrameWork(const dfea_mesh_view& v, void* base) {
         char* p = static_cast<char*>(base);
@@ -617,7 +699,7 @@ struct FrameWork {
         p += up((int64_t)v.nen * v.stride * 8);
         part = reinterpret_cast<double*>(p);
         norm_part = part + kMaxBlocks;
-        ticket = reinterpret_cast<unsigned*>(norm_part + kMaxBlocks);
+        ticket = reinterpret_cast<unsigned*>(norm_part + 2 * kMaxBlocks);
     }
 };
 
@@ -732,7 +814,7 @@ extern "C" int dfea_frame_moduli(const dfea_mesh_view* mesh, const double* u, co
 // the element pass of the residual and the node pass that follows it
 static int frame_residual(const dfea_mesh_view* mesh, const double* u, const double* theta, const MatArg& mat,
                           const double* f, double lf, double* R, double* out_norm2, double* out_energy, void* work,
-                          bool mask, cudaStream_t s) {
+                          bool mask, cudaStream_t s, const uint8_t* fixed = nullptr, double* reactions = nullptr) {
     const Mesh m = kernel_mesh(*mesh);
     FrameWork w(*mesh, work);
     int n_part = 0;
@@ -756,7 +838,10 @@ static int frame_residual(const dfea_mesh_view* mesh, const double* u, const dou
     pdl.pdl = true;
     const dim3 grid(grid_for(mesh->n_nodes, kThreads, 4));
     const RedSite site{w.norm_part, w.ticket, nullptr};
-    if (!mask)
+    if (reactions)
+        rc = launch_kernel(k_frame_node_reactions, grid, dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr, mesh->node_elem,
+                           (const double*)w.fe, fixed, site, reactions);
+    else if (!mask)
         rc = launch_kernel(k_frame_node_residual<false, false>, grid, dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr,
                            mesh->node_elem, (const double*)w.fe, f, lf, R, site, out_norm2, (const double*)w.part, n_part, out_energy);
     else if (out_norm2 || out_energy)
@@ -798,6 +883,19 @@ extern "C" int dfea_frame_internal_force(const dfea_mesh_view* mesh, const doubl
                           static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int dfea_frame_reactions(const dfea_mesh_view* mesh, const double* u, const double* theta,
+                                    const dfea_material* material, const double* mat_p, const uint8_t* mat_scalable,
+                                    const uint8_t* fixed, double* reactions, void* work, void* stream) {
+    int rc = validate_frame(mesh, "dfea_frame_reactions");
+    MatArg mat;
+    if (rc || (rc = validate_frame_material(material, mat_p, mat_scalable, &mat, "dfea_frame_reactions"))) return rc;
+    if (!u || !fixed || !reactions || !work || !mesh->node_elem_ptr || !mesh->node_elem)
+        return set_error(DFEA_ERR_INVALID, "dfea_frame_reactions: NULL pointer or no node incidence");
+    if (!al16(u) || !al16(work)) return set_error(DFEA_ERR_INVALID, "dfea_frame_reactions: alignment");
+    return frame_residual(mesh, u, theta, mat, nullptr, 0.0, nullptr, nullptr, nullptr, work, false,
+                          static_cast<cudaStream_t>(stream), fixed, reactions);
+}
+
 extern "C" int dfea_frame_sensitivity(const dfea_mesh_view* mesh, const double* u, const double* lam,
                                       const dfea_material* material, const double* mat_p, const uint8_t* mat_scalable,
                                       double* g, void* stream) {
@@ -835,27 +933,54 @@ extern "C" int dfea_frame_sensitivity(const dfea_mesh_view* mesh, const double* 
     return launch_check("dfea_frame_sensitivity");
 }
 
-extern "C" int dfea_frame_fields(const dfea_mesh_view* mesh, const double* u, const double* theta,
-                                 const dfea_material* material, const double* mat_p, const uint8_t* mat_scalable,
-                                 double* elem_out, void* stream) {
-    int rc = validate_frame(mesh, "dfea_frame_fields");
-    MatArg mat;
-    if (rc || (rc = validate_frame_material(material, mat_p, mat_scalable, &mat, "dfea_frame_fields"))) return rc;
-    if (!u || !elem_out) return set_error(DFEA_ERR_INVALID, "dfea_frame_fields: NULL pointer");
-    if (!al16(u)) return set_error(DFEA_ERR_INVALID, "dfea_frame_fields: u must be 16-byte aligned");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    rc = dispatch_element(mesh->nen, mesh->n_q, [&](auto nen_c, auto nq_c) -> int {
+static int frame_fields(const dfea_mesh_view* mesh, const double* u, const double* theta, const MatArg& mat,
+                        double* elem_out, double* part, int* n_part, cudaStream_t s) {
+    const int rc = dispatch_element(mesh->nen, mesh->n_q, [&](auto nen_c, auto nq_c) -> int {
         constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
         return dispatch_gen(mat.m.model, [&](auto gen_c) -> int {
             constexpr bool GEN = decltype(gen_c)::value;
-            k_frame_fields<NEN, NQ, GEN><<<frame_grid<NEN, NQ>(mesh->n_el), FrameCfg<NEN, NQ>::NT, 0, s>>>(
-                kernel_mesh(*mesh), mesh->frame, ref_grad_of<NEN, NQ>(*mesh), u, theta, mat, elem_out);
+            const int grid = *n_part = frame_grid<NEN, NQ>(mesh->n_el);
+            k_frame_fields<NEN, NQ, GEN><<<grid, FrameCfg<NEN, NQ>::NT, 0, s>>>(
+                kernel_mesh(*mesh), mesh->frame, ref_grad_of<NEN, NQ>(*mesh), u, theta, mat, elem_out, part);
             return DFEA_OK;
         });
     });
     if (rc) return rc;
     note_launches(1);
-    return launch_check("dfea_frame_fields");
+    return launch_check("frame fields");
+}
+
+extern "C" int dfea_frame_fields(const dfea_mesh_view* mesh, const double* u, const double* theta,
+                                 const dfea_material* material, const double* mat_p, const uint8_t* mat_scalable,
+                                 double* elem_out, void* stream) {
+    int rc = validate_frame(mesh, "dfea_frame_fields"), n_part;
+    MatArg mat;
+    if (rc || (rc = validate_frame_material(material, mat_p, mat_scalable, &mat, "dfea_frame_fields"))) return rc;
+    if (!u || !elem_out) return set_error(DFEA_ERR_INVALID, "dfea_frame_fields: NULL pointer");
+    if (!al16(u)) return set_error(DFEA_ERR_INVALID, "dfea_frame_fields: u must be 16-byte aligned");
+    return frame_fields(mesh, u, theta, mat, elem_out, nullptr, &n_part, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int dfea_frame_all_fields(const dfea_mesh_view* mesh, const double* u, const double* theta,
+                                     const dfea_material* material, const double* mat_p, const uint8_t* mat_scalable,
+                                     double* elem_out, double* node_out, double* scal_out, void* work, void* stream) {
+    int rc = validate_frame(mesh, "dfea_frame_all_fields"), n_part = 0;
+    MatArg mat;
+    if (rc || (rc = validate_frame_material(material, mat_p, mat_scalable, &mat, "dfea_frame_all_fields"))) return rc;
+    if (!u || !elem_out || !node_out || !scal_out || !work || !mesh->node_elem_ptr || !mesh->node_elem)
+        return set_error(DFEA_ERR_INVALID, "dfea_frame_all_fields: NULL pointer or no node incidence");
+    if (!al16(u) || !al16(work)) return set_error(DFEA_ERR_INVALID, "dfea_frame_all_fields: alignment");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    FrameWork w(*mesh, work);
+    if ((rc = frame_fields(mesh, u, theta, mat, elem_out, w.part, &n_part, s))) return rc;
+    LaunchOpts pdl;
+    pdl.pdl = true;
+    if ((rc = launch_kernel(k_frame_node_fields, dim3(grid_for(mesh->n_nodes, kThreads, 8)), dim3(kThreads), 0, s, pdl,
+                            kernel_mesh(*mesh), mesh->node_elem_ptr, mesh->node_elem, (const double*)elem_out, u, node_out,
+                            (const double*)w.part, n_part, scal_out)))
+        return rc;
+    note_launches(1);
+    return launch_check("dfea_frame_all_fields");
 }
 
 extern "C" int dfea_frame_push_forward(const dfea_mesh_view* mesh, const double* moduli_ref, double* moduli, void* stream) {

@@ -150,6 +150,10 @@ _PROTOS = {
                                               c_vp, c_vp]),
     "dfea_frame_fields": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, ctypes.POINTER(Material), c_vp, c_vp, c_vp,
                                          c_vp]),
+    "dfea_frame_all_fields": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, ctypes.POINTER(Material), c_vp, c_vp,
+                                             c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "dfea_frame_reactions": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, ctypes.POINTER(Material), c_vp, c_vp,
+                                            c_vp, c_vp, c_vp, c_vp]),
     "dfea_frame_push_forward": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_vp, c_vp]),
     "dfea_gather_work_bytes": (c_i64, [ctypes.POINTER(MeshView), c_i32]),
     "dfea_tangent_apply_gather": (ctypes.c_int, [ctypes.POINTER(MeshView), c_vp, c_i32, c_vp, c_vp, c_i32, c_vp,

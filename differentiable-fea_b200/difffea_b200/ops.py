@@ -20,6 +20,7 @@ Each op is a thin shim: it allocates its outputs through torch's caching allocat
                                         pcg_max_iter) -> (u, [converged, load factor, Newton, CG, cut-backs])
 the same on a mesh with a frame (CudaMesh.ensure_frame), in one element pass and one node pass:
     torch.ops.difffea_b200.frame_moduli / frame_residual / frame_internal_force / frame_sensitivity / frame_fields
+    torch.ops.difffea_b200.frame_all_fields / frame_reactions (compute_fields and support_reactions whole)
     torch.ops.difffea_b200.frame_push_forward(mesh_id, C) -> physical moduli
     torch.ops.difffea_b200.frame_residual_out / frame_moduli_out (caller buffers)
 and three forms that write into caller buffers, for the solver's preallocated workspace:
@@ -376,6 +377,44 @@ def frame_fields(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int,
 @frame_fields.register_fake
 def _(mesh_id, u, theta, model, scalable, mat_p, p_dev, s_dev):
     return u.new_empty(7, _mesh(mesh_id).n_el)
+
+
+@torch.library.custom_op("difffea_b200::frame_all_fields", mutates_args=(), device_types="cuda")
+def frame_all_fields(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int, mat_p: list[float],
+                     p_dev: Optional[torch.Tensor],
+                     s_dev: Optional[torch.Tensor]) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """Element rows (7, n_el), nodal rows (7, N; the last is |u|) and (strain energy, smallest J)."""
+    mesh = _frame_mesh(mesh_id, u, theta)
+    f64 = dict(dtype=torch.float64, device=mesh.device)
+    el, nodal, scal = torch.empty(7, mesh.n_el, **f64), torch.empty(7, mesh.n_nodes, **f64), torch.empty(2, **f64)
+    _lib.call("dfea_frame_all_fields", mesh.view_ref, ptr(u), ptr(theta),
+              *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev), ptr(el), ptr(nodal), ptr(scal),
+              ptr(mesh.frame_work()), stream_handle())
+    return el, nodal, scal
+
+
+@frame_all_fields.register_fake
+def _(mesh_id, u, theta, model, scalable, mat_p, p_dev, s_dev):
+    mesh = _mesh(mesh_id)
+    return u.new_empty(7, mesh.n_el), u.new_empty(7, mesh.n_nodes), u.new_empty(2)
+
+
+@torch.library.custom_op("difffea_b200::frame_reactions", mutates_args=(), device_types="cuda")
+def frame_reactions(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int, scalable: int, mat_p: list[float],
+                    p_dev: Optional[torch.Tensor], s_dev: Optional[torch.Tensor], fixed: torch.Tensor) -> torch.Tensor:
+    mesh = _frame_mesh(mesh_id, u, theta)
+    if fixed.dtype != torch.bool or fixed.numel() != mesh.n_dof or not fixed.is_contiguous() or fixed.device != mesh.device:
+        raise ValueError("fixed must be the contiguous (2N,) bool flags on the mesh's device")
+    out = torch.empty(2, dtype=torch.float64, device=mesh.device)
+    _lib.call("dfea_frame_reactions", mesh.view_ref, ptr(u), ptr(theta),
+              *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev), ptr(fixed), ptr(out), ptr(mesh.frame_work()),
+              stream_handle())
+    return out
+
+
+@frame_reactions.register_fake
+def _(mesh_id, u, theta, model, scalable, mat_p, p_dev, s_dev, fixed):
+    return u.new_empty(2)
 
 
 @torch.library.custom_op("difffea_b200::frame_push_forward", mutates_args=(), device_types="cuda")

@@ -37,12 +37,16 @@ def compute_fields(u, theta, params) -> dict:
         scalars (0-d):        strain_energy, min_J
     """
     mesh, mid = _prepare(u, theta, params)
-    el = element_fields(u, theta, params)
-    nodal = torch.ops.difffea_b200.node_fields(mid, el)
     un = _f64c(u).view(mesh.n_nodes, 2)
+    if mesh.ensure_frame() and mesh.n_el:
+        el, nodal, scal = ops.frame_all_fields(mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
+        u_mag, energy, min_J = nodal[6], scal[0], scal[1]
+    else:
+        el = element_fields(u, theta, params)
+        nodal = torch.ops.difffea_b200.node_fields(mid, el)
+        u_mag, energy, min_J = torch.linalg.norm(un, dim=1), torch.sum(el[6] * el[0]), el[1].min()
     out = {name: el[k + 1] for k, name in enumerate(ELEMENT_FIELDS)}
-    out.update(ux=un[:, 0], uy=un[:, 1], u_mag=torch.linalg.norm(un, dim=1),
-               strain_energy=torch.sum(el[6] * el[0]), min_J=el[1].min())
+    out.update(ux=un[:, 0], uy=un[:, 1], u_mag=u_mag, strain_energy=energy, min_J=min_J)
     for name in ("ux", "uy", "u_mag"):
         out[name + "_n"] = out[name]
     for k, name in enumerate(ELEMENT_FIELDS):
@@ -60,6 +64,10 @@ def internal_force(u, theta, params):
 
 def support_reactions(u, theta, params) -> torch.Tensor:
     """Total reaction (Rx, Ry) at the constrained DOFs; sum(reactions) + sum(applied loads) = 0 at equilibrium."""
+    mesh, mid = _prepare(u, theta, params)
+    if mesh.ensure_frame() and params["fixed"].numel() == mesh.n_dof:
+        fixed = params["fixed"].to(mesh.device, torch.bool).reshape(-1).contiguous()
+        return ops.frame_reactions(mid, _f64c(u), _f64c(theta), *ops.frame_material(params), fixed)
     R = internal_force(u, theta, params).view(-1, 2)
     fixed = params["fixed"].to(R.device).reshape(-1, 2).bool()
     return torch.sum(torch.where(fixed, R, torch.zeros_like(R)), dim=0)

@@ -354,6 +354,9 @@ int dfea_vec_norm2(const dfea_mesh_view* mesh, const double* x, double* out, voi
  *   dfea_frame_sensitivity     dfea_element_sensitivity_mat (parameters on the device: only models all of whose
  *                              parameters enter the energy as prefactors)
  *   dfea_frame_fields          dfea_element_fields_mat
+ *   dfea_frame_all_fields      dfea_frame_fields, then node_out: 7 rows of n_nodes doubles (dfea_node_fields' 6 and
+ *                              |u|), and scal_out: the strain energy (sum of psi x area) and the smallest mean J
+ *   dfea_frame_reactions       the internal force summed over the DOFs with fixed != 0 (2N bytes): (Rx, Ry)
  *   dfea_frame_push_forward    DFEA_F64 moduli from DFEA_F64REF ones
  */
 int64_t dfea_frame_work_bytes(const dfea_mesh_view* mesh);
@@ -370,6 +373,12 @@ int dfea_frame_sensitivity(const dfea_mesh_view* mesh, const double* u, const do
                            const double* mat_p, const uint8_t* mat_scalable, double* g, void* stream);
 int dfea_frame_fields(const dfea_mesh_view* mesh, const double* u, const double* theta, const dfea_material* material,
                       const double* mat_p, const uint8_t* mat_scalable, double* elem_out, void* stream);
+int dfea_frame_all_fields(const dfea_mesh_view* mesh, const double* u, const double* theta, const dfea_material* material,
+                          const double* mat_p, const uint8_t* mat_scalable, double* elem_out, double* node_out,
+                          double* scal_out, void* work, void* stream);
+int dfea_frame_reactions(const dfea_mesh_view* mesh, const double* u, const double* theta, const dfea_material* material,
+                         const double* mat_p, const uint8_t* mat_scalable, const uint8_t* fixed, double* reactions,
+                         void* work, void* stream);
 int dfea_frame_push_forward(const dfea_mesh_view* mesh, const double* moduli_ref, double* moduli, void* stream);
 
 /* ---------------------------------------------------------------- kernel (d) ------------------ */
