@@ -236,7 +236,7 @@ __device__ __forceinline__ bool apply_tiles(const Mesh& m, int64_t e0, int64_t e
 template <int NEN, int NQ, typename SD, typename T, bool DOT>
 __global__ void __launch_bounds__(128)
 k_apply(Mesh m, int64_t e0, int64_t e1, const SD* __restrict__ C, const SD* __restrict__ G,
-        const T* __restrict__ v, T* __restrict__ y, RedSite site, const int* __restrict__ done) {
+        const T* v, T* __restrict__ y, RedSite site, const int* __restrict__ done) {
     using T2 = v2_t<T>;
     extern __shared__ __align__(16) unsigned char smem[];
     T2* y2 = reinterpret_cast<T2*>(y);
@@ -251,7 +251,7 @@ k_apply(Mesh m, int64_t e0, int64_t e1, const SD* __restrict__ C, const SD* __re
             grid_dependents_launch();
             return true;
         },
-        [&](int n) { return __ldg(v2 + n); },
+        [&](int n) { return load_fresh(v2 + n); },
         [&](int64_t, const int (&node)[NEN], const int (&fix)[NEN], const T (&fx)[NEN], const T (&fy)[NEN]) {
 #pragma unroll
             for (int a = 0; a < NEN; ++a) {
@@ -276,7 +276,7 @@ k_apply(Mesh m, int64_t e0, int64_t e1, const SD* __restrict__ C, const SD* __re
 // into site.result[0].
 template <int NEN, int NQ, typename SD, typename T, bool DOT>
 __global__ void __launch_bounds__(128)
-k_apply_elem(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, const T* __restrict__ v,
+k_apply_elem(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, const T* v,
              T* __restrict__ fe, RedSite site, const int* __restrict__ done) {
     using T2 = v2_t<T>;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -292,7 +292,7 @@ k_apply_elem(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, const T
             grid_dependents_launch();
             return true;
         },
-        [&](int n) { return __ldg(v2 + n); },
+        [&](int n) { return load_fresh(v2 + n); },
         [&](int64_t e, const int (&)[NEN], const int (&)[NEN], const T (&fx)[NEN], const T (&fy)[NEN]) {
 #pragma unroll
             for (int a = 0; a < NEN; ++a) fe2[(int64_t)a * S + e] = make_v2<T>(fx[a], fy[a]);
@@ -315,12 +315,13 @@ __device__ __forceinline__ v2_t<T> node_sum(const int32_t* __restrict__ inc_ptr,
     int j = inc_ptr[n];
     const int j1 = inc_ptr[n + 1];
     for (; j + 4 <= j1; j += 4) {  // four loads in flight, added in order
-        const v2_t<T> f0 = fe2[inc[j]], f1 = fe2[inc[j + 1]], f2 = fe2[inc[j + 2]], f3 = fe2[inc[j + 3]];
+        const v2_t<T> f0 = load_fresh(fe2 + inc[j]), f1 = load_fresh(fe2 + inc[j + 1]);
+        const v2_t<T> f2 = load_fresh(fe2 + inc[j + 2]), f3 = load_fresh(fe2 + inc[j + 3]);
         sx = sx + f0.x + f1.x + f2.x + f3.x;
         sy = sy + f0.y + f1.y + f2.y + f3.y;
     }
     for (; j < j1; ++j) {
-        const v2_t<T> f = fe2[inc[j]];
+        const v2_t<T> f = load_fresh(fe2 + inc[j]);
         sx += f.x;
         sy += f.y;
     }
@@ -330,8 +331,8 @@ __device__ __forceinline__ v2_t<T> node_sum(const int32_t* __restrict__ inc_ptr,
 // Gather form, node pass of a plain product: y = (1 - m) v + m * sum of the element results.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_node_gather(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, const T* __restrict__ fe,
-              const T* __restrict__ v, T* __restrict__ y) {
+k_node_gather(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, const T* fe,
+              const T* v, T* __restrict__ y) {
     using T2 = v2_t<T>;
     grid_dependency_wait();
     grid_dependents_launch();
@@ -485,7 +486,7 @@ __device__ __forceinline__ bool apply_tiles_ref(const Mesh& m, int64_t e0, int64
 template <int NEN, int NQ, typename T, bool DOT>
 __global__ void __launch_bounds__(128)
 k_apply_ref(Mesh m, int64_t e0, int64_t e1, const float* __restrict__ C, const RefGrad<NEN, NQ> rg,
-            const T* __restrict__ v, T* __restrict__ y, RedSite site, const int* __restrict__ done) {
+            const T* v, T* __restrict__ y, RedSite site, const int* __restrict__ done) {
     using T2 = v2_t<T>;
     extern __shared__ __align__(16) unsigned char smem[];
     T2* y2 = reinterpret_cast<T2*>(y);
@@ -499,7 +500,7 @@ k_apply_ref(Mesh m, int64_t e0, int64_t e1, const float* __restrict__ C, const R
             grid_dependents_launch();
             return true;
         },
-        [&](int n) { return __ldg(v2 + n); },
+        [&](int n) { return load_fresh(v2 + n); },
         [&](int64_t, const int (&node)[NEN], const int (&fix)[NEN], const T (&fx)[NEN], const T (&fy)[NEN]) {
 #pragma unroll
             for (int a = 0; a < NEN; ++a) {
@@ -521,7 +522,7 @@ k_apply_ref(Mesh m, int64_t e0, int64_t e1, const float* __restrict__ C, const R
 // walk: one warp per Gauss point, results into fe[a][e].
 template <int NEN, int NQ, typename SD, typename T, bool DOT>
 __global__ void __launch_bounds__(FrameCfg<NEN, NQ>::NT, FrameCfg<NEN, NQ>::MINB)
-k_apply_ref_elem(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const T* __restrict__ v,
+k_apply_ref_elem(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const T* v,
                  T* __restrict__ fe, RedSite site, const int* __restrict__ done) {
     using T2 = v2_t<T>;
     constexpr int NT = FrameCfg<NEN, NQ>::NT;
@@ -538,7 +539,7 @@ k_apply_ref_elem(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, co
             grid_dependents_launch();
             return true;
         },
-        [&](int n) { return __ldg(v2 + n); },
+        [&](int n) { return load_fresh(v2 + n); },
         [&](int a, int64_t e, T2 f) { fe2[(int64_t)a * S + e] = f; }, blockIdx.x, gridDim.x);
     if (!ran) return;
     if (DOT) {

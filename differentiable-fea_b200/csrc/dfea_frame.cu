@@ -266,7 +266,7 @@ k_frame_moduli(Mesh m, const double* __restrict__ frame, RefGrad<NEN, NQ> rg, co
 // (B = M B_K M + (I - M) + 1e-12 I) as (Binv00, Binv01, Binv11, 0)
 __global__ void __launch_bounds__(kThreads)
 k_frame_node_diag(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
-                  const double* __restrict__ fe, const double* __restrict__ fb, double* __restrict__ diag,
+                  const double* fe, const double* fb, double* __restrict__ diag,
                   double* __restrict__ blocks) {
     grid_dependency_wait();
     grid_dependents_launch();
@@ -276,7 +276,7 @@ k_frame_node_diag(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __
         const double2 d = node_sum<double>(inc_ptr, inc, fe2, n);
         if (blocks != nullptr) {
             double c = 0.0;
-            for (int j = inc_ptr[n]; j < inc_ptr[n + 1]; ++j) c += fb[inc[j]];
+            for (int j = inc_ptr[n]; j < inc_ptr[n + 1]; ++j) c += load_fresh(fb + inc[j]);
             const bool fx = fix & 1, fy = fix & 2;
             const double a00 = (fx ? 1.0 : d.x) + 1e-12, a11 = (fy ? 1.0 : d.y) + 1e-12;
             const double a01 = (fx || fy) ? 0.0 : c;
@@ -363,7 +363,7 @@ k_frame_residual(Mesh m, const double* __restrict__ frame, RefGrad<NEN, NQ> rg, 
 // The internal force summed over the fixed DOFs (support reactions), without storing it
 __global__ void __launch_bounds__(kThreads)
 k_frame_node_reactions(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
-                       const double* __restrict__ fe, const uint8_t* __restrict__ fixed, RedSite site, double* __restrict__ out) {
+                       const double* fe, const uint8_t* __restrict__ fixed, RedSite site, double* __restrict__ out) {
     grid_dependency_wait();
     grid_dependents_launch();
     const double2* fe2 = reinterpret_cast<const double2*>(fe);
@@ -388,7 +388,7 @@ k_frame_node_reactions(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_
 template <bool MASK, bool NORM>
 __global__ void __launch_bounds__(kThreads)
 k_frame_node_residual(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
-                      const double* __restrict__ fe, const double* __restrict__ f, double lf, double* __restrict__ R,
+                      const double* fe, const double* __restrict__ f, double lf, double* __restrict__ R,
                       RedSite site, double* __restrict__ out_norm2, const double* __restrict__ part, int n_part,
                       double* __restrict__ out_energy) {
     grid_dependency_wait();
@@ -609,8 +609,8 @@ k_frame_fields(Mesh m, const double* __restrict__ frame, RefGrad<NEN, NQ> rg, co
 // 0 .. 6 of out; block 0 adds the element pass's energy partials and takes its smallest J
 __global__ void __launch_bounds__(kThreads)
 k_frame_node_fields(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
-                    const double* __restrict__ elem, const double* __restrict__ u, double* __restrict__ out,
-                    const double* __restrict__ part, int n_part, double* __restrict__ scal) {
+                    const double* elem, const double* __restrict__ u, double* __restrict__ out,
+                    const double* part, int n_part, double* __restrict__ scal) {
     grid_dependency_wait();
     grid_dependents_launch();
     const int64_t S = m.stride, n_el = m.n_el, N = m.n_nodes;
@@ -620,7 +620,7 @@ k_frame_node_fields(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* 
         for (int j = j0; j < j1; ++j) {
             const int64_t oe = m.orig[inc[j] % S];
 #pragma unroll
-            for (int k = 0; k < 6; ++k) acc[k] += elem[(k + 1) * n_el + oe];
+            for (int k = 0; k < 6; ++k) acc[k] += load_fresh(elem + (k + 1) * n_el + oe);
         }
         const double cnt = (j1 > j0) ? (double)(j1 - j0) : 1.0;
 #pragma unroll
@@ -632,8 +632,8 @@ k_frame_node_fields(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* 
         double E = 0.0, low = INFINITY;
         auto take = [](double a, double b) { return (b < a || b != b) ? ((a != a) ? a : b) : a; };
         for (int i = threadIdx.x; i < n_part; i += kThreads) {
-            E += part[i];
-            low = take(low, part[kMaxBlocks + i]);
+            E += load_fresh(part + i);
+            low = take(low, load_fresh(part + kMaxBlocks + i));
         }
         E = block_sum<kThreads>(E);
         __shared__ double lows[kThreads];

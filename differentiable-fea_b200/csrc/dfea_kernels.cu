@@ -8,6 +8,7 @@
 #include "dfea_apply.cuh"
 #include "dfea_common.cuh"
 #include "dfea_material.cuh"
+#include "dfea_mg.cuh"
 
 namespace dfea {
 
@@ -839,46 +840,156 @@ __global__ void __launch_bounds__(128) k_ref_frame(Mesh m, RefGrad<NEN, NQ> rg, 
     }
 }
 
-// Node pass of the gather-form product q = A v on the finite-element level of the multigrid V-cycle, with
-// the smoothing arithmetic that follows the product applied at the node (each node's q is complete here and
-// the element pass has finished reading v):
-//   MG_FE_STEP    (v = d): x += d, r -= q, d = c1 d + c2 r / D (d kept by the last step), coef = (c1, c2);
-//   MG_FE_RESTART (v = x): r = b - q, d = s r / D, coef = (s).
-// The expressions are those of k_node_gather followed by the multigrid's separate Chebyshev kernels, so the
-// iterates are bitwise the same.  d and v alias in MG_FE_STEP (read and written at the thread's own node).
-template <int MODE>
+// Node pass of the gather-form product q = A v on the finite-element level of the multigrid V-cycle, with the smoothing
+// arithmetic that follows the product applied at the node (each node's q is complete here and the element pass has
+// finished reading v):
+//   MG_FE_STEP    (v = d): x += d, r -= q, d = c1 d + c2 r / D;
+//   MG_FE_RESTART (v = x): r = b - q, d = s r / D.
+// With a.add the new direction goes into x at once and neither it nor the residual is stored: the last step of the
+// post-smoothing, whose product nobody reads.  DOT: x . rhs of the finished iterate, r.z of the PCG.  Bound by the two
+// dependent trips to L2 of a node's incidence list, so what can ride along is free (66k nodes of Q9: 8.2 us; the
+// separate r.z took 4.4 us more).
+template <int MODE, bool DOT>
 __global__ void __launch_bounds__(kThreads)
-k_node_gather_cheb(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, const double* __restrict__ fe,
-                   const double* v, double* __restrict__ x, double* __restrict__ r, double* d, const double* __restrict__ b,
-                   const double* __restrict__ diag, const double* __restrict__ coef, int last) {
+k_node_gather_cheb(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, const double* fe,
+                   const MgNodePass a, const double* __restrict__ rhs, MgPcgState* dot, double* dot_work) {
     grid_dependency_wait();
     grid_dependents_launch();
     const double2* fe2 = reinterpret_cast<const double2*>(fe);
-    const double c1 = (MODE == MG_FE_RESTART || last) ? 0.0 : coef[0];
-    const double c2 = (MODE == MG_FE_RESTART || last) ? 0.0 : coef[1];
-    const double sc = MODE == MG_FE_RESTART ? coef[0] : 0.0;
+    const bool next = a.d != nullptr || a.add;
+    const double c1 = next ? a.coef[0] : 0.0;
+    const double c2 = MODE == MG_FE_STEP && next ? a.coef[1] : 0.0;
+    double sum = 0.0;
     for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < m.n_nodes; n += (int64_t)gridDim.x * blockDim.x) {
         const int fix = m.node_fix[n];
         const double2 f = node_sum<double>(inc_ptr, inc, fe2, n);
-        const double2 vn = reinterpret_cast<const double2*>(v)[n];
+        const double2 vn = reinterpret_cast<const double2*>(a.v)[n];
         const double q0 = (fix & 1) ? vn.x : f.x, q1 = (fix & 2) ? vn.y : f.y;
-        const double2 Dn = reinterpret_cast<const double2*>(diag)[n];
+        const double2 rn = reinterpret_cast<const double2*>(a.r_in)[n];
+        const double r0 = rn.x - q0, r1 = rn.y - q1;
+        double2 xn = make_double2(0.0, 0.0), dn = xn;
         if (MODE == MG_FE_STEP) {
-            const double2 dn = reinterpret_cast<const double2*>(d)[n];
-            double2 xn = reinterpret_cast<const double2*>(x)[n];
+            if (!a.first) xn = reinterpret_cast<const double2*>(a.x)[n];
+            xn.x += vn.x;
+            xn.y += vn.y;
+        } else if (a.add) {
+            xn = vn;
+        }
+        if (next) {
+            const double2 Dn = reinterpret_cast<const double2*>(a.diag)[n];
+            dn = MODE == MG_FE_STEP ? make_double2(c1 * vn.x + c2 * r0 / Dn.x, c1 * vn.y + c2 * r1 / Dn.y)
+                                    : make_double2(c1 * r0 / Dn.x, c1 * r1 / Dn.y);
+        }
+        if (a.add) {
             xn.x += dn.x;
             xn.y += dn.y;
-            reinterpret_cast<double2*>(x)[n] = xn;
-            const double2 rn = reinterpret_cast<const double2*>(r)[n];
-            const double r0 = rn.x - q0, r1 = rn.y - q1;
-            reinterpret_cast<double2*>(r)[n] = make_double2(r0, r1);
-            if (!last) reinterpret_cast<double2*>(d)[n] = make_double2(c1 * dn.x + c2 * r0 / Dn.x, c1 * dn.y + c2 * r1 / Dn.y);
-        } else {
-            const double2 bn = reinterpret_cast<const double2*>(b)[n];
-            const double r0 = bn.x - q0, r1 = bn.y - q1;
-            reinterpret_cast<double2*>(r)[n] = make_double2(r0, r1);
-            reinterpret_cast<double2*>(d)[n] = make_double2(sc * r0 / Dn.x, sc * r1 / Dn.y);
         }
+        if (MODE == MG_FE_STEP || a.add) reinterpret_cast<double2*>(a.x)[n] = xn;
+        if (a.r_out) reinterpret_cast<double2*>(a.r_out)[n] = make_double2(r0, r1);
+        if (a.d) reinterpret_cast<double2*>(a.d)[n] = dn;
+        if (DOT) {
+            const double2 bn = reinterpret_cast<const double2*>(rhs)[n];
+            sum += xn.x * bn.x + xn.y * bn.y;
+        }
+    }
+    if (DOT) dot_finish<kThreads, MG_DOT_CYCLE>(sum, dot_work, reinterpret_cast<double*>(dot), nullptr, 0);
+}
+
+// Element pass of a conjugate-gradient step: the product with z + beta p, formed at the gather, and its curvature
+// (energy form; the fixed DOFs, whose rows are the identity, are added at their first slot).
+template <int NEN, int NQ, typename SD>
+__global__ void __launch_bounds__(FrameCfg<NEN, NQ>::NT, FrameCfg<NEN, NQ>::MINB)
+k_mg_cg_elem(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const double* z,
+             const double* p, const double* beta_at, double* __restrict__ fe,
+             const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, RedSite site) {
+    constexpr int NT = FrameCfg<NEN, NQ>::NT;
+    __shared__ FrameShared<NEN, NQ, double> sh;
+    const double2 *z2 = reinterpret_cast<const double2*>(z), *p2 = reinterpret_cast<const double2*>(p);
+    double2* fe2 = reinterpret_cast<double2*>(fe);
+    double curv = 0.0, beta = 0.0;
+    const auto direction = [&](int n) {
+        const double2 zn = load_fresh(z2 + n), pn = load_fresh(p2 + n);
+        return make_double2(zn.x + beta * pn.x, zn.y + beta * pn.y);
+    };
+    frame_product<NEN, NQ, SD, double, true>(
+        m, C, rg, sh, curv,
+        [&]() -> bool {
+            grid_dependency_wait();
+            beta = load_fresh(beta_at);
+            grid_dependents_launch();
+            return true;
+        },
+        direction,
+        [&](int a, int64_t e, double2 f) {
+            const int64_t slot = (int64_t)a * m.stride + e;
+            fe2[slot] = f;
+            const int c = __ldg(m.conn + slot);
+            if ((c & 3) && inc[inc_ptr[c >> 2]] == (int32_t)slot) {
+                const double2 pn = direction(c >> 2);
+                if (c & 1) curv += pn.x * pn.x;
+                if (c & 2) curv += pn.y * pn.y;
+            }
+        },
+        blockIdx.x, gridDim.x);
+    const double vals[1] = {block_sum<NT>(curv)};
+    double tot[1];
+    if (last_block_sum<NT, 1>(vals, site, tot) && threadIdx.x == 0) site.result[0] = tot[0];
+}
+
+// Node pass of a conjugate-gradient step, everything after the product: see MgCgStep.  (As separate launches -- product,
+// p.q, update, r.z or r.r, direction -- a step took 26 us on 66k nodes of Q9, in these two 16.)
+template <int KIND>
+__global__ void __launch_bounds__(kThreads)
+k_mg_cg_node(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, const double* fe,
+             const MgCgStep a, double* dot_work) {
+    grid_dependency_wait();
+    grid_dependents_launch();
+    const double2* fe2 = reinterpret_cast<const double2*>(fe);
+    const double curv = KIND == MG_CG_SOLVE ? a.st->curv : a.scal[0];
+    const double alpha = (KIND == MG_CG_SOLVE ? a.st->rz : a.scal[1]) / curv;
+    const double beta = KIND == MG_CG_SOLVE ? a.st->beta : a.scal[3];
+    const double scale = KIND == MG_CG_SOLVE ? *a.scale : 0.0;
+    const bool curved = KIND != MG_CG_SOLVE || curv > 0.0;
+    const bool take_z = KIND == MG_CG_SOLVE && !curved && a.st->k == 0;  // not SPD along the first direction: x = z
+    double sum = 0.0;
+    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < m.n_nodes; n += (int64_t)gridDim.x * blockDim.x) {
+        const double2 zn = reinterpret_cast<const double2*>(a.z)[n];
+        if (!curved) {
+            if (take_z) reinterpret_cast<double2*>(a.x)[n] = zn;
+            continue;
+        }
+        const int fix = m.node_fix[n];
+        const double2 f = node_sum<double>(inc_ptr, inc, fe2, n);
+        double2 pn = reinterpret_cast<const double2*>(a.p)[n], rn = reinterpret_cast<const double2*>(a.r)[n];
+        const double2 Dn = reinterpret_cast<const double2*>(a.diag)[n];
+        pn.x = zn.x + beta * pn.x;
+        pn.y = zn.y + beta * pn.y;
+        reinterpret_cast<double2*>(a.p)[n] = pn;
+        rn.x -= alpha * ((fix & 1) ? pn.x : f.x);
+        rn.y -= alpha * ((fix & 2) ? pn.y : f.y);
+        reinterpret_cast<double2*>(a.r)[n] = rn;
+        if (KIND == MG_CG_SOLVE) {
+            double2 xn = reinterpret_cast<const double2*>(a.x)[n];
+            xn.x += alpha * pn.x;
+            xn.y += alpha * pn.y;
+            reinterpret_cast<double2*>(a.x)[n] = xn;
+            reinterpret_cast<double2*>(a.d)[n] = make_double2(scale * rn.x / Dn.x, scale * rn.y / Dn.y);
+            sum += rn.x * rn.x + rn.y * rn.y;
+        } else {
+            const double2 zr = make_double2(rn.x / Dn.x, rn.y / Dn.y);
+            reinterpret_cast<double2*>(a.z)[n] = zr;
+            sum += rn.x * zr.x + rn.y * zr.y;
+        }
+    }
+    if (KIND == MG_CG_LANCZOS) {
+        dot_finish<kThreads, MG_DOT_LANCZOS>(sum, dot_work, a.scal, a.hist, a.k);
+        return;
+    }
+    const double vals[1] = {block_sum<kThreads>(sum)};
+    double tot[1];
+    if (last_block_sum<kThreads, 1>(vals, RedSite{dot_work, dot_ticket(dot_work), nullptr}, tot) && threadIdx.x == 0) {
+        const bool on = pcg_iteration_end(a.st, curved, tot[0]);
+        if (a.loop) cudaGraphSetConditional(a.cond, on ? 1u : 0u);
     }
 }
 
@@ -1208,17 +1319,15 @@ extern "C" int dfea_tangent_apply_gather(const dfea_mesh_view* mesh, const void*
     return launch_check("dfea_tangent_apply_gather");
 }
 
-int dfea::mg_fe_gather_cheb(const dfea_mesh_view* mesh, const void* moduli, int32_t moduli_dtype, void* fe_work, int mode,
-                           const double* v, double* x, double* r, double* d, const double* b, const double* diag,
-                           const double* coef, int last, cudaStream_t s) {
+int dfea::mg_fe_smooth(const dfea_mesh_view* mesh, const void* moduli, int32_t moduli_dtype, void* fe_work, int mode,
+                      const MgNodePass& a, const double* rhs, MgPcgState* dot, double* dot_work, cudaStream_t s) {
     int rc = validate_mesh(mesh, moduli_dtype == DFEA_F32);
     if (rc) return rc;
     if (!mesh->node_elem_ptr || !mesh->node_elem) return set_error(DFEA_ERR_INVALID, "multigrid smoothing: no node incidence");
-    if (!moduli || !v || !fe_work || !r || !d || !diag || (!last && !coef) || (mode == MG_FE_STEP && !x) ||
-        (mode == MG_FE_RESTART && !b))
+    if (!moduli || !a.v || !fe_work || !a.x || !a.r_in || !a.diag || ((a.d || a.add) && !a.coef) || (dot && (!rhs || !dot_work)))
         return set_error(DFEA_ERR_INVALID, "multigrid smoothing: NULL pointer");
-    if (!aligned16(moduli) || !aligned16(v) || !aligned16(fe_work))
-        return set_error(DFEA_ERR_INVALID, "multigrid smoothing: moduli, v and fe_work must be 16-byte aligned");
+    if (!aligned16(moduli) || !aligned16(a.v) || !aligned16(a.x) || !aligned16(a.r_in) || !aligned16(fe_work))
+        return set_error(DFEA_ERR_INVALID, "multigrid smoothing: moduli, vectors and fe_work must be 16-byte aligned");
     if (moduli_dtype != DFEA_F64 && moduli_dtype != DFEA_F32 && moduli_dtype != DFEA_F32REF && moduli_dtype != DFEA_F64REF)
         return set_error(DFEA_ERR_INVALID, "bad moduli dtype");
     const Mesh m = kernel_mesh(*mesh);
@@ -1230,26 +1339,67 @@ int dfea::mg_fe_gather_cheb(const dfea_mesh_view* mesh, const void* moduli, int3
     rc = dispatch_element(mesh->nen, mesh->n_q, [&](auto nen_c, auto nq_c) -> int {
         constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
         if (moduli_dtype == DFEA_F64REF)
-            return launch_apply_ref_elem<NEN, NQ, double, double, false>(*mesh, static_cast<const double*>(moduli), v, fe,
+            return launch_apply_ref_elem<NEN, NQ, double, double, false>(*mesh, static_cast<const double*>(moduli), a.v, fe,
                                                                         none, nullptr, s);
         if (moduli_dtype == DFEA_F32REF)
-            return launch_apply_ref_elem<NEN, NQ, float, double, false>(*mesh, static_cast<const float*>(moduli), v, fe,
+            return launch_apply_ref_elem<NEN, NQ, float, double, false>(*mesh, static_cast<const float*>(moduli), a.v, fe,
                                                                        none, nullptr, s);
         if (moduli_dtype == DFEA_F64)
             return launch_apply_elem<NEN, NQ, double, double, false>(*mesh, static_cast<const double*>(moduli), mesh->grad,
-                                                                    v, fe, none, nullptr, s);
-        return launch_apply_elem<NEN, NQ, float, double, false>(*mesh, static_cast<const float*>(moduli), mesh->grad32, v,
+                                                                    a.v, fe, none, nullptr, s);
+        return launch_apply_elem<NEN, NQ, float, double, false>(*mesh, static_cast<const float*>(moduli), mesh->grad32, a.v,
                                                                fe, none, nullptr, s);
     });
     if (rc) return rc;
-    rc = mode == MG_FE_STEP
-             ? launch_kernel(k_node_gather_cheb<MG_FE_STEP>, dim3(gn), dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr,
-                             mesh->node_elem, (const double*)fe, v, x, r, d, b, diag, coef, last)
-             : launch_kernel(k_node_gather_cheb<MG_FE_RESTART>, dim3(gn), dim3(kThreads), 0, s, pdl, m,
-                             mesh->node_elem_ptr, mesh->node_elem, (const double*)fe, v, x, r, d, b, diag, coef, last);
+    const auto node_pass = [&](auto kernel) {
+        return launch_kernel(kernel, dim3(gn), dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr, mesh->node_elem,
+                             (const double*)fe, a, rhs, dot, dot_work);
+    };
+    if (mode == MG_FE_STEP) rc = dot ? node_pass(k_node_gather_cheb<MG_FE_STEP, true>) : node_pass(k_node_gather_cheb<MG_FE_STEP, false>);
+    else rc = dot ? node_pass(k_node_gather_cheb<MG_FE_RESTART, true>) : node_pass(k_node_gather_cheb<MG_FE_RESTART, false>);
     if (rc) return rc;
     note_launches(2);
     return launch_check("multigrid smoothing");
+}
+
+bool dfea::mg_fe_cg_supported(const dfea_mesh_view* mesh, int32_t moduli_dtype) {
+    return (moduli_dtype == DFEA_F64REF || moduli_dtype == DFEA_F32REF) && mesh->node_elem_ptr && mesh->node_elem;
+}
+
+int dfea::mg_fe_cg_step(const dfea_mesh_view* mesh, const void* moduli, int32_t moduli_dtype, void* fe_work, int kind,
+                       const MgCgStep& a, double* dot_work, cudaStream_t s) {
+    int rc = validate_mesh(mesh, false);
+    if (rc) return rc;
+    if (!mg_fe_cg_supported(mesh, moduli_dtype)) return set_error(DFEA_ERR_INVALID, "multigrid CG step: reference-frame moduli only");
+    if (!moduli || !fe_work || !aligned16(moduli) || !aligned16(fe_work) || !aligned16(a.z) || !aligned16(a.p) ||
+        !aligned16(a.r) || (a.x && !aligned16(a.x)))
+        return set_error(DFEA_ERR_INVALID, "multigrid CG step: moduli, vectors and fe_work must be 16-byte aligned");
+    const Mesh m = kernel_mesh(*mesh);
+    LaunchOpts pdl;
+    pdl.pdl = true;
+    double* fe = static_cast<double*>(fe_work);
+    const double* beta = kind == MG_CG_SOLVE ? &a.st->beta : a.scal + 3;
+    const RedSite site{dot_work, dot_ticket(dot_work), kind == MG_CG_SOLVE ? &a.st->curv : a.scal};
+    rc = dispatch_element(mesh->nen, mesh->n_q, [&](auto nen_c, auto nq_c) -> int {
+        constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
+        const auto pass = [&](auto* C) -> int {
+            using SD = std::remove_const_t<std::remove_pointer_t<decltype(C)>>;
+            const int grid = frame_resident_grid<k_mg_cg_elem<NEN, NQ, SD>, NEN, NQ>(mesh->n_el);
+            return launch_kernel(k_mg_cg_elem<NEN, NQ, SD>, dim3(grid), dim3(FrameCfg<NEN, NQ>::NT), 0, s, pdl, m, C,
+                                 ref_grad_of<NEN, NQ>(*mesh), (const double*)a.z, (const double*)a.p, beta, fe,
+                                 mesh->node_elem_ptr, mesh->node_elem, site);
+        };
+        return moduli_dtype == DFEA_F64REF ? pass(static_cast<const double*>(moduli)) : pass(static_cast<const float*>(moduli));
+    });
+    if (rc) return rc;
+    const int gn = grid_for(mesh->n_nodes, kThreads, 4);
+    rc = kind == MG_CG_SOLVE ? launch_kernel(k_mg_cg_node<MG_CG_SOLVE>, dim3(gn), dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr,
+                                             mesh->node_elem, (const double*)fe, a, dot_work)
+                             : launch_kernel(k_mg_cg_node<MG_CG_LANCZOS>, dim3(gn), dim3(kThreads), 0, s, pdl, m,
+                                             mesh->node_elem_ptr, mesh->node_elem, (const double*)fe, a, dot_work);
+    if (rc) return rc;
+    note_launches(2);
+    return launch_check("multigrid CG step");
 }
 
 extern "C" int64_t dfea_reduce_work_bytes(const dfea_mesh_view* mesh) {

@@ -131,11 +131,11 @@ k_pcg_setup(Mesh m, const T* __restrict__ b, const T* __restrict__ d, T* __restr
 // form) in the incidence order, and takes p on its fixed DOFs (the identity rows).
 // The body of update 1 for block blk of nblk (one launch, or one solve's share of a batched launch).
 template <typename T, bool GATHER, bool BJ>
-__device__ __forceinline__ void pcg_update1_body(const Mesh& m, int n_colours, const T* __restrict__ p,
-                                                 const T* __restrict__ y, const T* __restrict__ d, T* __restrict__ x,
+__device__ __forceinline__ void pcg_update1_body(const Mesh& m, int n_colours, const T* p,
+                                                 const T* y, const T* __restrict__ d, T* __restrict__ x,
                                                  T* __restrict__ r, PcgState* st, const RedSite& site,
                                                  const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
-                                                 const T* __restrict__ fe, int64_t blk, int64_t nblk) {
+                                                 const T* fe, int64_t blk, int64_t nblk) {
     using T2 = v2_t<T>;
     if (st->done) return;
     double curv = st->pfix;
@@ -162,14 +162,14 @@ __device__ __forceinline__ void pcg_update1_body(const Mesh& m, int n_colours, c
     const T a = (T)alpha;
     double rr = 0.0, rz = 0.0;
     for (int64_t n = blk * (int64_t)blockDim.x + threadIdx.x; n < m.n_nodes; n += (int64_t)nblk * blockDim.x) {
-        const T2 pn = reinterpret_cast<const T2*>(p)[n];
+        const T2 pn = load_fresh(reinterpret_cast<const T2*>(p) + n);
         T2 yn;
         if constexpr (GATHER) {
             const int fix = m.node_fix[n];
             const T2 f = node_sum<T>(inc_ptr, inc, reinterpret_cast<const T2*>(fe), n);
             yn = make_v2<T>((fix & 1) ? pn.x : f.x, (fix & 2) ? pn.y : f.y);
         } else {
-            yn = reinterpret_cast<const T2*>(y)[n];
+            yn = load_fresh(reinterpret_cast<const T2*>(y) + n);
         }
         T2 xn = reinterpret_cast<const T2*>(x)[n];
         T2 rn = reinterpret_cast<const T2*>(r)[n];
@@ -194,9 +194,9 @@ __device__ __forceinline__ void pcg_update1_body(const Mesh& m, int n_colours, c
 
 template <typename T, bool GATHER, bool BJ>
 __global__ void __launch_bounds__(kThreads)
-k_pcg_update1(Mesh m, int n_colours, const T* __restrict__ p, const T* __restrict__ y, const T* __restrict__ d,
+k_pcg_update1(Mesh m, int n_colours, const T* p, const T* y, const T* __restrict__ d,
               T* __restrict__ x, T* __restrict__ r, PcgState* st, RedSite site, const int32_t* __restrict__ inc_ptr,
-              const int32_t* __restrict__ inc, const T* __restrict__ fe) {
+              const int32_t* __restrict__ inc, const T* fe) {
     grid_dependency_wait();  // launched with PDL: everything below reads the predecessors' results
     grid_dependents_launch();
     pcg_update1_body<T, GATHER, BJ>(m, n_colours, p, y, d, x, r, st, site, inc_ptr, inc, fe, blockIdx.x, gridDim.x);
@@ -204,7 +204,7 @@ k_pcg_update1(Mesh m, int n_colours, const T* __restrict__ p, const T* __restric
 
 // PIVOT: write Ap := (1 - m) p, the identity rows the colour passes then add to (the colour form).
 template <typename T, bool PIVOT, bool BJ>
-__device__ __forceinline__ void pcg_update2_body(const Mesh& m, const T* __restrict__ r, const T* __restrict__ d,
+__device__ __forceinline__ void pcg_update2_body(const Mesh& m, const T* r, const T* __restrict__ d,
                                                  T* __restrict__ p, T* __restrict__ y, PcgState* st,
                                                  const RedSite& site, int64_t blk, int64_t nblk) {
     using T2 = v2_t<T>;
@@ -225,7 +225,7 @@ __device__ __forceinline__ void pcg_update2_body(const Mesh& m, const T* __restr
     double pf = 0.0;
     for (int64_t n = blk * (int64_t)blockDim.x + threadIdx.x; n < m.n_nodes; n += (int64_t)nblk * blockDim.x) {
         const int fix = m.node_fix[n];
-        const T2 rn = reinterpret_cast<const T2*>(r)[n];
+        const T2 rn = load_fresh(reinterpret_cast<const T2*>(r) + n);
         const T2 zn = precond<BJ, T>(d, n, rn);
         T2 pn = reinterpret_cast<const T2*>(p)[n];
         pn.x = zn.x + bt * pn.x;
@@ -250,7 +250,7 @@ __device__ __forceinline__ void pcg_update2_body(const Mesh& m, const T* __restr
 
 template <typename T, bool PIVOT, bool BJ>
 __global__ void __launch_bounds__(kThreads)
-k_pcg_update2(Mesh m, const T* __restrict__ r, const T* __restrict__ d, T* __restrict__ p, T* __restrict__ y,
+k_pcg_update2(Mesh m, const T* r, const T* __restrict__ d, T* __restrict__ p, T* __restrict__ y,
               PcgState* st, RedSite site) {
     grid_dependency_wait();
     grid_dependents_launch();
@@ -275,14 +275,14 @@ template <typename T, bool BJ, int NEN>
 __device__ __forceinline__ void fused_scatter(int64_t e, int64_t S, const int (&node)[NEN], const int (&fix)[NEN],
                                               const T (&fx)[NEN], const T (&fy)[NEN], v2_t<T>* __restrict__ fe2,
                                               const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
-                                              const T* __restrict__ d, const v2_t<T>* __restrict__ r2,
-                                              const v2_t<T>* __restrict__ p2, T beta, double& pfix) {
+                                              const T* __restrict__ d, const v2_t<T>* r2,
+                                              const v2_t<T>* p2, T beta, double& pfix) {
 #pragma unroll
     for (int a = 0; a < NEN; ++a) fe2[(int64_t)a * S + e] = make_v2<T>(fx[a], fy[a]);
 #pragma unroll
     for (int a = 0; a < NEN; ++a) {
         if (fix[a] && inc[inc_ptr[node[a]]] == (int32_t)((int64_t)a * S + e)) {
-            const v2_t<T> pn = next_direction<BJ, T>(d, node[a], __ldg(r2 + node[a]), __ldg(p2 + node[a]), beta);
+            const v2_t<T> pn = next_direction<BJ, T>(d, node[a], load_fresh(r2 + node[a]), load_fresh(p2 + node[a]), beta);
             if (fix[a] & 1) pfix += (double)pn.x * pn.x;
             if (fix[a] & 2) pfix += (double)pn.y * pn.y;
         }
@@ -291,8 +291,8 @@ __device__ __forceinline__ void fused_scatter(int64_t e, int64_t S, const int (&
 
 template <int NEN, int NQ, typename SD, typename T, bool BJ>
 __global__ void __launch_bounds__(128)
-k_pcg_elem_fused(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, const T* __restrict__ r,
-                 const T* __restrict__ d, const T* __restrict__ p, T* __restrict__ fe, const int32_t* __restrict__ inc_ptr,
+k_pcg_elem_fused(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, const T* r,
+                 const T* __restrict__ d, const T* p, T* __restrict__ fe, const int32_t* __restrict__ inc_ptr,
                  const int32_t* __restrict__ inc, PcgState* st, RedSite site) {
     using T2 = v2_t<T>;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -310,7 +310,7 @@ k_pcg_elem_fused(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, con
             grid_dependents_launch();
             return true;
         },
-        [&](int n) { return next_direction<BJ, T>(d, n, __ldg(r2 + n), __ldg(p2 + n), beta); },
+        [&](int n) { return next_direction<BJ, T>(d, n, load_fresh(r2 + n), load_fresh(p2 + n), beta); },
         [&](int64_t e, const int (&node)[NEN], const int (&fix)[NEN], const T (&fx)[NEN], const T (&fy)[NEN]) {
             fused_scatter<T, BJ, NEN>(e, m.stride, node, fix, fx, fy, fe2, inc_ptr, inc, d, r2, p2, beta, pfix);
         });
@@ -322,8 +322,8 @@ k_pcg_elem_fused(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, con
 
 template <int NEN, int NQ, typename SD, typename T, bool BJ>
 __global__ void __launch_bounds__(FrameCfg<NEN, NQ>::NT, FrameCfg<NEN, NQ>::MINB)
-k_pcg_elem_fused_ref(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const T* __restrict__ r,
-                     const T* __restrict__ d, const T* __restrict__ p, T* __restrict__ fe,
+k_pcg_elem_fused_ref(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const T* r,
+                     const T* __restrict__ d, const T* p, T* __restrict__ fe,
                      const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, PcgState* st, RedSite site) {
     using T2 = v2_t<T>;
     constexpr int NT = FrameCfg<NEN, NQ>::NT;
@@ -342,13 +342,13 @@ k_pcg_elem_fused_ref(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg
             grid_dependents_launch();
             return true;
         },
-        [&](int n) { return next_direction<BJ, T>(d, n, __ldg(r2 + n), __ldg(p2 + n), beta); },
+        [&](int n) { return next_direction<BJ, T>(d, n, load_fresh(r2 + n), load_fresh(p2 + n), beta); },
         [&](int a, int64_t e, T2 f) {
             const int64_t slot = (int64_t)a * m.stride + e;
             fe2[slot] = f;
             const int c = __ldg(m.conn + slot);
             if ((c & 3) && inc[inc_ptr[c >> 2]] == (int32_t)slot) {  // a fixed DOF, counted by its first slot
-                const T2 pn = next_direction<BJ, T>(d, c >> 2, __ldg(r2 + (c >> 2)), __ldg(p2 + (c >> 2)), beta);
+                const T2 pn = next_direction<BJ, T>(d, c >> 2, load_fresh(r2 + (c >> 2)), load_fresh(p2 + (c >> 2)), beta);
                 if (c & 1) pfix += (double)pn.x * pn.x;
                 if (c & 2) pfix += (double)pn.y * pn.y;
             }
@@ -362,7 +362,7 @@ k_pcg_elem_fused_ref(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg
 
 template <typename T, bool BJ>
 __global__ void __launch_bounds__(kThreads)
-k_pcg_node_fused(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, const T* __restrict__ fe,
+k_pcg_node_fused(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, const T* fe,
                  const T* __restrict__ d, T* __restrict__ x, T* __restrict__ r, T* __restrict__ p, PcgState* st,
                  RedSite site) {
     using T2 = v2_t<T>;
@@ -1530,7 +1530,7 @@ k_batch_elem(const BatchSolve* __restrict__ solves, const int2* __restrict__ blo
             grid_dependents_launch();
             return true;
         },
-        [&](int n) { return __ldg(p2 + n); },
+        [&](int n) { return load_fresh(p2 + n); },
         [&](int a, int64_t e, double2 f) { fe2[(int64_t)a * Sd + e] = f; }, bm.y, S->elem_blocks);
     if (!ran) return;
     const double vals[1] = {block_sum<NT>(curv)};
