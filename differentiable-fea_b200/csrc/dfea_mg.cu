@@ -1663,6 +1663,8 @@ namespace dfea {
 // the graphs of one hierarchy, each bound to the buffers it was captured with
 struct MgGraphs {
     cudaStream_t capture = nullptr;
+    cudaStream_t branch[2] = {};  // of a captured set-up, with the events that fork and join them
+    cudaEvent_t fork[2] = {}, join[2] = {};
     // set-up: moduli, diag and the mesh arrays the level-0 product reads; with and without the Lanczos bounds
     const void* key_setup[6] = {};
     int32_t code_setup = -1;
@@ -1691,6 +1693,20 @@ struct MgGraphs {
         drop_setup();
         drop_pcg();
         if (capture) cudaStreamDestroy(capture);
+        for (int i = 0; i < 2; ++i) {
+            if (branch[i]) cudaStreamDestroy(branch[i]);
+            if (fork[i]) cudaEventDestroy(fork[i]);
+            if (join[i]) cudaEventDestroy(join[i]);
+        }
+    }
+    int make_branches() {
+        int rc = DFEA_OK;
+        for (int i = 0; !rc && i < 2; ++i) {
+            if (!branch[i]) rc = check_cuda(cudaStreamCreateWithFlags(&branch[i], cudaStreamNonBlocking), "cudaStreamCreate");
+            if (!rc && !fork[i]) rc = check_cuda(cudaEventCreateWithFlags(&fork[i], cudaEventDisableTiming), "cudaEventCreate");
+            if (!rc && !join[i]) rc = check_cuda(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming), "cudaEventCreate");
+        }
+        return rc;
     }
 };
 
@@ -1700,15 +1716,96 @@ static bool same_key(const void* const* a, const void* const* b, int n) {
     return true;
 }
 
-// the device part of a set-up: coarse operators, coarsest inverse, Lanczos coefficients into mg->lhist
+// Lanczos of level l by launches (p in x, z in d), on reduction scratch w
+static int level_lanczos(const dfea_mesh_view* mesh, const dfea_mg* mg, const void* moduli, int32_t code, int l, double* w,
+                         cudaStream_t s) {
+    const dfea_mg_level& lv = mg->level[l];
+    const int64_t n = lv.n;
+    double *sc = mg->lscal + 4 * l, *hist = mg->lhist + (int64_t)2 * mg->lanczos_steps * l;
+    const int nb = mg_dot_blocks(n);
+    int rc;
+    k_mg_lanczos_start<<<nb, kMgDotThreads, 0, s>>>(n, lv.r, lv.d, lv.x, lv.diag, sc, w);
+    note_launches(1);
+    if ((rc = launch_check("dfea_mg_setup: Lanczos start"))) return rc;
+    const bool fused = l == 0 && fe_gather(mesh, mg) && mg_fe_cg_supported(mesh, code);
+    double *p = lv.x, *p_next = lv.b;
+    for (int k = 0; k < mg->lanczos_steps; ++k) {
+        if (fused) {
+            MgCgStep a = {};
+            a.z = lv.d, a.p = lv.x, a.r = lv.r, a.diag = lv.diag, a.scal = sc, a.hist = hist, a.k = k;
+            if ((rc = mg_fe_cg_step(mesh, moduli, code, mg->fe_work, MG_CG_LANCZOS, a, w, s))) return rc;
+            continue;
+        }
+        if (l == 0) {
+            if ((rc = mg_apply(mesh, mg, moduli, code, 0, lv.x, lv.q, s)) ||
+                (rc = mg_dot1<MG_DOT_PLAIN>(n, lv.x, lv.q, sc, w, s)))
+                return rc;
+        } else {
+            rc = launch_kernel(k_mg_lanczos_apply, dim3(grid_for(n / 2, kMgDotThreads, 8)), dim3(kMgDotThreads), 0, s,
+                               overlapping(), level_grid(mg, l), (const double*)lv.d, (const double*)p, p_next, lv.q, sc, w);
+            if (rc) return rc;
+            note_launches(1);
+            std::swap(p, p_next);
+        }
+        rc = launch_kernel(k_mg_lanczos_step_rz, dim3(nb), dim3(kMgDotThreads), 0, s, overlapping(), n, (const double*)lv.q,
+                           lv.r, lv.d, (const double*)lv.diag, sc, w, hist, k);
+        if (rc) return rc;
+        note_launches(1);
+        if (l == 0) {
+            k_mg_lanczos_p<<<grid_for(n, kThreads, 8), kThreads, 0, s>>>(n, lv.x, lv.d, sc);
+            note_launches(1);
+        }
+    }
+    return launch_check("dfea_mg_setup: Lanczos");
+}
+
+// Lanczos of the small levels t .. L-2, one cluster per level
+static int tail_lanczos(const dfea_mg* mg, int t, cudaStream_t s) {
+    const int L = mg->n_levels;
+    MgLanczosTail T = {};
+    T.steps = mg->lanczos_steps;
+    T.size = mg_cluster_size(mg->level[t].n / 2);
+    int most = 0, rc;
+    for (int k = 0; k < L - 1 - t; ++k) {
+        const dfea_mg_level& lv = mg->level[t + k];
+        const int n_nodes = (int)(lv.n / 2), nb = (n_nodes + T.size - 1) / T.size;
+        T.lv[k] = MgLanczosLevel{level_grid(mg, t + k), n_nodes, nb, lv.diag, mg->lscal + 4 * (t + k),
+                                 mg->lhist + (int64_t)2 * mg->lanczos_steps * (t + k)};
+        most = nb > most ? nb : most;
+    }
+    if ((rc = launch_clusters<k_mg_tail_lanczos>(L - 1 - t, T.size, (size_t)(4 * 16 + 36 * 8) * most, false, s, T))) return rc;
+    note_launches(1);
+    return launch_check("dfea_mg_setup: Lanczos of the small levels");
+}
+
+// The device part of a set-up: coarse operators, coarsest inverse, Lanczos coefficients into mg->lhist.  The estimate of
+// level 0 needs no coarse operator and those of the large coarse levels no coarsest inverse: chains of short launches
+// that leave most of the GPU idle, so a captured set-up (g) runs them on branches beside the rest -- the same launches,
+// the same results.  128 x 128 Q9: 450 us in line, 250 us in branches.
 static int setup_device_part(const dfea_mesh_view* mesh, const dfea_mg* mg, const void* moduli, int32_t moduli_dtype,
-                             const double* diag, cudaStream_t s, bool lanczos) {
+                             const double* diag, cudaStream_t s, bool lanczos, MgGraphs* g) {
     int rc;
     const int L = mg->n_levels;
-    if ((rc = check_cuda(cudaMemsetAsync(dot_ticket(mg->dot_work), 0, sizeof(unsigned), s), "cudaMemsetAsync")) ||
-        (rc = check_cuda(cudaMemcpyAsync(mg->level[0].diag, diag, mg->level[0].n * sizeof(double), cudaMemcpyDeviceToDevice, s),
+    const int t = tail_start(mg) < L - 1 ? tail_start(mg) : L - 1;
+    double* scratch[2] = {mg->dot_work, mg->dot_work + kMgDotScratch};
+    cudaStream_t on[2] = {s, s};
+    const auto fork = [&](int i) -> int {
+        if (!g) return DFEA_OK;
+        on[i] = g->branch[i];
+        const int e = check_cuda(cudaEventRecord(g->fork[i], s), "cudaEventRecord");
+        return e ? e : check_cuda(cudaStreamWaitEvent(on[i], g->fork[i], 0), "cudaStreamWaitEvent");
+    };
+    const auto join = [&](int i) -> int {
+        if (on[i] == s) return DFEA_OK;
+        const int e = check_cuda(cudaEventRecord(g->join[i], on[i]), "cudaEventRecord");
+        return e ? e : check_cuda(cudaStreamWaitEvent(s, g->join[i], 0), "cudaStreamWaitEvent");
+    };
+    for (double* w : scratch)
+        if ((rc = check_cuda(cudaMemsetAsync(dot_ticket(w), 0, sizeof(unsigned), s), "cudaMemsetAsync"))) return rc;
+    if ((rc = check_cuda(cudaMemcpyAsync(mg->level[0].diag, diag, mg->level[0].n * sizeof(double), cudaMemcpyDeviceToDevice, s),
                          "cudaMemcpyAsync")))
         return rc;
+    if (lanczos && t > 0 && ((rc = fork(0)) || (rc = level_lanczos(mesh, mg, moduli, moduli_dtype, 0, scratch[0], on[0])))) return rc;
     for (int l = 1; l < L; ++l) {
         const int32_t* gn;
         const uint8_t* ffix;
@@ -1729,67 +1826,15 @@ static int setup_device_part(const dfea_mesh_view* mesh, const dfea_mg* mg, cons
         }
         if (rc) return rc;
     }
-    if ((rc = dfea_mg_dense_inverse(&mg->level[L - 1].grid, mg->dense_work, mg->Ainv, s))) return rc;
-    if (!lanczos) return DFEA_OK;
-    // Lanczos on every smoothed level (p in x, z in d): one cluster per small level, two launches a step on the others
-    // (level 0 on moduli in another form than the reference frame's: a launch per operation)
-    const int t = tail_start(mg) < L - 1 ? tail_start(mg) : L - 1;
-    if (t < L - 1) {
-        MgLanczosTail T = {};
-        T.steps = mg->lanczos_steps;
-        T.size = mg_cluster_size(mg->level[t].n / 2);
-        int most = 0;
-        for (int k = 0; k < L - 1 - t; ++k) {
-            const dfea_mg_level& lv = mg->level[t + k];
-            const int n_nodes = (int)(lv.n / 2), nb = (n_nodes + T.size - 1) / T.size;
-            T.lv[k] = MgLanczosLevel{level_grid(mg, t + k), n_nodes, nb, lv.diag, mg->lscal + 4 * (t + k),
-                                     mg->lhist + (int64_t)2 * mg->lanczos_steps * (t + k)};
-            most = nb > most ? nb : most;
-        }
-        if ((rc = launch_clusters<k_mg_tail_lanczos>(L - 1 - t, T.size, (size_t)(4 * 16 + 36 * 8) * most, false, s, T))) return rc;
-        note_launches(1);
-        if ((rc = launch_check("dfea_mg_setup: Lanczos of the small levels"))) return rc;
+    if (lanczos && t > 1) {
+        if ((rc = fork(1))) return rc;
+        for (int l = 1; l < t; ++l)
+            if ((rc = level_lanczos(mesh, mg, moduli, moduli_dtype, l, scratch[1], on[1]))) return rc;
     }
-    for (int l = 0; l < t; ++l) {
-        const dfea_mg_level& lv = mg->level[l];
-        const int64_t n = lv.n;
-        double *sc = mg->lscal + 4 * l, *hist = mg->lhist + (int64_t)2 * mg->lanczos_steps * l, *w = mg->dot_work;
-        const int nb = mg_dot_blocks(n);
-        k_mg_lanczos_start<<<nb, kMgDotThreads, 0, s>>>(n, lv.r, lv.d, lv.x, lv.diag, sc, w);
-        note_launches(1);
-        if ((rc = launch_check("dfea_mg_setup: Lanczos start"))) return rc;
-        const bool fused = l == 0 && fe_gather(mesh, mg) && mg_fe_cg_supported(mesh, moduli_dtype);
-        double *p = lv.x, *p_next = lv.b;
-        for (int k = 0; k < mg->lanczos_steps; ++k) {
-            if (fused) {
-                MgCgStep a = {};
-                a.z = lv.d, a.p = lv.x, a.r = lv.r, a.diag = lv.diag, a.scal = sc, a.hist = hist, a.k = k;
-                if ((rc = mg_fe_cg_step(mesh, moduli, moduli_dtype, mg->fe_work, MG_CG_LANCZOS, a, w, s))) return rc;
-                continue;
-            }
-            if (l == 0) {
-                if ((rc = mg_apply(mesh, mg, moduli, moduli_dtype, 0, lv.x, lv.q, s)) ||
-                    (rc = mg_dot1<MG_DOT_PLAIN>(n, lv.x, lv.q, sc, w, s)))
-                    return rc;
-            } else {
-                rc = launch_kernel(k_mg_lanczos_apply, dim3(grid_for(n / 2, kMgDotThreads, 8)), dim3(kMgDotThreads), 0, s,
-                                   overlapping(), level_grid(mg, l), (const double*)lv.d, (const double*)p, p_next, lv.q, sc, w);
-                if (rc) return rc;
-                note_launches(1);
-                std::swap(p, p_next);
-            }
-            rc = launch_kernel(k_mg_lanczos_step_rz, dim3(nb), dim3(kMgDotThreads), 0, s, overlapping(), n, (const double*)lv.q,
-                               lv.r, lv.d, (const double*)lv.diag, sc, w, hist, k);
-            if (rc) return rc;
-            note_launches(1);
-            if (l == 0) {
-                k_mg_lanczos_p<<<grid_for(n, kThreads, 8), kThreads, 0, s>>>(n, lv.x, lv.d, sc);
-                note_launches(1);
-            }
-        }
-        if ((rc = launch_check("dfea_mg_setup: Lanczos"))) return rc;
-    }
-    return DFEA_OK;
+    if ((rc = dfea_mg_dense_inverse(&mg->level[L - 1].grid, mg->dense_work, mg->Ainv, s)) ||
+        (lanczos && t < L - 1 && (rc = tail_lanczos(mg, t, s))))
+        return rc;
+    return (rc = join(0)) ? rc : join(1);
 }
 
 // Capture `body(stream)` into a new graph on the hierarchy's capture stream and instantiate it; the kernels
@@ -2032,17 +2077,18 @@ extern "C" int dfea_mg_setup(const dfea_mesh_view* mesh, dfea_mg* mg, const void
         }
         const int v = lanczos ? 1 : 0;
         if (g->calls_setup[v]++ == 0) {
-            rc = setup_device_part(mesh, mg, moduli, moduli_dtype, diag, s, lanczos);   // direct, the first time
+            rc = setup_device_part(mesh, mg, moduli, moduli_dtype, diag, s, lanczos, nullptr);   // direct, the first time
         } else {
             if (!g->setup[v] &&
-                (rc = capture_exec(g, [&](cudaStream_t cs) { return setup_device_part(mesh, mg, moduli, moduli_dtype, diag, cs, lanczos); },
-                                   &g->setup[v], &g->kernels_setup[v])))
+                ((rc = g->make_branches()) ||
+                 (rc = capture_exec(g, [&](cudaStream_t cs) { return setup_device_part(mesh, mg, moduli, moduli_dtype, diag, cs, lanczos, g); },
+                                    &g->setup[v], &g->kernels_setup[v]))))
                 return rc;
             rc = check_cuda(cudaGraphLaunch(g->setup[v], s), "cudaGraphLaunch");
             note_launches(g->kernels_setup[v]);
         }
     } else {
-        rc = setup_device_part(mesh, mg, moduli, moduli_dtype, diag, s, lanczos);
+        rc = setup_device_part(mesh, mg, moduli, moduli_dtype, diag, s, lanczos, nullptr);
     }
     if (rc) return rc;
     if (!lanczos) return DFEA_OK;   // bounds, coefficients and lam[] of the last estimate stay in force

@@ -12,10 +12,12 @@ struct MgPcgState {
 };
 static_assert(sizeof(MgPcgState) <= 16 * sizeof(double), "pcg_state holds 16 doubles");
 
-// dfea_mg.dot_work: block partials, the reduction ticket, the state of a host-driven solve (doubles, 256-byte padded).
-constexpr int kMgDotWork = kMaxBlocks + 32 + 16;
+// dfea_mg.dot_work (doubles): two reduction scratches of block partials and a ticket (a set-up's branches reduce side by
+// side), then the state of a host-driven solve; the tickets are zeroed at every set-up.
+constexpr int kMgDotScratch = kMaxBlocks + 32;
+constexpr int kMgDotWork = 2 * kMgDotScratch + 16;
 __host__ __device__ inline unsigned* dot_ticket(double* work) { return reinterpret_cast<unsigned*>(work + kMaxBlocks); }
-inline MgPcgState* host_driven_state(double* work) { return reinterpret_cast<MgPcgState*>(work + kMaxBlocks + 32); }
+inline MgPcgState* host_driven_state(double* work) { return reinterpret_cast<MgPcgState*>(work + 2 * kMgDotScratch); }
 
 // What a sum over the grid is for; stored by thread 0 of the block that holds the total.
 enum {
