@@ -1658,6 +1658,103 @@ static int read_scalars(double* host, const double* dev, int k, cudaStream_t s) 
 namespace dfea {
 
 // ------------------------------------------------------------------------------------------
+// the grid behind a structured mesh
+// ------------------------------------------------------------------------------------------
+// What a hierarchy needs to know of its mesh, from the device connectivity.  (Built on the host and compared with and
+// copied to the device: 3.9 ms of a 384 x 384 Q4 hierarchy's construction, 1.4 ms of a 128 x 128 Q9 one's; here 0.1 ms.)
+struct GridNumbering {
+    int span, gx, gy, nen, k;  // k: 0 by columns, 1 by rows
+    __device__ __forceinline__ GridNumbering(int nen_, int ncx, int ncy, int k_)
+        : span(nen_ == 4 || nen_ == 3 ? 1 : 2), gx(span * ncx), gy(span * ncy), nen(nen_), k(k_) {}
+    __device__ __forceinline__ int64_t operator()(int i, int j) const {
+        if (k == 1) return i + (int64_t)j * (gx + 1);
+        if (nen != 8) return (int64_t)i * (gy + 1) + j;
+        // Q8: odd columns hold the nodes of even j only
+        const int64_t pair = (gy + 1) + (gy / 2 + 1);
+        return (i & 1) ? ((j & 1) ? -1 : (i / 2) * pair + gy + 1 + j / 2) : (i / 2) * pair + j;
+    }
+};
+
+// positions (di, dj) of an element's nodes in its cell: quadrilaterals, the lower and the upper triangle
+__device__ __forceinline__ void grid_corner(int nen, int half, int a, int& di, int& dj) {
+    // corners counter-clockwise, mid-sides, centre, in half cells
+    constexpr int qi[9] = {0, 2, 2, 0, 1, 2, 1, 0, 1}, qj[9] = {0, 0, 2, 2, 0, 1, 2, 1, 1};
+    constexpr int t3[2][3] = {{0, 1, 3}, {1, 2, 3}}, t6[2][6] = {{0, 1, 3, 4, 8, 7}, {1, 2, 3, 5, 6, 8}};
+    const int m = nen == 3 ? t3[half][a] : nen == 6 ? t6[half][a] : a;
+    const int div = nen == 4 || nen == 3 ? 2 : 1;
+    di = qi[m] / div;
+    dj = qj[m] / div;
+}
+
+struct GridCandidates {
+    int n, ncx[DFEA_GRID_CANDIDATES], ncy[DFEA_GRID_CANDIDATES];
+};
+
+__global__ void __launch_bounds__(256) k_grid_match(int64_t n_el, int nen, const int64_t* __restrict__ conn, GridCandidates c,
+                                                    int32_t* __restrict__ mismatch) {
+    const bool triangles = nen == 3 || nen == 6;
+    const int numberings = nen == 4 || nen == 9 ? 2 : 1;
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n_el; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t e = base + threadIdx.x;
+        for (int i = 0; i < c.n; ++i) {
+            const int64_t n_cells = (int64_t)c.ncx[i] * c.ncy[i];
+            const int half = triangles && e >= n_cells ? 1 : 0;
+            const int64_t cell = e - half * n_cells;
+            for (int k = 0; k < numberings; ++k) {
+                bool differs = false;
+                if (e < n_el) {
+                    const GridNumbering id(nen, c.ncx[i], c.ncy[i], k);
+                    const int ci = (int)(cell / c.ncy[i]) * id.span, cj = (int)(cell % c.ncy[i]) * id.span;
+                    for (int a = 0; a < nen; ++a) {
+                        int di, dj;
+                        grid_corner(nen, half, a, di, dj);
+                        differs |= conn[e * nen + a] != id(ci + di, cj + dj);
+                    }
+                }
+                if (__any_sync(0xffffffffu, differs) && (threadIdx.x & 31) == 0) mismatch[2 * i + k] = 1;
+            }
+        }
+    }
+    if (numberings == 1 && blockIdx.x == 0 && threadIdx.x < c.n) mismatch[2 * threadIdx.x + 1] = 1;
+}
+
+__global__ void __launch_bounds__(256) k_grid_nodes(int nen, int ncx, int ncy, int numbering, int32_t* __restrict__ gnode,
+                                                    int2* __restrict__ node_ij) {
+    const GridNumbering id(nen, ncx, ncy, numbering);
+    const int64_t n = (int64_t)(id.gx + 1) * (id.gy + 1);
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+        const int i = (int)(t / (id.gy + 1)), j = (int)(t % (id.gy + 1));
+        const int64_t node = id(i, j);
+        gnode[t] = (int32_t)node;
+        if (node >= 0) node_ij[node] = make_int2(i, j);
+    }
+}
+
+struct GridLines {
+    int n;
+    int gx[DFEA_MG_MAX_LEVELS], gy[DFEA_MG_MAX_LEVELS];
+    int32_t* at[DFEA_MG_MAX_LEVELS][4];  // line_x, line_y, cell_x, cell_y of level l >= 1
+};
+
+__global__ void __launch_bounds__(256) k_mg_maps(Mesh m, int n_cells, int epc, int32_t* __restrict__ cell_slot,
+                                                 const __grid_constant__ GridLines g) {
+    const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t slot = first; slot < m.n_el; slot += step) {
+        const int e = m.orig[slot], k = e / n_cells;
+        cell_slot[(int64_t)(e - k * n_cells) * epc + k] = (int32_t)slot;
+    }
+    for (int l = 1; l < g.n; ++l)
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            const int fine = d ? g.gy[l - 1] : g.gx[l - 1], coarse = d ? g.gy[l] : g.gx[l];
+            for (int64_t i = first; i <= fine; i += step) {
+                if (i <= coarse) g.at[l][d][i] = 2 * (int)i < fine ? 2 * (int)i : fine;
+                g.at[l][2 + d][i] = (int)i / 2 < coarse - 1 ? (int)i / 2 : coarse - 1;
+            }
+        }
+}
+
+// ------------------------------------------------------------------------------------------
 // graph-driven mode: the captured set-up and the device-side PCG loop
 // ------------------------------------------------------------------------------------------
 // the graphs of one hierarchy, each bound to the buffers it was captured with
@@ -2051,6 +2148,71 @@ static int pcg_graph_solve(MgGraphs* g, const dfea_mg* mg, double rtol, int32_t 
 }
 
 }  // namespace dfea
+
+extern "C" int dfea_grid_match(int64_t n_el, int32_t nen, const int64_t* conn, int32_t n_cand, const int32_t* ncx,
+                               const int32_t* ncy, int32_t* mismatch, void* stream) {
+    const bool known = nen == 4 || nen == 9 || nen == 8 || nen == 3 || nen == 6;
+    if (n_el < 1 || !known || !conn || n_cand < 1 || n_cand > DFEA_GRID_CANDIDATES || !ncx || !ncy || !mismatch)
+        return set_error(DFEA_ERR_INVALID, "dfea_grid_match: bad arguments");
+    GridCandidates c = {};
+    c.n = n_cand;
+    for (int i = 0; i < n_cand; ++i) {
+        c.ncx[i] = ncx[i];
+        c.ncy[i] = ncy[i];
+        if (ncx[i] < 1 || ncy[i] < 1 || (int64_t)ncx[i] * ncy[i] * (nen == 3 || nen == 6 ? 2 : 1) != n_el)
+            return set_error(DFEA_ERR_INVALID, "dfea_grid_match: candidate %d does not have the element count", i);
+    }
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int rc = check_cuda(cudaMemsetAsync(mismatch, 0, 2 * DFEA_GRID_CANDIDATES * sizeof(int32_t), s), "cudaMemsetAsync");
+    if (rc) return rc;
+    k_grid_match<<<grid_for(n_el, 256, 8), 256, 0, s>>>(n_el, nen, conn, c, mismatch);
+    note_launches(1);
+    return launch_check("dfea_grid_match");
+}
+
+extern "C" int dfea_grid_nodes(int32_t nen, int32_t ncx, int32_t ncy, int32_t numbering, int32_t* gnode, int32_t* node_ij,
+                               void* stream) {
+    const bool known = nen == 4 || nen == 9 || nen == 8 || nen == 3 || nen == 6;
+    const int span = nen == 4 || nen == 3 ? 1 : 2;
+    if (!known || ncx < 1 || ncy < 1 || numbering < 0 || numbering > (nen == 4 || nen == 9 ? 1 : 0) || !gnode || !node_ij ||
+        (reinterpret_cast<uintptr_t>(node_ij) & 7))
+        return set_error(DFEA_ERR_INVALID, "dfea_grid_nodes: bad arguments");
+    const int64_t n = ((int64_t)span * ncx + 1) * ((int64_t)span * ncy + 1);
+    if (n >= (int64_t(1) << 31)) return set_error(DFEA_ERR_INVALID, "dfea_grid_nodes: too many nodes");
+    k_grid_nodes<<<grid_for(n, 256, 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(nen, ncx, ncy, numbering, gnode,
+                                                                                     reinterpret_cast<int2*>(node_ij));
+    note_launches(1);
+    return launch_check("dfea_grid_nodes");
+}
+
+extern "C" int dfea_mg_maps(const dfea_mesh_view* mesh, const dfea_mg* mg, void* stream) {
+    int rc = validate_mesh(mesh, false);
+    if (rc) return rc;
+    if (!mg || mg->n_levels < 2 || mg->n_levels > DFEA_MG_MAX_LEVELS || !mg->cell_slot || mg->span < 1 || mg->span > 2)
+        return set_error(DFEA_ERR_INVALID, "dfea_mg_maps: bad hierarchy parameters");
+    GridLines g = {};
+    g.n = mg->n_levels;
+    for (int l = 0; l < g.n; ++l) {
+        const dfea_mg_grid& lv = mg->level[l].grid;
+        g.gx[l] = lv.gx;
+        g.gy[l] = lv.gy;
+        const int32_t* at[4] = {lv.line_x, lv.line_y, lv.cell_x, lv.cell_y};
+        for (int k = 0; k < 4; ++k) {
+            if (l > 0 && !at[k]) return set_error(DFEA_ERR_INVALID, "dfea_mg_maps: NULL map");
+            g.at[l][k] = const_cast<int32_t*>(at[k]);
+        }
+        // a level's lines lie among twice as many finer ones
+        if (lv.gx < 1 || lv.gy < 1 || (l > 0 && (lv.gx > g.gx[l - 1] || lv.gy > g.gy[l - 1])))
+            return set_error(DFEA_ERR_INVALID, "dfea_mg_maps: level %d", l);
+    }
+    const int64_t n_cells = (int64_t)(g.gx[0] / mg->span) * (g.gy[0] / mg->span);
+    const int64_t epc = n_cells > 0 ? mesh->n_el / n_cells : 0;
+    if (epc < 1 || epc * n_cells != mesh->n_el) return set_error(DFEA_ERR_INVALID, "dfea_mg_maps: level 0 is not the mesh's grid");
+    k_mg_maps<<<grid_for(mesh->n_el, 256, 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        kernel_mesh(*mesh), (int)n_cells, (int)epc, const_cast<int32_t*>(mg->cell_slot), g);
+    note_launches(1);
+    return launch_check("dfea_mg_maps");
+}
 
 extern "C" int dfea_mg_setup(const dfea_mesh_view* mesh, dfea_mg* mg, const void* moduli, int32_t moduli_dtype,
                              const double* diag, void* stream) {

@@ -171,6 +171,9 @@ _PROTOS = {
     "dfea_mg_galerkin": (ctypes.c_int, [_MGP, _MGP, c_vp]),
     "dfea_mg_restrict": (ctypes.c_int, [_MGP, _MGP, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "dfea_mg_prolong_add": (ctypes.c_int, [_MGP, _MGP, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "dfea_grid_match": (ctypes.c_int, [c_i64, c_i32, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp]),
+    "dfea_grid_nodes": (ctypes.c_int, [c_i32, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp]),
+    "dfea_mg_maps": (ctypes.c_int, [ctypes.POINTER(MeshView), ctypes.POINTER(Mg), c_vp]),
     "dfea_mg_apply": (ctypes.c_int, [_MGP, c_vp, c_vp, c_vp]),
     "dfea_mg_diag": (ctypes.c_int, [_MGP, c_vp, c_vp]),
     "dfea_mg_cheb_start": (ctypes.c_int, [c_i64, c_vp, c_vp, c_vp, c_vp, c_vp]),

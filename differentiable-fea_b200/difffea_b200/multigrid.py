@@ -30,6 +30,7 @@ import numpy as np
 import torch
 
 from difffea_b200 import _lib, ops
+from difffea_b200.cuda_mesh import ptr, stream_handle
 
 COARSEST_NODES = 48           # levels are coarsened until a level has at most this many nodes (96 DOFs: the
                               # dense Gauss-Jordan of the coarsest operator then runs in shared memory)
@@ -84,13 +85,36 @@ def _candidates(n_cells, n_nodes, span, q8):
     return out
 
 
+def _device_grid(conn, n_nodes, n_cells, span, epc):
+    """structured_grid of a device connectivity: one launch and one read for the match, one launch for the maps."""
+    n_el, nen = conn.shape
+    cells = _candidates(n_cells, n_nodes, span, nen == 8)
+    if not cells:
+        return None
+    with torch.cuda.device(conn.device):
+        mismatch = torch.empty(4, dtype=torch.int32, device=conn.device)
+        host = [(ctypes.c_int32 * len(cells))(*t) for t in zip(*cells)]
+        _lib.call("dfea_grid_match", n_el, nen, ptr(conn), len(cells), host[0], host[1], ptr(mismatch), stream_handle())
+        for i, differs in enumerate(mismatch.tolist()[:2 * len(cells)]):
+            if differs:
+                continue
+            ncx, ncy = cells[i // 2]
+            gx, gy = span * ncx, span * ncy
+            gnode = torch.empty((gx + 1) * (gy + 1), dtype=torch.int32, device=conn.device)
+            node_ij = torch.empty(n_nodes, 2, dtype=torch.int32, device=conn.device)
+            _lib.call("dfea_grid_nodes", nen, ncx, ncy, i % 2, ptr(gnode), ptr(node_ij), stream_handle())
+            return dict(span=span, epc=epc, ncx=ncx, ncy=ncy, gx=gx, gy=gy, gnode=gnode, node_ij=node_ij)
+    return None
+
+
 def structured_grid(conn, n_nodes):
     """
     The logical grid of a structured mesh (any element type of the library), or None: the element count
     and the node count fix at most two cell counts ncx x ncy; each is tried with the node numbering of the
     rectangle mesher (grid node (i, j) = i (gy + 1) + j, Q8 without the cell centres) and, for Q4 / Q9, of
-    the quarter-plate mesher (i + j (gx + 1)), and accepted if the connectivity matches exactly.  The
-    candidate connectivity is built on the host and compared with ``conn`` where it lies (one comparison).
+    the quarter-plate mesher (i + j (gx + 1)), and accepted if the connectivity matches exactly.  A connectivity
+    on the GPU is compared there with every candidate in one launch (dfea_grid_match) and its maps are written
+    there; on the host the candidate connectivities are built and compared one after the other.
     Returns dict(span, epc (elements per cell), ncx, ncy, gx, gy, gnode (grid node -> FE node, -1 for a
     Q8 cell centre), node_ij (FE node -> grid position)), the tensors on ``conn``'s device.
     """
@@ -102,6 +126,8 @@ def structured_grid(conn, n_nodes):
         return None
     n_cells = n_el // epc
     dev = conn.device
+    if dev.type == "cuda" and conn.dtype == torch.int64:
+        return _device_grid(conn.contiguous(), n_nodes, n_cells, span, epc)
     for ncx, ncy in _candidates(n_cells, n_nodes, span, nen == 8):
         gx, gy = span * ncx, span * ncy
         lex = np.arange((gx + 1) * (gy + 1), dtype=np.int64)
@@ -199,29 +225,15 @@ class Multigrid:
         if last.n > int(_lib.load().dfea_mg_dense_max()):
             raise ValueError("multigrid: the coarsest level is too large for the dense solve")
         L = len(self.levels)
-        # Integer maps, built on the host and copied in one transfer: the element slot of every cell's elements
-        # (cell c holds elements c + k n_cells, k < epc: one quadrilateral, or the lower then the upper
-        # triangle, numbered like the mesher's) and per coarse level its line and cell maps -- line I of a
-        # level lies on line min(2 I, fgx) of the finer one, finer line i lies in cell min(i // 2, gx - 1).
-        n_cells = g["ncx"] * g["ncy"]
-        inv_perm = np.empty_like(mesh.perm_host)
-        inv_perm[mesh.perm_host] = np.arange(mesh.perm_host.size)
-        elems = np.arange(n_cells)[:, None] + n_cells * np.arange(g["epc"])[None, :]
-        pieces = {"cell_slot": inv_perm[elems.reshape(-1)]}
+        # Integer maps in one allocation, written on the device (dfea_mg_maps): the element slots of every cell and
+        # per coarse level its line and cell maps
+        ia = _Arena(4)
+        ia.add("cell_slot", g["ncx"] * g["ncy"] * g["epc"])
         for l in range(1, L):
             f, lv = self.levels[l - 1], self.levels[l]
-            pieces[(l, "line_x")] = np.minimum(2 * np.arange(lv.gx + 1), f.gx)
-            pieces[(l, "line_y")] = np.minimum(2 * np.arange(lv.gy + 1), f.gy)
-            pieces[(l, "cell_x")] = np.minimum(np.arange(f.gx + 1) // 2, lv.gx - 1)
-            pieces[(l, "cell_y")] = np.minimum(np.arange(f.gy + 1) // 2, lv.gy - 1)
-        ia = _Arena(4)
-        for k, v in pieces.items():
-            ia.add(k, v.size)
-        host = np.zeros(ia.size, dtype=np.int32)
-        for k, v in pieces.items():
-            o, c = ia.at[k]
-            host[o:o + c] = v
-        self._ints = torch.from_numpy(host).to(dev)
+            for name, count in (("line_x", lv.gx + 1), ("line_y", lv.gy + 1), ("cell_x", f.gx + 1), ("cell_y", f.gy + 1)):
+                ia.add((l, name), count)
+        self._ints = torch.empty(ia.size, dtype=torch.int32, device=dev)
         # Float64 buffers in one allocation, the zero-initialised ones first: coefficients, Lanczos scalars and
         # history, dot partials, PCG scalars and the graph-driven loop's state; then the coarsest inverse and
         # its work, the PCG vectors and every level's vectors and element matrices.
@@ -269,6 +281,7 @@ class Multigrid:
                 setattr(dst, name, fptr((l, name)))
         for name in ("Ainv", "dense_work", "coef", "lscal", "lhist", "dot_work", "scal", "stencil"):
             setattr(h, name, fptr(name))
+        _lib.call("dfea_mg_maps", mesh.view_ref, ctypes.byref(h), stream_handle())
         h.pcg = fptr("pcg")
         h.pcg_state = fptr("pcg_state") if graphs else None
         h.graphs = None
@@ -279,6 +292,8 @@ class Multigrid:
             self.fe_work = torch.empty(int(_lib.load().dfea_gather_work_bytes(mesh.view_ref, _lib.DFEA_F64)),
                                        dtype=torch.uint8, device=dev)
             h.fe_work = self.fe_work.data_ptr()
+        with torch.cuda.device(dev):     # the maps are there before another stream's set-up may read them
+            torch.cuda.current_stream().synchronize()
         self.C, self.code = None, None
         self.id = ops.register_handle(self)
         self.generation = 0          # set-ups so far: a preconditioner closure checks that it is still current

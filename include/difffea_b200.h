@@ -442,6 +442,15 @@ int dfea_mg_restrict(const dfea_mg_grid* fine, const dfea_mg_grid* coarse, const
 /* x += P~ ec. */
 int dfea_mg_prolong_add(const dfea_mg_grid* fine, const dfea_mg_grid* coarse, const int32_t* gnode,
                         const uint8_t* fine_fix, const double* ec, double* x, void* stream);
+/* Is a device connectivity (n_el x nen, row-major int64) that of a structured mesh?  For candidate i < n_cand (at most
+ * DFEA_GRID_CANDIDATES; ncx[i] x ncy[i] cells, host arrays; ncx ncy (elements per cell) = n_el) and numbering k -- 0: grid node
+ * (i, j) = i (gy + 1) + j, Q8 without the cell centres; 1: i + j (gx + 1), Q4 and Q9 -- mismatch[2 i + k] (device) becomes
+ * 0 if every element's nodes are the grid's, else 1 (1 where the numbering is not defined). */
+#define DFEA_GRID_CANDIDATES 2
+int dfea_grid_match(int64_t n_el, int32_t nen, const int64_t* conn, int32_t n_cand, const int32_t* ncx, const int32_t* ncy,
+                    int32_t* mismatch, void* stream);
+/* gnode (grid node -> node, -1 at a Q8 cell centre) and node_ij (node -> grid position, 2 per node) of that numbering. */
+int dfea_grid_nodes(int32_t nen, int32_t ncx, int32_t ncy, int32_t numbering, int32_t* gnode, int32_t* node_ij, void* stream);
 /* y = K v + (I - M) v on a coarse level; dfea_mg_diag: its diagonal. */
 int dfea_mg_apply(const dfea_mg_grid* grid, const double* v, double* y, void* stream);
 int dfea_mg_diag(const dfea_mg_grid* grid, double* diag, void* stream);
@@ -529,6 +538,10 @@ typedef struct dfea_mg {
     double* stencil;
 } dfea_mg;
 
+/* Fill the hierarchy's integer maps on the device: cell_slot (cell c's elements c + k n_cells, one quadrilateral or the
+ * lower then the upper triangle) and every coarse level's line_x, line_y, cell_x, cell_y -- line I of a level lies on line
+ * min(2 I, fgx) of the finer one, finer line i in cell min(i / 2, gx - 1). */
+int dfea_mg_maps(const dfea_mesh_view* mesh, const dfea_mg* mg, void* stream);
 /* Set-up at a linearisation: coarse operators from the moduli, coarsest inverse, Lanczos estimates,
  * Chebyshev coefficients (one host synchronisation). */
 int dfea_mg_setup(const dfea_mesh_view* mesh, dfea_mg* mg, const void* moduli, int32_t moduli_dtype,
