@@ -329,6 +329,8 @@ __device__ __forceinline__ v2_t<T> node_sum(const int32_t* __restrict__ inc_ptr,
 }
 
 // Gather form, node pass of a plain product: y = (1 - m) v + m * sum of the element results.
+// Two dependent trips to L2 or DRAM per node: launched with all the warps an SM holds (8 blocks of 256; product of a
+// million Q4 105.5 us with 4 blocks -> 99.3, 400 x 400 Q9 60.4 -> 56.3, 640,000 Tri3 cells 66.6 -> 60.4).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_node_gather(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc, const T* fe,

@@ -836,7 +836,7 @@ static int frame_residual(const dfea_mesh_view* mesh, const double* u, const dou
     if (rc) return rc;
     LaunchOpts pdl;
     pdl.pdl = true;
-    const dim3 grid(grid_for(mesh->n_nodes, kThreads, 4));
+    const dim3 grid(grid_for(mesh->n_nodes, kThreads, 8));
     const RedSite site{w.norm_part, w.ticket, nullptr};
     if (reactions)
         rc = launch_kernel(k_frame_node_reactions, grid, dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr, mesh->node_elem,

@@ -1276,7 +1276,7 @@ extern "C" int dfea_tangent_apply_gather(const dfea_mesh_view* mesh, const void*
         return set_error(DFEA_ERR_INVALID, "FP32 vectors need FP32 moduli");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const Mesh m = kernel_mesh(*mesh);
-    const int gn = grid_for(mesh->n_nodes, kThreads, 4);
+    const int gn = grid_for(mesh->n_nodes, kThreads, 8);
     const RedSite none{nullptr, nullptr, nullptr};
     LaunchOpts pdl;
     pdl.pdl = true;
@@ -1331,7 +1331,7 @@ int dfea::mg_fe_smooth(const dfea_mesh_view* mesh, const void* moduli, int32_t m
     if (moduli_dtype != DFEA_F64 && moduli_dtype != DFEA_F32 && moduli_dtype != DFEA_F32REF && moduli_dtype != DFEA_F64REF)
         return set_error(DFEA_ERR_INVALID, "bad moduli dtype");
     const Mesh m = kernel_mesh(*mesh);
-    const int gn = grid_for(mesh->n_nodes, kThreads, 4);
+    const int gn = grid_for(mesh->n_nodes, kThreads, 8);
     const RedSite none{nullptr, nullptr, nullptr};
     LaunchOpts pdl;
     pdl.pdl = true;
@@ -1392,7 +1392,7 @@ int dfea::mg_fe_cg_step(const dfea_mesh_view* mesh, const void* moduli, int32_t 
         return moduli_dtype == DFEA_F64REF ? pass(static_cast<const double*>(moduli)) : pass(static_cast<const float*>(moduli));
     });
     if (rc) return rc;
-    const int gn = grid_for(mesh->n_nodes, kThreads, 4);
+    const int gn = grid_for(mesh->n_nodes, kThreads, 8);
     rc = kind == MG_CG_SOLVE ? launch_kernel(k_mg_cg_node<MG_CG_SOLVE>, dim3(gn), dim3(kThreads), 0, s, pdl, m, mesh->node_elem_ptr,
                                              mesh->node_elem, (const double*)fe, a, dot_work)
                              : launch_kernel(k_mg_cg_node<MG_CG_LANCZOS>, dim3(gn), dim3(kThreads), 0, s, pdl, m,

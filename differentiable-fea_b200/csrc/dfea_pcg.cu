@@ -878,7 +878,7 @@ int launch_iteration(const dfea_pcg& h, cudaStream_t s, cudaGraphConditionalHand
     const T* d = static_cast<const T*>(h.diag);
     T* x = static_cast<T*>(h.x);
     PcgState* st = h.state();
-    const int gn = capped(grid_for(mv.n_nodes, kThreads, 4), h.grid_cap);
+    const int gn = capped(grid_for(mv.n_nodes, kThreads, 8), h.grid_cap);
     LaunchOpts pdl;
     pdl.pdl = true;
     int rc;
