@@ -88,5 +88,7 @@ def compute_implicit_vjp(u_star, theta, params, lambda_adj):
     """dL/dtheta (n_el,) = -lambda^T dR/dtheta (theta enters linearly, so no theta dependence remains)."""
     mesh, mid = _prepare(u_star, theta, params)
     if mesh.ensure_frame():
-        return ops.frame_sensitivity(mid, _f64c(u_star), _f64c(lambda_adj), *ops.frame_material(params, linear_only=True))
-    return ops.element_sensitivity(mid, _f64c(u_star), _f64c(lambda_adj), *ops.material_args(device_material(params)))
+        return ops.run(ops.frame_sensitivity, mid, _f64c(u_star), _f64c(lambda_adj),
+                       *ops.frame_material(params, linear_only=True))
+    return ops.run(ops.element_sensitivity, mid, _f64c(u_star), _f64c(lambda_adj),
+                   *ops.material_args(device_material(params)))

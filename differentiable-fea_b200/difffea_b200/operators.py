@@ -55,8 +55,8 @@ def _residual(u, theta, params, load_factor, scalars):
     mesh, mid = _prepare(u, theta, params)
     u, theta, f = _f64c(u), _f64c(theta), _f64c(params["f"])
     if mesh.ensure_frame():
-        return ops.frame_residual(mid, u, theta, *ops.frame_material(params), f, float(load_factor), scalars)
-    R, n2, W = ops.residual(mid, u, theta, *ops.material_args(device_material(params)), f, float(load_factor))
+        return ops.run(ops.frame_residual, mid, u, theta, *ops.frame_material(params), f, float(load_factor), scalars)
+    R, n2, W = ops.run(ops.residual, mid, u, theta, *ops.material_args(device_material(params)), f, float(load_factor))
     return R, (n2, W)
 
 
@@ -94,14 +94,14 @@ class CudaTangentOperator:
     def C(self):
         """The 16 physical moduli per Gauss point; from the reference-frame ones on first use."""
         if self._physical is None:
-            self._physical = ops.frame_push_forward(self.mesh_id, self.moduli)
+            self._physical = ops.run(ops.frame_push_forward, self.mesh_id, self.moduli)
         return self._physical
 
     def __call__(self, v):
         """A(v); FP32 moduli apply to FP32 vectors, or to FP64 vectors with FP64 arithmetic."""
         if v.dtype != self.dtype and not (self.dtype == torch.float32 and v.dtype == torch.float64):
             raise ValueError(f"this operator applies {self.dtype} vectors, got {v.dtype}")
-        return ops.tangent_apply(self.mesh_id, self.moduli, v.contiguous())
+        return ops.run(ops.tangent_apply, self.mesh_id, self.moduli, v.contiguous())
 
     @property
     def dtype(self):
@@ -152,10 +152,10 @@ def make_A_operator_cuda(u, theta, params, precision="fp64"):
         if mesh.nen * mesh.stride < 2 ** 31:
             mesh.ensure_node_incidence()
     if precision == "fp64" and mesh.ensure_frame():
-        C, diag, _ = ops.frame_moduli(mid, _f64c(u), _f64c(theta), *ops.frame_material(params), True, False)
+        C, diag, _ = ops.run(ops.frame_moduli, mid, _f64c(u), _f64c(theta), *ops.frame_material(params), True, False)
     else:
-        C, diag = ops.qp_moduli(mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)),
-                                precision == "fp32", True)
+        C, diag = ops.run(ops.qp_moduli, mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)),
+                          precision == "fp32", True)
     _LAST_DIAG.clear()
     _LAST_DIAG[_diag_key(u, theta, mesh)] = (weakref.ref(u), weakref.ref(theta), diag)
     return CudaTangentOperator(mesh, mid, C, diag, precision)
@@ -211,7 +211,7 @@ def _preconditioner_data(mesh, mid, u, theta, params, with_blocks):
     """(diag, blocks or None) at (u, theta), without storing moduli."""
     u64, th64 = _f64c(u), _f64c(theta)
     if mesh.ensure_frame():
-        _, diag, blocks = ops.frame_moduli(mid, u64, th64, *ops.frame_material(params), False, with_blocks)
+        _, diag, blocks = ops.run(ops.frame_moduli, mid, u64, th64, *ops.frame_material(params), False, with_blocks)
         return diag, blocks
     diag = torch.empty(mesh.n_dof, dtype=torch.float64, device=mesh.device)
     blocks = torch.empty(2 * mesh.n_dof if with_blocks else 0, dtype=torch.float64, device=mesh.device)

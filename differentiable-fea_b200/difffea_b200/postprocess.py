@@ -25,8 +25,8 @@ def element_fields(u, theta, params):
     """(7, n_el) per original element: area, then the weighted means J, sxx, syy, sxy, mises, psi."""
     mesh, mid = _prepare(u, theta, params)
     if mesh.ensure_frame():
-        return ops.frame_fields(mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
-    return ops.element_fields(mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)))
+        return ops.run(ops.frame_fields, mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
+    return ops.run(ops.element_fields, mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)))
 
 
 def compute_fields(u, theta, params) -> dict:
@@ -39,7 +39,7 @@ def compute_fields(u, theta, params) -> dict:
     mesh, mid = _prepare(u, theta, params)
     un = _f64c(u).view(mesh.n_nodes, 2)
     if mesh.ensure_frame() and mesh.n_el:
-        el, nodal, scal = ops.frame_all_fields(mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
+        el, nodal, scal = ops.run(ops.frame_all_fields, mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
         u_mag, energy, min_J = nodal[6], scal[0], scal[1]
     else:
         el = element_fields(u, theta, params)
@@ -58,8 +58,8 @@ def internal_force(u, theta, params):
     """R_int(u) at every DOF, the constrained ones included (no mask, no external load)."""
     mesh, mid = _prepare(u, theta, params)
     if mesh.ensure_frame():
-        return ops.frame_internal_force(mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
-    return ops.internal_force(mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)))
+        return ops.run(ops.frame_internal_force, mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
+    return ops.run(ops.internal_force, mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)))
 
 
 def support_reactions(u, theta, params) -> torch.Tensor:
@@ -67,7 +67,7 @@ def support_reactions(u, theta, params) -> torch.Tensor:
     mesh, mid = _prepare(u, theta, params)
     if mesh.ensure_frame() and params["fixed"].numel() == mesh.n_dof:
         fixed = params["fixed"].to(mesh.device, torch.bool).reshape(-1).contiguous()
-        return ops.frame_reactions(mid, _f64c(u), _f64c(theta), *ops.frame_material(params), fixed)
+        return ops.run(ops.frame_reactions, mid, _f64c(u), _f64c(theta), *ops.frame_material(params), fixed)
     R = internal_force(u, theta, params).view(-1, 2)
     fixed = params["fixed"].to(R.device).reshape(-1, 2).bool()
     return torch.sum(torch.where(fixed, R, torch.zeros_like(R)), dim=0)
