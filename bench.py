@@ -28,7 +28,7 @@ Beside the headline (ours):
   latency_ms        p50 / p99 of (finish - arrival) over all 2,000 requests of the stream (this rank's shard)
                     replayed with Poisson arrivals at 80 % of the full window's measured capacity, FIFO
   roofline          the tangent product (kernel (b), FP64 stored moduli) at the microbench size,
-                    structured Q4 1600 x 1600 = 2.56M elements (inputs 2.2 GB >> L2), CUDA-event timed
+                    structured Q4 1600 x 1600 = 2.56M elements (inputs 0.9 GB >> L2), CUDA-event timed
   cpu_baseline      the oracle on the first 24 requests of the sample, on this host's cores
 
 Workload "plain": one step = one complete FP64 solve of the 100 x 100 Q4 unit-square problem (left edge
@@ -56,11 +56,11 @@ METRIC = "solves/s + p50/p99 latency, batched vs plain, at <=1e-8 rel err; A(v) 
 PLAIN = dict(element_type="quad4", nx=100, ny=100, width=1.0, height=1.0, E=1.0, nu=0.3, load=(0.1, 0.0),
              n_load_steps=3, tol=1e-10)
 MATVEC_N = 1600
-# DRAM bytes of one FP64 product at 2.56M Q4 elements, from ncu (dram__bytes_read.sum + dram__bytes_write.sum of
-# the four colour passes, L2 state kept, two products averaged: 2,335.1 MB read + 131.0 MB written; the pass that
-# initialises y with the Dirichlet pivot is not counted) against 2,130.1 MB algorithmic: 1.158 per byte, the
-# excess being v gathered and y read back by every colour pass
-DRAM_BYTES_PER_PRODUCT = 2.466e9
+# DRAM bytes of one FP64 product at 2.56M Q4 elements, from ncu (dram__bytes_read.sum + dram__bytes_write.sum, L2 state
+# kept, two products averaged): the element pass 995.8 MB read + 142.7 MB written, the node pass 253.5 + 65.3, against
+# 944.8 MB algorithmic: 1.54 per byte, the excess being the element results (164 MB written and read, part of it in L2)
+# and the node incidence
+DRAM_BYTES_PER_PRODUCT = 1.457e9
 SERVE = dict(stream=2000, seed=0, batch=32, slots=32, compare=64, sample_nx=64, sample_per_step=4,
              cpu_baseline_requests=24, latency_load=0.8)
 
@@ -178,14 +178,10 @@ def plain_solve(params, theta, ws=None):
 
 def matvec_roofline(device, reps=20):
     """
-    Time kernel (b) (FP64 stored moduli) at 2.56M Q4 elements with CUDA events on its launch stream.
-    v and y live in one allocation, as the PCG's Krylov vectors do, so the L2 window covers both.
-    Algorithmic bytes per product: n_el*n_q*16*8 (moduli) + n_el*n_q*nen*2*8 (gradients) + n_el*nen*4
-    (connectivity) + 3*2N*8 (v read, y written, mask).
+    Time the tangent product A(v) (FP64 stored moduli, an element and a node pass) at 2.56M Q4 elements with CUDA
+    events on its launch stream.  Algorithmic bytes per product: n_el*n_q*10*8 (symmetric reference-frame moduli) +
+    n_el*nen*4 (connectivity) + 2*2N*8 (v read, y written) + N (fixed-DOF bits).
     """
-    import ctypes
-    from difffea_b200 import _lib
-    from difffea_b200.cuda_mesh import ptr, stream_handle
     from difffea_b200.operators import make_tangent_operator
     from difffea_b200.problem import build_rectangle_problem
     n = MATVEC_N
@@ -195,16 +191,12 @@ def matvec_roofline(device, reps=20):
     u = (((torch.rand(N2, dtype=torch.float64, generator=g) * 2 - 1) * 0.05).to(device)) * p["m"]
     th = torch.ones(p["conn"].shape[0], dtype=torch.float64, device=device)
     A = make_tangent_operator("cuda", u, th, p)
-    pad = (N2 + 3) // 4 * 4
-    buf = torch.empty(2 * pad, dtype=torch.float64, device=device)
-    v, y = buf[:N2], buf[pad:pad + N2]
-    v.copy_(torch.randn(N2, dtype=torch.float64, generator=g).to(device))
+    v = torch.randn(N2, dtype=torch.float64, generator=g).to(device)
     n_el, nen, nq = p["conn"].shape[0], 4, 4
-    alg_bytes = n_el * nq * 16 * 8 + n_el * nq * nen * 2 * 8 + n_el * nen * 4 + 3 * N2 * 8
+    alg_bytes = n_el * nq * 10 * 8 + n_el * nen * 4 + 2 * N2 * 8 + N2 // 2
 
     def product():
-        _lib.call("dfea_tangent_apply", A.mesh.view_ref, ptr(A.C), _lib.DFEA_F64, ptr(v), ptr(y), _lib.DFEA_F64,
-                  stream_handle())
+        return A(v)
     for _ in range(3):
         product()
     torch.cuda.synchronize()
@@ -216,11 +208,9 @@ def matvec_roofline(device, reps=20):
     t1.record(s)
     torch.cuda.synchronize()
     ms = t0.elapsed_time(t1) / reps
-    y_ref = A(v)
-    ok = bool(torch.equal(y_ref, y))
-    del A, p, buf
+    del A, p
     torch.cuda.empty_cache()
-    return dict(n_el=n_el, bytes=alg_bytes, ms=ms, gbs=alg_bytes / (ms * 1e-3) / 1e9, same_as_op=ok)
+    return dict(n_el=n_el, bytes=alg_bytes, ms=ms, gbs=alg_bytes / (ms * 1e-3) / 1e9)
 
 
 def cpu_oracle_solve(params_cpu, theta_cpu, n_load_steps, tol, pcg_max_iter=500):
@@ -241,7 +231,7 @@ def serve_config(steps):
                         f"axial load 0.01..0.05, 1 load step, tol 1e-10 ||f||), {S} requests per step, {steps * S} "
                         f"timed; nx 16..512 stream window under full_stream",
             "parallelism": "replicas (stream sharded by request id)",
-            "l2": "serving working sets stream from HBM; roofline leg inputs 2.2 GB > 126 MB L2"}
+            "l2": "serving working sets stream from HBM; roofline leg inputs 0.9 GB > 126 MB L2"}
 
 
 def stream_shard(rank, world):
@@ -433,7 +423,7 @@ def run_serve(args):
                                     "plain_host_sync": "spin" if (plain_spin or not blocking) else "blocking",
                                     "plain": "newton_krylov_solve defaults, one request after another: FP64 "
                                              "moduli and gradients, Jacobi-PCG in 8-iteration graphs, product "
-                                             "form by mesh size (fused gather below 1.5M elements)",
+                                             "form by mesh size (fused gather below 300k nodes)",
                                     "reading": "ratio_jacobi isolates the engine (batching, FP32 operator); "
                                                "ratio_auto adds the multigrid preconditioner"},
                "serving_hbm": {"achieved_gbs": pcg_bytes / (full_ms * 1e-3) / 1e9,
@@ -446,8 +436,8 @@ def run_serve(args):
                               "arrival_rate_per_s": rate, "load": SERVE["latency_load"], "order": "fifo"},
                "roofline": {"bound": "hbm", "achieved": roof["gbs"], "peak": hbm, "unit": "GB/s",
                             "frac": roof["gbs"] / hbm, "traffic": DRAM_BYTES_PER_PRODUCT, "peak_kind": kind,
-                            "traffic_source": "ncu capture of the same product at the same size (four colour passes)",
-                            "kernel": "k_apply<4,4,double,double> (A(v), FP64 stored moduli)",
+                            "traffic_source": "ncu capture of the same product at the same size (element and node pass)",
+                            "kernel": "k_apply_ref_elem<4,4,double,double> + k_node_gather<double> (A(v), FP64 stored moduli)",
                             "workload": f"structured Q4 {MATVEC_N}x{MATVEC_N} = {roof['n_el']} elements",
                             "alg_bytes_per_launch": roof["bytes"], "ms_per_product": roof["ms"]},
                "cpu_baseline": {"value": len(cpu_reqs) / cpu_s, "unit": "solves/s", "cores": os.cpu_count(),
@@ -528,8 +518,8 @@ def run_plain_workload(args):
                                        "newton_oracle": info_ref["total_newton"], "cg_oracle": info_ref["total_cg"]},
                           "roofline": {"bound": "hbm", "achieved": roof["gbs"], "peak": hbm, "unit": "GB/s",
                                        "frac": roof["gbs"] / hbm, "traffic": DRAM_BYTES_PER_PRODUCT, "peak_kind": kind,
-                            "traffic_source": "ncu capture of the same product at the same size (four colour passes)",
-                                       "kernel": "k_apply<4,4,double,double>",
+                            "traffic_source": "ncu capture of the same product at the same size (element and node pass)",
+                                       "kernel": "k_apply_ref_elem<4,4,double,double> + k_node_gather<double>",
                                        "workload": f"structured Q4 {MATVEC_N}x{MATVEC_N}",
                                        "alg_bytes_per_launch": roof["bytes"], "ms_per_product": roof["ms"]},
                           "cpu_baseline": {"value": 1.0 / cpu_dt, "unit": "solves/s", "cores": os.cpu_count(),

@@ -18,9 +18,9 @@
 // element in FP64 -- and STAGES items are in flight per thread, so each SM keeps ~100 KB of loads
 // outstanding without spending registers on them.  Each thread copies and later reads only its own
 // element's slots (layout [row][thread], conflict-free), so the pipeline needs no block barrier.
-// The copies bypass L1 and stream through L2 once.  The DOF vectors (a few % of the traffic, but
-// gathered and scattered once per colour pass) are kept in L2 across the passes by an access-policy
-// window on the launch that marks them persisting (see `l2_window`).
+// The copies bypass L1 and stream through L2 once.  Nothing is marked persisting: a set-aside for the DOF vectors is a
+// limit of the whole process that takes that part of L2 from every other kernel for good (residual, moduli and product
+// of 640,000 Q4: 366 us instead of 215 once any product had set it).
 #pragma once
 
 #include <mutex>
@@ -610,19 +610,6 @@ int apply_ref_elem_grid(int64_t n_elements) {
     return frame_resident_grid<k_apply_ref_elem<NEN, NQ, SD, T, DOT>, NEN, NQ>(n_elements);
 }
 
-// The byte range of the DOF vectors a product gathers (v) and scatters (y): both when they are
-// adjacent (one allocation, as in the PCG work buffer), else y alone.
-struct L2Window {
-    const void* base = nullptr;
-    size_t bytes = 0;
-};
-inline L2Window l2_window(const void* v, const void* y, size_t vec_bytes) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(v), b = reinterpret_cast<uintptr_t>(y);
-    const uintptr_t lo = a < b ? a : b, hi = (a < b ? b : a) + vec_bytes;
-    if (hi - lo <= 2 * vec_bytes + 4096) return L2Window{reinterpret_cast<const void*>(lo), hi - lo};
-    return L2Window{y, vec_bytes};
-}
-
 // Launch the colour passes of one product on `stream` (the pivot init is launched by the caller).
 // With DOT, colour c reduces into sites[c] (result = curvature of that colour).
 template <int NEN, int NQ, typename SD, typename T, bool DOT>
@@ -631,17 +618,8 @@ int launch_apply_colours(const dfea_mesh_view& mv, const SD* C, const SD* G, con
                          int grid_cap = 0) {
     using Cfg = ApplyCfg<NEN, SD>;
     const Mesh m = kernel_mesh(mv);
-    long long max_window = 0;
-    const long long setaside = persisting_l2_bytes(&max_window);
-    L2Window w = l2_window(v, y, (size_t)(2 * mv.n_nodes) * sizeof(T));
-    if ((long long)w.bytes > max_window) w.bytes = (size_t)max_window;
     LaunchOpts opts;
     opts.pdl = true;
-    if (setaside > 0 && w.bytes > 0) {
-        opts.win_base = w.base;
-        opts.win_bytes = w.bytes;
-        opts.hit_ratio = setaside >= (long long)w.bytes ? 1.0f : (float)((double)setaside / (double)w.bytes);
-    }
     for (int c = 0; c < mv.n_colours; ++c) {
         const int64_t e0 = mv.colour_begin[c], e1 = mv.colour_begin[c + 1];
         if (e1 <= e0) continue;
@@ -655,25 +633,15 @@ int launch_apply_colours(const dfea_mesh_view& mv, const SD* C, const SD* G, con
     return launch_check("k_apply");
 }
 
-// Gather form: the element pass over all elements (results into fe), launched with the L2 window on v.  The node
-// pass is launched by the caller.  pdl: the pass requests its first moduli before it waits for its predecessor, so
+// Gather form: the element pass over all elements (results into fe).  The node pass is launched by the caller.  pdl: the pass requests its first moduli before it waits for its predecessor, so
 // it may overlap one only where that predecessor cannot be the writer of the moduli.
 template <int NEN, int NQ, typename SD, typename T, bool DOT>
 int launch_apply_elem(const dfea_mesh_view& mv, const SD* C, const SD* G, const T* v, T* fe, RedSite site,
                       const int* done, cudaStream_t stream, int grid_cap = 0, bool pdl = true) {
     using Cfg = ApplyCfg<NEN, SD>;
     const Mesh m = kernel_mesh(mv);
-    long long max_window = 0;
-    const long long setaside = persisting_l2_bytes(&max_window);
-    size_t wb = (size_t)(2 * mv.n_nodes) * sizeof(T);
-    if ((long long)wb > max_window) wb = (size_t)max_window;
     LaunchOpts opts;
     opts.pdl = pdl;
-    if (setaside > 0 && wb > 0) {
-        opts.win_base = v;
-        opts.win_bytes = wb;
-        opts.hit_ratio = setaside >= (long long)wb ? 1.0f : (float)((double)setaside / (double)wb);
-    }
     const int grid = capped(apply_elem_grid<NEN, NQ, SD, T, DOT>(mv.n_el), grid_cap);
     const int rc = launch_kernel(k_apply_elem<NEN, NQ, SD, T, DOT>, dim3(grid), dim3(Cfg::NT), Cfg::SMEM, stream, opts, m,
                                  C, G, v, fe, site, done);
@@ -681,24 +649,14 @@ int launch_apply_elem(const dfea_mesh_view& mv, const SD* C, const SD* G, const 
     return launch_check("k_apply_elem");
 }
 
-// Reference-frame launches: colour passes (y read-modify-write) or the element pass (results into fe).  The element
-// pass marks nothing persisting: it reads v once, and the L2 the set-aside would take keeps fe for the node pass.
+// Reference-frame launches: colour passes (y read-modify-write) or the element pass (results into fe).
 template <int NEN, int NQ, typename T, bool DOT>
 int launch_apply_ref_colours(const dfea_mesh_view& mv, const float* C, const T* v, T* y, const RedSite* sites,
                              const int* done, cudaStream_t stream, int grid_cap = 0) {
     const Mesh m = kernel_mesh(mv);
     const RefGrad<NEN, NQ> rg = ref_grad_of<NEN, NQ>(mv);
-    long long max_window = 0;
-    const long long setaside = persisting_l2_bytes(&max_window);
-    L2Window w = l2_window(v, y, (size_t)(2 * mv.n_nodes) * sizeof(T));
-    if ((long long)w.bytes > max_window) w.bytes = (size_t)max_window;
     LaunchOpts opts;
     opts.pdl = true;
-    if (setaside > 0 && w.bytes > 0) {
-        opts.win_base = w.base;
-        opts.win_bytes = w.bytes;
-        opts.hit_ratio = setaside >= (long long)w.bytes ? 1.0f : (float)((double)setaside / (double)w.bytes);
-    }
     for (int c = 0; c < mv.n_colours; ++c) {
         const int64_t e0 = mv.colour_begin[c], e1 = mv.colour_begin[c + 1];
         if (e1 <= e0) continue;
@@ -730,7 +688,6 @@ template <int NEN, int NQ, typename SD, typename T>
 void prepare_apply_ref() {
     if constexpr (sizeof(SD) == 4) (void)apply_ref_grid<NEN, NQ, T, true>(1);
     (void)apply_ref_elem_grid<NEN, NQ, SD, T, true>(1);
-    (void)persisting_l2_bytes(nullptr);
 }
 
 // Configure the instantiations a solver launches (shared-memory size, occupancy) before any stream capture.
@@ -740,7 +697,6 @@ void prepare_apply() {
     (void)apply_grid<NEN, NQ, SD, T, false>(1);
     (void)apply_elem_grid<NEN, NQ, SD, T, true>(1);
     (void)apply_elem_grid<NEN, NQ, SD, T, false>(1);
-    (void)persisting_l2_bytes(nullptr);
 }
 
 }  // namespace dfea

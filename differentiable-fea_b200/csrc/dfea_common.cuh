@@ -29,7 +29,6 @@ void note_launches(long long n);
 long long thread_launch_count();  // launches noted by the calling thread (kernels captured into a graph are
                                   // noted while capturing; the capture subtracts them again)
 int device_sm_count();
-long long persisting_l2_bytes(long long* max_window);
 // copy `bytes` from the device to `host` once stream `s` reaches the copy, through a pooled page-locked block
 int read_to_host(void* host, const void* dev, size_t bytes, cudaStream_t s);
 
@@ -115,37 +114,21 @@ __device__ __forceinline__ T load_fresh(const T* p) { return *p; }
 
 struct LaunchOpts {
     bool pdl = false;               // allow this launch to overlap its predecessor's tail
-    const void* win_base = nullptr; // L2 access-policy window marked persisting (0 bytes: none)
-    size_t win_bytes = 0;
-    float hit_ratio = 0.f;
 };
 
 template <typename... KArgs, typename... Args>
 int launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                   const LaunchOpts& o, Args... args) {
-    cudaLaunchAttribute attr[2];
-    unsigned n = 0;
-    if (o.pdl) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n].val.programmaticStreamSerializationAllowed = 1;
-        ++n;
-    }
-    if (o.win_bytes > 0 && o.hit_ratio > 0.f) {
-        attr[n].id = cudaLaunchAttributeAccessPolicyWindow;
-        attr[n].val.accessPolicyWindow.base_ptr = const_cast<void*>(o.win_base);
-        attr[n].val.accessPolicyWindow.num_bytes = o.win_bytes;
-        attr[n].val.accessPolicyWindow.hitRatio = o.hit_ratio;
-        attr[n].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
-        attr[n].val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
-        ++n;
-    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cfg.attrs = n ? attr : nullptr;
-    cfg.numAttrs = n;
+    cfg.attrs = attr;
+    cfg.numAttrs = o.pdl ? 1 : 0;
     return check_cuda(cudaLaunchKernelEx(&cfg, kernel, args...), "cudaLaunchKernelEx");
 }
 

@@ -886,18 +886,6 @@ int launch_iteration(const dfea_pcg& h, cudaStream_t s, cudaGraphConditionalHand
         T* fe = reinterpret_cast<T*>(h.work + h.layout.off_fe);
         rc = dispatch_element(mv.nen, mv.n_q, [&](auto nen_c, auto nq_c) -> int {
             constexpr int NEN = decltype(nen_c)::value, NQ = decltype(nq_c)::value;
-            long long max_window = 0;
-            const long long setaside = persisting_l2_bytes(&max_window);
-            LaunchOpts opts;
-            opts.pdl = true;
-            // r and p (adjacent in the work buffer) are gathered by every element: keep them in L2
-            L2Window w = l2_window(r, p, (size_t)(2 * mv.n_nodes) * sizeof(T));
-            if ((long long)w.bytes > max_window) w.bytes = (size_t)max_window;
-            if (setaside > 0 && w.bytes > 0) {
-                opts.win_base = w.base;
-                opts.win_bytes = w.bytes;
-                opts.hit_ratio = setaside >= (long long)w.bytes ? 1.0f : (float)((double)setaside / (double)w.bytes);
-            }
             if constexpr (REF) {
                 const int grid = capped(frame_resident_grid<k_pcg_elem_fused_ref<NEN, NQ, S, T, BJ>, NEN, NQ>(mv.n_el),
                                         h.grid_cap);
@@ -908,7 +896,7 @@ int launch_iteration(const dfea_pcg& h, cudaStream_t s, cudaGraphConditionalHand
                 using Cfg = ApplyCfg<NEN, S>;
                 const int grid = capped(resident_grid<k_pcg_elem_fused<NEN, NQ, S, T, BJ>, Cfg::SMEM, Cfg::NT>(mv.n_el),
                                         h.grid_cap);
-                return launch_kernel(k_pcg_elem_fused<NEN, NQ, S, T, BJ>, dim3(grid), dim3(Cfg::NT), Cfg::SMEM, s, opts,
+                return launch_kernel(k_pcg_elem_fused<NEN, NQ, S, T, BJ>, dim3(grid), dim3(Cfg::NT), Cfg::SMEM, s, pdl,
                                      m, C, G, (const T*)r, d, (const T*)p, fe, mv.node_elem_ptr, mv.node_elem, st,
                                      h.site(0, 1));
             }

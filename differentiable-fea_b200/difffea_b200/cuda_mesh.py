@@ -155,11 +155,6 @@ class CudaMesh:
             self.view.grad32 = self.grad32.data_ptr()
         return self.grad32
 
-    # Products of physical moduli below this many elements run in the gather form (two launches) where the mesh has its
-    # incidence: a launch per colour leaves most of the chip idle on a mid-sized mesh.  FP32, B200, colour / gather us:
-    # 65k Tri6 54 / 30, 90k Q4 43 / 31, 99k Q9 48 / 36, 410k Q4 51 / 46, 1M Q4 100 / 107, 980k Tri3 54 / 50.
-    GATHER_MAX_ELEMENTS = 700_000
-
     def ensure_node_incidence(self):
         """
         Build the node -> element incidence of the gather form once: the slots of node n are the flat

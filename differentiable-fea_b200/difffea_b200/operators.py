@@ -113,6 +113,7 @@ class CudaTangentOperator:
         the Jacobi diagonal, or with preconditioner="block_jacobi" the (4N,) inverse node blocks.
         """
         from difffea_b200.krylov import DevicePCG
+        from difffea_b200.workspace import pcg_form_for
         vt = b.dtype if self.dtype == torch.float32 else torch.float64   # FP32 moduli: FP64 or FP32 vectors
         if preconditioner == "block_jacobi":
             vt = torch.float64
@@ -124,7 +125,9 @@ class CudaTangentOperator:
             xx = torch.empty(n, dtype=vt, device=self.mesh.device)
             if self._pcg is not None:
                 self._pcg.close()
-            ref = dict(form="fused", moduli="ref", use_graph=2, cluster=True) if self.code == _lib.DFEA_F64REF else {}
+            ref = {}
+            if self.code == _lib.DFEA_F64REF:
+                ref = dict(form=pcg_form_for(self.mesh), moduli="ref", use_graph=2, cluster=True)
             self._pcg = DevicePCG(self.mesh, self.moduli, d, bb, xx, preconditioner=preconditioner, **ref)
             self._pcg_diag_src = diag
         self._pcg.b.copy_(b)

@@ -18,20 +18,21 @@ from difffea_b200.krylov import DevicePCG
 from difffea_b200.materials import device_material
 
 
-# Launch forms for meshes too large for the cluster form.  Physical moduli: below this many elements the fused gather
-# form of the PCG iteration (2 kernels) is faster than the colour form (n_colours + 2 kernels); above it the colour
-# form's lower traffic wins (measured on B200, FP64, per iteration: 23.0 vs 40.2 us at 16k Q4 elements, 27.5 vs 46.5 at
-# 40k, 171 vs 174 at 640k, 608 vs 550 at 2.56M).  Reference-frame moduli: fused, 54 us at 262k, 135 us at 655k.
-GATHER_FORM_MAX_ELEMENTS = 1_500_000
+# Launch forms for meshes too large for the cluster form: below this many nodes the fused gather form of a PCG iteration
+# (2 kernels), above it the gather form (3), whose element pass gathers one vector instead of rebuilding p from three.
+# Microseconds an iteration, FP64 reference-frame moduli, fused / gather: 40k Q4 nodes 20 / 22, 250k Q4 42 / 45, 250k Q9
+# 41 / 43, 250k Tri6 43 / 43, 360k Q4 53 / 55, 640k Q4 93 / 89, 2M Q9 241 / 201, 2.6M Q4 378 / 339, 3.2M Tri6 494 / 357.  The
+# colour form (n_colours + 2 kernels) is behind at every size: 39 against 18 - 22 at 22k, 301 against 271 at 2.6M (FP32).
+FUSED_FORM_MAX_NODES = 300_000
 
 
-def pcg_form_for(mesh, pcg_form="auto", moduli_code=_lib.DFEA_F64):
-    """The PCG product form: "colour", "gather", "fused", or "auto" (fused below GATHER_FORM_MAX_ELEMENTS; above it
-    colour, or gather for FP64 reference-frame moduli, which have no colour form)."""
+def pcg_form_for(mesh, pcg_form="auto"):
+    """The PCG product form: "colour", "gather", "fused", or "auto" (fused below FUSED_FORM_MAX_NODES, else gather; colour
+    where the mesh is too large for its node incidence)."""
     if pcg_form == "auto":
-        if mesh.n_el < GATHER_FORM_MAX_ELEMENTS:
-            return "fused"
-        return "gather" if moduli_code == _lib.DFEA_F64REF else "colour"
+        if mesh.nen * mesh.stride >= 2 ** 31:
+            return "colour"
+        return "fused" if mesh.n_nodes < FUSED_FORM_MAX_NODES else "gather"
     if pcg_form not in ("colour", "gather", "fused"):
         raise ValueError("pcg_form must be 'auto', 'colour', 'gather' or 'fused'")
     return pcg_form
@@ -101,7 +102,7 @@ class NewtonWorkspace:
             self.pcg = None
         else:
             self.pcg = DevicePCG(mesh, self.C, self.diag if self.blocks is None else self.blocks, self.b, self.du,
-                                 use_graph=use_graph, form=pcg_form_for(mesh, pcg_form, self.moduli_code),
+                                 use_graph=use_graph, form=pcg_form_for(mesh, pcg_form),
                                  moduli=self.moduli_kind, max_blocks=max_blocks, preconditioner=preconditioner,
                                  cluster=pcg_form == "auto" if cluster is None else cluster)
         self.work = mesh.reduce_work()
