@@ -119,9 +119,9 @@ def with_arrivals(requests, rate, seed=1):
 
 
 # "auto" preconditioner: geometric multigrid from this many nodes up (structured rectangles), Jacobi below.
-# Measured crossover on B200 (one request, FP32 operator, 1 load step, tol 1e-10 ||f||): Q4 64 x 16 (1,105
-# nodes) 15.6 ms Jacobi vs 18.1 ms multigrid, Q4 128 x 32 (4,257) 28.2 vs 21.0, Q9 64 x 16 (4,257) 40.0 vs
-# 24.0, Q9 512 x 128 (263,169) 381 vs 49.
+# Measured on B200 (FP32 operator, 1 load step, tol 1e-10 ||f||), requests/s through 16 slots, Jacobi / multigrid: Q4 96 x 24
+# (2,425 nodes) 521 / 552, Q4 112 x 28 (3,277) 459 / 591, Q9 48 x 12 (2,425) 437 / 579, Q9 128 x 32 (16,705) 146 / 522; one
+# request alone 7.4 / 4.2 ms, 9.5 / 4.2, 7.7 / 4.0, 27.9 / 4.3.
 MULTIGRID_MIN_NODES = 2500
 
 
@@ -390,8 +390,8 @@ def solve_request(req, device, precision="fp32", n_load_steps=1, tol_rel=1e-10, 
     """
     Build (or copy from ``host_params``) and solve one request on the current stream; returns
     (u on device, info).  ``pcg_graph`` is the PCG launch form (2: unrolled graph, the default for
-    a request solved alone; 1: conditional-loop graph; 0: direct launches, the serving engine's default); ``pcg_form`` the product form inside
-    it ("auto", "colour" or "gather", see DevicePCG and workspace.pcg_form_for) of a mesh too large for the cluster
+    a request solved alone; 1: conditional-loop graph; 0: direct launches, the serving engine's default); ``pcg_form``
+    the product form inside it ("auto", "colour" or "gather", see DevicePCG and workspace.pcg_form_for) of a mesh too large for the cluster
     form, which solves the smaller ones in one launch; ``fp32_moduli`` the FP32
     operator's moduli ("ref": reference frame, no gradients read; "physical"); ``max_blocks`` the most blocks
     per PCG launch (0: the whole GPU); ``preconditioner`` "jacobi", "block_jacobi", "multigrid" or "auto"
