@@ -106,9 +106,10 @@ inline int grid_for(int64_t n, int threads, int blocks_per_sm) {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-// A load of what the predecessor wrote, after the wait.  Such a pointer is no const __restrict__ parameter and is not
-// read with __ldg: the read-only path and its hoisting assume data that does not change while the kernel is resident,
-// and a kernel that started early may share an SM's L1 with a predecessor that read a line before another SM wrote it.
+// A load of what the predecessor wrote, after the wait.  Such a pointer is no __restrict__ parameter and is not read with
+// __ldg: a restricted pointer's loads may be hoisted above the wait (nothing else seems to write there), the read-only
+// path assumes data that does not change while the kernel is resident, and a kernel that started early may share an SM's
+// L1 with a predecessor that read a line before another SM wrote it.
 template <typename T>
 __device__ __forceinline__ T load_fresh(const T* p) { return *p; }
 

@@ -431,7 +431,7 @@ __device__ __forceinline__ void mg_prolong_node(const MgGrid& fg, const MgGrid& 
 }
 
 __global__ void k_mg_prolong_add(MgGrid fg, MgGrid cg, const int32_t* __restrict__ gnode, const uint8_t* __restrict__ ffix,
-                                 const double* ec, double* __restrict__ x) {
+                                 const double* ec, double* x) {
     grid_dependency_wait();
     grid_dependents_launch();
     const int n_nodes = (fg.gx + 1) * (fg.gy + 1);
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(256) k_mg_residual_restart(MgGrid g, const dou
 // one Chebyshev step on a coarse level with its product computed at the node: q = A d_in, x += d_in, r = r_in - q,
 // d_out = c1 d_in + c2 r / D (double-buffered: neighbouring nodes read d_in).  last: no next direction; add: the next
 // direction goes into x at once and neither it nor r is stored; first: x = d_in.
-__global__ void __launch_bounds__(256) k_mg_cheb_apply_step(MgGrid g, double* __restrict__ x, const double* r_in, double* r,
+__global__ void __launch_bounds__(256) k_mg_cheb_apply_step(MgGrid g, double* x, const double* r_in, double* r,
                                                             const double* d_in, double* __restrict__ d_out,
                                                             const double* __restrict__ diag, const double* __restrict__ c,
                                                             int first, int last, int add) {
@@ -667,9 +667,9 @@ static int mg_dot1(int64_t n, const double* x, const double* y, double* out, dou
 // k_mg_lanczos_step and the following r.z in one launch: r -= alpha q, z = r / D with alpha = s[1] / s[0], then the CG
 // step's bookkeeping
 __global__ void __launch_bounds__(kMgDotThreads) k_mg_lanczos_step_rz(int64_t n, const double* q,
-                                                                       double* __restrict__ r, double* __restrict__ z,
+                                                                       double* r, double* z,
                                                                        const double* __restrict__ diag,
-                                                                       double* __restrict__ s, double* __restrict__ work,
+                                                                       double* s, double* __restrict__ work,
                                                                        double* __restrict__ hist, int k) {
     grid_dependency_wait();
     grid_dependents_launch();
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(kMgDotThreads) k_mg_lanczos_start(int64_t n, d
 // nodes read p_in)
 __global__ void __launch_bounds__(kMgDotThreads) k_mg_lanczos_apply(MgGrid g, const double* z,
                                                                      const double* p_in, double* __restrict__ p_out,
-                                                                     double* __restrict__ q, double* __restrict__ s,
+                                                                     double* __restrict__ q, double* s,
                                                                      double* __restrict__ work) {
     grid_dependency_wait();
     grid_dependents_launch();
@@ -1535,7 +1535,7 @@ static int mg_cheb_steps(const dfea_mesh_view* mesh, const dfea_mg* mg, const vo
     return rc;
 }
 
-// first level (>= 1) of the one-block tail: levels shrink, so every level from it on is small enough
+// first level (>= 1) of the cluster tail: levels shrink, so every level from it on is small enough
 static int tail_start(const dfea_mg* mg) {
     if (!mg->stencil) return mg->n_levels;
     for (int l = 1; l < mg->n_levels; ++l)

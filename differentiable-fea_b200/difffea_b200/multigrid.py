@@ -15,8 +15,8 @@ Coarse operators are Galerkin products assembled element by element on the devic
 C (B P~) from the fine moduli, then sum P^T K P), P~ the bilinear interpolation with fixed fine DOFs
 zeroed, so every coarse operator is P~^T A P~ exactly (to rounding) and SPD.  Smoothing is Chebyshev
 with the Jacobi diagonal of each level on [lambda / 10, lambda], lambda = 1.1 x the lambda_max of D^-1 A from
-10 Lanczos steps per level and linearisation (the coefficients of Jacobi-preconditioned CG, all levels in
-lockstep with their scalars on the device, one host read): power iteration converges too slowly for the
+10 Lanczos steps per level and linearisation (the coefficients of Jacobi-preconditioned CG, their scalars on
+the device, one host read): power iteration converges too slowly for the
 dense top of this spectrum (26 % low after 10 steps on a 256 x 64 Q4 cantilever, measured, which made the
 smoother amplify the highest modes), Lanczos is within 1 % after 10.  The same polynomial runs before and
 after the coarse correction, so the V-cycle is a symmetric positive definite preconditioner for PCG.
@@ -33,7 +33,7 @@ from difffea_b200 import _lib, ops
 from difffea_b200.cuda_mesh import ptr, stream_handle
 
 COARSEST_NODES = 48           # levels are coarsened until a level has at most this many nodes (96 DOFs: the
-                              # dense Gauss-Jordan of the coarsest operator then runs in shared memory)
+                              # dense Gauss-Jordan of the coarsest operator then runs in registers)
 CHEB_DEGREE = 2
 CHEB_RATIO = 10.0             # smoothing interval [lambda_max / ratio, 1.1 lambda_max]
 LANCZOS_STEPS = 10

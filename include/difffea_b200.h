@@ -511,7 +511,7 @@ typedef struct dfea_mg {
     double* lhist;                             /* [n_levels][2 lanczos_steps] Lanczos coefficients      */
     double* dot_work;                          /* dfea_mg_dot_work() doubles                            */
     double* pcg;                               /* 4 x level[0].n: the PCG's r, z, p, q                  */
-    double* scal;                              /* 4 device doubles                                      */
+    double* scal;                              /* 4 device doubles (kept for callers; not written)      */
     double lam[DFEA_MG_MAX_LEVELS];            /* out: the lambda_max estimates of the last set-up      */
     /* Graph-driven mode (optional): with pcg_state set, dfea_mg_setup replays its launch sequence as a CUDA
      * graph and dfea_mg_pcg runs its iteration as a device-side loop (scalars on the device, one graph
