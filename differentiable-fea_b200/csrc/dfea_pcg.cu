@@ -878,7 +878,9 @@ int launch_iteration(const dfea_pcg& h, cudaStream_t s, cudaGraphConditionalHand
     const T* d = static_cast<const T*>(h.diag);
     T* x = static_cast<T*>(h.x);
     PcgState* st = h.state();
-    const int gn = capped(grid_for(mv.n_nodes, kThreads, 8), h.grid_cap);
+    // node passes with all the warps an SM holds; the colour form's two updates stream vectors, and keep the four blocks per
+    // SM that its sums (and so its iterates, bit for bit) were always divided over
+    const int gn = capped(grid_for(mv.n_nodes, kThreads, h.gather ? 8 : 4), h.grid_cap);
     LaunchOpts pdl;
     pdl.pdl = true;
     int rc;

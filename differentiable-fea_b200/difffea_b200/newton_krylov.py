@@ -44,15 +44,17 @@ def pcg(A_fn, b, Minv_fn, rtol=1e-5, max_iter=500):
 
     Stops when ||r|| <= rtol ||b||, returns (0, 0) for b = 0, and on non-positive curvature p.Ap <= 0
     returns z = M^-1 b at the first iteration and the current x otherwise.  With the GPU operator and
-    Jacobi preconditioner of this package the whole loop runs on the device (kernel (c), one CUDA
-    graph); any other pair of closures runs the same recurrences step by step.
+    Jacobi preconditioner of this package the whole loop runs on the device (kernel (c)); any other pair of
+    closures runs the same recurrences step by step.  ``A_fn.last_status`` says how a device solve ended; the x
+    of a "negative_curvature" is determined by rounding, and the same whichever device form met it.
     """
     if (isinstance(A_fn, CudaTangentOperator) and isinstance(Minv_fn, CudaJacobiPreconditioner)
             and Minv_fn.mesh is A_fn.mesh and b.is_cuda):
-        return A_fn.pcg_solve(b, Minv_fn.diag, rtol, max_iter)
+        return A_fn.pcg_solve(b, Minv_fn.diag, rtol, max_iter, diag_point=Minv_fn.point)
     if (isinstance(A_fn, CudaTangentOperator) and isinstance(Minv_fn, CudaBlockJacobiPreconditioner)
             and Minv_fn.mesh is A_fn.mesh and b.is_cuda):
-        return A_fn.pcg_solve(b, Minv_fn.blocks, rtol, max_iter, preconditioner="block_jacobi")
+        return A_fn.pcg_solve(b, Minv_fn.blocks, rtol, max_iter, preconditioner="block_jacobi",
+                              diag_point=Minv_fn.point)
     return _pcg_steps(A_fn, b, Minv_fn, rtol, max_iter)
 
 

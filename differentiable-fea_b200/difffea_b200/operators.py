@@ -74,15 +74,59 @@ def strain_energy(u, theta, params):
 # ---------------------------------------------------------------------------------------------
 # tangent operator
 # ---------------------------------------------------------------------------------------------
+def _version(t):
+    """The tensor's version counter, or None where torch keeps none."""
+    return None if t.is_inference() else t._version
+
+
+class _Linearisation:
+    """
+    The point (u, theta, material) an operator or preconditioner was made at: what its physical moduli, diagonal or
+    blocks are computed from when a solve asks for them later.  Holds the tensors themselves; ``unchanged`` is False
+    once one of them was written to (or where torch keeps no version of it).
+    """
+
+    def __init__(self, u, theta, params):
+        self.u, self.theta = (t.detach() if t.requires_grad else t for t in (u, theta))
+        self.material = {k: params[k] for k in ("material", "mat_p", "mat_scalable", "mu0", "lmbda0", "nodes") if k in params}
+        self.versions = self._versions()
+
+    def _versions(self):
+        tensors = (self.u, self.theta, *(t for t in self.material.values() if torch.is_tensor(t)))
+        return [_version(t) for t in tensors]
+
+    @property
+    def unchanged(self):
+        return None not in self.versions and self.versions == self._versions()
+
+    def physical(self, mesh_id):
+        """(the 16 physical moduli per Gauss point, the Jacobi diagonal) by the kernels that read dN/dX."""
+        return ops.run(ops.qp_moduli, mesh_id, _f64c(self.u), _f64c(self.theta),
+                       *ops.material_args(device_material(self.material)), False, True)
+
+    def physical_preconditioner(self, mesh, mesh_id, with_blocks):
+        """(diag, blocks or None) by the same kernels, without storing moduli."""
+        diag = torch.empty(mesh.n_dof, dtype=torch.float64, device=mesh.device)
+        blocks = torch.empty(2 * mesh.n_dof if with_blocks else 0, dtype=torch.float64, device=mesh.device)
+        torch.ops.difffea_b200.qp_moduli_out(mesh_id, _f64c(self.u), _f64c(self.theta),
+                                             *ops.material_args(device_material(self.material)),
+                                             torch.empty(0, dtype=torch.float64, device=mesh.device), _lib.DFEA_F64, diag,
+                                             blocks)
+        return diag, blocks if with_blocks else None
+
+
 class CudaTangentOperator:
     """
     v -> A(v) from moduli stored at the Gauss points (kernel (b)).  Holds the moduli of its linearisation point
     (``moduli``, layout ``code``: FP64 in the element reference frame where the mesh has one, else the 16 physical
-    entries) and the Jacobi diagonal computed in the same pass of kernel (a).
+    entries) and the Jacobi diagonal computed in the same pass of kernel (a); ``point`` is that linearisation point, where
+    the operator was made from one.
     """
 
-    def __init__(self, mesh, mesh_id, moduli, diag, precision="fp64"):
+    def __init__(self, mesh, mesh_id, moduli, diag, precision="fp64", point=None):
         self.mesh, self.mesh_id, self.moduli, self.diag, self.precision = mesh, mesh_id, moduli, diag, precision
+        self.point = point
+        self._indefinite = None
         self.code = (_lib.DFEA_F32 if moduli.dtype == torch.float32 else
                      _lib.DFEA_F64REF if moduli.numel() == mesh.moduli_numel_ref() else _lib.DFEA_F64)
         self._physical = None if self.code == _lib.DFEA_F64REF else moduli
@@ -107,13 +151,16 @@ class CudaTangentOperator:
     def dtype(self):
         return self.moduli.dtype
 
-    def pcg_solve(self, b, diag, rtol, max_iter, preconditioner="jacobi"):
+    def pcg_solve(self, b, diag, rtol, max_iter, preconditioner="jacobi", diag_point=None):
         """
         PCG on the device (kernel (c)) with this operator; returns (x in b's dtype, iterations).  ``diag`` is
-        the Jacobi diagonal, or with preconditioner="block_jacobi" the (4N,) inverse node blocks.
+        the Jacobi diagonal, or with preconditioner="block_jacobi" the (4N,) inverse node blocks, and ``diag_point`` the
+        linearisation point it was made at.
         """
         from difffea_b200.krylov import DevicePCG
         from difffea_b200.workspace import pcg_form_for
+        if self._indefinite is not None and self._indefinite[0] is diag and self._indefinite[1] == _version(diag):
+            return self._run_pcg(self._indefinite[2], b, rtol, max_iter)
         vt = b.dtype if self.dtype == torch.float32 else torch.float64   # FP32 moduli: FP64 or FP32 vectors
         if preconditioner == "block_jacobi":
             vt = torch.float64
@@ -130,10 +177,45 @@ class CudaTangentOperator:
                 ref = dict(form=pcg_form_for(self.mesh), moduli="ref", use_graph=2, cluster=True)
             self._pcg = DevicePCG(self.mesh, self.moduli, d, bb, xx, preconditioner=preconditioner, **ref)
             self._pcg_diag_src = diag
-        self._pcg.b.copy_(b)
-        iters, status = self._pcg.solve(rtol, max_iter)
+        out = self._run_pcg(self._pcg, b, rtol, max_iter)
+        if self.last_status == "negative_curvature" and self.code == _lib.DFEA_F64REF:
+            physical = self._physical_pcg(diag, preconditioner, diag_point)
+            if physical is not None:
+                self._indefinite = (diag, _version(diag), physical)
+                return self._run_pcg(physical, b, rtol, max_iter)
+        return out
+
+    def _run_pcg(self, solver, b, rtol, max_iter):
+        solver.b.copy_(b)
+        iters, status = solver.solve(rtol, max_iter)
         self.last_status = status
-        return self._pcg.x.to(b.dtype, copy=True), iters
+        return solver.x.to(b.dtype, copy=True), iters
+
+    def _physical_pcg(self, diag, preconditioner, diag_point):
+        """
+        The solver of an operator that is not positive definite: physical moduli, one launch per colour.  On such an
+        operator the iterate at the first non-positive curvature is amplified rounding -- two orders of summation
+        leave 1e-4 to 1 of it different -- so the forms of a solve would give different answers.  All of them end
+        here instead, with one answer.  None (the first solve's answer stands) where the point the operator was made
+        at is gone or there is no memory for its physical moduli.
+        """
+        from difffea_b200.krylov import DevicePCG
+        if self.point is None or not self.point.unchanged:
+            return None
+        try:
+            C, own = self.point.physical(self.mesh_id)
+            d = diag.detach().to(torch.float64).contiguous()
+            as_made = _version(diag) == 0                # not a diagonal the caller has written to
+            if as_made and diag is self.diag:
+                d = own
+            elif as_made and diag_point is not None and diag_point.unchanged:
+                blocks = preconditioner == "block_jacobi"
+                d = diag_point.physical_preconditioner(self.mesh, self.mesh_id, blocks)[1 if blocks else 0]
+            n = self.mesh.n_dof
+            b, x = (torch.empty(n, dtype=torch.float64, device=self.mesh.device) for _ in range(2))
+            return DevicePCG(self.mesh, C, d, b, x, preconditioner=preconditioner)
+        except torch.cuda.OutOfMemoryError:
+            return None
 
 
 # (weakref(u), u._version, weakref(theta), theta._version, mesh id) -> diag of the last linearisation,
@@ -161,7 +243,7 @@ def make_A_operator_cuda(u, theta, params, precision="fp64"):
                           precision == "fp32", True)
     _LAST_DIAG.clear()
     _LAST_DIAG[_diag_key(u, theta, mesh)] = (weakref.ref(u), weakref.ref(theta), diag)
-    return CudaTangentOperator(mesh, mid, C, diag, precision)
+    return CudaTangentOperator(mesh, mid, C, diag, precision, _Linearisation(u, theta, params))
 
 
 def make_tangent_operator(kind, u, theta, params):
@@ -194,8 +276,8 @@ def make_AT_operator(u, theta, params):
 class CudaJacobiPreconditioner:
     """r -> r / diag(K) with diag clamped to >= 1e-6 on free DOFs and 1 on fixed DOFs."""
 
-    def __init__(self, mesh, diag):
-        self.mesh, self.diag = mesh, diag
+    def __init__(self, mesh, diag, point=None):
+        self.mesh, self.diag, self.point = mesh, diag, point
 
     def __call__(self, r):
         return r / self.diag.to(r.dtype)
@@ -212,21 +294,15 @@ def compute_jacobi_diagonal(u, theta, params):
 
 def _preconditioner_data(mesh, mid, u, theta, params, with_blocks):
     """(diag, blocks or None) at (u, theta), without storing moduli."""
-    u64, th64 = _f64c(u), _f64c(theta)
     if mesh.ensure_frame():
-        _, diag, blocks = ops.run(ops.frame_moduli, mid, u64, th64, *ops.frame_material(params), False, with_blocks)
+        _, diag, blocks = ops.run(ops.frame_moduli, mid, _f64c(u), _f64c(theta), *ops.frame_material(params), False, with_blocks)
         return diag, blocks
-    diag = torch.empty(mesh.n_dof, dtype=torch.float64, device=mesh.device)
-    blocks = torch.empty(2 * mesh.n_dof if with_blocks else 0, dtype=torch.float64, device=mesh.device)
-    torch.ops.difffea_b200.qp_moduli_out(mid, u64, th64, *ops.material_args(device_material(params)),
-                                         torch.empty(0, dtype=torch.float64, device=mesh.device), _lib.DFEA_F64, diag,
-                                         blocks)
-    return diag, blocks
+    return _Linearisation(u, theta, params).physical_preconditioner(mesh, mid, with_blocks)
 
 
 def make_jacobi_preconditioner(u, theta, params):
     mesh = cuda_mesh(params)
-    return CudaJacobiPreconditioner(mesh, compute_jacobi_diagonal(u, theta, params))
+    return CudaJacobiPreconditioner(mesh, compute_jacobi_diagonal(u, theta, params), _Linearisation(u, theta, params))
 
 
 class CudaBlockJacobiPreconditioner:
@@ -235,8 +311,8 @@ class CudaBlockJacobiPreconditioner:
     fixed DOFs and + 1e-12 I (operators.py:598-625); ``blocks`` = (Binv00, Binv01, Binv11, 0) per node.
     """
 
-    def __init__(self, mesh, blocks):
-        self.mesh, self.blocks = mesh, blocks
+    def __init__(self, mesh, blocks, point=None):
+        self.mesh, self.blocks, self.point = mesh, blocks, point
 
     def __call__(self, r):
         B = self.blocks.view(-1, 4).to(r.dtype)
@@ -253,7 +329,7 @@ def compute_block_jacobi(u, theta, params):
 
 def make_block_jacobi_preconditioner(u, theta, params):
     mesh = cuda_mesh(params)
-    return CudaBlockJacobiPreconditioner(mesh, compute_block_jacobi(u, theta, params))
+    return CudaBlockJacobiPreconditioner(mesh, compute_block_jacobi(u, theta, params), _Linearisation(u, theta, params))
 
 
 class CudaMultigridPreconditioner:
