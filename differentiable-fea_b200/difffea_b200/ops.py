@@ -322,10 +322,11 @@ def frame_moduli(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: int,
     C = torch.empty(mesh.moduli_numel_ref() if with_moduli else 0, **f64)
     diag = torch.empty(mesh.n_dof, **f64)
     blocks = torch.empty(2 * mesh.n_dof if with_blocks else 0, **f64)
+    work = mesh.frame_work()        # a local: the call's own until its launches are made
     _lib.call("dfea_frame_moduli", mesh.view_ref, ptr(u), ptr(theta),
               *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev),
               ptr(C if with_moduli else None), _lib.DFEA_F64REF, ptr(diag), ptr(blocks if with_blocks else None),
-              ptr(mesh.frame_work()), stream_handle())
+              ptr(work), stream_handle())
     return C, diag, blocks
 
 
@@ -345,10 +346,11 @@ def frame_residual(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: in
     _f64(f, mesh, mesh.n_dof)
     R = torch.empty_like(u)
     out = torch.empty(2 if scalars else 0, dtype=torch.float64, device=mesh.device)
+    work = mesh.frame_work()        # a local: the call's own until its launches are made
     _lib.call("dfea_frame_residual", mesh.view_ref, ptr(u), ptr(theta),
               *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev), ptr(f), float(load_factor), ptr(R),
               ptr(out if scalars else None), ptr(out[1:] if scalars else None),
-              ptr(mesh.frame_work()), stream_handle())
+              ptr(work), stream_handle())
     return R, out
 
 
@@ -363,9 +365,10 @@ def frame_internal_force(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, mod
                  p_dev: Optional[torch.Tensor], s_dev: Optional[torch.Tensor]) -> torch.Tensor:
     mesh = _frame_mesh(mesh_id, u, theta)
     R = torch.empty_like(u)
+    work = mesh.frame_work()        # a local: the call's own until its launches are made
     _lib.call("dfea_frame_internal_force", mesh.view_ref, ptr(u), ptr(theta),
               *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev),
-              ptr(R), ptr(mesh.frame_work()), stream_handle())
+              ptr(R), ptr(work), stream_handle())
     return R
 
 
@@ -417,9 +420,10 @@ def frame_all_fields(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: 
     mesh = _frame_mesh(mesh_id, u, theta)
     f64 = dict(dtype=torch.float64, device=mesh.device)
     el, nodal, scal = torch.empty(7, mesh.n_el, **f64), torch.empty(7, mesh.n_nodes, **f64), torch.empty(2, **f64)
+    work = mesh.frame_work()        # a local: the call's own until its launches are made
     _lib.call("dfea_frame_all_fields", mesh.view_ref, ptr(u), ptr(theta),
               *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev), ptr(el), ptr(nodal), ptr(scal),
-              ptr(mesh.frame_work()), stream_handle())
+              ptr(work), stream_handle())
     return el, nodal, scal
 
 
@@ -436,8 +440,9 @@ def frame_reactions(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, model: i
     if fixed.dtype != torch.bool or fixed.numel() != mesh.n_dof or not fixed.is_contiguous() or fixed.device != mesh.device:
         raise ValueError("fixed must be the contiguous (2N,) bool flags on the mesh's device")
     out = torch.empty(2, dtype=torch.float64, device=mesh.device)
+    work = mesh.frame_work()        # a local: the call's own until its launches are made
     _lib.call("dfea_frame_reactions", mesh.view_ref, ptr(u), ptr(theta),
-              *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev), ptr(fixed), ptr(out), ptr(mesh.frame_work()),
+              *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev), ptr(fixed), ptr(out), ptr(work),
               stream_handle())
     return out
 
