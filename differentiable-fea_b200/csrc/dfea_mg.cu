@@ -773,6 +773,7 @@ __global__ void k_mg_lanczos_p(int64_t n, double* __restrict__ p, const double* 
 // The tail of a 128 x 128 Q9 cycle (levels of 4,225 nodes down to 25): 100 us in one block, plus 44 us of launches for
 // the 4,225-node level, -> 54 us; the Lanczos estimates of these levels 247 -> 51 us, the clusters side by side.
 constexpr int kMgTailNodes = 6000;
+constexpr int kMgTailNodeBytes = 6 * 16 + 36 * 8;  // of a tail level: b, x, r, d, q, 1 / D and the node's rows
 constexpr int kMgClusterThreads = 512;
 constexpr int kMgClusterWarps = kMgClusterThreads / 32;
 
@@ -1185,11 +1186,11 @@ __global__ void __launch_bounds__(kMgClusterThreads, 1) k_mg_tail(const __grid_c
     cluster_barrier();  // no block leaves while another may read its shared memory
 }
 
-// A launch of clusters of `size` blocks (a power of two of at most kClusterMax).
-template <auto Kernel, typename... Args>
-static int launch_clusters(int n_clusters, int size, size_t smem, bool pdl, cudaStream_t s, const Args&... args) {
+// The kernel set up for clusters on the current device: *bytes becomes the dynamic shared memory a block may take.
+template <auto Kernel>
+static int cluster_configure(int64_t* bytes) {
     static std::once_flag once[64];
-    static int result[64] = {0};
+    static int result[64] = {0}, most_bytes[64] = {0};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     std::call_once(once[dev], [dev] {
@@ -1197,12 +1198,21 @@ static int launch_clusters(int n_clusters, int size, size_t smem, bool pdl, cuda
         int rc = check_cuda(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
         cudaFuncAttributes fa;
         if (!rc) rc = check_cuda(cudaFuncGetAttributes(&fa, Kernel), "cudaFuncGetAttributes");
-        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                      most - (int)fa.sharedSizeBytes), "cudaFuncSetAttribute");
+        if (!rc) most_bytes[dev] = most - (int)fa.sharedSizeBytes;
+        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most_bytes[dev]),
+                                 "cudaFuncSetAttribute");
         if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "cudaFuncSetAttribute");
         result[dev] = rc;
     });
-    if (result[dev]) return result[dev];
+    if (bytes) *bytes = most_bytes[dev];
+    return result[dev];
+}
+
+// A launch of clusters of `size` blocks (a power of two of at most kClusterMax).
+template <auto Kernel, typename... Args>
+static int launch_clusters(int n_clusters, int size, size_t smem, bool pdl, cudaStream_t s, const Args&... args) {
+    const int rc = cluster_configure<Kernel>(nullptr);
+    if (rc) return rc;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = size;
@@ -1219,10 +1229,10 @@ static int launch_clusters(int n_clusters, int size, size_t smem, bool pdl, cuda
     return check_cuda(cudaLaunchKernelEx(&cfg, Kernel, args...), "cudaLaunchKernelEx");
 }
 
-// blocks for a largest level of n nodes: about 64 nodes a block, 16 blocks at the most
-static int mg_cluster_size(int64_t n_nodes) {
+// blocks for a largest level of n nodes: about 64 nodes a block, 16 blocks (or the fewer that are allowed) at the most
+static int mg_cluster_size(int64_t n_nodes, int most = kClusterMax) {
     int size = 1;
-    while (size < kClusterMax && (int64_t)size * 64 < n_nodes) size *= 2;
+    while (2 * size <= most && (int64_t)size * 64 < n_nodes) size *= 2;
     return size;
 }
 
@@ -1535,12 +1545,23 @@ static int mg_cheb_steps(const dfea_mesh_view* mesh, const dfea_mg* mg, const vo
     return rc;
 }
 
-// first level (>= 1) of the cluster tail: levels shrink, so every level from it on is small enough
-static int tail_start(const dfea_mg* mg) {
-    if (!mg->stencil) return mg->n_levels;
-    for (int l = 1; l < mg->n_levels; ++l)
-        if (mg->level[l].n / 2 <= kMgTailNodes) return l;
+// First level (>= 1) of the cluster tail, n_levels: none.  A block holds its nodes of all the tail's levels.  Where both
+// directions coarsen, the levels after the first add a third to it; on a thin strip one direction is soon a single cell,
+// the levels only halve and double it (a 2,945 x 6 strip: 235 KB from its level of 5,892 nodes on), so the sum decides.
+static int tail_level(const dfea_mg* mg, int blocks, int64_t bytes) {
+    for (int l = 1; l < mg->n_levels; ++l) {
+        if (mg->level[l].n / 2 > kMgTailNodes) continue;
+        const int size = mg_cluster_size(mg->level[l].n / 2, blocks);
+        int64_t need = 0;
+        for (int k = l; k < mg->n_levels; ++k) need += (mg->level[k].n / 2 + size - 1) / size * kMgTailNodeBytes;
+        if (need <= bytes) return l;
+    }
     return mg->n_levels;
+}
+static int tail_start(const dfea_mg* mg) {
+    int64_t bytes = 0;
+    if (!mg->stencil || cluster_configure<k_mg_tail>(&bytes)) return mg->n_levels;
+    return tail_level(mg, kClusterMax, bytes);
 }
 
 // restriction of level l's residual, the cycle of levels l + 1 .. L - 1 and the prolongation into x, in one launch
@@ -1560,7 +1581,7 @@ static int launch_tail(const dfea_mesh_view* mesh, const dfea_mg* mg, int l, dou
         const dfea_mg_level& c = mg->level[l + 1 + k];
         const int n_nodes = (int)(c.n / 2), nb = (n_nodes + size - 1) / size;
         T.lv[k] = MgTailLevel{level_grid(mg, l + 1 + k), n_nodes, nb, at, c.diag, mg->coef + (int64_t)(l + 1 + k) * 2 * DFEA_MG_MAX_DEGREE};
-        at += (6 * 16 + 36 * 8) * nb;
+        at += kMgTailNodeBytes * nb;
     }
     const int rc = launch_clusters<k_mg_tail>(1, size, at, true, s, T);
     if (rc) return rc;
@@ -2212,6 +2233,11 @@ extern "C" int dfea_mg_maps(const dfea_mesh_view* mesh, const dfea_mg* mg, void*
         kernel_mesh(*mesh), (int)n_cells, (int)epc, const_cast<int32_t*>(mg->cell_slot), g);
     note_launches(1);
     return launch_check("dfea_mg_maps");
+}
+
+extern "C" int32_t dfea_mg_tail_level(const dfea_mg* mg, int32_t blocks, int64_t bytes) {
+    if (!mg || mg->n_levels < 2 || mg->n_levels > DFEA_MG_MAX_LEVELS || blocks < 1 || bytes < 0) return -1;
+    return tail_level(mg, blocks < kClusterMax ? blocks : kClusterMax, bytes);
 }
 
 extern "C" int dfea_mg_setup(const dfea_mesh_view* mesh, dfea_mg* mg, const void* moduli, int32_t moduli_dtype,

@@ -182,6 +182,7 @@ _PROTOS = {
     "dfea_mg_dot": (ctypes.c_int, [c_i64, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "dfea_mg_lanczos_step": (ctypes.c_int, [c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_i32, c_vp, c_vp]),
     "dfea_mg_dense_max": (c_i64, []),
+    "dfea_mg_tail_level": (c_i32, [ctypes.POINTER(Mg), c_i32, c_i64]),
     "dfea_mg_lanczos_bound": (ctypes.c_double, [c_vp, c_i32]),
     "dfea_mg_setup": (ctypes.c_int, [ctypes.POINTER(MeshView), ctypes.POINTER(Mg), c_vp, c_i32, c_vp, c_vp]),
     "dfea_mg_vcycle": (ctypes.c_int, [ctypes.POINTER(MeshView), ctypes.POINTER(Mg), c_vp, c_i32, c_vp, c_vp, c_vp]),

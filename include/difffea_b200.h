@@ -550,6 +550,10 @@ int dfea_mg_setup(const dfea_mesh_view* mesh, dfea_mg* mg, const void* moduli, i
  * Jacobi-CG coefficients hist = (alpha_0, beta_0, alpha_1, ...), over the prefix before a breakdown (2.5 if
  * none), by Sturm-sequence bisection; -1 for bad arguments.  No GPU involved. */
 double dfea_mg_lanczos_bound(const double* hist, int32_t steps);
+/* Host arithmetic of the set-up: the first level whose cycle, with those below it, runs in one thread-block cluster of at
+ * most `blocks` blocks (a power of two, at most 16) with `bytes` of dynamic shared memory each, from level[].n; n_levels
+ * if none, -1 for bad arguments.  No GPU involved. */
+int32_t dfea_mg_tail_level(const dfea_mg* mg, int32_t blocks, int64_t bytes);
 /* z = one V-cycle applied to r (the moduli of the set-up). */
 int dfea_mg_vcycle(const dfea_mesh_view* mesh, const dfea_mg* mg, const void* moduli, int32_t moduli_dtype,
                    const double* r, double* z, void* stream);
