@@ -146,14 +146,32 @@ class CudaMesh:
     def n_dof(self):
         return 2 * self.n_nodes
 
+    def _finish(self):
+        """
+        Wait for the arrays just written: another thread may use them on another stream as soon as the attribute that
+        says they are there is set, which is therefore set last.  (Inside a graph capture nothing has run to wait for.)
+        """
+        with torch.cuda.device(self.device):
+            stream = torch.cuda.current_stream()
+            if not torch.cuda.is_current_stream_capturing():
+                stream.synchronize()
+
     def ensure_grad32(self):
         """Build the FP32 copy of the gradients (the geometry of the FP32 inner operator) once."""
-        if self.grad32 is None:
-            self.grad32 = torch.empty(self.n_q * self.nen * self.stride * 2, dtype=torch.float32, device=self.device)
-            with torch.cuda.device(self.device):
-                _lib.call("dfea_mesh_grad_to_f32", self.view_ref, ptr(self.grad32), stream_handle())
-            self.view.grad32 = self.grad32.data_ptr()
-        return self.grad32
+        with self._lock:
+            if self.grad32 is None:
+                grad32 = torch.empty(self.n_q * self.nen * self.stride * 2, dtype=torch.float32, device=self.device)
+                with torch.cuda.device(self.device):
+                    _lib.call("dfea_mesh_grad_to_f32", self.view_ref, ptr(grad32), stream_handle())
+                self._finish()
+                self.view.grad32 = grad32.data_ptr()
+                self.grad32 = grad32
+            return self.grad32
+
+    @property
+    def indexable(self):
+        """Whether the slots of the node incidence fit 32 bits."""
+        return self.nen * self.stride < 2 ** 31
 
     def ensure_node_incidence(self):
         """
@@ -161,22 +179,26 @@ class CudaMesh:
         indices a * stride + e of its (element, local node) pairs, in increasing order.
         """
         with self._lock:
-            return self._node_incidence()
+            if self.node_elem is None:
+                incidence = self._launch_incidence()
+                self._finish()
+                self._publish_incidence(*incidence)
+            return self.node_elem_ptr, self.node_elem
 
-    def _node_incidence(self):
-        if self.node_elem is None:
-            S, nen, n, N, dev = self.stride, self.nen, self.n_el, self.n_nodes, self.device
-            if nen * S >= 2 ** 31:
-                raise ValueError("mesh too large for 32-bit incidence indices")
-            i32 = dict(dtype=torch.int32, device=dev)
-            ptr_, inc, work = torch.empty(N + 1, **i32), torch.empty(max(nen * n, 1), **i32), torch.empty(N, **i32)
-            with torch.cuda.device(dev):
-                _lib.call("dfea_mesh_node_incidence", self.view_ref, ptr(ptr_), ptr(inc), ptr(work), stream_handle())
-            self.node_elem = inc[:nen * n]
-            self.node_elem_ptr = ptr_
-            self.view.node_elem_ptr = self.node_elem_ptr.data_ptr()
-            self.view.node_elem = self.node_elem.data_ptr()
-        return self.node_elem_ptr, self.node_elem
+    def _launch_incidence(self):
+        """(ptr, slots), on their way on the current stream."""
+        if not self.indexable:
+            raise ValueError("mesh too large for 32-bit incidence indices")
+        slots, i32 = self.nen * self.n_el, dict(dtype=torch.int32, device=self.device)
+        ptr_, inc, work = (torch.empty(n, **i32) for n in (self.n_nodes + 1, max(slots, 1), self.n_nodes))
+        with torch.cuda.device(self.device):
+            _lib.call("dfea_mesh_node_incidence", self.view_ref, ptr(ptr_), ptr(inc), ptr(work), stream_handle())
+        return ptr_, inc[:slots]
+
+    def _publish_incidence(self, ptr_, inc):
+        self.view.node_elem_ptr, self.view.node_elem = ptr_.data_ptr(), inc.data_ptr()
+        self.node_elem_ptr = ptr_
+        self.node_elem = inc
 
     # A Gauss point's dN/dX is taken as Jinv^T dN/dxi when the fitted Jinv reproduces it to this, relative to its
     # largest entry: rounding leaves ~1e-15, and what is below the tolerance stays far inside FP64 parity (1e-11).
@@ -191,20 +213,23 @@ class CudaMesh:
         """
         with self._lock:
             if self._frame_check is None:
-                if self.nen * self.stride >= 2 ** 31:                   # no 32-bit incidence
+                if not self.indexable:
                     self._frame_check = (float("inf"), 0.0, float("inf"))
                     return False
-                self._node_incidence()
+                incidence = self._launch_incidence() if self.node_elem is None else None
                 dev, S, nq = self.device, self.stride, self.n_q
                 nodes = self._nodes.detach().to(dev, torch.float64).contiguous()
                 frame = torch.empty(nq * 2 * S * 2, dtype=torch.float64, device=dev)
                 check = torch.empty(3, dtype=torch.float64, device=dev)
                 with torch.cuda.device(dev):
                     _lib.call("dfea_mesh_frame", self.view_ref, ptr(nodes), ptr(frame), ptr(check), stream_handle())
-                self._frame_check = tuple(check.tolist())
-                if not self.n_el or self._frame_check[2] <= self.FRAME_TOLERANCE:
-                    self.frame = frame
+                    result = tuple(check.tolist())               # waits for the frame and the incidence too
+                if incidence is not None:
+                    self._publish_incidence(*incidence)
+                if not self.n_el or result[2] <= self.FRAME_TOLERANCE:
                     self.view.frame = frame.data_ptr()
+                    self.frame = frame
+                self._frame_check = result
             return self.frame is not None
 
     def ensure_ref_frame(self):
@@ -230,8 +255,8 @@ class CudaMesh:
                 if self.n_el and diff > 1e-9 * scale:
                     raise ValueError("dN_dX does not match this package's reference gradients and quadrature; "
                                      "the reference-frame operator cannot be used for this problem")
+                self.view.jinv = jinv.data_ptr()
                 self.jinv = jinv.view(nq, 2, S, 2)
-                self.view.jinv = self.jinv.data_ptr()
             return self.jinv
 
     def moduli_numel_ref(self):

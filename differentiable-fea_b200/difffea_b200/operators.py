@@ -120,12 +120,13 @@ class CudaTangentOperator:
     v -> A(v) from moduli stored at the Gauss points (kernel (b)).  Holds the moduli of its linearisation point
     (``moduli``, layout ``code``: FP64 in the element reference frame where the mesh has one, else the 16 physical
     entries) and the Jacobi diagonal computed in the same pass of kernel (a); ``point`` is that linearisation point, where
-    the operator was made from one.
+    the operator was made from one.  ``gather``: physical moduli are applied in the gather form; chosen when the operator
+    is made, so that its sums are grouped alike for as long as it lives.
     """
 
-    def __init__(self, mesh, mesh_id, moduli, diag, precision="fp64", point=None):
+    def __init__(self, mesh, mesh_id, moduli, diag, precision="fp64", point=None, gather=False):
         self.mesh, self.mesh_id, self.moduli, self.diag, self.precision = mesh, mesh_id, moduli, diag, precision
-        self.point = point
+        self.point, self.gather = point, gather
         self._indefinite = None
         self.code = (_lib.DFEA_F32 if moduli.dtype == torch.float32 else
                      _lib.DFEA_F64REF if moduli.numel() == mesh.moduli_numel_ref() else _lib.DFEA_F64)
@@ -145,7 +146,7 @@ class CudaTangentOperator:
         """A(v); FP32 moduli apply to FP32 vectors, or to FP64 vectors with FP64 arithmetic."""
         if v.dtype != self.dtype and not (self.dtype == torch.float32 and v.dtype == torch.float64):
             raise ValueError(f"this operator applies {self.dtype} vectors, got {v.dtype}")
-        return ops.run(ops.tangent_apply, self.mesh_id, self.moduli, v.contiguous())
+        return ops.run(ops.tangent_apply, self.mesh_id, self.moduli, v.contiguous(), self.gather)
 
     @property
     def dtype(self):
@@ -234,7 +235,7 @@ def make_A_operator_cuda(u, theta, params, precision="fp64"):
     mesh, mid = _prepare(u, theta, params)
     if precision == "fp32":
         mesh.ensure_grad32()
-        if mesh.nen * mesh.stride < 2 ** 31:
+        if mesh.indexable:
             mesh.ensure_node_incidence()
     if precision == "fp64" and mesh.ensure_frame():
         C, diag, _ = ops.run(ops.frame_moduli, mid, _f64c(u), _f64c(theta), *ops.frame_material(params), True, False)
@@ -243,7 +244,7 @@ def make_A_operator_cuda(u, theta, params, precision="fp64"):
                           precision == "fp32", True)
     _LAST_DIAG.clear()
     _LAST_DIAG[_diag_key(u, theta, mesh)] = (weakref.ref(u), weakref.ref(theta), diag)
-    return CudaTangentOperator(mesh, mid, C, diag, precision, _Linearisation(u, theta, params))
+    return CudaTangentOperator(mesh, mid, C, diag, precision, _Linearisation(u, theta, params), mesh.indexable)
 
 
 def make_tangent_operator(kind, u, theta, params):

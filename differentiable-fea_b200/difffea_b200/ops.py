@@ -6,7 +6,7 @@ Each op is a thin shim: it allocates its outputs through torch's caching allocat
 (``register_mesh``) because a mesh is a bundle of device arrays, not one tensor.
 
     torch.ops.difffea_b200.qp_moduli(mesh_id, u, theta, model, scalable, mat_p, fp32, with_diag) -> (C, diag)
-    torch.ops.difffea_b200.tangent_apply(mesh_id, C, v) -> y               kernel (b)
+    torch.ops.difffea_b200.tangent_apply(mesh_id, C, v, gather=False) -> y   kernel (b)
     torch.ops.difffea_b200.residual(mesh_id, u, theta, model, scalable, mat_p, f, load_factor) -> (R, |R|^2, energy)
     torch.ops.difffea_b200.element_sensitivity(mesh_id, u, lam, model, scalable, mat_p) -> g      kernel (d)
     torch.ops.difffea_b200.element_fields(mesh_id, u, theta, model, scalable, mat_p) -> (7, n_el)
@@ -150,7 +150,8 @@ def _(mesh_id, u, theta, model, scalable, mat_p, fp32, with_diag):
 
 
 @_functional_op("tangent_apply")
-def tangent_apply(mesh_id: int, C: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
+def tangent_apply(mesh_id: int, C: torch.Tensor, v: torch.Tensor, gather: bool = False) -> torch.Tensor:
+    """A(v); ``gather``: physical moduli too in the gather form, which needs the mesh's node incidence."""
     mesh = _mesh(mesh_id)
     fp32 = v.dtype == torch.float32
     if C.dtype == torch.float32:
@@ -169,7 +170,8 @@ def tangent_apply(mesh_id: int, C: torch.Tensor, v: torch.Tensor) -> torch.Tenso
         return y
     dt = _lib.DFEA_F32 if fp32 else _lib.DFEA_F64
     cdt = _lib.DFEA_F32 if C.dtype == torch.float32 else _lib.DFEA_F64
-    if mesh.node_elem is not None:
+    if gather:
+        mesh.ensure_node_incidence()
         # two launches, at every size: FP32 colour / gather us: 65k Tri6 54 / 17, 90k Q4 43 / 13, 640k Q4 74 / 63, 810k Q9
         # 283 / 222, 1M Q4 109 / 97, 4M Q4 356 / 351, 3.9M Tri3 171 / 144
         fe = torch.empty(int(_lib.load().dfea_gather_work_bytes(mesh.view_ref, dt)), dtype=torch.uint8, device=mesh.device)
@@ -180,7 +182,7 @@ def tangent_apply(mesh_id: int, C: torch.Tensor, v: torch.Tensor) -> torch.Tenso
 
 
 @tangent_apply.register_fake
-def _(mesh_id, C, v):
+def _(mesh_id, C, v, gather=False):
     return torch.empty_like(v)
 
 
