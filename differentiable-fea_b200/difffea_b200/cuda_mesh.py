@@ -185,6 +185,24 @@ class CudaMesh:
                 self._publish_incidence(*incidence)
             return self.node_elem_ptr, self.node_elem
 
+    def ensure_gather(self):
+        """Whether the gather form can be used; builds its incidence, but not inside a graph capture."""
+        if self.node_elem is None and self.indexable and not torch.cuda.is_current_stream_capturing():
+            self.ensure_node_incidence()
+        return self.node_elem is not None
+
+    def gather_view(self):
+        """
+        (reference to a view with the node incidence, what has to live until the call is made).  Inside a capture of a
+        mesh that has none yet it is built by the graph, for this call only: eager calls must not see it.
+        """
+        if self.node_elem is not None or self.ensure_gather():
+            return self.view_ref, None
+        ptr_, inc = self._launch_incidence()
+        view = _lib.MeshView.from_buffer_copy(self.view)
+        view.node_elem_ptr, view.node_elem = ptr_.data_ptr(), inc.data_ptr()
+        return ctypes.byref(view), (view, ptr_, inc)
+
     def _launch_incidence(self):
         """(ptr, slots), on their way on the current stream."""
         if not self.indexable:
@@ -209,10 +227,13 @@ class CudaMesh:
         The FP64 frame of the mesh (Jinv of every Gauss point, fitted to the packed dN/dX) with the node incidence
         its node passes need, built once; returns whether the frame kernels can be used.  A problem whose dN/dX is
         not Jinv^T dN/dxi with this package's reference gradients (another quadrature, FP32 geometry) keeps the
-        kernels that read dN/dX.
+        kernels that read dN/dX.  So does a call inside a graph capture before the frame was built: the fit is read
+        on the host.
         """
         with self._lock:
             if self._frame_check is None:
+                if torch.cuda.is_current_stream_capturing():
+                    return False
                 if not self.indexable:
                     self._frame_check = (float("inf"), 0.0, float("inf"))
                     return False

@@ -235,16 +235,16 @@ def make_A_operator_cuda(u, theta, params, precision="fp64"):
     mesh, mid = _prepare(u, theta, params)
     if precision == "fp32":
         mesh.ensure_grad32()
-        if mesh.indexable:
-            mesh.ensure_node_incidence()
-    if precision == "fp64" and mesh.ensure_frame():
+    framed = precision == "fp64" and mesh.ensure_frame()
+    gather = mesh.ensure_gather()
+    if framed:
         C, diag, _ = ops.run(ops.frame_moduli, mid, _f64c(u), _f64c(theta), *ops.frame_material(params), True, False)
     else:
         C, diag = ops.run(ops.qp_moduli, mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)),
                           precision == "fp32", True)
     _LAST_DIAG.clear()
     _LAST_DIAG[_diag_key(u, theta, mesh)] = (weakref.ref(u), weakref.ref(theta), diag)
-    return CudaTangentOperator(mesh, mid, C, diag, precision, _Linearisation(u, theta, params), mesh.indexable)
+    return CudaTangentOperator(mesh, mid, C, diag, precision, _Linearisation(u, theta, params), gather)
 
 
 def make_tangent_operator(kind, u, theta, params):

@@ -161,21 +161,21 @@ def tangent_apply(mesh_id: int, C: torch.Tensor, v: torch.Tensor, gather: bool =
     y = torch.empty_like(v)
     if C.numel() == mesh.moduli_numel_ref():
         # reference-frame moduli: the gather form, with its element results in scratch of this call
-        mesh.ensure_node_incidence()
+        view, keep = mesh.gather_view()
         fe = torch.empty(int(_lib.load().dfea_gather_work_bytes(mesh.view_ref, _lib.DFEA_F64)), dtype=torch.uint8,
                          device=mesh.device)
         code = _lib.DFEA_F64REF if C.dtype == torch.float64 else _lib.DFEA_F32REF
-        _lib.call("dfea_tangent_apply_gather", mesh.view_ref, ptr(C), code, ptr(v), ptr(y),
+        _lib.call("dfea_tangent_apply_gather", view, ptr(C), code, ptr(v), ptr(y),
                   _lib.DFEA_F32 if fp32 else _lib.DFEA_F64, ptr(fe), stream_handle())
         return y
     dt = _lib.DFEA_F32 if fp32 else _lib.DFEA_F64
     cdt = _lib.DFEA_F32 if C.dtype == torch.float32 else _lib.DFEA_F64
     if gather:
-        mesh.ensure_node_incidence()
+        view, keep = mesh.gather_view()
         # two launches, at every size: FP32 colour / gather us: 65k Tri6 54 / 17, 90k Q4 43 / 13, 640k Q4 74 / 63, 810k Q9
         # 283 / 222, 1M Q4 109 / 97, 4M Q4 356 / 351, 3.9M Tri3 171 / 144
         fe = torch.empty(int(_lib.load().dfea_gather_work_bytes(mesh.view_ref, dt)), dtype=torch.uint8, device=mesh.device)
-        _lib.call("dfea_tangent_apply_gather", mesh.view_ref, ptr(C), cdt, ptr(v), ptr(y), dt, ptr(fe), stream_handle())
+        _lib.call("dfea_tangent_apply_gather", view, ptr(C), cdt, ptr(v), ptr(y), dt, ptr(fe), stream_handle())
         return y
     _lib.call("dfea_tangent_apply", mesh.view_ref, ptr(C), cdt, ptr(v), ptr(y), dt, stream_handle())
     return y
@@ -247,9 +247,9 @@ def node_fields(mesh_id: int, elem: torch.Tensor) -> torch.Tensor:
     mesh = _mesh(mesh_id)
     if elem.shape != (7, mesh.n_el) or elem.dtype != torch.float64 or not elem.is_contiguous():
         raise ValueError("elem must be the contiguous (7, n_el) float64 output of element_fields")
-    mesh.ensure_node_incidence()
+    view, keep = mesh.gather_view()
     out = torch.empty(6, mesh.n_nodes, dtype=torch.float64, device=mesh.device)
-    _lib.call("dfea_node_fields", mesh.view_ref, ptr(elem), ptr(out), stream_handle())
+    _lib.call("dfea_node_fields", view, ptr(elem), ptr(out), stream_handle())
     return out
 
 

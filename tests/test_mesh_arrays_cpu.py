@@ -63,6 +63,18 @@ def test_nothing_is_announced_before_the_wait(log, build, launch, attributes):
     assert len(events) == 2                        # once
 
 
+def test_inside_a_capture_nothing_is_announced(log, monkeypatch):
+    """What a graph would write is there after its first replay only: such a call takes the forms that need none of it."""
+    mesh, events = log
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    assert not mesh.ensure_frame() and not mesh.ensure_gather() and not events
+    view, keep = mesh.gather_view()                # an incidence of this call's own
+    assert events == [("dfea_mesh_node_incidence", [])] and view._obj.node_elem == keep[2].data_ptr()
+    assert mesh.node_elem is None and not mesh.view.node_elem
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    assert mesh.ensure_frame() and mesh.ensure_gather() and mesh.gather_view()[1] is None
+
+
 def test_the_frame_and_its_incidence_are_announced_after_their_read(log):
     mesh, events = log
     assert mesh.ensure_frame()                     # reading the fit error waits for both
@@ -79,8 +91,8 @@ def test_the_product_form_does_not_depend_on_what_the_mesh_has_built(monkeypatch
     C, v = torch.zeros(16, dtype=torch.float64), torch.zeros(18, dtype=torch.float64)
     for incidence in (None, torch.zeros(16, dtype=torch.int32)):
         mesh = SimpleNamespace(device=v.device, n_dof=18, node_elem=incidence, view_ref=ctypes.byref(_mesh().view),
-                               moduli_numel_ref=lambda: 10, moduli_numel=lambda *a: 16,
-                               ensure_node_incidence=lambda: None, ensure_grad32=lambda: None)
+                               moduli_numel_ref=lambda: 10, moduli_numel=lambda *a: 16, ensure_grad32=lambda: None)
+        mesh.gather_view = lambda: (mesh.view_ref, None)
         monkeypatch.setattr(ops, "_mesh", lambda mesh_id: mesh)
         ops.tangent_apply.implementation(0, C, v, gather)
     assert called == 2 * ["dfea_tangent_apply_gather" if gather else "dfea_tangent_apply"]
