@@ -2,6 +2,8 @@
 // hardware barrier, and sums over the cluster that ride on it.
 #pragma once
 
+#include <mutex>
+
 #include "dfea_common.cuh"
 
 namespace dfea {
@@ -83,5 +85,45 @@ struct ClusterExchange {
     }
     __device__ __forceinline__ void two(double v0, double v1, double& t0, double& t1) { run<true>(v0, v1, t0, t1); }
 };
+
+// What clusters of a kernel can be on the current device: the dynamic shared memory a block may take, and the most blocks
+// (a power of two) of a cluster that can be resident with that much each.  16 blocks and 225 KB on a whole B200; on a
+// partition of one a large cluster may find no place, and its launch would fail.  Nothing: the kernel cannot be set up.
+struct ClusterRoom {
+    int blocks = 0, bytes = 0;
+};
+template <auto Kernel>
+const ClusterRoom& cluster_room(int threads) {
+    static std::once_flag once[64];
+    static ClusterRoom room[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    std::call_once(once[dev], [dev, threads] {
+        int most = 0;
+        cudaFuncAttributes fa;
+        if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+            cudaFuncGetAttributes(&fa, Kernel) == cudaSuccess &&
+            cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes) == cudaSuccess &&
+            cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.blockDim = dim3(threads);
+            cfg.dynamicSmemBytes = most - fa.sharedSizeBytes;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            for (int size = kClusterMax; size >= 1 && room[dev].blocks == 0; size /= 2) {
+                int clusters = 0;
+                attr[0].val.clusterDim.x = size;
+                cfg.gridDim = dim3(size);
+                if (cudaOccupancyMaxActiveClusters(&clusters, Kernel, &cfg) == cudaSuccess && clusters > 0) room[dev].blocks = size;
+            }
+            room[dev].bytes = most - (int)fa.sharedSizeBytes;
+        }
+        (void)cudaGetLastError();  // a size that finds no place is no error of the caller's
+    });
+    return room[dev];
+}
 
 }  // namespace dfea

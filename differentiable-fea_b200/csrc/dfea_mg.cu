@@ -13,7 +13,6 @@
 // Everything here is deterministic: node-centric gathers in a fixed order, single-block reductions.
 #include <cmath>
 #include <cstdio>
-#include <mutex>
 #include <new>
 #include <utility>
 
@@ -1186,33 +1185,11 @@ __global__ void __launch_bounds__(kMgClusterThreads, 1) k_mg_tail(const __grid_c
     cluster_barrier();  // no block leaves while another may read its shared memory
 }
 
-// The kernel set up for clusters on the current device: *bytes becomes the dynamic shared memory a block may take.
-template <auto Kernel>
-static int cluster_configure(int64_t* bytes) {
-    static std::once_flag once[64];
-    static int result[64] = {0}, most_bytes[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-    std::call_once(once[dev], [dev] {
-        int most = 0;
-        int rc = check_cuda(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
-        cudaFuncAttributes fa;
-        if (!rc) rc = check_cuda(cudaFuncGetAttributes(&fa, Kernel), "cudaFuncGetAttributes");
-        if (!rc) most_bytes[dev] = most - (int)fa.sharedSizeBytes;
-        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most_bytes[dev]),
-                                 "cudaFuncSetAttribute");
-        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "cudaFuncSetAttribute");
-        result[dev] = rc;
-    });
-    if (bytes) *bytes = most_bytes[dev];
-    return result[dev];
-}
-
-// A launch of clusters of `size` blocks (a power of two of at most kClusterMax).
+// A launch of clusters of `size` blocks (a power of two of at most cluster_room's).
 template <auto Kernel, typename... Args>
 static int launch_clusters(int n_clusters, int size, size_t smem, bool pdl, cudaStream_t s, const Args&... args) {
-    const int rc = cluster_configure<Kernel>(nullptr);
-    if (rc) return rc;
+    if (size > cluster_room<Kernel>(kMgClusterThreads).blocks)
+        return set_error(DFEA_ERR_UNSUPPORTED, "multigrid: clusters of %d blocks find no place on this device", size);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = size;
@@ -1230,7 +1207,7 @@ static int launch_clusters(int n_clusters, int size, size_t smem, bool pdl, cuda
 }
 
 // blocks for a largest level of n nodes: about 64 nodes a block, 16 blocks (or the fewer that are allowed) at the most
-static int mg_cluster_size(int64_t n_nodes, int most = kClusterMax) {
+static int mg_cluster_size(int64_t n_nodes, int most) {
     int size = 1;
     while (2 * size <= most && (int64_t)size * 64 < n_nodes) size *= 2;
     return size;
@@ -1558,10 +1535,14 @@ static int tail_level(const dfea_mg* mg, int blocks, int64_t bytes) {
     }
     return mg->n_levels;
 }
+// blocks of the tail's clusters, 0: none (the Lanczos kernel needs less shared memory per node than the cycle's)
+static int tail_blocks() {
+    const int a = cluster_room<k_mg_tail>(kMgClusterThreads).blocks, b = cluster_room<k_mg_tail_lanczos>(kMgClusterThreads).blocks;
+    return a < b ? a : b;
+}
 static int tail_start(const dfea_mg* mg) {
-    int64_t bytes = 0;
-    if (!mg->stencil || cluster_configure<k_mg_tail>(&bytes)) return mg->n_levels;
-    return tail_level(mg, kClusterMax, bytes);
+    if (!mg->stencil || tail_blocks() == 0) return mg->n_levels;
+    return tail_level(mg, tail_blocks(), cluster_room<k_mg_tail>(kMgClusterThreads).bytes);
 }
 
 // restriction of level l's residual, the cycle of levels l + 1 .. L - 1 and the prolongation into x, in one launch
@@ -1575,7 +1556,7 @@ static int launch_tail(const dfea_mesh_view* mesh, const dfea_mg* mg, int l, dou
     T.Ainv = mg->Ainv;
     T.n_levels = mg->n_levels - (l + 1);
     T.degree = mg->degree;
-    const int size = mg_cluster_size(mg->level[l + 1].n / 2);
+    const int size = mg_cluster_size(mg->level[l + 1].n / 2, tail_blocks());
     int at = 0;
     for (int k = 0; k < T.n_levels; ++k) {
         const dfea_mg_level& c = mg->level[l + 1 + k];
@@ -1882,7 +1863,7 @@ static int tail_lanczos(const dfea_mg* mg, int t, cudaStream_t s) {
     const int L = mg->n_levels;
     MgLanczosTail T = {};
     T.steps = mg->lanczos_steps;
-    T.size = mg_cluster_size(mg->level[t].n / 2);
+    T.size = mg_cluster_size(mg->level[t].n / 2, tail_blocks());
     int most = 0, rc;
     for (int k = 0; k < L - 1 - t; ++k) {
         const dfea_mg_level& lv = mg->level[t + k];

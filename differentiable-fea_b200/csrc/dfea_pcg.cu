@@ -967,34 +967,16 @@ int launch_iteration_any(const dfea_pcg& h, cudaStream_t s, cudaGraphConditional
     return launch_iteration<float, float>(h, s, cond, with_cond);
 }
 
-template <auto Kernel>
-int cluster_configure() {
-    static std::once_flag once[64];
-    static int result[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-    std::call_once(once[dev], [dev] {
-        int most = 0;
-        int rc = check_cuda(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
-        cudaFuncAttributes fa;
-        if (!rc) rc = check_cuda(cudaFuncGetAttributes(&fa, Kernel), "cudaFuncGetAttributes");
-        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                      most - (int)fa.sharedSizeBytes), "cudaFuncSetAttribute");
-        if (!rc) rc = check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "cudaFuncSetAttribute");
-        result[dev] = rc;
-    });
-    return result[dev];
-}
-
 constexpr int kClusterSmem = 220 * 1024;  // dynamic shared memory a block may take (of 227 KB)
 
-// The cluster of a mesh: blocks (a power of two) and shared memory, or 0 blocks where
+// The cluster of a mesh: blocks (a power of two, at most `most`) and shared memory, or 0 blocks where
 // the mesh does not fit.  max_slots(blocks, nb, slices): the most fe entries of a block's node range.
 template <int NEN, int NQ, bool SPLIT, typename MaxSlots>
-int cluster_layout(const dfea_mesh_view& mv, bool block_jacobi, ClusterLayout* out, MaxSlots&& max_slots) {
+int cluster_layout(const dfea_mesh_view& mv, bool block_jacobi, int most, ClusterLayout* out, MaxSlots&& max_slots) {
     using Cfg = ClusterCfg<NEN, NQ, SPLIT>;
+    if (most < 1) return 0;
     int blocks = 1;
-    while (blocks < kClusterMax && (int64_t)blocks * Cfg::TEAMS * 32 < mv.n_el) blocks *= 2;
+    while (2 * blocks <= most && (int64_t)blocks * Cfg::TEAMS * 32 < mv.n_el) blocks *= 2;
     const int64_t nb = (mv.n_nodes + blocks - 1) / blocks;
     if (nb >= (1 << 16) || 96 * nb > kClusterSmem) return 0;  // five vectors and an entry per node at the least
     const int slices = (int)((nb + 31) / 32);
@@ -1039,8 +1021,6 @@ int launch_cluster(const dfea_pcg& h, cudaStream_t s, double rtol, int max_iter)
         const auto launch = [&](auto split_c) -> int {
             constexpr bool SPLIT = decltype(split_c)::value;
             constexpr auto kernel = k_pcg_cluster<NEN, NQ, SD, BJ, SPLIT>;
-            const int rc2 = cluster_configure<kernel>();
-            if (rc2) return rc2;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = h.cluster_blocks;
@@ -1074,6 +1054,7 @@ int launch_cluster_any(const dfea_pcg& h, cudaStream_t s, double rtol, int max_i
 }
 
 // Lay the cluster out (exact entry counts of the node ranges, read once) and write the slot map of the handle.
+template <typename SD, bool BJ>
 int prepare_cluster(dfea_pcg* h) {
     const dfea_mesh_view& mv = h->mesh;
     cudaStream_t s = cudaStreamPerThread;
@@ -1094,17 +1075,30 @@ int prepare_cluster(dfea_pcg* h) {
             for (int i = 0; i < blocks; ++i) most = total[i] > most ? total[i] : most;
             return most;
         };
-        return cluster_split<NEN, NQ>(mv.n_el) ? cluster_layout<NEN, NQ, true>(mv, h->block, &h->cluster, max_slots)
-                                               : cluster_layout<NEN, NQ, false>(mv, h->block, &h->cluster, max_slots);
+        const auto layout = [&](auto split_c) -> int {
+            constexpr bool SPLIT = decltype(split_c)::value;
+            constexpr auto kernel = k_pcg_cluster<NEN, NQ, SD, BJ, SPLIT>;
+            const ClusterRoom& room = cluster_room<kernel>(ClusterCfg<NEN, NQ, SPLIT>::NT);
+            if (room.bytes < kClusterSmem) return 0;
+            return cluster_layout<NEN, NQ, SPLIT>(mv, BJ, capped(room.blocks, h->grid_cap), &h->cluster, max_slots);
+        };
+        if constexpr (NQ > 1)
+            if (cluster_split<NEN, NQ>(mv.n_el)) return layout(std::true_type{});
+        return layout(std::false_type{});
     });
     if (rc) return rc;
     if (h->cluster_blocks == 0)
-        return set_error(DFEA_ERR_UNSUPPORTED, "dfea_pcg_create: the mesh does not fit the shared memory of a cluster");
+        return set_error(DFEA_ERR_UNSUPPORTED, "dfea_pcg_create: the mesh does not fit the shared memory of a cluster on this device");
     k_pcg_cluster_map<<<grid_for(mv.n_nodes, kThreads, 8), kThreads, 0, s>>>(
         kernel_mesh(mv), h->cluster.nb, h->cluster.slices, h->slice_base(), mv.node_elem_ptr, mv.node_elem, h->slot_map());
     note_launches(1);
     if ((rc = launch_check("cluster PCG map"))) return rc;
     return check_cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+}
+
+int prepare_cluster_any(dfea_pcg* h) {
+    if (h->vec_dtype == DFEA_F64REF) return h->block ? prepare_cluster<double, true>(h) : prepare_cluster<double, false>(h);
+    return h->block ? prepare_cluster<float, true>(h) : prepare_cluster<float, false>(h);
 }
 
 template <typename T, bool BJ = false>
@@ -1244,7 +1238,7 @@ extern "C" int dfea_pcg_create(const dfea_mesh_view* mesh, const void* moduli, c
         return set_error(DFEA_ERR_INVALID, "dfea_pcg_create: the gather form needs the mesh's node incidence");
     }
     if (h->clustered) {  // captures nothing, and every solve resets the state it uses
-        rc = prepare_cluster(h);
+        rc = prepare_cluster_any(h);
         if (!rc) {
             *out = h;
             return DFEA_OK;

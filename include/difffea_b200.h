@@ -72,8 +72,9 @@ extern "C" {
                                 * (implies DFEA_PCG_GATHER) */
 #define DFEA_PCG_CLUSTER 128   /* dfea_pcg_create flag: the whole solve in one launch of a thread-block cluster with
                                 * its vectors in distributed shared memory (DFEA_F32REF or DFEA_F64REF moduli, node
-                                * incidence; no block cap).  Alone: DFEA_ERR_UNSUPPORTED for a mesh that does not
-                                * fit; beside DFEA_PCG_GATHER or _FUSED: taken where the mesh fits, else that form.
+                                * incidence), of at most 16 blocks, DFEA_PCG_MAX_BLOCKS and what the device can
+                                * place.  Alone: DFEA_ERR_UNSUPPORTED for a mesh that does not fit such a cluster;
+                                * beside DFEA_PCG_GATHER or _FUSED: taken where the mesh fits, else that form.
                                 * The creation reads the mesh's incidence, which has to be complete by then. */
 /* dfea_pcg_create option: at most n blocks per launch (n < 2^23; 0 = as many as the GPU holds at
  * once).  For solves that share the GPU with solves on other streams. */
