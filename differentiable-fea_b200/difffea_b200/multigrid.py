@@ -281,7 +281,6 @@ class Multigrid:
                 setattr(dst, name, fptr((l, name)))
         for name in ("Ainv", "dense_work", "coef", "lscal", "lhist", "dot_work", "scal", "stencil"):
             setattr(h, name, fptr(name))
-        _lib.call("dfea_mg_maps", mesh.view_ref, ctypes.byref(h), stream_handle())
         h.pcg = fptr("pcg")
         h.pcg_state = fptr("pcg_state") if graphs else None
         h.graphs = None
@@ -293,6 +292,7 @@ class Multigrid:
                                        dtype=torch.uint8, device=dev)
             h.fe_work = self.fe_work.data_ptr()
         with torch.cuda.device(dev):     # the maps are there before another stream's set-up may read them
+            _lib.call("dfea_mg_maps", mesh.view_ref, ctypes.byref(h), stream_handle())
             torch.cuda.current_stream().synchronize()
         self.C, self.code = None, None
         self.id = ops.register_handle(self)
