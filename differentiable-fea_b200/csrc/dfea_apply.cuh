@@ -236,7 +236,7 @@ __device__ __forceinline__ bool apply_tiles(const Mesh& m, int64_t e0, int64_t e
 template <int NEN, int NQ, typename SD, typename T, bool DOT>
 __global__ void __launch_bounds__(128)
 k_apply(Mesh m, int64_t e0, int64_t e1, const SD* __restrict__ C, const SD* __restrict__ G,
-        const T* v, T* __restrict__ y, RedSite site, const int* __restrict__ done) {
+        const T* v, T* y, RedSite site, const int* done) {
     using T2 = v2_t<T>;
     extern __shared__ __align__(16) unsigned char smem[];
     T2* y2 = reinterpret_cast<T2*>(y);
@@ -247,7 +247,7 @@ k_apply(Mesh m, int64_t e0, int64_t e1, const SD* __restrict__ C, const SD* __re
         [&]() -> bool {
             // from here on v, y and the solver state may come from the predecessor (PDL)
             grid_dependency_wait();
-            if (DOT && done != nullptr && *done) return false;  // solve finished: no-op iteration of the graph
+            if (DOT && done != nullptr && load_fresh(done)) return false;  // solve finished: no-op iteration of the graph
             grid_dependents_launch();
             return true;
         },
@@ -255,7 +255,7 @@ k_apply(Mesh m, int64_t e0, int64_t e1, const SD* __restrict__ C, const SD* __re
         [&](int64_t, const int (&node)[NEN], const int (&fix)[NEN], const T (&fx)[NEN], const T (&fy)[NEN]) {
 #pragma unroll
             for (int a = 0; a < NEN; ++a) {
-                T2 t = y2[node[a]];
+                T2 t = load_fresh(y2 + node[a]);
                 if (!(fix[a] & 1)) t.x += fx[a];
                 if (!(fix[a] & 2)) t.y += fy[a];
                 y2[node[a]] = t;
@@ -277,7 +277,7 @@ k_apply(Mesh m, int64_t e0, int64_t e1, const SD* __restrict__ C, const SD* __re
 template <int NEN, int NQ, typename SD, typename T, bool DOT>
 __global__ void __launch_bounds__(128)
 k_apply_elem(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, const T* v,
-             T* __restrict__ fe, RedSite site, const int* __restrict__ done) {
+             T* __restrict__ fe, RedSite site, const int* done) {
     using T2 = v2_t<T>;
     extern __shared__ __align__(16) unsigned char smem[];
     T2* fe2 = reinterpret_cast<T2*>(fe);
@@ -288,7 +288,7 @@ k_apply_elem(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, const T
         m, 0, m.n_el, C, G, smem, curv,
         [&]() -> bool {
             grid_dependency_wait();
-            if (DOT && done != nullptr && *done) return false;
+            if (DOT && done != nullptr && load_fresh(done)) return false;
             grid_dependents_launch();
             return true;
         },
@@ -310,7 +310,7 @@ k_apply_elem(Mesh m, const SD* __restrict__ C, const SD* __restrict__ G, const T
 // incidence order (fixed, so the sum is reproducible).
 template <typename T>
 __device__ __forceinline__ v2_t<T> node_sum(const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
-                                            const v2_t<T>* __restrict__ fe2, int64_t n) {
+                                            const v2_t<T>* fe2, int64_t n) {
     T sx = T(0), sy = T(0);
     int j = inc_ptr[n];
     const int j1 = inc_ptr[n + 1];
@@ -488,7 +488,7 @@ __device__ __forceinline__ bool apply_tiles_ref(const Mesh& m, int64_t e0, int64
 template <int NEN, int NQ, typename T, bool DOT>
 __global__ void __launch_bounds__(128)
 k_apply_ref(Mesh m, int64_t e0, int64_t e1, const float* __restrict__ C, const RefGrad<NEN, NQ> rg,
-            const T* v, T* __restrict__ y, RedSite site, const int* __restrict__ done) {
+            const T* v, T* y, RedSite site, const int* done) {
     using T2 = v2_t<T>;
     extern __shared__ __align__(16) unsigned char smem[];
     T2* y2 = reinterpret_cast<T2*>(y);
@@ -498,7 +498,7 @@ k_apply_ref(Mesh m, int64_t e0, int64_t e1, const float* __restrict__ C, const R
         m, e0, e1, C, rg, smem, curv,
         [&]() -> bool {
             grid_dependency_wait();
-            if (DOT && done != nullptr && *done) return false;
+            if (DOT && done != nullptr && load_fresh(done)) return false;
             grid_dependents_launch();
             return true;
         },
@@ -506,7 +506,7 @@ k_apply_ref(Mesh m, int64_t e0, int64_t e1, const float* __restrict__ C, const R
         [&](int64_t, const int (&node)[NEN], const int (&fix)[NEN], const T (&fx)[NEN], const T (&fy)[NEN]) {
 #pragma unroll
             for (int a = 0; a < NEN; ++a) {
-                T2 t = y2[node[a]];
+                T2 t = load_fresh(y2 + node[a]);
                 if (!(fix[a] & 1)) t.x += fx[a];
                 if (!(fix[a] & 2)) t.y += fy[a];
                 y2[node[a]] = t;
@@ -525,7 +525,7 @@ k_apply_ref(Mesh m, int64_t e0, int64_t e1, const float* __restrict__ C, const R
 template <int NEN, int NQ, typename SD, typename T, bool DOT>
 __global__ void __launch_bounds__(FrameCfg<NEN, NQ>::NT, FrameCfg<NEN, NQ>::MINB)
 k_apply_ref_elem(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, const T* v,
-                 T* __restrict__ fe, RedSite site, const int* __restrict__ done) {
+                 T* __restrict__ fe, RedSite site, const int* done) {
     using T2 = v2_t<T>;
     constexpr int NT = FrameCfg<NEN, NQ>::NT;
     __shared__ FrameShared<NEN, NQ, T> sh;
@@ -537,7 +537,7 @@ k_apply_ref_elem(Mesh m, const SD* __restrict__ C, const RefGrad<NEN, NQ> rg, co
         m, C, rg, sh, curv,
         [&]() -> bool {
             grid_dependency_wait();
-            if (DOT && done != nullptr && *done) return false;
+            if (DOT && done != nullptr && load_fresh(done)) return false;
             grid_dependents_launch();
             return true;
         },

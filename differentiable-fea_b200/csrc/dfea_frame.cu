@@ -389,7 +389,7 @@ template <bool MASK, bool NORM>
 __global__ void __launch_bounds__(kThreads)
 k_frame_node_residual(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
                       const double* fe, const double* __restrict__ f, double lf, double* __restrict__ R,
-                      RedSite site, double* __restrict__ out_norm2, const double* __restrict__ part, int n_part,
+                      RedSite site, double* __restrict__ out_norm2, const double* part, int n_part,
                       double* __restrict__ out_energy) {
     grid_dependency_wait();
     grid_dependents_launch();
@@ -414,7 +414,7 @@ k_frame_node_residual(Mesh m, const int32_t* __restrict__ inc_ptr, const int32_t
             if (threadIdx.x == 0 && out_norm2) *out_norm2 = tot[0];
             if (out_energy) {
                 double E = 0.0;
-                for (int i = threadIdx.x; i < n_part; i += kThreads) E += __ldcg(part + i);
+                for (int i = threadIdx.x; i < n_part; i += kThreads) E += load_fresh(part + i);
                 E = block_sum<kThreads>(E);
                 if (threadIdx.x == 0) *out_energy = E;
             }
