@@ -74,9 +74,12 @@ def strain_energy(u, theta, params):
 # ---------------------------------------------------------------------------------------------
 # tangent operator
 # ---------------------------------------------------------------------------------------------
-def _version(t):
-    """The tensor's version counter, or None where torch keeps none."""
-    return None if t.is_inference() else t._version
+def _versions(*tensors):
+    """The tensors' version counters, or None where torch keeps none (inference mode)."""
+    try:
+        return [getattr(t, "_version", 0) for t in tensors]
+    except RuntimeError:
+        return None
 
 
 class _Linearisation:
@@ -85,19 +88,18 @@ class _Linearisation:
     blocks are computed from when a solve asks for them later.  Holds the tensors themselves; ``unchanged`` is False
     once one of them was written to (or where torch keeps no version of it).
     """
+    __slots__ = ("u", "theta", "material", "versions", "__weakref__")
 
     def __init__(self, u, theta, params):
-        self.u, self.theta = (t.detach() if t.requires_grad else t for t in (u, theta))
-        self.material = {k: params[k] for k in ("material", "mat_p", "mat_scalable", "mu0", "lmbda0", "nodes") if k in params}
-        self.versions = self._versions()
-
-    def _versions(self):
-        tensors = (self.u, self.theta, *(t for t in self.material.values() if torch.is_tensor(t)))
-        return [_version(t) for t in tensors]
+        self.u = u.detach() if u.requires_grad else u
+        self.theta = theta.detach() if theta.requires_grad else theta
+        keys = ("material", "mat_p", "mat_scalable") if "material" in params else ("mu0", "lmbda0", "nodes")
+        self.material = {k: params[k] for k in keys}
+        self.versions = _versions(self.u, self.theta, *self.material.values())
 
     @property
     def unchanged(self):
-        return None not in self.versions and self.versions == self._versions()
+        return self.versions is not None and self.versions == _versions(self.u, self.theta, *self.material.values())
 
     def physical(self, mesh_id):
         """(the 16 physical moduli per Gauss point, the Jacobi diagonal) by the kernels that read dN/dX."""
@@ -160,7 +162,7 @@ class CudaTangentOperator:
         """
         from difffea_b200.krylov import DevicePCG
         from difffea_b200.workspace import pcg_form_for
-        if self._indefinite is not None and self._indefinite[0] is diag and self._indefinite[1] == _version(diag):
+        if self._indefinite is not None and self._indefinite[0] is diag and self._indefinite[1] == _versions(diag):
             return self._run_pcg(self._indefinite[2], b, rtol, max_iter)
         vt = b.dtype if self.dtype == torch.float32 else torch.float64   # FP32 moduli: FP64 or FP32 vectors
         if preconditioner == "block_jacobi":
@@ -182,7 +184,7 @@ class CudaTangentOperator:
         if self.last_status == "negative_curvature" and self.code == _lib.DFEA_F64REF:
             physical = self._physical_pcg(diag, preconditioner, diag_point)
             if physical is not None:
-                self._indefinite = (diag, _version(diag), physical)
+                self._indefinite = (diag, _versions(diag), physical)
                 return self._run_pcg(physical, b, rtol, max_iter)
         return out
 
@@ -206,7 +208,7 @@ class CudaTangentOperator:
         try:
             C, own = self.point.physical(self.mesh_id)
             d = diag.detach().to(torch.float64).contiguous()
-            as_made = _version(diag) == 0                # not a diagonal the caller has written to
+            as_made = _versions(diag) == [0]             # not a diagonal the caller has written to
             if as_made and diag is self.diag:
                 d = own
             elif as_made and diag_point is not None and diag_point.unchanged:
@@ -219,7 +221,7 @@ class CudaTangentOperator:
             return None
 
 
-# (weakref(u), u._version, weakref(theta), theta._version, mesh id) -> diag of the last linearisation,
+# (weakref(u), u._version, weakref(theta), theta._version, mesh id) -> diag and point of the last linearisation,
 # so that make_preconditioner right after make_tangent_operator at the same point reuses kernel (a)'s pass
 _LAST_DIAG = {}
 
@@ -243,8 +245,9 @@ def make_A_operator_cuda(u, theta, params, precision="fp64"):
         C, diag = ops.run(ops.qp_moduli, mid, _f64c(u), _f64c(theta), *ops.material_args(device_material(params)),
                           precision == "fp32", True)
     _LAST_DIAG.clear()
-    _LAST_DIAG[_diag_key(u, theta, mesh)] = (weakref.ref(u), weakref.ref(theta), diag)
-    return CudaTangentOperator(mesh, mid, C, diag, precision, _Linearisation(u, theta, params), gather)
+    point = _Linearisation(u, theta, params)
+    _LAST_DIAG[_diag_key(u, theta, mesh)] = (weakref.ref(u), weakref.ref(theta), diag, weakref.ref(point))
+    return CudaTangentOperator(mesh, mid, C, diag, precision, point, gather)
 
 
 def make_tangent_operator(kind, u, theta, params):
@@ -285,12 +288,17 @@ class CudaJacobiPreconditioner:
 
 
 def compute_jacobi_diagonal(u, theta, params):
-    """diag(K) without forming K (kernel (a)'s element diagonals, scattered by colour), shape (2N,)."""
+    """diag(K) without forming K (kernel (a)'s element diagonals, summed at the nodes), shape (2N,)."""
+    return _jacobi(u, theta, params)[1]
+
+
+def _jacobi(u, theta, params):
+    """(mesh, diagonal, the point it was made at)."""
     mesh, mid = _prepare(u, theta, params)
     hit = _LAST_DIAG.get(_diag_key(u, theta, mesh))
     if hit is not None and hit[0]() is u and hit[1]() is theta:
-        return hit[2]
-    return _preconditioner_data(mesh, mid, u, theta, params, False)[0]
+        return mesh, hit[2], hit[3]() or _Linearisation(u, theta, params)
+    return mesh, _preconditioner_data(mesh, mid, u, theta, params, False)[0], _Linearisation(u, theta, params)
 
 
 def _preconditioner_data(mesh, mid, u, theta, params, with_blocks):
@@ -302,8 +310,7 @@ def _preconditioner_data(mesh, mid, u, theta, params, with_blocks):
 
 
 def make_jacobi_preconditioner(u, theta, params):
-    mesh = cuda_mesh(params)
-    return CudaJacobiPreconditioner(mesh, compute_jacobi_diagonal(u, theta, params), _Linearisation(u, theta, params))
+    return CudaJacobiPreconditioner(*_jacobi(u, theta, params))
 
 
 class CudaBlockJacobiPreconditioner:
