@@ -24,9 +24,15 @@ from difffea_b200.elements import default_rule, element_quadrature, quadrature_g
 _SUPPORTED = {(4, 4): "quad4", (9, 9): "quad9", (3, 1): "tri3", (6, 6): "tri6", (8, 9): "quad8"}
 
 
+# the raw handle without a Stream object around it (1 us a call), where this torch has the private function
+_RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_handle():
     """cudaStream_t of torch's current stream (every launch goes there)."""
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    if _RAW_STREAM is None:
+        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(_RAW_STREAM(torch.cuda.current_device()))
 
 
 def ptr(t):

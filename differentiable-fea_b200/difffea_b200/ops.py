@@ -86,12 +86,28 @@ def _functional_op(name):
     return register
 
 
+def _interpreter_probes():
+    """The functions of torch that tell _observed what lies on the dispatcher's stacks; None if this torch lacks one."""
+    try:
+        torch.autograd.forward_ad._current_level
+        return (torch.compiler.is_compiling, torch._C._len_torch_dispatch_stack, torch._C._len_torch_function_stack,
+                torch._C._autograd._profiler_enabled, torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state)
+    except AttributeError:
+        return None
+
+
+_PROBES = _interpreter_probes()
+
+
 def _observed(args):
     """True if the dispatcher has something to do between a call of a functional op and its CUDA implementation: a trace,
-    a mode, a functorch or forward-mode level, the profiler, autograd, a tensor subclass, another device."""
-    if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
-            or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0
-            or torch._C._get_tracing_state() is not None or torch._C._autograd._profiler_enabled()):
+    a mode, a functorch or forward-mode level, the profiler, autograd, a tensor subclass, another device.  Also where
+    torch does not say: its probes are private."""
+    if _PROBES is None:
+        return True
+    compiling, modes, functions, profiler, functorch, tracing = _PROBES
+    if (compiling() or modes() or functions() or functorch() is not None or torch.autograd.forward_ad._current_level >= 0
+            or tracing() is not None or profiler()):
         return True
     for t in args:
         if isinstance(t, torch.Tensor) and (type(t) is not torch.Tensor or t.requires_grad or not t.is_cuda or t.is_neg()):
