@@ -138,9 +138,9 @@ def hbm_estimate(req, precision="fp32", preconditioner="jacobi"):
     nen, nq = NEN[req.element_type], NQ[req.element_type]
     per_el = (8 * nen + 16 * nq * nen + 8 * nq          # problem dictionary: conn, dN_dX, w_detJ
               + 4 * nen + 4 + 16 * nq * nen + 8 * nq + 8  # packed mesh (FP64 gradients)
-              + ((40 + 32) * nq if precision == "fp32"  # reference-frame FP32 moduli + inverse Jacobians
-                 else 128 * nq)                         # FP64 moduli
+              + ((40 if precision == "fp32" else 80) + 32) * nq  # reference-frame moduli + inverse Jacobians
               + 16 * nen + 4 * nen                      # gather form: element results, node incidence
+              + 24 * nen                                # scratch of the frame calls: element results and couplings
               + 32 * nen)                               # int64 keys, values and order of the incidence sort
     per_node = 16 + 2 * 8 * 14 + 2 * 4 * 6 + 1 + 4      # nodes, ~14 f64 and ~6 f32 DOF vectors, fix bits, ptr
     if preconditioner_for(req, preconditioner) == "multigrid":
