@@ -240,7 +240,7 @@ class CudaMesh:
             if self._frame_check is None:
                 if torch.cuda.is_current_stream_capturing():
                     return False
-                if not self.indexable:
+                if not self.indexable or not self.n_el:
                     self._frame_check = (float("inf"), 0.0, float("inf"))
                     return False
                 incidence = self._launch_incidence() if self.node_elem is None else None
@@ -253,7 +253,7 @@ class CudaMesh:
                     result = tuple(check.tolist())               # waits for the frame and the incidence too
                 if incidence is not None:
                     self._publish_incidence(*incidence)
-                if not self.n_el or result[2] <= self.FRAME_TOLERANCE:
+                if result[2] <= self.FRAME_TOLERANCE:
                     self.view.frame = frame.data_ptr()
                     self.frame = frame
                 self._frame_check = result
