@@ -382,7 +382,7 @@ def frame_internal_force(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, mod
                          mat_p: list[float],
                  p_dev: Optional[torch.Tensor], s_dev: Optional[torch.Tensor]) -> torch.Tensor:
     mesh = _frame_mesh(mesh_id, u, theta)
-    R = torch.empty_like(u)
+    R = torch.empty(mesh.n_dof, dtype=torch.float64, device=mesh.device)
     work = mesh.frame_work()        # a local: the call's own until its launches are made
     _lib.call("dfea_frame_internal_force", mesh.view_ref, ptr(u), ptr(theta),
               *_frame_args(mesh, model, scalable, mat_p, p_dev, s_dev),
@@ -392,7 +392,7 @@ def frame_internal_force(mesh_id: int, u: torch.Tensor, theta: torch.Tensor, mod
 
 @frame_internal_force.register_fake
 def _(mesh_id, u, theta, model, scalable, mat_p, p_dev, s_dev):
-    return torch.empty_like(u)
+    return u.new_empty(_mesh(mesh_id).n_dof)
 
 
 @_functional_op("frame_sensitivity")
