@@ -37,13 +37,13 @@ def compute_fields(u, theta, params) -> dict:
         scalars (0-d):        strain_energy, min_J
     """
     mesh, mid = _prepare(u, theta, params)
-    un = _f64c(u).view(mesh.n_nodes, 2)
-    if mesh.ensure_frame() and mesh.n_el:
+    if mesh.ensure_frame():
         el, nodal, scal = ops.run(ops.frame_all_fields, mid, _f64c(u), _f64c(theta), *ops.frame_material(params))
-        u_mag, energy, min_J = nodal[6], scal[0], scal[1]
+        un, u_mag, energy, min_J = _f64c(u).view(mesh.n_nodes, 2), nodal[6], scal[0], scal[1]
     else:
         el = element_fields(u, theta, params)
         nodal = torch.ops.difffea_b200.node_fields(mid, el)
+        un = _f64c(u).view(mesh.n_nodes, 2)
         u_mag, energy, min_J = torch.linalg.norm(un, dim=1), torch.sum(el[6] * el[0]), el[1].min()
     out = {name: el[k + 1] for k, name in enumerate(ELEMENT_FIELDS)}
     out.update(ux=un[:, 0], uy=un[:, 1], u_mag=u_mag, strain_energy=energy, min_J=min_J)
