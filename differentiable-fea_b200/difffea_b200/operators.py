@@ -101,6 +101,11 @@ class _Linearisation:
     def unchanged(self):
         return self.versions is not None and self.versions == _versions(self.u, self.theta, *self.material.values())
 
+    def holds(self, params):
+        """Whether this is a point of the problem's material, none of it written to since."""
+        return (("material" in params) == ("material" in self.material)
+                and all(params.get(k) is t for k, t in self.material.items()) and self.unchanged)
+
     def physical(self, mesh_id):
         """(the 16 physical moduli per Gauss point, the Jacobi diagonal) by the kernels that read dN/dX."""
         return ops.run(ops.qp_moduli, mesh_id, _f64c(self.u), _f64c(self.theta),
@@ -297,7 +302,9 @@ def _jacobi(u, theta, params):
     mesh, mid = _prepare(u, theta, params)
     hit = _LAST_DIAG.get(_diag_key(u, theta, mesh))
     if hit is not None and hit[0]() is u and hit[1]() is theta:
-        return mesh, hit[2], hit[3]() or _Linearisation(u, theta, params)
+        point = hit[3]()
+        if point is not None and point.holds(params):
+            return mesh, hit[2], point
     return mesh, _preconditioner_data(mesh, mid, u, theta, params, False)[0], _Linearisation(u, theta, params)
 
 
