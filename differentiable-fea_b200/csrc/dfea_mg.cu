@@ -1651,6 +1651,13 @@ static int validate_mg(const dfea_mesh_view* mesh, const dfea_mg* mg, const char
     return DFEA_OK;
 }
 
+// The passes over level 0 read and write nodal pairs.  A caller's vector that starts between two pairs stands in level 0's
+// right-hand side, which nothing else uses.
+static bool paired(const double* v) { return (reinterpret_cast<uintptr_t>(v) & 15u) == 0; }
+static int copy_vector(double* to, const double* from, int64_t n, cudaStream_t s) {
+    return check_cuda(cudaMemcpyAsync(to, from, n * sizeof(double), cudaMemcpyDeviceToDevice, s), "cudaMemcpyAsync");
+}
+
 static int read_scalars(double* host, const double* dev, int k, cudaStream_t s) {
     return read_to_host(host, dev, k * sizeof(double), s);
 }
@@ -2305,17 +2312,17 @@ extern "C" int dfea_mg_vcycle(const dfea_mesh_view* mesh, const dfea_mg* mg, con
     int rc = validate_mg(mesh, mg, "dfea_mg_vcycle");
     if (rc) return rc;
     if (!moduli || !r || !z) return set_error(DFEA_ERR_INVALID, "dfea_mg_vcycle: NULL pointer");
-    return mg_vcycle(mesh, mg, moduli, moduli_dtype, 0, r, z, CycleUse(), static_cast<cudaStream_t>(stream));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (!paired(r)) {
+        if ((rc = copy_vector(mg->level[0].b, r, mg->level[0].n, s))) return rc;
+        r = mg->level[0].b;
+    }
+    return mg_vcycle(mesh, mg, moduli, moduli_dtype, 0, r, z, CycleUse(), s);
 }
 
-extern "C" int dfea_mg_pcg(const dfea_mesh_view* mesh, const dfea_mg* mg, const void* moduli, int32_t moduli_dtype,
-                           const double* b, double* x, double rtol, int32_t max_iter, int32_t* iterations,
-                           int32_t* status, void* stream) {
-    int rc = validate_mg(mesh, mg, "dfea_mg_pcg");
-    if (rc) return rc;
-    if (!moduli || !b || !x || !iterations || !status || max_iter < 0)
-        return set_error(DFEA_ERR_INVALID, "dfea_mg_pcg: bad arguments");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
+static int mg_pcg(const dfea_mesh_view* mesh, const dfea_mg* mg, const void* moduli, int32_t moduli_dtype, const double* b,
+                  double* x, double rtol, int32_t max_iter, int32_t* iterations, int32_t* status, cudaStream_t s) {
+    int rc;
     if (mg->pcg_state && mg->graphs) {
         // graph-driven: the second solve with the same buffers captures the loop, later ones replay it
         MgGraphs* g = static_cast<MgGraphs*>(mg->graphs);
@@ -2347,4 +2354,17 @@ extern "C" int dfea_mg_pcg(const dfea_mesh_view* mesh, const dfea_mg* mg, const 
             (rc = read_to_host(&host, st, sizeof(host), s)))
             return rc;
     return pcg_result(host, iterations, status);
+}
+
+extern "C" int dfea_mg_pcg(const dfea_mesh_view* mesh, const dfea_mg* mg, const void* moduli, int32_t moduli_dtype,
+                           const double* b, double* x, double rtol, int32_t max_iter, int32_t* iterations,
+                           int32_t* status, void* stream) {
+    int rc = validate_mg(mesh, mg, "dfea_mg_pcg");
+    if (rc) return rc;
+    if (!moduli || !b || !x || !iterations || !status || max_iter < 0)
+        return set_error(DFEA_ERR_INVALID, "dfea_mg_pcg: bad arguments");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    double* own = paired(x) ? x : mg->level[0].b;
+    rc = mg_pcg(mesh, mg, moduli, moduli_dtype, b, own, rtol, max_iter, iterations, status, s);
+    return rc || own == x ? rc : copy_vector(x, own, mg->level[0].n, s);
 }
