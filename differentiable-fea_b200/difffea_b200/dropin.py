@@ -75,7 +75,7 @@ def register(package=None):
     def pcg(A_fn, b, Minv_fn, rtol=1e-5, max_iter=500):
         if isinstance(A_fn, CudaTangentOperator) and b.is_cuda:
             if isinstance(Minv_fn, CudaJacobiPreconditioner) and Minv_fn.mesh is A_fn.mesh:
-                return A_fn.pcg_solve(b, Minv_fn.diag, rtol, max_iter)
+                return A_fn.pcg_solve(b, Minv_fn.diag, rtol, max_iter, diag_point=Minv_fn.point)
             if isinstance(Minv_fn, CudaMultigridPreconditioner) and Minv_fn.mesh is A_fn.mesh:
                 Minv_fn.refresh()                       # the hierarchy at this closure's linearisation
                 x = torch.empty_like(b, dtype=torch.float64)
