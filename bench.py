@@ -404,7 +404,7 @@ def run_serve(args):
                "data": "synthetic (seeded request stream)", "config": serve_config(args.steps),
                "engine": f"{SERVE['slots']} slots, largest waiting request first, problems written by the library "
                          f"on the device, multigrid-preconditioned from 2500 nodes (gather-form level 0), Jacobi "
-                         f"below (direct launches), the C++ Newton driver per request, host sync "
+                         f"below (cluster PCG, one launch a solve), the C++ Newton driver per request, host sync "
                          f"{'blocking' if blocking else 'spin (blocking sync refused)'}",
                "all_converged": ok and lat_ok,
                "e2e": {"value": world * len(timed_s) / e2e_s, "unit": "solves/s", "requests": len(timed_s),
@@ -422,8 +422,9 @@ def run_serve(args):
                                     "max_rel_err_auto": err, "max_rel_err_jacobi": err_j,
                                     "plain_host_sync": "spin" if (plain_spin or not blocking) else "blocking",
                                     "plain": "newton_krylov_solve defaults, one request after another: FP64 "
-                                             "moduli and gradients, Jacobi-PCG in 8-iteration graphs, product "
-                                             "form by mesh size (fused gather below 300k nodes)",
+                                             "reference-frame moduli, Jacobi-PCG in one cluster launch where "
+                                             "the mesh fits, else in 8-iteration graphs (fused form below "
+                                             "300k nodes, gather above)",
                                     "reading": "ratio_jacobi isolates the engine (batching, FP32 operator); "
                                                "ratio_auto adds the multigrid preconditioner"},
                "serving_hbm": {"achieved_gbs": pcg_bytes / (full_ms * 1e-3) / 1e9,

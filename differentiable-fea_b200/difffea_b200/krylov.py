@@ -1,10 +1,11 @@
 """
-Device-resident Jacobi-PCG (kernel (c)) bound to fixed buffers.
+Device-resident PCG (kernel (c)) bound to fixed buffers.
 
-``DevicePCG`` owns a ``dfea_pcg`` handle: one PCG iteration (the colour passes of the tangent product
-with the curvature fused in, two fused vector-update kernels, the loop condition) captured once in a
-CUDA graph with a device-side while-loop, so a whole solve is one graph launch and one read-back of
-(status, iterations).  The buffers it binds (moduli, diagonal, right-hand side, solution and a work
+``DevicePCG`` owns a ``dfea_pcg`` handle, in one of four forms.  Cluster: the whole solve in one launch of a thread-block
+cluster, on meshes whose vectors fit its shared memory.  Fused, gather and colour: two, three or n_colours + 2 launches
+an iteration (the tangent product with the curvature fused in, the vector updates), captured in a CUDA graph of eight
+iterations or of a device-side while-loop, or launched one by one.  Each ends with one read-back of (status, iterations).
+The buffers it binds (moduli, diagonal, right-hand side, solution and a work
 area for the Krylov vectors and partial sums) stay allocated for the life of the object; their
 contents may change between solves.
 """
@@ -30,7 +31,9 @@ class DevicePCG:
     per-node sums fused into the first vector update: 3 kernels per iteration; needs the mesh's node
     incidence, built here) or "fused" (the gather form with the direction update moved into the next
     element pass: 2 kernels per iteration) or "cluster" (the whole solve in one launch of a thread-block cluster,
-    its vectors in distributed shared memory; reference-frame moduli, meshes that fit).  Each form is reproducible; they agree to rounding.
+    its vectors in distributed shared memory; reference-frame moduli, meshes that fit).  Each form is reproducible; they
+    agree to rounding (on an operator that is not positive definite, where the iterate of the first non-positive curvature
+    is amplified rounding, CudaTangentOperator.pcg_solve ends them all in the colour form).
     moduli: "physical" (C with the packed dN/dX: FP64, FP32, or FP32 on FP64 vectors) or "ref" (FP32 or FP64
     moduli pulled back to the element reference frame, 10 per Gauss point, FP64 vectors; the product
     reads no gradients; FP64: the gather and fused forms).  max_blocks: at most this many blocks per launch (0: the whole GPU), for solves

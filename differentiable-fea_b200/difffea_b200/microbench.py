@@ -30,6 +30,10 @@ nu = 0.3, h = 1.  Algorithmic bytes count every array a kernel must touch once:
 ``precision``: fp64 (FP64 moduli, gradients and vectors), fp32 (all FP32), mixed (FP32 moduli and
 gradients on FP64 vectors) or ref (FP32 moduli in the element reference frame, 10 per Gauss point, on
 FP64 vectors: the serving operator; the product reads no gradients, its bytes count 10 moduli).
+
+moduli, residual, sensitivity, fields and the fp64 / fp32 / mixed products are the physical forms, which read the packed
+gradients: what a mesh without a frame runs.  The functional operators of a mesh with one run the frame kernels;
+perf/cases.py times those through the calls that use them.
 """
 import argparse
 import json

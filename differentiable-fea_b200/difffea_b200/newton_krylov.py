@@ -19,7 +19,7 @@ and (status, iterations) per linear solve.
 operators.py:586-625), both applied inside the device PCG.
 
 Extra keyword arguments (not in the reference): ``pcg_max_iter``; ``precision`` = "fp64" (default) or
-"fp32" (the PCG applies FP32 moduli and gradients -- the bytes that dominate the operator -- to FP64
+"fp32" (the PCG applies FP32 moduli -- the bytes that dominate the operator -- to FP64
 Krylov vectors; the residual, line search, convergence test and state update stay FP64, so each Newton
 step is an iterative-refinement correction of the FP64 state computed with an FP32 operator);
 ``workspace`` to reuse device buffers across solves of the same problem.
