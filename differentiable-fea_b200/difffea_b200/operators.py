@@ -75,9 +75,11 @@ def strain_energy(u, theta, params):
 # tangent operator
 # ---------------------------------------------------------------------------------------------
 def _versions(*tensors):
-    """The tensors' version counters, or None where torch keeps none (inference mode)."""
+    """The tensors' version counters (0 for what is no tensor), or None where torch keeps none (inference mode)."""
     try:
-        return [getattr(t, "_version", 0) for t in tensors]
+        return tuple([t._version for t in tensors])
+    except AttributeError:
+        return _versions(*(t for t in tensors if torch.is_tensor(t)))
     except RuntimeError:
         return None
 
@@ -88,23 +90,32 @@ class _Linearisation:
     blocks are computed from when a solve asks for them later.  Holds the tensors themselves; ``unchanged`` is False
     once one of them was written to (or where torch keeps no version of it).
     """
-    __slots__ = ("u", "theta", "material", "versions", "__weakref__")
+    __slots__ = ("u", "theta", "keys", "values", "versions", "__weakref__")
+    MATERIAL, LEGACY = ("mat_p", "mat_scalable", "material"), ("nodes", "mu0", "lmbda0")
 
     def __init__(self, u, theta, params):
         self.u = u.detach() if u.requires_grad else u
         self.theta = theta.detach() if theta.requires_grad else theta
-        keys = ("material", "mat_p", "mat_scalable") if "material" in params else ("mu0", "lmbda0", "nodes")
-        self.material = {k: params[k] for k in keys}
-        self.versions = _versions(self.u, self.theta, *self.material.values())
+        self.keys = self.MATERIAL if "material" in params else self.LEGACY
+        a, b, c = self.keys
+        self.values = a, b, c = params[a], params[b], params[c]
+        self.versions = _versions(u, theta, a, b) if c.__class__ is str else _versions(u, theta, a, b, c)
 
     @property
     def unchanged(self):
-        return self.versions is not None and self.versions == _versions(self.u, self.theta, *self.material.values())
+        a, b, c = self.values
+        now = _versions(self.u, self.theta, a, b) if c.__class__ is str else _versions(self.u, self.theta, a, b, c)
+        return now is not None and now == self.versions
 
     def holds(self, params):
         """Whether this is a point of the problem's material, none of it written to since."""
-        return (("material" in params) == ("material" in self.material)
-                and all(params.get(k) is t for k, t in self.material.items()) and self.unchanged)
+        (a, b, c), (x, y, z) = self.keys, self.values
+        return (params.get(a) is x and params.get(b) is y and params.get(c) is z
+                and ("material" in params) == (self.keys is self.MATERIAL) and self.unchanged)
+
+    @property
+    def material(self):
+        return dict(zip(self.keys, self.values))
 
     def physical(self, mesh_id):
         """(the 16 physical moduli per Gauss point, the Jacobi diagonal) by the kernels that read dN/dX."""
@@ -213,7 +224,7 @@ class CudaTangentOperator:
         try:
             C, own = self.point.physical(self.mesh_id)
             d = diag.detach().to(torch.float64).contiguous()
-            as_made = _versions(diag) == [0]             # not a diagonal the caller has written to
+            as_made = _versions(diag) == (0,)           # not a diagonal the caller has written to
             if as_made and diag is self.diag:
                 d = own
             elif as_made and diag_point is not None and diag_point.unchanged:
